@@ -12,7 +12,7 @@ from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int6
 
 import torch
 
-from .build import LIB_PATH
+from .build import HOST_PATH, LIB_PATH
 
 F32, F16, BF16 = 0, 1, 2
 DENSE_PAGE, QUANTIZED_PAGE, MIXED_PAGE = 0, 1, 2
@@ -158,6 +158,19 @@ def _load() -> ctypes.CDLL:
 
 
 LIB = _load()
+
+
+def _load_host():
+    """The per-call host path (``csrc/host_path.cpp``): append and decode without ctypes in between."""
+
+    if not os.path.exists(HOST_PATH):
+        raise ImportError(f"{HOST_PATH} is missing: build it with `python -m dartkv_b200.build`")
+    from . import _dartkv_host
+
+    return _dartkv_host
+
+
+HOST = _load_host()
 
 
 class DartKVError(RuntimeError):

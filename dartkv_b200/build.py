@@ -1,9 +1,8 @@
-"""Compile the CUDA sources of this package into ``libdartkv_b200.so`` (sm_100a only).
+"""Compile the native code of this package: the CUDA sources into ``libdartkv_b200.so`` (sm_100a only) and the
+per-call host path into the CPython extension ``_dartkv_host.so``, which links against it.
 
 ``python dartkv_b200/build.py [--force] [-v]``; ``-v`` prints ptxas resource usage.  Extra nvcc flags can be
-passed in ``DARTKV_NVCC_FLAGS`` (the decode kernels have build-time knobs for timing experiments: unroll factors
-``-DPEROP_QK_UNROLL=`` / ``-DFUSED_PV_UNROLL=`` ..., and parts that can be compiled out, ``-DFUSED_SKIP_QK``,
-``-DFUSED_SKIP_PV``, ``-DFUSED_SKIP_SETUP``, ``-DDENSE_SKIP``; a library built with the latter computes garbage).
+passed in ``DARTKV_NVCC_FLAGS``.
 """
 
 from __future__ import annotations
@@ -12,10 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PACKAGE_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PACKAGE_DIR, "csrc")
 LIB_PATH = os.path.join(PACKAGE_DIR, "libdartkv_b200.so")
+HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
+HOST_PATH = os.path.join(PACKAGE_DIR, "_dartkv_host.so")
 SOURCES = ("quantize.cu", "cache_append.cu", "append_fast.cu", "decode_attention.cu", "decode_fast.cu", "decode_fused32.cu",
            "decode_wide.cu")
 NVCC_FLAGS = (
@@ -40,15 +42,55 @@ def _stale(sources) -> bool:
     return any(os.path.exists(p) and os.path.getmtime(p) > built for p in deps)
 
 
+def _start_host_build(force: bool):
+    """Start compiling the CPython extension (``None`` when it is up to date)."""
+
+    header = os.path.join(PACKAGE_DIR, "..", "include", "dartkv_b200.h")
+    if not force and os.path.exists(HOST_PATH) and all(
+            os.path.getmtime(p) <= os.path.getmtime(HOST_PATH) for p in (HOST_SOURCE, header)):
+        return None
+    import torch
+    from torch.utils import cpp_extension
+
+    includes = [*cpp_extension.include_paths("cuda"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-c", HOST_SOURCE, "-o", os.path.join(PACKAGE_DIR, "build", "host_path.o"),
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{path}" for path in includes]]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
+def _finish_host_build(proc) -> None:
+    """Link the extension against the library beside it and torch's own libraries."""
+
+    from torch.utils import cpp_extension
+
+    out, _ = proc.communicate()
+    if proc.returncode:
+        print(out, file=sys.stderr)
+        raise RuntimeError("g++ failed; see the compiler output above")
+    libraries = [f"-L{path}" for path in cpp_extension.library_paths("cuda")]
+    subprocess.run(["g++", "-shared", "-o", HOST_PATH, os.path.join(PACKAGE_DIR, "build", "host_path.o"), f"-L{PACKAGE_DIR}",
+                    "-ldartkv_b200", "-Wl,-rpath,$ORIGIN", *libraries, "-ltorch_python", "-ltorch", "-ltorch_cpu",
+                    "-lc10", "-lc10_cuda"], check=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Build the shared library in-tree and return its path (no-op when up to date)."""
+    """Build both shared objects in-tree and return the library's path (no-op when up to date)."""
+
+    os.makedirs(os.path.join(PACKAGE_DIR, "build"), exist_ok=True)
+    host = _start_host_build(force)
+    path = _build_library(force, verbose)
+    if host is not None:
+        _finish_host_build(host)
+    return path
+
+
+def _build_library(force: bool, verbose: bool) -> str:
 
     sources = [os.path.join(CSRC, name) for name in SOURCES if os.path.exists(os.path.join(CSRC, name))]
     if not force and not _stale(sources):
         return LIB_PATH
     objects = []
     build_dir = os.path.join(PACKAGE_DIR, "build")
-    os.makedirs(build_dir, exist_ok=True)
     procs = []
     for src in sources:
         obj = os.path.join(build_dir, os.path.basename(src) + ".o")

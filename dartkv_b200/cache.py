@@ -151,6 +151,26 @@ class DartKVCache:
         self._c_cfg = _lib.LifecycleConfig(cfg.page_size, cfg.sink_tokens, cfg.local_tokens, cfg.value_local_tokens,
                                            int(cfg.hold_partial_pages))
         self._c_state = _lib.LifecycleStateC()
+        # what the native host path needs of this cache, as plain integers (see _bind_native)
+        self._append_args: Optional[tuple] = None
+        self._decode_args: Optional[tuple] = None
+
+    def _bind_native(self) -> None:
+        """Addresses for the native append path: descriptor, lifecycle structs (their fields change in place, the
+        structs stay where they are) and the finite-input flag."""
+
+        cfg = self.config
+        address = ctypes.addressof
+        self._decode_args = None
+        self._append_args = None
+        if cfg.promote_ratio <= 0.0 or cfg.channel_selection == "magnitude":
+            self._append_args = (address(self._desc), address(self._c_cfg), address(self._c_state), address(self._plan),
+                                 self._pools["nonfinite"].data_ptr())
+
+    def _set_c_state(self, state) -> None:
+        mine = self._c_state
+        mine.seen, mine.k_packed_end, mine.v_packed_end, mine.key_pages = (
+            state.seen, state.k_packed_end, state.v_packed_end, state.key_pages)
 
     # ------------------------------------------------------------------ simple accessors
     @property
@@ -250,6 +270,7 @@ class DartKVCache:
                      "page_tokens", "state"):
             setattr(d, name, old[name].data_ptr())
         self._workspace = None
+        self._bind_native()
 
     # ------------------------------------------------------------------ append / update
     def update(self, key_states: torch.Tensor, value_states: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -267,6 +288,13 @@ class DartKVCache:
         with a recorded reference run.
         """
 
+        if self._append_args is not None and channel_indices is None:
+            rc = _lib.HOST.append(key_states, value_states, *self._append_args)
+            if rc == 0:
+                self._note_step()
+                return
+            if rc != _lib.HOST.SLOW_PATH and rc != _lib.ELIMIT:
+                check(rc)
         self._validate_inputs(key_states, value_states)
         device = require_cuda(key_states, value_states)
         keys = key_states.detach()
@@ -334,15 +362,19 @@ class DartKVCache:
                 check(LIB.dartkv_cache_append(
                     ctypes.byref(d), ctypes.byref(plan), ptr(keys), ptr(values), keys.stride(0), keys.stride(1),
                     keys.stride(2), ptr(idx), ptr(self._pools["nonfinite"]), stream_ptr(device)))
-            self._c_state = state
-        # the step was accepted: bring the host-side segment bookkeeping up to date from its plan
-        life = self._life
+            self._set_c_state(state)
+        self._note_step()
+
+    def _note_step(self) -> None:
+        """The step in ``self._plan`` was accepted: bring the host-side segment bookkeeping up to date."""
+
+        life, plan = self._life, self._plan
         if plan.sink_copy:
             life.sink_pieces.append((plan.chunk_start, plan.sink_copy))
-        page = cfg.page_size
-        for i in range(plan.num_pages):
-            life.pages.append((plan.page_token_start + i * page,
-                               plan.last_page_tokens if i == plan.num_pages - 1 else page))
+        if plan.num_pages:
+            page, start = self.config.page_size, plan.page_token_start
+            life.pages.extend((start + i * page, page) for i in range(plan.num_pages - 1))
+            life.pages.append((start + (plan.num_pages - 1) * page, plan.last_page_tokens))
         life.seen = plan.seen_after
         life.k_packed_end = plan.k_packed_end_after
         life.v_packed_end = plan.v_packed_end_after
@@ -409,22 +441,10 @@ class DartKVCache:
         return state
 
     def _commit_step(self, state) -> None:
-        """The step in ``self._plan`` was accepted: bring the host-side bookkeeping up to date."""
+        """The device-planned step in ``self._plan`` was accepted: advance the host's copy of the state."""
 
-        cfg, plan = self.config, self._plan
-        self._c_state = state
-        life = self._life
-        if plan.sink_copy:
-            life.sink_pieces.append((plan.chunk_start, plan.sink_copy))
-        page = cfg.page_size
-        for i in range(plan.num_pages):
-            life.pages.append((plan.page_token_start + i * page,
-                               plan.last_page_tokens if i == plan.num_pages - 1 else page))
-        life.seen = plan.seen_after
-        life.k_packed_end = plan.k_packed_end_after
-        life.v_packed_end = plan.v_packed_end_after
-        self._layout_version += 1
-        self._invalidate_page_descriptors()
+        self._set_c_state(state)
+        self._note_step()
 
     def _host_selected_indices(self, keys: torch.Tensor, chunk: int) -> Optional[torch.Tensor]:
         """Promoted channels for the 'random' and 'variance' strategies, chosen with the functional API.
@@ -699,6 +719,7 @@ class DartKVCache:
                          "page_tokens", "state"):
                 setattr(self._desc, name, self._pools[name].data_ptr())
             self._workspace = None
+            self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
         return self
@@ -727,6 +748,7 @@ class DartKVCache:
         self._desc.batch = int(indices.numel())
         self._shape = (self._desc.batch, self._shape[1], self._shape[2])
         self._workspace = None
+        self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
         return self
@@ -736,8 +758,10 @@ class DartKVCache:
         self._layout_version += 1
 
     def _invalidate_page_descriptors(self) -> None:
-        self._page_table_cache.clear()
-        self._page_run_cache.clear()
+        if self._page_table_cache:
+            self._page_table_cache.clear()
+        if self._page_run_cache:
+            self._page_run_cache.clear()
 
     def _validate_inputs(self, key_states: torch.Tensor, value_states: torch.Tensor) -> None:
         if key_states.ndim != 4 or value_states.ndim != 4:
@@ -771,9 +795,24 @@ class DartKVCache:
         if self._workspace is None or self._workspace[0] != key:
             nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), query_heads, capacity)
             with device_guard(self._device):
-                buf = torch.zeros(max(16, nbytes), dtype=torch.uint8, device=self._device)
+                buf = torch.empty(max(16, nbytes), dtype=torch.uint8, device=self._device)
+                buf[:16].zero_()        # status word and counters; the partials need no initial value
             self._workspace = (key, buf)
+        self._decode_args = (ctypes.addressof(d), self._workspace[1].data_ptr(), self._workspace[1].numel(), query_heads)
         return self._workspace[1], capacity
+
+    def decode_native(self, query: torch.Tensor, scale: Optional[float], flavour: int, row_start: Optional[torch.Tensor]):
+        """One decode call through the native host path: the output shaped like ``query``, or ``None`` when the call
+        is not an ordinary one (first call on this cache, other shapes or devices, wide query groups)."""
+
+        args = self._decode_args
+        if args is None:
+            return None
+        out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,
+                               flavour, row_start)
+        if type(out) is int:
+            check(out)
+        return out
 
     def decode_status(self) -> int:
         """0 unless a decode kernel gave up on a bounded wait for an async copy (synchronizes)."""

@@ -34,6 +34,10 @@ def decode_attention(query: torch.Tensor, cache: DartKVCache, *, scale: Optional
     rank of the node and the gathered tensor ``[B_total, Hq_total, D]`` of the step is returned instead.
     """
 
+    if token_capacity is None and out is None and peer_gather is None and query.ndim == 3:
+        result = cache.decode_native(query, scale, flavour, row_start)
+        if result is not None:
+            return result
     if cache.shape is None or cache.seen_tokens == 0:
         raise ValueError("cache is empty")
     batch, kv_heads, seen, head_dim = cache.shape
@@ -135,6 +139,11 @@ def fused_dart_attention(
     the result) serve calls captured in a CUDA graph: see ``decode_attention``.
     """
 
+    if page_table is None and page_runs is None and token_capacity is None and out is None:
+        # the ordinary call, through the native host path; whatever it leaves (and every error) is handled below
+        result = cache.decode_native(query, scale, flavour, row_start) if query.ndim == 4 else None
+        if result is not None:
+            return result
     if query.ndim != 4:
         raise ValueError("query must have shape [B, Hq, 1, D]")
     if query.shape[-2] != 1:
