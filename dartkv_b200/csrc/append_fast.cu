@@ -1,32 +1,43 @@
-// Page-shaped quantize+pack kernels for the common geometry: head_dim 128, 16-bit data,
-// full 128-token key pages with one 128-token key group, value groups of 32/64/128 channels.
+// Append step for the common geometry: head_dim 128, 16-bit data, 128-token key pages with one 128-token key group,
+// value groups of 16/32/64/128 channels.  One kernel does a whole step: quantize + pack the key pages, quantize +
+// pack the value rows, copy the dense sink / ring rows and publish the page table and the state words.
 //
-// Keys (one block of 64 threads per (batch*head, page)): the page is staged in shared memory
-// with 16-byte async copies; thread p owns the channel pair (2p, 2p+1), which moves through both
-// passes as one packed 16-bit pair: a pass for min / max / sum|k|, a block-wide rank for the
-// promoted channels, a pass that emits the codes and packs them in registers, then 16-byte row
-// stores.  Values: eight lanes per token row (16 channels per lane), group min/max by
-// xor-shuffles, packed bytes and metadata written coalesced.
+// Grid (head, batch row, page of the step and role): a block of 256 threads takes the 128 key tokens of a page or the 128
+// value rows beside it.  The ring rows a step reads are those of its first page only, so the block of that page also
+// writes the step's dense rows of its side, after a block barrier: no ordering between blocks is needed, and a
+// generation-time append is one launch instead of three.
+//
+// Keys: thread (tq, p) owns the channel pair (2p, 2p+1) of 32 tokens (quarter tq of the page) and keeps them in
+// registers as packed 16-bit pairs: one pass for min / max / sum|k|, the splits' statistics combined in shared
+// memory, the rank of the 128 channels by one integer key, then the codes.  Values: four lanes per token row
+// (32 channels per lane), group min/max by xor-shuffles.
+//
+// What bounds it: the instruction stream.  Per pair of elements the quantizer needs a subtract, two unpacks, two
+// multiplies, a pack, the rounding add and a cap; gathering the codes is one shift-add per pair (the magic exponents
+// are subtracted once per register, and 4-bit codes split into their low and high plane once per eight tokens).
 // HBM traffic per page: 64 KiB read (K and V rows), 10.6 KiB written (2-bit, 32 promoted).
 // The arithmetic is the reference's per-op rounding in the data dtype
 // (src/dart/quantization.py:178-186, src/dart/mixed.py:200-209).
 
 #include "common.cuh"
+#include "append_common.cuh"
 
 namespace {
 
 constexpr int kD = 128;
 constexpr int kP = 128;
+constexpr int kThreads = 256;
+constexpr int kSplits = 4;              // token splits of a key page
+constexpr int kTok = kP / kSplits;      // tokens per thread
 
 struct RowSource {
   const void* chunk;
   const void* ring;
   int64_t sb, sh, st;
-  int chunk_start, ring_tokens, kv_heads;
-  // base pointers for one (batch, head): chunk rows then ring rows
+  int chunk_start, ring_tokens;
+  // base pointers of this block's (batch, head): chunk rows then ring rows
   __device__ __forceinline__ void bases(int bh, const uint16_t*& chunk_base, const uint16_t*& ring_base) const {
-    int b = bh / kv_heads, h = bh % kv_heads;
-    chunk_base = reinterpret_cast<const uint16_t*>(chunk) + (int64_t)b * sb + (int64_t)h * sh;
+    chunk_base = reinterpret_cast<const uint16_t*>(chunk) + (int64_t)blockIdx.y * sb + (int64_t)blockIdx.x * sh;
     ring_base = reinterpret_cast<const uint16_t*>(ring) + (int64_t)bh * ring_tokens * kD;
   }
   __device__ __forceinline__ const uint16_t* row_from(const uint16_t* chunk_base, const uint16_t* ring_base, int t) const {
@@ -34,12 +45,6 @@ struct RowSource {
     return ring_base + (t % ring_tokens) * kD;
   }
 };
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // range / qmax rounded to the data dtype.  For bf16 the quotient of two 8-bit significands is never within
 // 2^-17 of a rounding boundary (see below), so a multiply by the fp32 reciprocal rounds to the same bf16.
@@ -52,24 +57,33 @@ __device__ __forceinline__ float scale_of(float mn, float mx, float qmax) {
   if (DT == DARTKV_BF16) return rnd<DT>(__fmul_rn(range, inv_qmax));
   return rnd<DT>(__fdiv_rn(range, qmax));
 }
-// 1 / scale for the reciprocal-multiply quotient (bf16 only): the approximate reciprocal is within 2^-22
-template <int DT>
+// 1 / scale for the quotients below: the approximate reciprocal is within 2^-22 (0 for an infinite scale)
 __device__ __forceinline__ float inverse_scale(float scale) {
-  if (DT != DARTKV_BF16) return 0.0f;   // fp16 takes the true division
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(scale));
   return r;
 }
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // ---- packed code computation -------------------------------------------------------------------
 // Two elements that share (min, scale) travel as one 16-bit pair.  The reference computes
 //   code = clamp(rint(r16(r16(x - min) / scale)), 0, qmax)        (r16 = round to the data dtype)
 // which is evaluated here as
 //   a2   = x2 - min2                      packed subtract, one rounding (exact for the 16-bit formats)
-//   q    = a * (1/scale)  (bf16)          the quotient of two 8-bit significands is never within 2^-17
-//          a / scale      (fp16)          of a bf16 rounding boundary and never on one, so a reciprocal
-//                                         multiply rounds to the same bf16 as the IEEE quotient; fp16
-//                                         significands are too long for that and take the true division
+//   q    = a * (1/scale)         bf16: the quotient of two 8-bit significands is never within 2^-17 of a bf16
+//                                rounding boundary and never on one, so a reciprocal multiply rounds to the
+//                                same bf16 as the IEEE quotient
+//          q + (a - q*scale)/scale   fp16: a boundary b between two fp16 numbers has a 12-bit odd significand N, so
+//                                a = b * scale would need 11 bits to hold N * (odd part of scale) >= 2^11 + 1:
+//                                never on a boundary, and |a - b*scale| is at least one unit of a product below
+//                                2^23, i.e. the quotient stays 2^-23 (relative) away from every boundary, while
+//                                one exact-residual step leaves q within 2^-24.  An infinite scale (the range of
+//                                the group overflows fp16) enters as scale = 1/scale = 0.
 //   r2   = r16(q) packed
 //   m2   = r2 + magic                     magic = 128 (bf16) / 1024 (fp16): the sum has unit ulp, so the
 //                                         packed add rounds half-to-even to an integer = rint
@@ -87,21 +101,31 @@ template <> struct Pack16<DARTKV_BF16> {
   static __device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) {
     uint32_t d; asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
+  static __device__ __forceinline__ uint32_t cap2(uint32_t a, uint32_t b) {   // a NaN becomes the cap
+    uint32_t d; asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
+  // count + (1.0 in each half where a > b)
+  static __device__ __forceinline__ uint32_t count_greater(uint32_t count, uint32_t a, uint32_t b) {
+    uint32_t d; asm("set.gt.bf16x2.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return add(count, d);
   }
   static __device__ __forceinline__ float lo(uint32_t v) { return __uint_as_float(v << 16); }
   static __device__ __forceinline__ float hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
   static __device__ __forceinline__ uint32_t pack(float hi_v, float lo_v) {
     uint32_t d; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi_v), "f"(lo_v)); return d;
   }
-  static __device__ __forceinline__ float quotient(float a, float s, float inv) { (void)s; return __fmul_rn(a, inv); }
-  static __device__ __forceinline__ uint16_t bits(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
-  // |x| as a double, from the 15 magnitude bits (subnormal inputs count as zero)
-  static __device__ __forceinline__ double abs_double(uint32_t b) {
-    const uint32_t mag = b & 0x7FFFu;
-    return __hiloint2double(mag >= 0x80u ? (int)(mag * 8192u + 0x38000000u) : 0, 0);
+  // the quotients of a pair, rounded to bf16: both products in one packed fp32 multiply
+  static __device__ __forceinline__ uint32_t quotients(uint32_t a2, float, float, float inv_lo, float inv_hi) {
+    uint32_t d;
+    asm("{\n.reg .b64 a, b, q;\n.reg .f32 ql, qh;\n"
+        "mov.b64 a, {%1, %2};\nmov.b64 b, {%3, %4};\nmul.rn.f32x2 q, a, b;\nmov.b64 {ql, qh}, q;\n"
+        "cvt.rn.bf16x2.f32 %0, qh, ql;\n}"
+        : "=r"(d) : "f"(lo(a2)), "f"(hi(a2)), "f"(inv_lo), "f"(inv_hi));
+    return d;
   }
+  static __device__ __forceinline__ uint16_t bits(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
 };
 template <> struct Pack16<DARTKV_F16> {
   static constexpr uint32_t kMagic = 0x64006400u;   // 1024.0 | 1024.0
@@ -114,158 +138,208 @@ template <> struct Pack16<DARTKV_F16> {
   static __device__ __forceinline__ uint32_t min2(uint32_t a, uint32_t b) {
     uint32_t d; asm("min.NaN.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
+  static __device__ __forceinline__ uint32_t cap2(uint32_t a, uint32_t b) {
+    uint32_t d; asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
+  static __device__ __forceinline__ uint32_t count_greater(uint32_t count, uint32_t a, uint32_t b) {
+    uint32_t d; asm("set.gt.f16x2.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return add(count, d);
   }
   static __device__ __forceinline__ float lo(uint32_t v) { return __half2float(__ushort_as_half((uint16_t)(v & 0xFFFFu))); }
   static __device__ __forceinline__ float hi(uint32_t v) { return __half2float(__ushort_as_half((uint16_t)(v >> 16))); }
   static __device__ __forceinline__ uint32_t pack(float hi_v, float lo_v) {
     uint32_t d; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi_v), "f"(lo_v)); return d;
   }
-  static __device__ __forceinline__ float quotient(float a, float s, float inv) { (void)inv; return __fdiv_rn(a, s); }
+  static __device__ __forceinline__ float quotient(float a, float s, float inv) {
+    const float q = __fmul_rn(a, inv);
+    return __fmaf_rn(__fmaf_rn(-q, s, a), inv, q);
+  }
+  static __device__ __forceinline__ uint32_t quotients(uint32_t a2, float s_lo, float s_hi, float inv_lo, float inv_hi) {
+    return pack(quotient(hi(a2), s_hi, inv_hi), quotient(lo(a2), s_lo, inv_lo));
+  }
   static __device__ __forceinline__ uint16_t bits(float v) { return __half_as_ushort(__float2half_rn(v)); }
-  static __device__ __forceinline__ double abs_double(uint32_t b) {
-    const uint32_t mag = b & 0x7FFFu;
-    if (mag < 0x400u) return (double)__half2float(__ushort_as_half((uint16_t)mag));   // zero / subnormal
-    return __hiloint2double((int)(mag * 1024u + 0x3F000000u), 0);
+};
+
+
+// magic exponents in the codes of a pair (none where scalar rint produced them)
+template <int DT, int BITS>
+__host__ __device__ constexpr uint32_t pair_magic() {
+  return DT == DARTKV_BF16 && BITS == 8 ? 0u : (DT == DARTKV_BF16 ? 0x43004300u : 0x64006400u);
+}
+// largest code of a pair, as pair_codes() compares it
+template <int DT>
+__device__ __forceinline__ uint32_t cap_pair(float qmax_lo, float qmax_hi) {
+  constexpr float kBase = DT == DARTKV_BF16 ? 128.0f : 1024.0f;
+  return (uint32_t)Pack16<DT>::bits(kBase + qmax_lo) | ((uint32_t)Pack16<DT>::bits(kBase + qmax_hi) << 16);
+}
+// codes of a pair, plus pair_magic(): low element in bits [15:0], high element in bits [31:16]
+template <int DT, int BITS>
+__device__ __forceinline__ uint32_t pair_codes(uint32_t x2, uint32_t mn2, float s_lo, float s_hi, float inv_lo, float inv_hi,
+                                               uint32_t cap2) {
+  using P = Pack16<DT>;
+  const uint32_t r2 = P::quotients(P::sub(x2, mn2), s_lo, s_hi, inv_lo, inv_hi);
+  if (DT == DARTKV_BF16 && BITS == 8)
+    return (uint32_t)fminf(rintf(P::lo(r2)), 255.0f) | ((uint32_t)fminf(rintf(P::hi(r2)), 255.0f) << 16);
+  return P::cap2(P::add(r2, P::kMagic), cap2);
+}
+
+// sum of 4^... shifted magic exponents of a gather register: `count` pairs, `step` bits apart (modulo 2^32)
+__host__ __device__ constexpr uint32_t magic_sum(uint32_t magic, int count, int step) {
+  uint32_t sum = 0;
+  for (int i = 0; i < count; ++i) sum += magic << (step * i);
+  return sum;
+}
+
+// acc + (codes << shift) as one multiply-add
+__device__ __forceinline__ uint32_t gather(uint32_t acc, uint32_t codes, int shift) {
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(codes), "r"(1u << shift), "r"(acc));
+  return d;
+}
+
+// two neighbouring metadata values (scale or zero point), rounded to the metadata dtype
+__device__ __forceinline__ void store_pair(void* p, int md, int64_t pair, float a, float b) {
+  if (md == DARTKV_F32) reinterpret_cast<float2*>(p)[pair] = make_float2(a, b);
+  else if (md == DARTKV_F16) reinterpret_cast<uint32_t*>(p)[pair] = Pack16<DARTKV_F16>::pack(b, a);
+  else reinterpret_cast<uint32_t*>(p)[pair] = Pack16<DARTKV_BF16>::pack(b, a);
+}
+
+// The dense rows of a step for one (batch, head) and side, 64 rows at a time with 16 lanes per row: load() brings
+// a batch into registers (beside the loads of the page, so that a small step waits for memory once), store() puts
+// it into the sink and ring rows once the block has read the ring.
+template <int DT>
+struct DenseBatch {
+  static constexpr int ROWS = 4;   // rows per thread
+  uint4 v[ROWS];
+  const uint16_t* chunk;
+  uint4 *sink, *ring;
+  int sink_copy, ring_first, rows, ring_begin, chunk_start, ring_tokens;
+  int64_t st;
+
+  __device__ __forceinline__ void init(const dartkv_cache_desc& d, const RowSource& src, const dartkv_append_plan& plan,
+                                       int bh, int role) {
+    const DenseRows r = dense_rows(plan);
+    const uint16_t* ring_base;
+    src.bases(bh, chunk, ring_base);
+    sink = reinterpret_cast<uint4*>(role == 0 ? d.k_sink : d.v_sink) + (int64_t)bh * d.sink_tokens * 16;
+    ring = reinterpret_cast<uint4*>(role == 0 ? d.k_ring : d.v_ring) + (int64_t)bh * d.ring_tokens * 16;
+    sink_copy = plan.sink_copy; ring_first = r.ring_first; rows = r.rows;
+    ring_begin = role == 0 ? plan.ring_begin : plan.value_end;
+    chunk_start = src.chunk_start; ring_tokens = src.ring_tokens; st = src.st;
+  }
+  __device__ __forceinline__ int chunk_row(int r) const { return r < sink_copy ? r : ring_first + (r - sink_copy); }
+  __device__ __forceinline__ void load(int first) {
+    const int piece = threadIdx.x & 15;
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const int r = first + (threadIdx.x >> 4) + 16 * k;
+      if (r < rows) v[k] = reinterpret_cast<const uint4*>(chunk + (int64_t)chunk_row(r) * st)[piece];
+    }
+  }
+  __device__ __forceinline__ bool store(int first) {   // whether a stored element is Inf or NaN
+    const int piece = threadIdx.x & 15;
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const int r = first + (threadIdx.x >> 4) + 16 * k;
+      if (r >= rows) continue;
+      const int t = chunk_start + chunk_row(r);
+      if (r >= sink_copy && t < ring_begin) continue;
+      bad |= piece_nonfinite(v[k], DT);
+      if (r < sink_copy) sink[t * 16 + piece] = v[k];
+      else ring[(t % ring_tokens) * 16 + piece] = v[k];
+    }
+    return bad;
+  }
+  // the batch in registers, then whatever rows are left
+  __device__ __forceinline__ bool store_all() {
+    bool bad = store(0);
+    for (int first = 16 * ROWS; first < rows; first += 16 * ROWS) {
+      load(first);
+      bad |= store(first);
+    }
+    return bad;
   }
 };
 
-// codes of a pair in bits [7:0] (low element) and [23:16] (high element)
-template <int DT, int BITS>
-__device__ __forceinline__ uint32_t pair_codes(uint32_t x2, uint32_t mn2, float s, float inv, uint32_t cap2) {
+struct KeySmem {
+  __align__(16) uint32_t page[kP * 64];   // [token][channel pair]
+  uint32_t mn[kSplits][64], mx[kSplits][64];
+  float sum[2][kSplits][64];        // [low | high channel]
+  double exact[2][kSplits][64];
+  __align__(16) uint32_t score[64];
+  int rank[kSplits][kD];            // [block of 32 others][channel]
+};
+
+// One key page.  KBITS: 0 = mixed 2+2-bit keys, else uniform keys with KBITS bits.
+template <int DT, int KBITS>
+__device__ __forceinline__ bool key_page(const dartkv_cache_desc& d, const RowSource& src, KeySmem& sm, int bh, int pg,
+                                         int first_slot, int num_pages, int page_token_start,
+                                         const int32_t* __restrict__ indices, DenseBatch<DT>& dense) {
   using P = Pack16<DT>;
-  const uint32_t a2 = P::sub(x2, mn2);
-  const float q_lo = P::quotient(P::lo(a2), s, inv), q_hi = P::quotient(P::hi(a2), s, inv);
-  if (DT == DARTKV_BF16 && BITS == 8) {
-    const uint32_t r2 = P::pack(q_hi, q_lo);
-    const uint32_t c_lo = (uint32_t)fminf(rintf(P::lo(r2)), 255.0f), c_hi = (uint32_t)fminf(rintf(P::hi(r2)), 255.0f);
-    return c_lo | (c_hi << 16);
-  }
-  const uint32_t m2 = P::min2(P::add(P::pack(q_hi, q_lo), P::kMagic), cap2);   // magic + code, capped at magic + qmax
-  return m2 & (DT == DARTKV_BF16 ? 0x007F007Fu : 0x03FF03FFu);
-}
-
-template <int DT>
-__device__ __forceinline__ uint32_t cap_pair(float qmax) {
-  const uint32_t one = Pack16<DT>::bits((DT == DARTKV_BF16 ? 128.0f : 1024.0f) + qmax);
-  return one * 0x00010001u;
-}
-
-__device__ __forceinline__ uint32_t umin16x2(uint32_t a, uint32_t b) {
-  uint32_t d; asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
-}
-
-// |x| of a normal 16-bit float, from its 15 magnitude bits, as the high word of a double (low word 0)
-template <int DT>
-__device__ __forceinline__ double normal_abs_as_double(uint32_t magnitude) {
-  constexpr uint32_t kShift = DT == DARTKV_BF16 ? 8192u : 1024u;
-  constexpr uint32_t kBias = DT == DARTKV_BF16 ? 0x38000000u : 0x3F000000u;
-  return __hiloint2double((int)(magnitude * kShift + kBias), 0);
-}
-// any magnitude, zero and subnormals included
-template <int DT>
-__device__ __forceinline__ double any_abs_as_double(uint32_t magnitude) {
-  constexpr uint32_t kMinNormal = DT == DARTKV_BF16 ? 0x80u : 0x400u;
-  constexpr double kUnit = DT == DARTKV_BF16 ? 9.183549615799121e-41 : 5.9604644775390625e-08;   // 2^-133, 2^-24
-  return magnitude >= kMinNormal ? normal_abs_as_double<DT>(magnitude) : (double)(int)magnitude * kUnit;
-}
-
-// KBITS: 0 = mixed 2+2-bit keys, else uniform keys with KBITS bits.
-// One block of 64 * TQ threads per (batch*head, page); thread (tq, p) owns the adjacent channels 2p, 2p+1, which
-// travel together as one packed pair through both passes, for the tokens of quarter tq (TQ = 1, 2 or 4 splits
-// of the page's 128 tokens).  The splits meet twice in shared memory: for the channel statistics after pass 1
-// and for the ranks of the promoted channels.  More threads per page mean more resident warps per SM (the page
-// staging, 32 KiB, is what limits the pages per SM) and a shorter critical path when a step brings few pages.
-template <int DT, int KBITS, int TQ>
-__global__ void __launch_bounds__(64 * TQ) fast_key_pages_kernel(dartkv_cache_desc d, RowSource src, int first_slot,
-                                                                 int num_pages, int page_token_start,
-                                                                 const int32_t* __restrict__ indices, int32_t* nonfinite,
-                                                                 const dartkv_append_plan* device_plan) {
-  using P = Pack16<DT>;
-  constexpr int TOK = kP / TQ;   // tokens per thread and pass
-  if (device_plan) {
-    // the step was planned on the device (the grid is the most pages such a step can bring): take the step's
-    // numbers from there; blocks beyond its pages have nothing to do
-    first_slot = device_plan->first_page;
-    num_pages = device_plan->num_pages;
-    page_token_start = device_plan->page_token_start;
-    src.chunk_start = device_plan->chunk_start;
-    if ((int)blockIdx.y >= num_pages) return;
-  }
-  __shared__ __align__(16) uint32_t s_page[kP * 64];   // [token][channel pair]
-  __shared__ __align__(16) uint32_t s_key[kD];
-  __shared__ uint32_t s_part[TQ > 1 ? 3 * TQ * 64 : 1];      // [min | max | smallest magnitude][split][pair]
-  __shared__ double s_sum[TQ > 1 ? 2 * TQ * 64 : 1];         // [low | high channel][split][pair]
-  __shared__ int s_rank[TQ > 1 ? TQ * kD : 1];               // [split][channel]
-  const int bh = blockIdx.x, pg = blockIdx.y, p = threadIdx.x & 63, tq = threadIdx.x >> 6;
-  const int t0 = page_token_start + pg * kP;
+  const int p = threadIdx.x & 63, tq = threadIdx.x >> 6;
   const uint16_t *chunk_base, *ring_base;
   src.bases(bh, chunk_base, ring_base);
-  // stage the page: 2048 16-byte pieces (thread: piece tid%16 of rows tid/16, tid/16 + 4*TQ, ...)
+  // stage the page: piece threadIdx % 16 of rows threadIdx / 16, + 16, ...
   {
-    const int piece = threadIdx.x & 15, r0 = threadIdx.x >> 4;
-    char* dst = reinterpret_cast<char*>(s_page) + r0 * 256 + piece * 16;
-    if (t0 >= src.chunk_start) {
-      const char* from = reinterpret_cast<const char*>(chunk_base + (int64_t)(t0 - src.chunk_start + r0) * src.st) + piece * 16;
-      const int64_t step = src.st * (8 * TQ);   // 4 * TQ rows, in bytes
-#pragma unroll 8
-      for (int k = 0; k < kP / (4 * TQ); ++k) cp_async16(dst + k * (1024 * TQ), from + k * step);
-    } else {
-      for (int k = 0; k < kP / (4 * TQ); ++k)
-        cp_async16(dst + k * (1024 * TQ),
-                   reinterpret_cast<const char*>(src.row_from(chunk_base, ring_base, t0 + r0 + 4 * TQ * k)) + piece * 16);
+    const int piece = threadIdx.x & 15, r0 = threadIdx.x >> 4, first = page_token_start + pg * kP;
+    uint32_t* to = sm.page + r0 * 64 + piece * 4;
+    if (first >= src.chunk_start) {
+      const uint16_t* from = chunk_base + (int64_t)(first - src.chunk_start + r0) * src.st + piece * 8;
+      if (src.st == kD) {   // rows of one head lie together: every address is the first one plus a constant
+#pragma unroll
+        for (int k = 0; k < kP / 16; ++k) cp_async16(to + k * 1024, from + k * 16 * kD);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kP / 16; ++k, from += 16 * src.st) cp_async16(to + k * 1024, from);
+      }
+    } else {                // the first tokens of the page wait in the ring
+#pragma unroll
+      for (int k = 0; k < kP / 16; ++k)
+        cp_async16(to + k * 1024, src.row_from(chunk_base, ring_base, first + r0 + 16 * k) + piece * 8);
     }
   }
+  if (dense.rows > 0) dense.load(0);
   cp_async_wait_all();
   __syncthreads();
-
+  bool bad = false;
+  if (dense.rows > 0) bad = dense.store_all();   // every ring row of the page has been read
+  const uint32_t* x = sm.page + (tq * kTok) * 64 + p;   // + 64 * token
   uint8_t* page = d.k_pages + ((int64_t)bh * d.max_key_pages + first_slot + pg) * d.key_page_bytes;
-  const uint32_t* col = s_page + p;
-  // pass 1: packed min / max (NaN-propagating, so Inf/NaN inputs surface in them) and, for mixed pages,
-  // sum |k| per channel in double (exact for 16-bit inputs).  The loop takes every magnitude for a normal
-  // number; the smallest magnitude seen says whether a channel has to be summed again with care.
-  uint32_t mn2 = col[tq * TOK * 64], mx2 = mn2, min_mag2 = 0xFFFFFFFFu;
-  constexpr uint32_t kMinNormal = DT == DARTKV_BF16 ? 0x80u : 0x400u;
-  double sum_lo = 0.0, sum_hi = 0.0;
-#pragma unroll 8
-  for (int t = tq * TOK; t < (tq + 1) * TOK; ++t) {
-    const uint32_t x2 = col[t * 64];
-    mn2 = P::min2(mn2, x2);
-    mx2 = P::max2(mx2, x2);
-    if (KBITS == 0) {
-      const uint32_t mag2 = x2 & 0x7FFF7FFFu;
-      min_mag2 = umin16x2(min_mag2, mag2);
-      sum_lo += normal_abs_as_double<DT>(mag2 & 0xFFFFu);
-      sum_hi += normal_abs_as_double<DT>(mag2 >> 16);
-    }
-  }
-  if (TQ > 1) {
-    // the splits of a channel pair exchange their partial statistics; every split then holds the page's values
-    s_part[(0 * TQ + tq) * 64 + p] = mn2;
-    s_part[(1 * TQ + tq) * 64 + p] = mx2;
-    if (KBITS == 0) {
-      s_part[(2 * TQ + tq) * 64 + p] = min_mag2;
-      s_sum[(0 * TQ + tq) * 64 + p] = sum_lo;
-      s_sum[(1 * TQ + tq) * 64 + p] = sum_hi;
-    }
-    __syncthreads();
-    mn2 = s_part[(0 * TQ) * 64 + p];
-    mx2 = s_part[(1 * TQ) * 64 + p];
-    if (KBITS == 0) { min_mag2 = s_part[(2 * TQ) * 64 + p]; sum_lo = s_sum[p]; sum_hi = s_sum[TQ * 64 + p]; }
+  // the scores are only needed when the kernel ranks the channels itself
+  const bool ranked = KBITS == 0 && indices == nullptr && d.promoted > 0 && d.promoted < kD;
+
+  // pass 1: packed min / max (NaN-propagating, so Inf/NaN inputs surface in them) and sum |k| per channel.  The score
+  // is the exact sum rounded to fp32, divided and rounded to the data dtype.  bf16: an fp32 sum decides it unless the
+  // rounding boundary lies within the sum's error (about 1 page in 16 has such a channel), then the block sums again in
+  // double; fp16 scores have 11 bits and almost
+  // every page would, so they are summed in double at once.
+  uint32_t mn2 = x[0], mx2 = mn2;
+  float part_lo[2] = {0.0f, 0.0f}, part_hi[2] = {0.0f, 0.0f};
+  double e_lo = 0.0, e_hi = 0.0;
 #pragma unroll
-    for (int o = 1; o < TQ; ++o) {
-      mn2 = P::min2(mn2, s_part[(0 * TQ + o) * 64 + p]);
-      mx2 = P::max2(mx2, s_part[(1 * TQ + o) * 64 + p]);
-      if (KBITS == 0) {
-        min_mag2 = umin16x2(min_mag2, s_part[(2 * TQ + o) * 64 + p]);
-        sum_lo += s_sum[(0 * TQ + o) * 64 + p];     // sums of 16-bit magnitudes are exact in double: any order
-        sum_hi += s_sum[(1 * TQ + o) * 64 + p];
-      }
-    }
+  for (int j = 0; j < kTok; ++j) {
+    const uint32_t v = x[64 * j];
+    mn2 = P::min2(mn2, v);
+    mx2 = P::max2(mx2, v);
+    if (KBITS == 0 && DT == DARTKV_BF16) { part_lo[j & 1] += fabsf(P::lo(v)); part_hi[j & 1] += fabsf(P::hi(v)); }
+    if (KBITS == 0 && DT == DARTKV_F16) { e_lo += (double)fabsf(P::lo(v)); e_hi += (double)fabsf(P::hi(v)); }
   }
+  float sum_lo = part_lo[0] + part_lo[1], sum_hi = part_hi[0] + part_hi[1];
+  sm.mn[tq][p] = mn2;
+  sm.mx[tq][p] = mx2;
+  if (KBITS == 0 && DT == DARTKV_BF16) { sm.sum[0][tq][p] = sum_lo; sm.sum[1][tq][p] = sum_hi; }
+  if (KBITS == 0 && DT == DARTKV_F16) { sm.exact[0][tq][p] = e_lo; sm.exact[1][tq][p] = e_hi; }
+  __syncthreads();
+  mn2 = sm.mn[0][p];
+  mx2 = sm.mx[0][p];
+#pragma unroll
+  for (int o = 1; o < kSplits; ++o) { mn2 = P::min2(mn2, sm.mn[o][p]); mx2 = P::max2(mx2, sm.mx[o][p]); }
   const float mn_lo = P::lo(mn2), mn_hi = P::hi(mn2), mx_lo = P::lo(mx2), mx_hi = P::hi(mx2);
-  const bool bad = !(isfinite(mn_lo) && isfinite(mn_hi) && isfinite(mx_lo) && isfinite(mx_hi));
+  bad |= !(isfinite(mn_lo) && isfinite(mn_hi) && isfinite(mx_lo) && isfinite(mx_hi));
+
   int slot_lo = -1, slot_hi = -1;
   float qmax_lo, qmax_hi;
   if (KBITS == 0) {
@@ -279,43 +353,81 @@ __global__ void __launch_bounds__(64 * TQ) fast_key_pages_kernel(dartkv_cache_de
         if (ch == c_lo) slot_lo = k;
         if (ch == c_hi) slot_hi = k;
       }
-      for (int k = threadIdx.x; k < K; k += 64 * TQ) idx_field[k] = mine[k];
+      for (int k = threadIdx.x; k < K; k += kThreads) idx_field[k] = mine[k];
     } else if (K == kD) {
       slot_lo = c_lo; slot_hi = c_hi;
       if (tq == 0) { idx_field[c_lo] = c_lo; idx_field[c_hi] = c_hi; }
-    } else if (K > 0) {
-      if ((min_mag2 & 0xFFFFu) < kMinNormal || (min_mag2 >> 16) < kMinNormal) {   // zeros or subnormals: sum again
-        sum_lo = 0.0; sum_hi = 0.0;
-        for (int t = 0; t < kP; ++t) {
-          const uint32_t mag2 = col[t * 64] & 0x7FFF7FFFu;
-          sum_lo += any_abs_as_double<DT>(mag2 & 0xFFFFu);
-          sum_hi += any_abs_as_double<DT>(mag2 >> 16);
-        }
+    } else if (ranked) {
+      // score bits of a channel from its sum
+      auto score = [](float sum) -> uint32_t { return P::bits(__fmul_rn(sum, 1.0f / kP)); };   // a power of two: exact like the division
+      uint32_t score_lo = 0, score_hi = 0;
+      bool unsure = true;
+      if (DT == DARTKV_BF16) {
+        sum_lo = (sm.sum[0][0][p] + sm.sum[0][1][p]) + (sm.sum[0][2][p] + sm.sum[0][3][p]);
+        sum_hi = (sm.sum[1][0][p] + sm.sum[1][1][p]) + (sm.sum[1][2][p] + sm.sum[1][3][p]);
+        // 15 additions per partial sum and three more: at most 18 rounding errors of 2^-24 each, and one of the product
+        constexpr float kError = 20.0f / 16777216.0f, kBelow = 1.0f - kError, kAbove = 1.0f + kError;
+        score_lo = score(sum_lo * kBelow);
+        score_hi = score(sum_hi * kBelow);
+        unsure = score_lo != score(sum_lo * kAbove) || score_hi != score(sum_hi * kAbove) ||
+                 !(sum_lo < 1e37f) || !(sum_hi < 1e37f);
       }
-      // rank by (score descending, channel ascending): scores are non-negative 16-bit floats, so their bit
-      // patterns order like integers and one unsigned key carries both criteria
-      const uint32_t key_lo = ((uint32_t)P::bits(__fdiv_rn((float)sum_lo, (float)kP)) << 7) | (uint32_t)(kD - 1 - c_lo);
-      const uint32_t key_hi = ((uint32_t)P::bits(__fdiv_rn((float)sum_hi, (float)kP)) << 7) | (uint32_t)(kD - 1 - c_hi);
-      if (tq == 0) {
-        s_key[c_lo] = key_lo;
-        s_key[c_hi] = key_hi;
+      const bool exact = DT == DARTKV_F16 || __syncthreads_or(unsure);
+      if (exact) {
+        if (DT == DARTKV_BF16) {
+#pragma unroll 8
+          for (int j = 0; j < kTok; ++j) {
+            const uint32_t again = x[64 * j];
+            e_lo += (double)fabsf(P::lo(again));
+            e_hi += (double)fabsf(P::hi(again));
+          }
+          sm.exact[0][tq][p] = e_lo;
+          sm.exact[1][tq][p] = e_hi;
+          __syncthreads();
+        }
+        e_lo = (sm.exact[0][0][p] + sm.exact[0][1][p]) + (sm.exact[0][2][p] + sm.exact[0][3][p]);
+        e_hi = (sm.exact[1][0][p] + sm.exact[1][1][p]) + (sm.exact[1][2][p] + sm.exact[1][3][p]);
+        score_lo = score((float)e_lo);
+        score_hi = score((float)e_hi);
+      }
+      // Rank by (score descending, channel ascending).  The 128 x 128 comparisons go as 16 squares of 32 channels
+      // against 32 others, two squares per warp, lane = channel, two others per packed comparison; a channel with
+      // the same score counts if it comes first, i.e. against the next smaller number instead of the score.
+      if (tq == 0) sm.score[p] = score_lo | (score_hi << 16);
+      __syncthreads();
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int mine = warp >> 1, others = 2 * (warp & 1) + i;     // blocks of 32 channels
+        const uint32_t bits = reinterpret_cast<const uint16_t*>(sm.score)[32 * mine + lane];
+        const uint32_t above = bits * 0x00010001u, from = (bits == 0 ? 0x8001u : bits - 1u) * 0x00010001u;
+        uint32_t count = 0;
+        const uint4* o4 = reinterpret_cast<const uint4*>(sm.score) + 4 * others;
+        if (others != mine) {
+          const uint32_t than = others < mine ? from : above;
+#pragma unroll
+          for (int r4 = 0; r4 < 4; ++r4) {
+            const uint4 o = o4[r4];
+            count = P::count_greater(P::count_greater(count, o.x, than), o.y, than);
+            count = P::count_greater(P::count_greater(count, o.z, than), o.w, than);
+          }
+        } else {   // others 2r and 2r + 1 of the channel's own block come before it, after it, or on both sides
+          const uint32_t both = lane & 1 ? (from & 0xFFFFu) | (above & 0xFFFF0000u) : above;
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            const uint32_t o = sm.score[16 * others + r];
+            count = P::count_greater(count, o, r < lane >> 1 ? from : (r == lane >> 1 ? both : above));
+          }
+        }
+        sm.rank[others][32 * mine + lane] = (int)(P::lo(count) + P::hi(count));
       }
       __syncthreads();
-      // every split counts the larger keys among its share of the 128 channels
-      int rank_lo = 0, rank_hi = 0;
-#pragma unroll 4
-      for (int o = tq * (kD / 4 / TQ); o < (tq + 1) * (kD / 4 / TQ); ++o) {
-        const uint4 k4 = reinterpret_cast<const uint4*>(s_key)[o];
-        rank_lo += (k4.x > key_lo) + (k4.y > key_lo) + (k4.z > key_lo) + (k4.w > key_lo);
-        rank_hi += (k4.x > key_hi) + (k4.y > key_hi) + (k4.z > key_hi) + (k4.w > key_hi);
-      }
-      if (TQ > 1) {
-        s_rank[tq * kD + c_lo] = rank_lo;
-        s_rank[tq * kD + c_hi] = rank_hi;
-        __syncthreads();
-        rank_lo = 0; rank_hi = 0;
+      int rank_lo, rank_hi;
+      rank_lo = 0; rank_hi = 0;
 #pragma unroll
-        for (int o = 0; o < TQ; ++o) { rank_lo += s_rank[o * kD + c_lo]; rank_hi += s_rank[o * kD + c_hi]; }
+      for (int o = 0; o < kSplits; ++o) {
+        const int2 r = *reinterpret_cast<const int2*>(&sm.rank[o][c_lo]);
+        rank_lo += r.x; rank_hi += r.y;
       }
       if (rank_lo < K) { slot_lo = rank_lo; if (tq == 0) idx_field[rank_lo] = c_lo; }
       if (rank_hi < K) { slot_hi = rank_hi; if (tq == 0) idx_field[rank_hi] = c_hi; }
@@ -325,183 +437,267 @@ __global__ void __launch_bounds__(64 * TQ) fast_key_pages_kernel(dartkv_cache_de
   } else {
     qmax_lo = qmax_hi = (float)((1 << KBITS) - 1);
   }
-  const float scale_lo = scale_of<DT>(mn_lo, mx_lo, qmax_lo), scale_hi = scale_of<DT>(mn_hi, mx_hi, qmax_hi);
+  float scale_lo = scale_of<DT>(mn_lo, mx_lo, qmax_lo), scale_hi = scale_of<DT>(mn_hi, mx_hi, qmax_hi);
   if (tq == 0) {
-    store_f(page + d.key_off_scale, d.md_dtype, 2 * p, scale_lo);
-    store_f(page + d.key_off_scale, d.md_dtype, 2 * p + 1, scale_hi);
-    store_f(page + d.key_off_zero, d.md_dtype, 2 * p, mn_lo);
-    store_f(page + d.key_off_zero, d.md_dtype, 2 * p + 1, mn_hi);
+    store_pair(page + d.key_off_scale, d.md_dtype, p, scale_lo, scale_hi);
+    store_pair(page + d.key_off_zero, d.md_dtype, p, mn_lo, mn_hi);
   }
-  const float inv_lo = inverse_scale<DT>(scale_lo), inv_hi = inverse_scale<DT>(scale_hi);
-  const uint32_t cap2 = (uint32_t)P::bits((DT == DARTKV_BF16 ? 128.0f : 1024.0f) + qmax_lo) |
-                        ((uint32_t)P::bits((DT == DARTKV_BF16 ? 128.0f : 1024.0f) + qmax_hi) << 16);
+  const float inv_lo = inverse_scale(scale_lo), inv_hi = inverse_scale(scale_hi);
+  if (DT == DARTKV_F16) {   // an infinite scale enters the quotient as zero
+    scale_lo = isinf(scale_lo) ? 0.0f : scale_lo;
+    scale_hi = isinf(scale_hi) ? 0.0f : scale_hi;
+  }
+  const uint32_t cap2 = cap_pair<DT>(qmax_lo, qmax_hi);
 
-  // pass 2: codes of (channel 2p, channel 2p+1) for one token per step.  A plane's fields of both channels
-  // gather in one register (channel 2p in the low half, 2p+1 in the high half, 16/BITS tokens each); two such
-  // registers split into one 32-bit word per channel.  Split tq produces words [tq, tq+1) * WORDS / TQ.
+  // pass 2: the codes of a channel pair gather in registers, channel 2p in the low half and 2p+1 in the high half,
+  // 16 / BITS tokens each; two such registers split into one 32-bit word per channel.
   constexpr int BITS = KBITS == 0 ? 2 : KBITS;      // bits per stored plane
-  constexpr int CODE_BITS = KBITS == 0 ? 4 : KBITS; // bits the quantizer produces
   constexpr int PER_HALF = 16 / BITS;               // tokens per 16-bit half of a plane word
   constexpr int WORDS = kP / (2 * PER_HALF);        // 32-bit words per channel and plane
-  constexpr int MY_WORDS = WORDS / TQ;              // words of this split
-  constexpr int CHUNK = MY_WORDS < 4 ? MY_WORDS : 4;   // words per store
-  static_assert(MY_WORDS >= 2 && MY_WORDS % CHUNK == 0, "page words do not split this way");
-  constexpr uint32_t FIELD2 = ((1u << BITS) - 1u) * 0x00010001u;
-  uint32_t* low_lo = reinterpret_cast<uint32_t*>(page + (2 * p) * (WORDS * 4));
-  uint32_t* low_hi = low_lo + WORDS;
-  uint32_t* high_lo = (KBITS == 0 && slot_lo >= 0) ? reinterpret_cast<uint32_t*>(page + d.key_off_high + slot_lo * (WORDS * 4)) : nullptr;
-  uint32_t* high_hi = (KBITS == 0 && slot_hi >= 0) ? reinterpret_cast<uint32_t*>(page + d.key_off_high + slot_hi * (WORDS * 4)) : nullptr;
-#pragma unroll 1
-  for (int w4 = tq * MY_WORDS; w4 < (tq + 1) * MY_WORDS; w4 += CHUNK) {
+  constexpr int MY_WORDS = WORDS / kSplits;         // words of this split: 2, 4 or 8
+  constexpr uint32_t MAGIC = pair_magic<DT, KBITS == 0 ? 4 : KBITS>();
+  constexpr int CHUNK = MY_WORDS < 4 ? 2 : 4;       // words per store
+#pragma unroll
+  for (int w0 = 0; w0 < MY_WORDS; w0 += CHUNK) {
     uint32_t a_lo[CHUNK], a_hi[CHUNK], b_lo[CHUNK], b_hi[CHUNK];   // a: low plane, b: high plane
 #pragma unroll
-    for (int q = 0; q < CHUNK; ++q) {
+    for (int w = 0; w < CHUNK; ++w) {
       uint32_t acc_a[2], acc_b[2];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        uint32_t fa = 0, fb = 0;
-        const int base = ((w4 + q) * 2 + half) * PER_HALF;
+        const int base = (2 * (w0 + w) + half) * PER_HALF;
+        auto codes = [&](int j) {
+          return pair_codes<DT, KBITS == 0 ? 4 : KBITS>(x[64 * j], mn2, scale_lo, scale_hi, inv_lo, inv_hi, cap2);
+        };
+        if (KBITS == 0) {
+          // 4-bit codes of the even and of the odd tokens as nibbles, then the planes of all eight tokens at once
+          uint32_t even = 0u - magic_sum(MAGIC, 4, 4), odd = even;
 #pragma unroll
-        for (int u = 0; u < PER_HALF; ++u) {
-          const uint32_t x2 = col[(base + u) * 64];
-          const uint32_t a2 = P::sub(x2, mn2);
-          const float q_l = P::quotient(P::lo(a2), scale_lo, inv_lo), q_h = P::quotient(P::hi(a2), scale_hi, inv_hi);
-          uint32_t codes;
-          if (DT == DARTKV_BF16 && CODE_BITS == 8) {
-            const uint32_t r2 = P::pack(q_h, q_l);
-            codes = (uint32_t)fminf(rintf(P::lo(r2)), 255.0f) | ((uint32_t)fminf(rintf(P::hi(r2)), 255.0f) << 16);
-          } else {
-            codes = P::min2(P::add(P::pack(q_h, q_l), P::kMagic), cap2);
+          for (int u = 0; u < 4; ++u) {
+            even = gather(even, codes(base + 2 * u), 4 * u);
+            odd = gather(odd, codes(base + 2 * u + 1), 4 * u);
           }
-          fa += (codes & FIELD2) << (BITS * u);
-          if (KBITS == 0) fb += ((codes >> 2) & FIELD2) << (BITS * u);
+          acc_a[half] = (even & 0x33333333u) | ((odd << 2) & 0xCCCCCCCCu);
+          acc_b[half] = ((even >> 2) & 0x33333333u) | (odd & 0xCCCCCCCCu);
+        } else {
+          uint32_t acc = 0u - magic_sum(MAGIC, PER_HALF, BITS);
+#pragma unroll
+          for (int u = 0; u < PER_HALF; ++u) acc = gather(acc, codes(base + u), BITS * u);
+          acc_a[half] = acc;
+          acc_b[half] = 0;
         }
-        acc_a[half] = fa;
-        acc_b[half] = fb;
       }
-      a_lo[q] = __byte_perm(acc_a[0], acc_a[1], 0x5410);
-      a_hi[q] = __byte_perm(acc_a[0], acc_a[1], 0x7632);
-      if (KBITS == 0) {
-        b_lo[q] = __byte_perm(acc_b[0], acc_b[1], 0x5410);
-        b_hi[q] = __byte_perm(acc_b[0], acc_b[1], 0x7632);
-      }
+      a_lo[w] = __byte_perm(acc_a[0], acc_a[1], 0x5410);
+      a_hi[w] = __byte_perm(acc_a[0], acc_a[1], 0x7632);
+      b_lo[w] = __byte_perm(acc_b[0], acc_b[1], 0x5410);
+      b_hi[w] = __byte_perm(acc_b[0], acc_b[1], 0x7632);
     }
-    if (CHUNK == 4) {
-      reinterpret_cast<uint4*>(low_lo)[w4 / 4] = make_uint4(a_lo[0], a_lo[1], a_lo[2], a_lo[3]);
-      reinterpret_cast<uint4*>(low_hi)[w4 / 4] = make_uint4(a_hi[0], a_hi[1], a_hi[2], a_hi[3]);
-      if (KBITS == 0) {
-        if (high_lo) reinterpret_cast<uint4*>(high_lo)[w4 / 4] = make_uint4(b_lo[0], b_lo[1], b_lo[2], b_lo[3]);
-        if (high_hi) reinterpret_cast<uint4*>(high_hi)[w4 / 4] = make_uint4(b_hi[0], b_hi[1], b_hi[2], b_hi[3]);
-      }
-    } else {
-      reinterpret_cast<uint2*>(low_lo)[w4 / 2] = make_uint2(a_lo[0], a_lo[CHUNK - 1]);
-      reinterpret_cast<uint2*>(low_hi)[w4 / 2] = make_uint2(a_hi[0], a_hi[CHUNK - 1]);
-      if (KBITS == 0) {
-        if (high_lo) reinterpret_cast<uint2*>(high_lo)[w4 / 2] = make_uint2(b_lo[0], b_lo[CHUNK - 1]);
-        if (high_hi) reinterpret_cast<uint2*>(high_hi)[w4 / 2] = make_uint2(b_hi[0], b_hi[CHUNK - 1]);
-      }
+    auto store_words = [&](uint8_t* row, const uint32_t (&v)[CHUNK]) {
+      uint32_t* to = reinterpret_cast<uint32_t*>(row) + tq * MY_WORDS + w0;
+      if (CHUNK == 2) *reinterpret_cast<uint2*>(to) = make_uint2(v[0], v[1]);
+      else *reinterpret_cast<uint4*>(to) = make_uint4(v[0], v[1], v[CHUNK - 2], v[CHUNK - 1]);
+    };
+    store_words(page + (2 * p) * (WORDS * 4), a_lo);
+    store_words(page + (2 * p + 1) * (WORDS * 4), a_hi);
+    if (KBITS == 0) {
+      if (slot_lo >= 0) store_words(page + d.key_off_high + slot_lo * (WORDS * 4), b_lo);
+      if (slot_hi >= 0) store_words(page + d.key_off_high + slot_hi * (WORDS * 4), b_hi);
     }
   }
-  if (bad && nonfinite) *nonfinite = 1;
+  return bad;
 }
 
-// Values: eight lanes per token row (16 channels per lane), four rows per warp per step, two steps in
-// flight; grid (64-row blocks of one (batch, head), batch*head).  VBITS in {2,4,8}; lanes_per_group =
-// value_group / 16.
+// 128 value rows from `first` (relative to value_begin; rows past `count` are skipped): four lanes per token row,
+// 32 channels per lane, so a warp holds eight rows and a block goes twice over 64.  A group is half a lane
+// (value_group 16), one lane (32), or 2 / 4 neighbouring lanes.
 template <int DT, int VBITS>
-__global__ void __launch_bounds__(256) fast_value_rows_kernel(dartkv_cache_desc d, RowSource src, int value_begin,
-                                                              int count, int lanes_per_group, int32_t* nonfinite,
-                                                              const dartkv_append_plan* device_plan) {
+__device__ __forceinline__ bool value_rows(const dartkv_cache_desc& d, const RowSource& src, int bh, int first,
+                                           int value_begin, int count) {
   using P = Pack16<DT>;
-  constexpr int STEPS = 2;
-  if (device_plan) {   // planned on the device: the grid covers the most rows such a step can pack
-    value_begin = device_plan->value_begin;
-    count = device_plan->value_end - device_plan->value_begin;
-    src.chunk_start = device_plan->chunk_start;
-  }
-  const int bh = blockIdx.y, lane = threadIdx.x & 31;
-  const int sub = lane >> 3, part = lane & 7;   // row within the step, 16-channel slice of the row
-  const int first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * (4 * STEPS);
-  if (first >= count) return;
+  constexpr int ROWS = 2;               // rows per thread, all loads in flight together
+  const int lane = threadIdx.x & 31, part = lane & 3;
+  const int row0 = first + (threadIdx.x >> 2);
   const uint16_t *chunk_base, *ring_base;
   src.bases(bh, chunk_base, ring_base);
-  uint4 raw[STEPS][2];
-  int t_of[STEPS];
-  bool live[STEPS];
+  bool bad = false;
+  if (first + (threadIdx.x & ~31) / 4 >= count) return bad;   // the whole warp is past the end
+  const bool from_ring = value_begin + first < src.chunk_start;   // only blocks of the step's first rows
+  uint4 raw[ROWS][4];
 #pragma unroll
-  for (int s = 0; s < STEPS; ++s) {
-    const int row = first + 4 * s + sub;
-    live[s] = row < count;
-    t_of[s] = value_begin + (live[s] ? row : count - 1);
-    const uint4* ptr = reinterpret_cast<const uint4*>(src.row_from(chunk_base, ring_base, t_of[s]) + part * 16);
-    raw[s][0] = ptr[0];
-    raw[s][1] = ptr[1];
+  for (int s = 0; s < ROWS; ++s) {
+    const int t = value_begin + min(row0 + 64 * s, count - 1);
+    const uint16_t* row = chunk_base + (int64_t)(t - src.chunk_start) * src.st;
+    if (from_ring && t < src.chunk_start) row = ring_base + (t % src.ring_tokens) * kD;
+    const uint4* ptr = reinterpret_cast<const uint4*>(row + part * 32);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) raw[s][i] = ptr[i];
   }
   constexpr float qmax = (float)((1 << VBITS) - 1);
-  const uint32_t cap2 = cap_pair<DT>(qmax);
-  bool bad = false;
+  const uint32_t cap2 = cap_pair<DT>(qmax, qmax);
+  const bool half_lane = d.value_group == 16;
+  const int lanes = d.value_group >> 5;   // lanes per group
 #pragma unroll
-  for (int s = 0; s < STEPS; ++s) {
-    const uint32_t x[8] = {raw[s][0].x, raw[s][0].y, raw[s][0].z, raw[s][0].w, raw[s][1].x, raw[s][1].y, raw[s][1].z, raw[s][1].w};
-    uint32_t mn2 = x[0], mx2 = x[0];
+  for (int s = 0; s < ROWS; ++s) {
+    uint32_t x[16];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) {
-      mn2 = P::min2(mn2, x[i]);
-      mx2 = P::max2(mx2, x[i]);
+    for (int i = 0; i < 4; ++i) { x[4 * i] = raw[s][i].x; x[4 * i + 1] = raw[s][i].y; x[4 * i + 2] = raw[s][i].z; x[4 * i + 3] = raw[s][i].w; }
+    uint32_t mn2[2], mx2[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mn2[h] = mx2[h] = x[8 * h];
+#pragma unroll
+      for (int i = 1; i < 8; ++i) { mn2[h] = P::min2(mn2[h], x[8 * h + i]); mx2[h] = P::max2(mx2[h], x[8 * h + i]); }
     }
-    for (int off = 1; off < lanes_per_group; off <<= 1) {
-      mn2 = P::min2(mn2, __shfl_xor_sync(0xffffffffu, mn2, off));
-      mx2 = P::max2(mx2, __shfl_xor_sync(0xffffffffu, mx2, off));
+    if (!half_lane) {
+      mn2[0] = P::min2(mn2[0], mn2[1]);
+      mx2[0] = P::max2(mx2[0], mx2[1]);
+      for (int off = 1; off < lanes; off <<= 1) {
+        mn2[0] = P::min2(mn2[0], __shfl_xor_sync(0xffffffffu, mn2[0], off));
+        mx2[0] = P::max2(mx2[0], __shfl_xor_sync(0xffffffffu, mx2[0], off));
+      }
+      mn2[1] = mn2[0];
+      mx2[1] = mx2[0];
     }
-    // NaN-propagating min / max: any Inf or NaN of the group ends up in mn or mx
-    const uint32_t mn1 = P::min2(mn2, mn2 >> 16), mx1 = P::max2(mx2, mx2 >> 16);
-    const float mn = P::lo(mn1), mx = P::lo(mx1);
-    bad |= live[s] && !(isfinite(mn) && isfinite(mx));
-    const float scale = scale_of<DT>(mn, mx, qmax);
-    const float inv = inverse_scale<DT>(scale);
-    const uint32_t mnp = (mn1 & 0xFFFFu) * 0x00010001u;
-    // codes of 16/(2*VBITS) pairs gather in one register (even channels in the low half, odd in the high half)
+    float mn[2], scale[2], inv[2], s_q[2];
+    uint32_t mnp[2];
+    const bool live = row0 + 64 * s < count;
+    auto group = [&](int h) {
+      // NaN-propagating min / max: any Inf or NaN of the group ends up in mn or mx
+      const uint32_t mn1 = P::min2(mn2[h], mn2[h] >> 16), mx1 = P::max2(mx2[h], mx2[h] >> 16);
+      mn[h] = P::lo(mn1);
+      const float mx = P::lo(mx1);
+      bad |= live && !(isfinite(mn[h]) && isfinite(mx));
+      scale[h] = scale_of<DT>(mn[h], mx, qmax);
+      inv[h] = inverse_scale(scale[h]);
+      s_q[h] = DT == DARTKV_F16 && isinf(scale[h]) ? 0.0f : scale[h];
+      mnp[h] = (mn1 & 0xFFFFu) * 0x00010001u;
+    };
+    group(0);
+    if (half_lane) {
+      group(1);
+    } else {
+      mn[1] = mn[0]; scale[1] = scale[0]; inv[1] = inv[0]; s_q[1] = s_q[0]; mnp[1] = mnp[0];
+    }
+    // codes of 8 / VBITS pairs gather in one register (even channels in the low half, odd ones in the high half)
     constexpr int PAIRS = 8 / VBITS;                      // pairs per gather register
-    constexpr int GATHERS = 8 / PAIRS;
+    constexpr int GATHERS = 16 / PAIRS;
+    constexpr uint32_t MAGIC = pair_magic<DT, VBITS>();
     constexpr uint32_t LOMASK = VBITS == 2 ? 0x3333u : VBITS == 4 ? 0x0F0Fu : 0x00FFu;
     uint32_t half_word[GATHERS];
 #pragma unroll
     for (int g = 0; g < GATHERS; ++g) {
-      uint32_t acc = 0;
+      uint32_t acc = 0u - magic_sum(MAGIC, PAIRS, 2 * VBITS);
 #pragma unroll
-      for (int i = 0; i < PAIRS; ++i) acc += pair_codes<DT, VBITS>(x[g * PAIRS + i], mnp, scale, inv, cap2) << (2 * VBITS * i);
+      for (int i = 0; i < PAIRS; ++i) {
+        const int k = g * PAIRS + i, h = k / 8;
+        acc = gather(acc, pair_codes<DT, VBITS>(x[k], mnp[h], s_q[h], s_q[h], inv[h], inv[h], cap2), 2 * VBITS * i);
+      }
       half_word[g] = (acc & LOMASK) | ((acc >> (16 - VBITS)) & (LOMASK << VBITS));
     }
-    if (!live[s]) continue;
-    const int64_t out_row = (int64_t)bh * d.max_value_tokens + (t_of[s] - d.sink_tokens);
-    uint8_t* codes = d.v_codes + out_row * d.value_row_bytes;
+    if (!live) continue;
+    const int64_t out_row = (int64_t)bh * d.max_value_tokens + (value_begin + row0 + 64 * s - d.sink_tokens);
+    uint32_t* codes = reinterpret_cast<uint32_t*>(d.v_codes + out_row * d.value_row_bytes) + part * (GATHERS / 2);
     if (VBITS == 2) {
-      reinterpret_cast<uint32_t*>(codes)[part] = half_word[0] | (half_word[1] << 16);
-    } else if (VBITS == 4) {
-      reinterpret_cast<uint2*>(codes)[part] = make_uint2(half_word[0] | (half_word[1] << 16), half_word[2] | (half_word[3] << 16));
+      *reinterpret_cast<uint2*>(codes) = make_uint2(half_word[0] | (half_word[1] << 16), half_word[2] | (half_word[3] << 16));
     } else {
-      reinterpret_cast<uint4*>(codes)[part] = make_uint4(half_word[0] | (half_word[1] << 16), half_word[2] | (half_word[3] << 16),
-                                                         half_word[4] | (half_word[5] << 16), half_word[6] | (half_word[7] << 16));
+#pragma unroll
+      for (int g = 0; g + 7 < GATHERS; g += 8)
+        reinterpret_cast<uint4*>(codes)[g / 8] = make_uint4(half_word[g] | (half_word[g + 1] << 16), half_word[g + 2] | (half_word[g + 3] << 16),
+                                                            half_word[g + 4] | (half_word[g + 5] << 16), half_word[g + 6] | (half_word[g + 7] << 16));
     }
-    if ((part % lanes_per_group) == 0) {
-      const int g = part / lanes_per_group;
-      store_f(d.v_meta, d.md_dtype, (out_row * 2 + 0) * d.value_groups + g, scale);
-      store_f(d.v_meta, d.md_dtype, (out_row * 2 + 1) * d.value_groups + g, mn);
+    if (half_lane) {
+      const int64_t pair = out_row * d.value_groups + part;       // groups 2*part, 2*part + 1 of the scale row
+      store_pair(d.v_meta, d.md_dtype, pair, scale[0], scale[1]);
+      store_pair(d.v_meta, d.md_dtype, pair + d.value_groups / 2, mn[0], mn[1]);
+    } else if ((part & (lanes - 1)) == 0) {
+      const int g = part >> (lanes >> 1);   // lanes per group: 1, 2 or 4
+      store_f(d.v_meta, d.md_dtype, (out_row * 2 + 0) * d.value_groups + g, scale[0]);
+      store_f(d.v_meta, d.md_dtype, (out_row * 2 + 1) * d.value_groups + g, mn[0]);
     }
   }
-  if (bad && nonfinite) *nonfinite = 1;
+  return bad;
 }
 
-bool fast_common(const dartkv_cache_desc* d, int64_t sb, int64_t sh, int64_t st) {
-  return (d->dtype == DARTKV_F16 || d->dtype == DARTKV_BF16) && d->head_dim == kD && st % 8 == 0 && sb % 8 == 0 &&
-         sh % 8 == 0;
+struct StepArgs {
+  RowSource source;                        // strides of the chunk; pointers and first token are set per block
+  const void *keys, *values;
+  dartkv_append_plan plan;
+  const dartkv_append_plan* device_plan;   // where the plan was made on the device: *plan then only sizes the grid
+  const int32_t* indices;
+  int32_t* nonfinite;
+  int roles, role_begin;                   // 2: keys and values; 1: role_begin only (0 keys, 1 values)
+  int copies;                              // the step's dense rows and metadata are written here
+};
+
+// KBITS as in key_page().  Three blocks per SM: 24 warps whose loads (32 words per thread) are all in flight at once.
+template <int DT, int KBITS, int VBITS>
+__global__ void __launch_bounds__(kThreads, 4) append_step_kernel(const __grid_constant__ dartkv_cache_desc d,
+                                                                  const __grid_constant__ StepArgs a) {
+  __shared__ KeySmem sm;
+  // read through the pointer where it is needed: the plan's numbers are not kept in registers across the page code
+  const dartkv_append_plan& plan = a.device_plan ? *a.device_plan : a.plan;
+  // grid: (kv head, batch row, page and role): no division to find any of them
+  const int bh = blockIdx.y * gridDim.x + blockIdx.x;
+  const int pg = a.roles == 2 ? blockIdx.z >> 1 : blockIdx.z, role = a.roles == 2 ? (int)(blockIdx.z & 1) : a.role_begin;
+  RowSource src = a.source;
+  src.chunk = role == 0 ? a.keys : a.values;
+  src.ring = role == 0 ? d.k_ring : d.v_ring;
+  src.chunk_start = plan.chunk_start;
+  const bool writes_dense = a.copies && pg == 0;
+  if (writes_dense && bh == 0 && role == 0) publish_append(d, plan);
+  bool bad = false;
+  DenseBatch<DT> dense;
+  dense.rows = 0;
+  if (role == 0 && pg < plan.num_pages) {
+    if (writes_dense) dense.init(d, src, plan, bh, role);
+    bad = key_page<DT, KBITS>(d, src, sm, bh, pg, plan.first_page, plan.num_pages, plan.page_token_start, a.indices, dense);
+  } else {
+    if (role == 1 && pg * kP < plan.value_end - plan.value_begin)
+      bad = value_rows<DT, VBITS>(d, src, bh, pg * kP, plan.value_begin, plan.value_end - plan.value_begin);
+    if (writes_dense) {
+      // value blocks are done well before the key blocks: their dense rows come last
+      dense.init(d, src, plan, bh, role);
+      __syncthreads();   // every ring row of these values has been read
+      dense.load(0);
+      bad |= dense.store_all();
+    }
+  }
+  if (bad && a.nonfinite) *a.nonfinite = 1;
+}
+
+using StepKernel = void (*)(dartkv_cache_desc, StepArgs);
+template <int DT, int KBITS>
+StepKernel step_variant_v(int value_bits) {
+  return value_bits == 2 ? append_step_kernel<DT, KBITS, 2> : value_bits == 4 ? append_step_kernel<DT, KBITS, 4>
+                                                                              : append_step_kernel<DT, KBITS, 8>;
+}
+template <int DT>
+StepKernel step_variant_k(int key_bits, int value_bits) {
+  switch (key_bits) {
+    case 0: return step_variant_v<DT, 0>(value_bits);
+    case 2: return step_variant_v<DT, 2>(value_bits);
+    case 4: return step_variant_v<DT, 4>(value_bits);
+    default: return step_variant_v<DT, 8>(value_bits);
+  }
+}
+
+int launch_step(const dartkv_cache_desc& d, StepArgs a, int blocks, int roles, cudaStream_t stream) {
+  DARTKV_REQUIRE(blocks * roles <= 65535, "too many pages in one append (limit 32767)");
+  DARTKV_REQUIRE(d.batch <= 65535, "batch above 65535");
+  a.roles = roles;
+  const int key_bits = d.key_mode == DARTKV_MIXED_PAGE ? 0 : d.key_bits;
+  const StepKernel kernel = d.dtype == DARTKV_F16 ? step_variant_k<DARTKV_F16>(key_bits, d.value_bits)
+                                                  : step_variant_k<DARTKV_BF16>(key_bits, d.value_bits);
+  kernel<<<dim3(d.kv_heads, d.batch, blocks * roles), kThreads, 0, stream>>>(d, a);
+  DARTKV_LAUNCH_OK("append_step_kernel");
+  return DARTKV_OK;
 }
 
 }  // namespace
 
-// bit 0: keys can take the fast kernel; bit 1: values can
+// bit 0: the keys of the step have the geometry of this file; bit 1: its values have
 int dartkv_append_fast_supported(const dartkv_cache_desc* d, const dartkv_append_plan* p, int64_t st) {
-  if (!fast_common(d, 0, 0, st)) return 0;
+  if ((d->dtype != DARTKV_F16 && d->dtype != DARTKV_BF16) || d->head_dim != kD || st % 8) return 0;
   int ok = 0;
   if (d->page_size == kP && d->key_group == kP && (p->num_pages == 0 || p->last_page_tokens == kP) &&
       (d->key_mode == DARTKV_QUANTIZED_PAGE || d->promoted <= kD))
@@ -510,77 +706,51 @@ int dartkv_append_fast_supported(const dartkv_cache_desc* d, const dartkv_append
   return ok;
 }
 
-#ifndef APPEND_KEY_SPLITS
-#define APPEND_KEY_SPLITS 4
-#endif
-
-template <int DT, int TQ>
-static int launch_keys_split(const dartkv_cache_desc& d, const dartkv_append_plan& p, const RowSource& src,
-                             const int32_t* indices, int32_t* nonfinite, cudaStream_t stream,
-                             const dartkv_append_plan* device_plan) {
-  dim3 grid(d.batch * d.kv_heads, p.num_pages);
-  if (d.key_mode == DARTKV_MIXED_PAGE)
-    fast_key_pages_kernel<DT, 0, TQ><<<grid, 64 * TQ, 0, stream>>>(d, src, p.first_page, p.num_pages, p.page_token_start, indices, nonfinite, device_plan);
-  else if (d.key_bits == 2)
-    fast_key_pages_kernel<DT, 2, TQ><<<grid, 64 * TQ, 0, stream>>>(d, src, p.first_page, p.num_pages, p.page_token_start, indices, nonfinite, device_plan);
-  else if (d.key_bits == 4)
-    fast_key_pages_kernel<DT, 4, TQ><<<grid, 64 * TQ, 0, stream>>>(d, src, p.first_page, p.num_pages, p.page_token_start, indices, nonfinite, device_plan);
-  else
-    fast_key_pages_kernel<DT, 8, TQ><<<grid, 64 * TQ, 0, stream>>>(d, src, p.first_page, p.num_pages, p.page_token_start, indices, nonfinite, device_plan);
-  DARTKV_LAUNCH_OK("fast_key_pages_kernel");
-  return DARTKV_OK;
-}
-
-template <int DT>
-static int launch_keys(const dartkv_cache_desc& d, const dartkv_append_plan& p, const RowSource& src,
-                       const int32_t* indices, int32_t* nonfinite, cudaStream_t stream,
-                       const dartkv_append_plan* device_plan) {
-#ifdef APPEND_KEY_SPLITS_FIXED
-  return launch_keys_split<DT, APPEND_KEY_SPLITS>(d, p, src, indices, nonfinite, stream, device_plan);
-#else
-  // Four token splits per page give a step of few pages more warps and a shorter critical path; with thousands of
-  // pages in flight the splits' extra combine work costs more than it hides: two splits (measured on bulk appends
-  // of bf16 [16,8,4096,128]: 123 us against 132 us; a 128-token step replayed from a graph: 10.1 against 9.9 us).
-  if ((long long)d.batch * d.kv_heads * p.num_pages >= 2048)
-    return launch_keys_split<DT, 2>(d, p, src, indices, nonfinite, stream, device_plan);
-  return launch_keys_split<DT, APPEND_KEY_SPLITS>(d, p, src, indices, nonfinite, stream, device_plan);
-#endif
-}
-
-template <int DT>
-static int launch_values(const dartkv_cache_desc& d, const dartkv_append_plan& p, const RowSource& src,
-                         int32_t* nonfinite, cudaStream_t stream, const dartkv_append_plan* device_plan) {
-  const int count = p.value_end - p.value_begin;
-  DARTKV_REQUIRE(d.batch * d.kv_heads <= 65535, "batch * kv_heads above 65535");
-  const dim3 blocks((unsigned)((count + 63) / 64), d.batch * d.kv_heads);   // 8 warps per block, 8 rows per warp
-  const int lpg = d.value_group / 16;
-  if (d.value_bits == 2)
-    fast_value_rows_kernel<DT, 2><<<blocks, 256, 0, stream>>>(d, src, p.value_begin, count, lpg, nonfinite, device_plan);
-  else if (d.value_bits == 4)
-    fast_value_rows_kernel<DT, 4><<<blocks, 256, 0, stream>>>(d, src, p.value_begin, count, lpg, nonfinite, device_plan);
-  else
-    fast_value_rows_kernel<DT, 8><<<blocks, 256, 0, stream>>>(d, src, p.value_begin, count, lpg, nonfinite, device_plan);
-  DARTKV_LAUNCH_OK("fast_value_rows_kernel");
-  return DARTKV_OK;
-}
-
 // device_plan (optional): the step's plan in device memory, written by a kernel earlier on the stream; *p then
-// only sizes the grids (the most pages / rows the step can bring)
+// only sizes the grid (the most pages / rows the step can bring)
+static StepArgs step_args(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, const void* values,
+                          int64_t sb, int64_t sh, int64_t st, const int32_t* indices, int32_t* nonfinite,
+                          const dartkv_append_plan* device_plan) {
+  StepArgs a{};
+  a.source = RowSource{nullptr, nullptr, sb, sh, st, p->chunk_start, d->ring_tokens};
+  a.keys = keys;
+  a.values = values;
+  a.plan = *p;
+  a.device_plan = device_plan;
+  a.indices = indices;
+  a.nonfinite = nonfinite;
+  return a;
+}
+
+// Whether one launch can do the whole step: the value rows are those of the key pages, and no page but the first
+// reads the ring (a local window longer than a page leaves more than a page waiting there).
+int dartkv_append_fast_whole_step(const dartkv_append_plan* p) {
+  const bool same_rows = p->num_pages == 0 ? p->value_end <= p->value_begin
+                                           : p->value_begin == p->page_token_start &&
+                                                 p->value_end == p->page_token_start + p->num_pages * kP;
+  return same_rows && (p->num_pages <= 1 || p->page_token_start + kP >= p->chunk_start);
+}
+
+int dartkv_append_fast_step(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, const void* values,
+                            int64_t sb, int64_t sh, int64_t st, const int32_t* indices, int32_t* nonfinite,
+                            cudaStream_t stream, const dartkv_append_plan* device_plan) {
+  StepArgs a = step_args(d, p, keys, values, sb, sh, st, indices, nonfinite, device_plan);
+  a.copies = 1;
+  return launch_step(*d, a, max(1, p->num_pages), 2, stream);
+}
+
 int dartkv_append_fast_keys(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, int64_t sb,
                             int64_t sh, int64_t st, const int32_t* indices, int32_t* nonfinite, cudaStream_t stream,
                             const dartkv_append_plan* device_plan) {
   if (p->num_pages == 0) return DARTKV_OK;
-  DARTKV_REQUIRE(p->num_pages <= 65535, "too many pages in one append (limit 65535)");
-  RowSource src{keys, d->k_ring, sb, sh, st, p->chunk_start, d->ring_tokens, d->kv_heads};
-  return d->dtype == DARTKV_F16 ? launch_keys<DARTKV_F16>(*d, *p, src, indices, nonfinite, stream, device_plan)
-                                : launch_keys<DARTKV_BF16>(*d, *p, src, indices, nonfinite, stream, device_plan);
+  return launch_step(*d, step_args(d, p, keys, nullptr, sb, sh, st, indices, nonfinite, device_plan), p->num_pages, 1, stream);
 }
 
 int dartkv_append_fast_values(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* values, int64_t sb,
                               int64_t sh, int64_t st, int32_t* nonfinite, cudaStream_t stream,
                               const dartkv_append_plan* device_plan) {
   if (p->value_end <= p->value_begin) return DARTKV_OK;
-  RowSource src{values, d->v_ring, sb, sh, st, p->chunk_start, d->ring_tokens, d->kv_heads};
-  return d->dtype == DARTKV_F16 ? launch_values<DARTKV_F16>(*d, *p, src, nonfinite, stream, device_plan)
-                                : launch_values<DARTKV_BF16>(*d, *p, src, nonfinite, stream, device_plan);
+  StepArgs a = step_args(d, p, nullptr, values, sb, sh, st, nullptr, nonfinite, device_plan);
+  a.role_begin = 1;
+  return launch_step(*d, a, ceil_div(p->value_end - p->value_begin, kP), 1, stream);
 }

@@ -3,6 +3,7 @@
 // bookkeeping done by the host (dartkv_append_plan); everything that touches K/V data runs here.
 
 #include "common.cuh"
+#include "append_common.cuh"
 
 static inline int align16(int v) { return (v + 15) & ~15; }
 
@@ -57,33 +58,6 @@ struct TokenSource {
 };
 
 // ---------------------------------------------------------------------------- dense copies
-// ---------------------------------------------------------------------------- device-side metadata
-__device__ __forceinline__ void publish_append(const dartkv_cache_desc& d, const dartkv_append_plan& p) {
-  for (int pg = threadIdx.x; pg < p.num_pages; pg += blockDim.x) {
-    d.page_start[p.first_page + pg] = p.page_token_start + pg * d.page_size;
-    d.page_tokens[p.first_page + pg] = (pg == p.num_pages - 1) ? p.last_page_tokens : d.page_size;
-  }
-  if (threadIdx.x == 0) {
-    d.state[0] = p.seen_after;
-    d.state[1] = p.key_pages_after;
-    d.state[2] = p.k_packed_end_after;
-    d.state[3] = p.v_packed_end_after;
-    d.state[4] = min(p.seen_after, d.sink_tokens);
-  }
-}
-
-// true when a 16-byte piece of `dt` elements holds an Inf or NaN
-__device__ __forceinline__ bool piece_nonfinite(uint4 v, int dt) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  uint32_t flag = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if (dt == DARTKV_F32) flag |= ((w[i] & 0x7FFFFFFFu) + 0x00800000u) & 0x80000000u;
-    else flag |= ((w[i] & 0x7FFF7FFFu) + (dt == DARTKV_BF16 ? 0x00800080u : 0x04000400u)) & 0x80008000u;
-  }
-  return flag != 0;
-}
-
 constexpr int kCopyRows = 8;   // rows per block of the dense copy
 
 // grid (bh, blocks of kCopyRows copy rows, side): copies sink tokens into the sink rows and tail tokens into
@@ -97,45 +71,16 @@ __global__ void copy_dense_kernel(dartkv_cache_desc d, dartkv_append_plan p, con
                                   int32_t* nonfinite, const dartkv_append_plan* device_plan) {
   if (device_plan) {
     p = *device_plan;
-    const int chunk_end = p.chunk_start + p.chunk_tokens;
-    const bool copies = p.sink_copy > 0 || p.ring_begin < chunk_end || p.value_end < chunk_end;
-    ring_first = p.chunk_tokens;
-    rows = 0;
-    if (copies) {
-      ring_first = max(p.sink_copy, min(p.ring_begin, max(p.value_end, p.chunk_start)) - p.chunk_start);
-      rows = p.sink_copy + (p.chunk_tokens - ring_first);
-    }
+    const DenseRows r = dense_rows(p);
+    ring_first = r.ring_first;
+    rows = r.rows;
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) publish_append(d, p);
   const int bh = blockIdx.x, side = blockIdx.z;
   const int r_begin = blockIdx.y * kCopyRows, r_end = min(rows, r_begin + kCopyRows);
   if (r_begin >= r_end) return;
-  const int ring_begin = side == 0 ? p.ring_begin : p.value_end;  // values not packed by this step stay dense
-  const void* src = side == 0 ? keys : values;
-  const int b = bh / d.kv_heads, h = bh % d.kv_heads;
-  const int64_t src_base = (int64_t)b * sb + (int64_t)h * sh;
-  const int esize = dartkv_dtype_size(d.dtype);
-  const int pieces = vector_ok ? d.head_dim * esize / 16 : d.head_dim;   // units per row: 16-byte pieces or elements
-  bool bad = false;
-  for (int i = threadIdx.x; i < (r_end - r_begin) * pieces; i += blockDim.x) {
-    const int r = r_begin + i / pieces, c = i % pieces;
-    const int j = r < p.sink_copy ? r : ring_first + (r - p.sink_copy);
-    const int t = p.chunk_start + j;
-    const bool to_sink = j < p.sink_copy;
-    if (!to_sink && t < ring_begin) continue;
-    void* dst = to_sink ? (side == 0 ? d.k_sink : d.v_sink) : (side == 0 ? d.k_ring : d.v_ring);
-    const int64_t drow = to_sink ? ((int64_t)bh * d.sink_tokens + t) : ((int64_t)bh * d.ring_tokens + (t % d.ring_tokens));
-    const int64_t srow = src_base + (int64_t)j * st;
-    if (vector_ok) {
-      const uint4 v = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(src) + srow * esize)[c];
-      bad |= piece_nonfinite(v, d.dtype);
-      reinterpret_cast<uint4*>(reinterpret_cast<char*>(dst) + drow * d.head_dim * esize)[c] = v;
-    } else {
-      const float v = load_f(src, d.dtype, srow + c);
-      bad |= !isfinite(v);
-      store_f(dst, d.dtype, drow * d.head_dim + c, v);
-    }
-  }
+  const int64_t base = (int64_t)(bh / d.kv_heads) * sb + (int64_t)(bh % d.kv_heads) * sh;
+  const bool bad = copy_dense_rows(d, p, side == 0 ? keys : values, base, st, ring_first, r_begin, r_end, vector_ok, bh, side);
   if (bad && nonfinite) *nonfinite = 1;
 }
 
@@ -431,6 +376,10 @@ int dartkv_append_fast_keys(const dartkv_cache_desc* d, const dartkv_append_plan
 int dartkv_append_fast_values(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* values, int64_t sb,
                               int64_t sh, int64_t st, int32_t* nonfinite, cudaStream_t stream,
                               const dartkv_append_plan* device_plan = nullptr);
+int dartkv_append_fast_whole_step(const dartkv_append_plan* p);
+int dartkv_append_fast_step(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, const void* values,
+                            int64_t sb, int64_t sh, int64_t st, const int32_t* indices, int32_t* nonfinite,
+                            cudaStream_t stream, const dartkv_append_plan* device_plan = nullptr);
 
 static int validate_desc(const dartkv_cache_desc* d) {
   DARTKV_REQUIRE(d != nullptr, "null descriptor");
@@ -459,7 +408,6 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
                  "bad sink_copy");
   DARTKV_REQUIRE(p.num_pages == 0 || (p.last_page_tokens > 0 && p.last_page_tokens <= d.page_size), "bad last_page_tokens");
   const int bh = d.batch * d.kv_heads;
-  const int chunk_end = p.chunk_start + p.chunk_tokens;
   const size_t page_smem = (size_t)d.head_dim * (sizeof(float) + sizeof(int));
 
   const int32_t* new_page_indices = indices;
@@ -475,9 +423,10 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
     if (indices) new_page_indices = indices + (int64_t)bh * d.promoted;
   }
 
-  const bool copies = p.sink_copy > 0 || p.ring_begin < chunk_end || p.value_end < chunk_end;
   int fast = dartkv_append_fast_supported(desc, plan, stride_t);
   if (stride_b % 8 || stride_h % 8 || ((uintptr_t)keys | (uintptr_t)values) % 16) fast = 0;
+  if (fast == 3 && dartkv_append_fast_whole_step(plan))
+    return dartkv_append_fast_step(desc, plan, keys, values, stride_b, stride_h, stride_t, new_page_indices, nonfinite, stream);
   if (p.num_pages > 0) {
     if (fast & 1) {
       rc = dartkv_append_fast_keys(desc, plan, keys, stride_b, stride_h, stride_t, new_page_indices, nonfinite, stream);
@@ -507,11 +456,7 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
   }
   {
     // dense copies of the step (possibly none) and the step's metadata, one launch
-    int ring_first = p.chunk_tokens, rows = 0;
-    if (copies) {
-      ring_first = max(p.sink_copy, min(p.ring_begin, max(p.value_end, p.chunk_start)) - p.chunk_start);
-      rows = p.sink_copy + (p.chunk_tokens - ring_first);
-    }
+    const auto [ring_first, rows] = dense_rows(p);
     const int row_blocks = max(1, ceil_div(rows, kCopyRows));
     DARTKV_REQUIRE(row_blocks <= 65535, "append chunks this long must be split by the caller");
     const int esize = dartkv_dtype_size(d.dtype);
@@ -695,6 +640,9 @@ extern "C" int dartkv_cache_append_device_planned(const dartkv_cache_desc* desc,
   const dartkv_append_plan* device_plan = reinterpret_cast<const dartkv_append_plan*>(d.state + 8);
   plan_append_kernel<<<1, 1, 0, stream>>>(d, *cfg, chunk_tokens);
   DARTKV_LAUNCH_OK("plan_append_kernel");
+  // lifecycles whose value rows are those of the key pages, at most one page waiting in the ring: one launch
+  if (cfg->value_local_tokens == 0 && (cfg->local_tokens == 0 || chunk_tokens == 1))
+    return dartkv_append_fast_step(desc, &most, keys, values, stride_b, stride_h, stride_t, nullptr, nonfinite, stream, device_plan);
   rc = dartkv_append_fast_keys(desc, &most, keys, stride_b, stride_h, stride_t, nullptr, nonfinite, stream, device_plan);
   if (rc) return rc;
   rc = dartkv_append_fast_values(desc, &most, values, stride_b, stride_h, stride_t, nonfinite, stream, device_plan);
