@@ -27,8 +27,8 @@ CODE_DTYPE = {v: k for k, v in DTYPE_CODE.items()}
 #: every symbol ``include/dartkv_b200.h`` declares
 EXPORTS = (
     "dartkv_last_error", "dartkv_version", "dartkv_launch_count", "dartkv_pack", "dartkv_unpack", "dartkv_quantize", "dartkv_dequantize",
-    "dartkv_channel_scores", "dartkv_select_channels", "dartkv_quantize_key_mixed", "dartkv_dequantize_key_mixed",
-    "dartkv_cache_geometry", "dartkv_cache_append", "dartkv_cache_materialize", "dartkv_decode_workspace_bytes",
+    "dartkv_channel_scores", "dartkv_select_channels", "dartkv_promote_channels", "dartkv_quantize_key_mixed", "dartkv_dequantize_key_mixed",
+    "dartkv_cache_geometry", "dartkv_cache_append", "dartkv_cache_materialize", "dartkv_cache_materialize_both", "dartkv_decode_workspace_bytes",
     "dartkv_decode_attention", "dartkv_decode_plan", "dartkv_decode_status", "dartkv_builtin_scratch_bytes",
     "dartkv_decode_attention_builtin_scratch", "dartkv_shard_range", "dartkv_decode_split_override",
     "dartkv_lifecycle_plan", "dartkv_cache_append_step", "dartkv_decode_attention_scatter",
@@ -128,11 +128,13 @@ def _load() -> ctypes.CDLL:
     lib.dartkv_dequantize.argtypes = [p, p, p, i32, i64, i64, i64, i32, i32, i32, p, i32, i64, i64, i64, p]
     lib.dartkv_channel_scores.argtypes = [p, i32, i64, i64, i64, i64, i64, i32, p, p]
     lib.dartkv_select_channels.argtypes = [p, i32, i64, i64, i32, p, p]
+    lib.dartkv_promote_channels.argtypes = [p, i32, i64, i64, i64, i64, i64, i32, p, p, p]
     lib.dartkv_quantize_key_mixed.argtypes = [p, i32, i64, i64, i64, i64, i64, i32, p, i32, i32, p, p, p, p, p, p]
     lib.dartkv_dequantize_key_mixed.argtypes = [p, p, p, p, p, i32, i64, i64, i64, i32, i32, i32, p, i32, p]
     lib.dartkv_cache_geometry.argtypes = [POINTER(CacheDesc)]
     lib.dartkv_cache_append.argtypes = [POINTER(CacheDesc), POINTER(AppendPlan), p, p, i64, i64, i64, p, p, p]
     lib.dartkv_cache_materialize.argtypes = [POINTER(CacheDesc), i32, c_int32, c_int32, i32, p, i32, p]
+    lib.dartkv_cache_materialize_both.argtypes = [POINTER(CacheDesc), c_int32, c_int32, i32, p, p, i32, p]
     lib.dartkv_decode_workspace_bytes.argtypes = [POINTER(CacheDesc), i32, i32]
     lib.dartkv_decode_workspace_bytes.restype = c_int64
     lib.dartkv_decode_attention.argtypes = [POINTER(CacheDesc), p, i32, i32, c_float, i32, i32, p, i64, p, p]

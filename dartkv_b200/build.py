@@ -18,7 +18,7 @@ CSRC = os.path.join(PACKAGE_DIR, "csrc")
 LIB_PATH = os.path.join(PACKAGE_DIR, "libdartkv_b200.so")
 HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
 HOST_PATH = os.path.join(PACKAGE_DIR, "_dartkv_host.so")
-SOURCES = ("quantize.cu", "cache_append.cu", "append_fast.cu", "decode_attention.cu", "decode_fast.cu", "decode_fused32.cu",
+SOURCES = ("quantize.cu", "quantize_fast.cu", "cache_append.cu", "append_fast.cu", "materialize.cu", "decode_attention.cu", "decode_fast.cu", "decode_fused32.cu",
            "decode_wide.cu")
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -70,7 +70,7 @@ def _finish_host_build(proc) -> None:
     libraries = [f"-L{path}" for path in cpp_extension.library_paths("cuda")]
     subprocess.run(["g++", "-shared", "-o", HOST_PATH, os.path.join(PACKAGE_DIR, "build", "host_path.o"), f"-L{PACKAGE_DIR}",
                     "-ldartkv_b200", "-Wl,-rpath,$ORIGIN", *libraries, "-ltorch_python", "-ltorch", "-ltorch_cpu",
-                    "-lc10", "-lc10_cuda"], check=True)
+                    "-lc10", "-lc10_cuda", "-lcudart"], check=True)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -52,7 +52,9 @@ class DartPageMetadata:
     value: DartSegmentLayout
 
 
-_PLAN_FIELDS = tuple(name for name, _ in AppendPlan._fields_ if name != "reserved")
+#: the pools of a cache, in the order the native allocation returns them
+_POOL_NAMES = ("k_sink", "v_sink", "k_ring", "v_ring", "state", "nonfinite", "k_pages", "page_start", "page_tokens",
+               "v_codes", "v_meta")
 
 
 @dataclass(frozen=True)
@@ -225,17 +227,24 @@ class DartKVCache:
         d.max_value_tokens = 1
         check(LIB.dartkv_cache_geometry(ctypes.byref(d)))
         self._desc = d
+        hint = self._max_tokens_hint or max(2 * first_chunk, first_chunk + 1024)
+        pages, rows = -(-hint // cfg.page_size) + 1, -(-hint // 128) * 128
+        pools = _lib.HOST.allocate(ctypes.addressof(d), device.index if device.index is not None else -1, pages, rows)
+        if pools is not None:
+            self._pools = dict(zip(_POOL_NAMES, pools))
+            self._bind_native()
+            return
         with device_guard(device):
+            words = torch.zeros(64, dtype=torch.int32, device=device)
             self._pools = {
                 "k_sink": torch.empty((batch, heads, max(1, cfg.sink_tokens), head_dim), dtype=dtype, device=device),
                 "v_sink": torch.empty((batch, heads, max(1, cfg.sink_tokens), head_dim), dtype=dtype, device=device),
                 "k_ring": torch.empty((batch, heads, d.ring_tokens, head_dim), dtype=dtype, device=device),
                 "v_ring": torch.empty((batch, heads, d.ring_tokens, head_dim), dtype=dtype, device=device),
-                "state": torch.zeros(32, dtype=torch.int32, device=device),   # 8 state words, then plan scratch
-                "nonfinite": torch.zeros(1, dtype=torch.int32, device=device),
+                "state": words[:32],   # 8 state words, then plan scratch
+                "nonfinite": words[32:33],
             }
-        hint = self._max_tokens_hint or max(2 * first_chunk, first_chunk + 1024)
-        self._ensure_capacity(-(-hint // cfg.page_size) + 1, hint)
+        self._ensure_capacity(pages, rows)
 
     def _ensure_capacity(self, need_pages: int, need_rows: int) -> None:
         """(Re)allocate the key page slots / packed value rows so that they hold at least the given counts."""
@@ -288,13 +297,8 @@ class DartKVCache:
         with a recorded reference run.
         """
 
-        if self._append_args is not None and channel_indices is None:
-            rc = _lib.HOST.append(key_states, value_states, *self._append_args)
-            if rc == 0:
-                self._note_step()
-                return
-            if rc != _lib.HOST.SLOW_PATH and rc != _lib.ELIMIT:
-                check(rc)
+        if self._append_args is not None and channel_indices is None and self._append_native(key_states, value_states):
+            return
         self._validate_inputs(key_states, value_states)
         device = require_cuda(key_states, value_states)
         keys = key_states.detach()
@@ -308,6 +312,8 @@ class DartKVCache:
         if self._desc is None:
             self._device = device
             self._allocate(batch, heads, head_dim, keys.dtype, device, chunk)
+            if self._append_args is not None and channel_indices is None and self._append_native(keys, values):
+                return
         # the kernels index chunk tokens with 16 bits: longer chunks are appended in pieces, which the lifecycle
         # treats exactly like one append of the whole chunk (pages are cut at the same absolute positions) as long
         # as the first piece carries the whole sink prefix
@@ -364,6 +370,17 @@ class DartKVCache:
                     keys.stride(2), ptr(idx), ptr(self._pools["nonfinite"]), stream_ptr(device)))
             self._set_c_state(state)
         self._note_step()
+
+    def _append_native(self, key_states: torch.Tensor, value_states: torch.Tensor) -> bool:
+        """The step through the native host path; ``False`` when it is not an ordinary one (nothing launched then)."""
+
+        rc = _lib.HOST.append(key_states, value_states, *self._append_args)
+        if rc == 0:
+            self._note_step()
+            return True
+        if rc != _lib.HOST.SLOW_PATH and rc != _lib.ELIMIT:
+            check(rc)
+        return False
 
     def _note_step(self) -> None:
         """The step in ``self._plan`` was accepted: bring the host-side segment bookkeeping up to date."""
@@ -488,20 +505,21 @@ class DartKVCache:
         b, h, d = self._shape
         out = torch.empty((b, h, stop - start, d), dtype=self._dtype, device=self._device)
         with device_guard(self._device):
-            for lo in range(start, stop, 32768):
-                hi = min(stop, lo + 32768)
-                piece = out if (lo == start and hi == stop) else torch.empty(
-                    (b, h, hi - lo, d), dtype=self._dtype, device=self._device)
-                check(LIB.dartkv_cache_materialize(ctypes.byref(self._desc), side, lo, hi, flavour, ptr(piece),
-                                                   _lib.DTYPE_CODE[self._dtype], stream_ptr(self._device)))
-                if piece is not out:
-                    out[:, :, lo - start: hi - start].copy_(piece)
+            check(LIB.dartkv_cache_materialize(ctypes.byref(self._desc), side, start, stop, flavour, ptr(out),
+                                               _lib.DTYPE_CODE[self._dtype], stream_ptr(self._device)))
         return out
 
     def get(self) -> Tuple[torch.Tensor, torch.Tensor]:
         if self._life.seen == 0:
             raise RuntimeError("DartKVCache is empty; call update() before get()")
-        return self._materialize(0, 0, self._life.seen), self._materialize(1, 0, self._life.seen)
+        b, h, d = self._shape
+        keys = torch.empty((b, h, self._life.seen, d), dtype=self._dtype, device=self._device)
+        values = torch.empty_like(keys)
+        with device_guard(self._device):
+            check(LIB.dartkv_cache_materialize_both(ctypes.byref(self._desc), 0, self._life.seen, _lib.DEQUANT_PER_OP,
+                                                    ptr(keys), ptr(values), _lib.DTYPE_CODE[self._dtype],
+                                                    stream_ptr(self._device)))
+        return keys, values
 
     @property
     def key_states(self) -> torch.Tensor:

@@ -78,3 +78,12 @@ __device__ __forceinline__ bool copy_dense_rows(const dartkv_cache_desc& d, cons
   }
   return bad;
 }
+
+static inline int validate_desc(const dartkv_cache_desc* d) {
+  DARTKV_REQUIRE(d != nullptr, "null descriptor");
+  DARTKV_REQUIRE(d->key_page_bytes > 0 && d->value_row_bytes > 0, "descriptor geometry not filled (call dartkv_cache_geometry)");
+  DARTKV_REQUIRE(d->k_ring && d->v_ring && d->k_pages && d->v_codes && d->v_meta && d->page_start && d->page_tokens && d->state,
+                 "descriptor has a null pool pointer");
+  DARTKV_REQUIRE(d->sink_tokens == 0 || (d->k_sink && d->v_sink), "descriptor has a null sink pointer");
+  return DARTKV_OK;
+}

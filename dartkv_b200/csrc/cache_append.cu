@@ -276,73 +276,6 @@ __device__ __forceinline__ float page_key_element(const dartkv_cache_desc& d, co
   return affine_restore((float)code, s, z, d.md_dtype, d.dtype, flavour);
 }
 
-__device__ __forceinline__ float packed_value_element(const dartkv_cache_desc& d, int bh, int t, int c, int flavour) {
-  int64_t row = (int64_t)bh * d.max_value_tokens + (t - d.sink_tokens);
-  const int bits = d.value_bits, vpb = 8 / bits, g = c / d.value_group;
-  uint32_t code = (d.v_codes[row * d.value_row_bytes + c / vpb] >> ((c % vpb) * bits)) & ((1u << bits) - 1u);
-  float s = load_f(d.v_meta, d.md_dtype, (row * 2 + 0) * d.value_groups + g);
-  float z = load_f(d.v_meta, d.md_dtype, (row * 2 + 1) * d.value_groups + g);
-  return affine_restore((float)code, s, z, d.md_dtype, d.dtype, flavour);
-}
-
-// first page whose range ends after token t (pages are contiguous from sink_tokens)
-__device__ __forceinline__ int find_page(const dartkv_cache_desc& d, int pages, int t) {
-  int lo = 0, hi = pages - 1;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (d.page_start[mid] + d.page_tokens[mid] > t) hi = mid; else lo = mid + 1;
-  }
-  return lo;
-}
-
-// grid (bh, token); out [B*H, t1-t0, D]
-__global__ void materialize_kernel(dartkv_cache_desc d, int side, int t0, int t1, int flavour, void* out, int out_dt) {
-  extern __shared__ int s_slot[];
-  __shared__ int s_page;
-  const int bh = blockIdx.x, t = t0 + blockIdx.y, D = d.head_dim;
-  const int sink_filled = d.state[4];
-  const int packed_end = side == 0 ? d.state[2] : d.state[3];
-  int64_t orow = ((int64_t)bh * (t1 - t0) + (t - t0)) * D;
-  if (t < sink_filled || t >= packed_end) {
-    const void* src;
-    int64_t row;
-    if (t < sink_filled) {
-      src = side == 0 ? d.k_sink : d.v_sink;
-      row = (int64_t)bh * d.sink_tokens + t;
-    } else {
-      src = side == 0 ? d.k_ring : d.v_ring;
-      row = (int64_t)bh * d.ring_tokens + (t % d.ring_tokens);
-    }
-    for (int c = threadIdx.x; c < D; c += blockDim.x)
-      store_f(out, out_dt, orow + c, rnd_rt(load_f(src, d.dtype, row * D + c), out_dt));
-    return;
-  }
-  if (side == 1) {
-    for (int c = threadIdx.x; c < D; c += blockDim.x)
-      store_f(out, out_dt, orow + c, rnd_rt(packed_value_element(d, bh, t, c, flavour), out_dt));
-    return;
-  }
-  if (threadIdx.x == 0) s_page = find_page(d, d.state[1], t);
-  __syncthreads();
-  const int pg = s_page;
-  const uint8_t* page = d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes;
-  if (d.key_mode == DARTKV_MIXED_PAGE) {
-    const int32_t* idx = reinterpret_cast<const int32_t*>(page + d.key_off_index);
-    for (int c = threadIdx.x; c < D; c += blockDim.x) s_slot[c] = -1;
-    __syncthreads();
-    for (int k = threadIdx.x; k < d.promoted; k += blockDim.x) {
-      int c = idx[k];
-      if (c >= 0 && c < D) s_slot[c] = k;
-    }
-    __syncthreads();
-  }
-  const int n = d.page_tokens[pg], j = t - d.page_start[pg];
-  for (int c = threadIdx.x; c < D; c += blockDim.x) {
-    int slot = d.key_mode == DARTKV_MIXED_PAGE ? s_slot[c] : -1;
-    store_f(out, out_dt, orow + c, rnd_rt(page_key_element(d, page, n, j, c, slot, flavour), out_dt));
-  }
-}
-
 // dequantize one key page back into the ring rows of its tokens (first half of the boundary
 // re-quantization of src/dart/cache.py:427-439); grid (bh, token of the page)
 __global__ void page_to_ring_kernel(dartkv_cache_desc d, int slot_index, int page_token_start, int n) {
@@ -380,15 +313,6 @@ int dartkv_append_fast_whole_step(const dartkv_append_plan* p);
 int dartkv_append_fast_step(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, const void* values,
                             int64_t sb, int64_t sh, int64_t st, const int32_t* indices, int32_t* nonfinite,
                             cudaStream_t stream, const dartkv_append_plan* device_plan = nullptr);
-
-static int validate_desc(const dartkv_cache_desc* d) {
-  DARTKV_REQUIRE(d != nullptr, "null descriptor");
-  DARTKV_REQUIRE(d->key_page_bytes > 0 && d->value_row_bytes > 0, "descriptor geometry not filled (call dartkv_cache_geometry)");
-  DARTKV_REQUIRE(d->k_ring && d->v_ring && d->k_pages && d->v_codes && d->v_meta && d->page_start && d->page_tokens && d->state,
-                 "descriptor has a null pool pointer");
-  DARTKV_REQUIRE(d->sink_tokens == 0 || (d->k_sink && d->v_sink), "descriptor has a null sink pointer");
-  return DARTKV_OK;
-}
 
 extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_append_plan* plan, const void* keys,
                                    const void* values, int64_t stride_b, int64_t stride_h, int64_t stride_t,
@@ -468,24 +392,6 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
   }
   return DARTKV_OK;
 }
-
-extern "C" int dartkv_cache_materialize(const dartkv_cache_desc* desc, int side, int32_t t0, int32_t t1, int flavour,
-                                        void* out, int out_dtype, void* stream) {
-  int rc = validate_desc(desc);
-  if (rc) return rc;
-  DARTKV_REQUIRE(side == 0 || side == 1, "side must be 0 (keys) or 1 (values)");
-  DARTKV_REQUIRE(t0 >= 0 && t1 >= t0, "bad token range");
-  DARTKV_REQUIRE(dartkv_valid_dtype(out_dtype), "unsupported output dtype");
-  DARTKV_REQUIRE(flavour == DARTKV_DEQUANT_PER_OP || flavour == DARTKV_DEQUANT_FP32, "unknown dequant flavour %d", flavour);
-  if (t1 == t0) return DARTKV_OK;
-  DARTKV_REQUIRE(out != nullptr, "materialize received a null output");
-  DARTKV_REQUIRE(t1 - t0 <= 65535, "materialize at most 65535 tokens per call");
-  const int bh = desc->batch * desc->kv_heads;
-  materialize_kernel<<<dim3(bh, t1 - t0), 128, desc->head_dim * sizeof(int), (cudaStream_t)stream>>>(*desc, side, t0, t1, flavour, out, out_dtype);
-  DARTKV_LAUNCH_OK("materialize_kernel");
-  return DARTKV_OK;
-}
-
 
 // ---------------------------------------------------------------------------- host-side lifecycle planner
 // The integer bookkeeping of the reference's cache lifecycle (src/dart/cache.py:168-190, 403-470) as a host

@@ -1,8 +1,8 @@
 // Per-call host path of the cache as a CPython extension: append and decode calls go from the Python tensor objects
 // straight into the C ABI.  One generation step makes two such calls per layer, each of a few microseconds of GPU
 // work, so what the host does per call decides the step time of small batches; reading a tensor's fields from
-// Python and converting ctypes arguments cost 15-25 us per call, this file about one (B200 host, 128-token appends:
-// 26 -> 15 us per call, the three kernel launches included).
+// Python and converting ctypes arguments cost 15-25 us per call, a call here 3 us for an append (one launch) and 7 us
+// for a decode (two launches and the output tensor).
 //
 // Every function answers "not for me" (kSlowPath / None) for anything out of the ordinary -- other devices, odd
 // strides, wrong shapes, pools that have to grow -- before it launches anything; the Python code then takes its
@@ -13,6 +13,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/dartkv_b200.h"
@@ -115,7 +116,180 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return THPVariable_Wrap(std::move(out));
 }
 
+at::ScalarType scalar_type(int code) {
+  return code == DARTKV_F32 ? at::kFloat : code == DARTKV_F16 ? at::kHalf : at::kBFloat16;
+}
+
+// allocate(desc, device_index, key_pages, value_rows): the pools of a new cache, in the order of `kPoolNames` on the
+// Python side, with the descriptor's pointers set; None when the device is not the current one.  Only the state words
+// and the finite-input flag start at zero (one fill for both); everything else is written before it is read.
+PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 4) { PyErr_SetString(PyExc_TypeError, "allocate takes 4 arguments"); return nullptr; }
+  auto* d = static_cast<dartkv_cache_desc*>(PyLong_AsVoidPtr(args[0]));
+  const long device = PyLong_AsLong(args[1]), pages = PyLong_AsLong(args[2]), rows = PyLong_AsLong(args[3]);
+  if (PyErr_Occurred()) return nullptr;
+  if (device != c10::cuda::current_device()) Py_RETURN_NONE;
+  try {
+    const int64_t b = d->batch, h = d->kv_heads, hd = d->head_dim, sinks = d->sink_tokens > 0 ? d->sink_tokens : 1;
+    const auto options = at::TensorOptions().device(at::Device(at::kCUDA, (c10::DeviceIndex)device));
+    const auto dense = options.dtype(scalar_type(d->dtype));
+    at::Tensor words = at::zeros({64}, options.dtype(at::kInt)), table = at::empty({2, pages}, options.dtype(at::kInt));
+    at::Tensor pools[] = {
+        at::empty({b, h, sinks, hd}, dense), at::empty({b, h, sinks, hd}, dense),
+        at::empty({b, h, d->ring_tokens, hd}, dense), at::empty({b, h, d->ring_tokens, hd}, dense),
+        words.narrow(0, 0, 32), words.narrow(0, 32, 1),
+        at::empty({b, h, pages, d->key_page_bytes}, options.dtype(at::kByte)), table.select(0, 0), table.select(0, 1),
+        at::empty({b, h, rows, d->value_row_bytes}, options.dtype(at::kByte)),
+        at::empty({b, h, rows, 2, d->value_groups}, options.dtype(scalar_type(d->md_dtype)))};
+    d->k_sink = pools[0].data_ptr(); d->v_sink = pools[1].data_ptr();
+    d->k_ring = pools[2].data_ptr(); d->v_ring = pools[3].data_ptr();
+    d->state = (int32_t*)pools[4].data_ptr();
+    d->k_pages = (uint8_t*)pools[6].data_ptr();
+    d->page_start = (int32_t*)pools[7].data_ptr(); d->page_tokens = (int32_t*)pools[8].data_ptr();
+    d->v_codes = (uint8_t*)pools[9].data_ptr(); d->v_meta = pools[10].data_ptr();
+    d->max_key_pages = (int32_t)pages; d->max_value_tokens = (int32_t)rows;
+    constexpr int kPools = sizeof(pools) / sizeof(pools[0]);
+    PyObject* out = PyTuple_New(kPools);
+    if (!out) return nullptr;
+    for (int i = 0; i < kPools; ++i) PyTuple_SET_ITEM(out, i, THPVariable_Wrap(pools[i]));
+    return out;
+  } catch (const c10::OutOfMemoryError&) {
+    Py_RETURN_NONE;   // the Python path allocates the same pools and raises torch's own error
+  }
+}
+
+// Finite-input flag of a synchronous call: one pinned word per thread that the kernels write through its device
+// mapping.  Such a call ends with a wait for its own stream anyway; the word saves the fill kernel before it and the
+// copy after it.
+struct HostFlag {
+  int32_t* word = nullptr;
+  HostFlag() {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) word = static_cast<int32_t*>(p);
+  }
+  ~HostFlag() {
+    if (word) cudaFreeHost(word);
+  }
+};
+int32_t* host_flag() {
+  thread_local HostFlag flag;
+  if (flag.word) *reinterpret_cast<volatile int32_t*>(flag.word) = 0;
+  return flag.word;
+}
+
+// What a call with a finite-input check returns: the tuple, a return code, or False where the input was not finite.
+PyObject* finish(PyObject* tuple, int rc, const int32_t* flag, void* stream) {
+  if (rc == 0 && flag) {
+    cudaError_t err;
+    Py_BEGIN_ALLOW_THREADS
+    err = cudaStreamSynchronize((cudaStream_t)stream);
+    Py_END_ALLOW_THREADS
+    if (err != cudaSuccess) {
+      Py_DECREF(tuple);
+      PyErr_Format(PyExc_RuntimeError, "CUDA error while waiting for the finite-input check: %s", cudaGetErrorString(err));
+      return nullptr;
+    }
+    if (*reinterpret_cast<const volatile int32_t*>(flag)) {
+      Py_DECREF(tuple);
+      Py_RETURN_FALSE;
+    }
+  }
+  if (rc != 0) {
+    Py_DECREF(tuple);
+    return PyLong_FromLong(rc);
+  }
+  return tuple;
+}
+
+PyObject* tensors(std::initializer_list<at::Tensor> list) {
+  PyObject* out = PyTuple_New((Py_ssize_t)list.size());
+  Py_ssize_t i = 0;
+  for (const at::Tensor& t : list) PyTuple_SET_ITEM(out, i++, THPVariable_Wrap(t));
+  return out;
+}
+
+bool dense_here(const at::Tensor& t) { return t.is_contiguous() && on_current_device(t); }
+
+// quantize(data, bits, group, axis, metadata dtype code, division, check) -> (values, scale, zero); data contiguous
+PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 7) { PyErr_SetString(PyExc_TypeError, "quantize takes 7 arguments"); return nullptr; }
+  if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const int bits = (int)PyLong_AsLong(args[1]);
+  const int64_t group = PyLong_AsLongLong(args[2]);
+  const int64_t axis = PyLong_AsLongLong(args[3]);
+  const int md = (int)PyLong_AsLong(args[4]), division = (int)PyLong_AsLong(args[5]), wanted = (int)PyLong_AsLong(args[6]);
+  if (PyErr_Occurred()) return nullptr;
+  const int code = dtype_code(x.scalar_type());
+  if (code < 0 || !dense_here(x) || x.numel() == 0 || group > INT32_MAX) Py_RETURN_NONE;
+  int64_t outer = 1, inner = 1;
+  at::SmallVector<int64_t, 6> shape;
+  for (int64_t i = 0; i < x.dim(); ++i) {
+    if (i < axis) outer *= x.size(i);
+    if (i > axis) inner *= x.size(i);
+    if (i != axis) shape.push_back(x.size(i));
+  }
+  const int64_t len = x.size(axis), groups = (len + group - 1) / group, vpb = 8 / bits;
+  shape.push_back((groups * group + vpb - 1) / vpb);
+  const auto options = x.options().requires_grad(false);
+  at::Tensor values = at::empty(shape, options.dtype(at::kByte));
+  shape.back() = groups;
+  at::Tensor scale = at::empty(shape, options.dtype(scalar_type(md))), zero = at::empty(shape, options.dtype(scalar_type(md)));
+  int32_t* flag = wanted ? host_flag() : nullptr;
+  if (wanted && !flag) Py_RETURN_NONE;
+  void* stream = stream_of(x);
+  const int rc = dartkv_quantize(x.data_ptr(), code, outer, len, inner, len * inner, inner, 1, bits, (int)group, md, division,
+                                 (uint8_t*)values.data_ptr(), scale.data_ptr(), zero.data_ptr(), flag, stream);
+  return finish(tensors({values, scale, zero}), rc, flag, stream);
+}
+
+// quantize_mixed(keys, group, promoted count, metadata dtype code, indices | None, check)
+//   -> (low, high, indices, scale, zero); keys [B,H,T,D] contiguous, indices int32 contiguous
+PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 6) { PyErr_SetString(PyExc_TypeError, "quantize_mixed takes 6 arguments"); return nullptr; }
+  if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
+  const at::Tensor& k = THPVariable_Unpack(args[0]);
+  const int64_t group = PyLong_AsLongLong(args[1]), count = PyLong_AsLongLong(args[2]);
+  const int md = (int)PyLong_AsLong(args[3]), wanted = (int)PyLong_AsLong(args[5]);
+  if (PyErr_Occurred()) return nullptr;
+  const int code = dtype_code(k.scalar_type());
+  if (code < 0 || !dense_here(k) || k.dim() != 4 || k.numel() == 0 || group > INT32_MAX) Py_RETURN_NONE;
+  const int64_t b = k.size(0), h = k.size(1), t = k.size(2), d = k.size(3), groups = (t + group - 1) / group, packed = (group + 3) / 4;
+  const auto options = k.options().requires_grad(false);
+  void* stream = stream_of(k);
+  at::Tensor index;
+  int rc = 0;
+  if (args[4] != Py_None) {
+    if (!THPVariable_Check(args[4])) Py_RETURN_NONE;
+    index = THPVariable_Unpack(args[4]);
+    if (index.scalar_type() != at::kInt || !dense_here(index)) Py_RETURN_NONE;
+  } else {
+    index = at::empty({b, h, count}, options.dtype(at::kInt));
+    at::Tensor scores;
+    // the one-launch selection takes 16-bit keys of an even number of channels up to 128 and needs no score buffer
+    if (code == DARTKV_F32 || d > 128 || d % 2 || (uintptr_t)k.data_ptr() % 4 || b * h > INT32_MAX)
+      scores = at::empty({b, h, d}, options);
+    rc = dartkv_promote_channels(k.data_ptr(), code, b * h, t, d, t * d, d, (int)count,
+                                 scores.defined() ? scores.data_ptr() : index.data_ptr(), (int32_t*)index.data_ptr(), stream);
+    if (rc) return PyLong_FromLong(rc);
+  }
+  const int64_t promoted = index.size(-1);
+  at::Tensor low = at::empty({b, h, d, groups, packed}, options.dtype(at::kByte));
+  at::Tensor high = at::empty({b, h, promoted, groups, packed}, options.dtype(at::kByte));
+  at::Tensor scale = at::empty({b, h, d, groups}, options.dtype(scalar_type(md)));
+  at::Tensor zero = at::empty({b, h, d, groups}, options.dtype(scalar_type(md)));
+  int32_t* flag = wanted ? host_flag() : nullptr;
+  if (wanted && !flag) Py_RETURN_NONE;
+  rc = dartkv_quantize_key_mixed(k.data_ptr(), code, b * h, t, d, t * d, d, (int)group,
+                                 promoted ? (const int32_t*)index.data_ptr() : nullptr, (int)promoted, md, (uint8_t*)low.data_ptr(),
+                                 promoted ? (uint8_t*)high.data_ptr() : nullptr, scale.data_ptr(), zero.data_ptr(), flag, stream);
+  return finish(tensors({low, high, index, scale, zero}), rc, flag, stream);
+}
+
 PyMethodDef methods[] = {
+    {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "group-wise quantizer"},
+    {"quantize_mixed", (PyCFunction)(void (*)(void))quantize_mixed, METH_FASTCALL, "mixed key quantizer"},
+    {"allocate", (PyCFunction)(void (*)(void))allocate, METH_FASTCALL, "the pools of a new cache"},
     {"append", (PyCFunction)(void (*)(void))append, METH_FASTCALL, "one append step of a cache"},
     {"decode", (PyCFunction)(void (*)(void))decode, METH_FASTCALL, "one decode attention call on a cache"},
     {nullptr, nullptr, 0, nullptr}};

@@ -108,6 +108,22 @@ extern "C" int dartkv_unpack(const uint8_t* packed, int64_t rows, int64_t packed
   return DARTKV_OK;
 }
 
+// ---------------------------------------------------------------------------- shapes with kernels of their own
+// quantize_fast.cu: 1 when the launch was made, 0 when the shape is not one of that file, negative on failure
+int dartkv_quantize_columns_fast(const void* x, int dtype, int64_t outer, int64_t n, int64_t inner, int64_t so, int64_t sn,
+                                 int key_bits, int group, int md, uint8_t* values, uint8_t* high, const int32_t* indices,
+                                 int promoted, void* scale, void* zero, int32_t* nonfinite, cudaStream_t stream);
+int dartkv_quantize_rows_fast(const void* x, int dtype, int64_t rows, int64_t n, int64_t so, int bits, int group, int md,
+                              uint8_t* values, void* scale, void* zero, int32_t* nonfinite, cudaStream_t stream);
+int dartkv_score_select_fast(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t d, int64_t sbh, int64_t st,
+                             int count, void* scores, int32_t* indices, cudaStream_t stream);
+int dartkv_restore_columns_fast(const uint8_t* values, const uint8_t* high, const int32_t* indices, int promoted,
+                                const void* scale, const void* zero, int md, int64_t outer, int64_t n, int64_t inner,
+                                int key_bits, int group, int flavour, void* out, int out_dtype, int64_t so, int64_t sn,
+                                cudaStream_t stream);
+int dartkv_restore_rows_fast(const uint8_t* values, const void* scale, const void* zero, int md, int64_t rows, int64_t n, int bits,
+                             int group, int flavour, void* out, int out_dtype, int64_t so, cudaStream_t stream);
+
 // ---------------------------------------------------------------------------- uniform quantizer
 // One thread per (row, unit).  A unit is lcm(group, values-per-byte) consecutive codes, so it
 // holds whole groups and whole bytes and no two threads share a byte.
@@ -181,6 +197,16 @@ extern "C" int dartkv_quantize(const void* x, int dtype, int64_t outer, int64_t 
   DARTKV_REQUIRE(div_mode == DARTKV_DIV_TRUE || div_mode == DARTKV_DIV_RECIPROCAL, "unknown div_mode %d", div_mode);
   if (outer == 0 || inner == 0) return DARTKV_OK;
   DARTKV_REQUIRE(x && values && scale && zero, "quantize received a null pointer");
+  if (div_mode == DARTKV_DIV_TRUE) {
+    int made = 0;
+    if (inner == 1 && stride_n == 1)
+      made = dartkv_quantize_rows_fast(x, dtype, outer, n, stride_outer, bits, group_size, md_dtype, values, scale, zero, nonfinite,
+                                       (cudaStream_t)stream);
+    else if (stride_inner == 1)
+      made = dartkv_quantize_columns_fast(x, dtype, outer, n, inner, stride_outer, stride_n, bits, group_size, md_dtype, values,
+                                          nullptr, nullptr, 0, scale, zero, nonfinite, (cudaStream_t)stream);
+    if (made) return made > 0 ? DARTKV_OK : made;
+  }
   QuantArgs a;
   a.x = x; a.dtype = dtype; a.outer = outer; a.n = n; a.inner = inner;
   a.so = stride_outer; a.sn = stride_n; a.si = stride_inner;
@@ -228,6 +254,14 @@ extern "C" int dartkv_dequantize(const uint8_t* values, const void* scale, const
   DARTKV_REQUIRE(n > 0 && outer >= 0 && inner >= 0, "bad extents");
   if (outer == 0 || inner == 0) return DARTKV_OK;
   DARTKV_REQUIRE(values && scale && zero && out, "dequantize received a null pointer");
+  int made = 0;
+  if (inner == 1 && stride_n == 1)
+    made = dartkv_restore_rows_fast(values, scale, zero, md_dtype, outer, n, bits, group_size, flavour, out, out_dtype, stride_outer,
+                                    (cudaStream_t)stream);
+  else if (stride_inner == 1)
+    made = dartkv_restore_columns_fast(values, nullptr, nullptr, 0, scale, zero, md_dtype, outer, n, inner, bits, group_size, flavour,
+                                       out, out_dtype, stride_outer, stride_n, (cudaStream_t)stream);
+  if (made) return made > 0 ? DARTKV_OK : made;
   int64_t groups = ceil_div64(n, group_size);
   int64_t packed_bytes = ceil_div64(groups * group_size, 8 / bits);
   dequantize_kernel<<<grid_for(outer * n * inner, 256), 256, 0, (cudaStream_t)stream>>>(
@@ -275,6 +309,11 @@ extern "C" int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, in
                  "strategy must be 'magnitude', 'random', or 'variance'");
   if (bh == 0) return DARTKV_OK;
   DARTKV_REQUIRE(keys && scores, "channel_scores received a null pointer");
+  if (strategy == DARTKV_SCORE_MAGNITUDE) {
+    const int made = dartkv_score_select_fast(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, 0, scores, nullptr,
+                                              (cudaStream_t)stream);
+    if (made) return made > 0 ? DARTKV_OK : made;
+  }
   channel_scores_kernel<<<grid_for(bh * head_dim, 128), 128, 0, (cudaStream_t)stream>>>(
       keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, strategy, scores);
   DARTKV_LAUNCH_OK("channel_scores_kernel");
@@ -310,6 +349,22 @@ extern "C" int dartkv_select_channels(const void* scores, int dtype, int64_t bh,
                                                                                              count, indices);
   DARTKV_LAUNCH_OK("select_channels_kernel");
   return DARTKV_OK;
+}
+
+// Scores and selection by magnitude in one launch where the shape allows it, else through `scores` in two.
+extern "C" int dartkv_promote_channels(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t head_dim,
+                                       int64_t stride_bh, int64_t stride_token, int count, void* scores, int32_t* indices,
+                                       void* stream) {
+  DARTKV_REQUIRE(dartkv_valid_dtype(dtype), "key_states must be floating point");
+  DARTKV_REQUIRE(tokens > 0 && head_dim > 0 && head_dim <= 8192, "bad key_states extents");
+  DARTKV_REQUIRE(count >= 0 && count <= head_dim, "count must be in [0, head_dim]");
+  if (bh == 0 || count == 0) return DARTKV_OK;
+  DARTKV_REQUIRE(keys && scores && indices, "promote_channels received a null pointer");
+  const int made = dartkv_score_select_fast(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, count, nullptr, indices,
+                                            (cudaStream_t)stream);
+  if (made) return made > 0 ? DARTKV_OK : made;
+  const int rc = dartkv_channel_scores(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, DARTKV_SCORE_MAGNITUDE, scores, stream);
+  return rc ? rc : dartkv_select_channels(scores, dtype, bh, head_dim, count, indices, stream);
 }
 
 // ---------------------------------------------------------------------------- mixed key quantizer
@@ -383,6 +438,9 @@ extern "C" int dartkv_quantize_key_mixed(const void* keys, int dtype, int64_t bh
   if (bh == 0) return DARTKV_OK;
   DARTKV_REQUIRE(keys && low && scale && zero && (promoted == 0 || (indices && high)),
                  "quantize_key_mixed received a null pointer");
+  const int made = dartkv_quantize_columns_fast(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, 0, group_size, md_dtype,
+                                                low, high, indices, promoted, scale, zero, nonfinite, (cudaStream_t)stream);
+  if (made) return made > 0 ? DARTKV_OK : made;
   int64_t groups = ceil_div64(tokens, group_size);
   dim3 grid((unsigned)bh, grid_for(head_dim * groups, 128));
   quantize_key_mixed_kernel<<<grid, 128, head_dim * sizeof(int), (cudaStream_t)stream>>>(
@@ -431,6 +489,9 @@ extern "C" int dartkv_dequantize_key_mixed(const uint8_t* low, const uint8_t* hi
   if (bh == 0) return DARTKV_OK;
   DARTKV_REQUIRE(low && scale && zero && out && (promoted == 0 || (indices && high)),
                  "dequantize_key_mixed received a null pointer");
+  const int made = dartkv_restore_columns_fast(low, high, indices, promoted, scale, zero, md_dtype, bh, tokens, head_dim, 0, group_size,
+                                               flavour, out, out_dtype, tokens * head_dim, head_dim, (cudaStream_t)stream);
+  if (made) return made > 0 ? DARTKV_OK : made;
   dim3 grid((unsigned)bh, grid_for(tokens * head_dim, 256));
   dequantize_key_mixed_kernel<<<grid, 256, head_dim * sizeof(int), (cudaStream_t)stream>>>(
       low, high, indices, scale, zero, md_dtype, tokens, head_dim, group_size, promoted, flavour, out, out_dtype);

@@ -1,0 +1,446 @@
+// Functional quantizers and dequantizers for 16-bit data whose groups fill whole 32-bit words: the shapes a model's
+// keys (groups along the tokens, channels contiguous) and values (groups along the channels) have.  Any other shape
+// keeps the kernels of quantize.cu, which handle one group (or element) per thread.
+//
+// All of these are bound by memory latency and by the few instructions per element, not by capacity: a group's tokens
+// are split over up to four threads per channel pair, loads run eight deep, codes gather in registers (quant_math.cuh)
+// and leave as whole words.  fp16 [8,8,1024,128], 2-bit + promoted keys / 2-bit values, before -> now:
+// keys 52 -> 7 us, values 68 -> 5 us, channel scores 77 -> 8 us, dequantize 80 -> 7 us each (B200).
+
+#include "common.cuh"
+#include "quant_math.cuh"
+
+namespace {
+
+constexpr int kSlab = 128;   // columns per block: 64 threads, two neighbouring columns each
+
+// ---------------------------------------------------------------------------- groups along a strided axis
+struct ColumnArgs {
+  const uint16_t* x;
+  int64_t so, sn;                      // element strides of the outer index and of the quantized axis
+  int n, inner, group, groups;
+  int64_t packed_bytes;                // per (outer, column) row, all groups
+  uint8_t *values, *high;              // mixed keys: low plane and promoted high plane
+  const int32_t* indices;              // mixed keys: [outer][promoted]
+  int promoted, md;
+  void *scale, *zero;
+  int32_t* nonfinite;
+};
+
+// grid (group, slab of columns, outer); 64 threads per token split.  KB: 0 = mixed 2+2-bit keys, else the code width.
+template <int DT, int KB>
+__global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_constant__ ColumnArgs a) {
+  using P = Pack16<DT>;
+  constexpr int PB = KB == 0 ? 2 : KB, CODE_BITS = KB == 0 ? 4 : KB;
+  constexpr int PER_HALF = 16 / PB;
+  constexpr uint32_t MAGIC = pair_magic<DT, CODE_BITS>();
+  __shared__ int s_slot[KB == 0 ? kSlab : 1];
+  __shared__ uint32_t s_mn[4][64], s_mx[4][64];
+  const int p = threadIdx.x & 63, split = threadIdx.x >> 6, splits = blockDim.x >> 6;
+  const int g = blockIdx.x, c0 = blockIdx.y * kSlab + 2 * p;
+  const int64_t o = blockIdx.z;
+  const bool live = c0 < a.inner;      // the column count is even
+  if (KB == 0) {
+    for (int i = threadIdx.x; i < kSlab; i += blockDim.x) s_slot[i] = -1;
+    __syncthreads();
+    for (int k = threadIdx.x; k < a.promoted; k += blockDim.x) {
+      const int c = a.indices[o * a.promoted + k] - (int)blockIdx.y * kSlab;
+      if (c >= 0 && c < kSlab) s_slot[c] = k;
+    }
+  }
+  const int words = a.group * PB / 32, mine = words / splits;           // words per group and plane, of this thread
+  const int tok = mine * 2 * PER_HALF, t_begin = g * a.group + split * tok;
+  const uint16_t* col = a.x + o * a.so + (live ? c0 : 0);
+  // the last group is padded by repeating the final element
+  auto at = [&](int t) { return __ldg(reinterpret_cast<const uint32_t*>(col + (int64_t)min(t, a.n - 1) * a.sn)); };
+  uint32_t mn2 = at(t_begin), mx2 = mn2;
+#pragma unroll 8
+  for (int j = 1; j < tok; ++j) {
+    const uint32_t v = at(t_begin + j);
+    mn2 = P::min2(mn2, v);
+    mx2 = P::max2(mx2, v);
+  }
+  s_mn[split][p] = mn2;
+  s_mx[split][p] = mx2;
+  __syncthreads();
+  for (int s = 0; s < splits; ++s) { mn2 = P::min2(mn2, s_mn[s][p]); mx2 = P::max2(mx2, s_mx[s][p]); }
+  if (!live) return;
+  const float mn_lo = P::lo(mn2), mn_hi = P::hi(mn2), mx_lo = P::lo(mx2), mx_hi = P::hi(mx2);
+  if (a.nonfinite && !(isfinite(mn_lo) && isfinite(mn_hi) && isfinite(mx_lo) && isfinite(mx_hi))) *a.nonfinite = 1;
+  const int slot_lo = KB == 0 ? s_slot[2 * p] : -1, slot_hi = KB == 0 ? s_slot[2 * p + 1] : -1;
+  const float qmax_lo = KB == 0 ? (slot_lo >= 0 ? 15.0f : 3.0f) : (float)((1 << CODE_BITS) - 1);
+  const float qmax_hi = KB == 0 ? (slot_hi >= 0 ? 15.0f : 3.0f) : (float)((1 << CODE_BITS) - 1);
+  float scale_lo = scale_of<DT>(mn_lo, mx_lo, qmax_lo), scale_hi = scale_of<DT>(mn_hi, mx_hi, qmax_hi);
+  const int64_t row = o * a.inner + c0;
+  if (split == 0) {
+    store_f(a.scale, a.md, row * a.groups + g, scale_lo);
+    store_f(a.scale, a.md, (row + 1) * a.groups + g, scale_hi);
+    store_f(a.zero, a.md, row * a.groups + g, mn_lo);
+    store_f(a.zero, a.md, (row + 1) * a.groups + g, mn_hi);
+  }
+  const float inv_lo = inverse_scale(scale_lo), inv_hi = inverse_scale(scale_hi);
+  if (DT == DARTKV_F16) {
+    scale_lo = isinf(scale_lo) ? 0.0f : scale_lo;
+    scale_hi = isinf(scale_hi) ? 0.0f : scale_hi;
+  }
+  const uint32_t cap2 = cap_pair<DT>(qmax_lo, qmax_hi);
+  auto word_at = [&](uint8_t* plane, int64_t r, int w) -> uint32_t& {
+    return reinterpret_cast<uint32_t*>(plane + r * a.packed_bytes + (int64_t)g * words * 4)[split * mine + w];
+  };
+#pragma unroll 1
+  for (int w = 0; w < mine; ++w) {
+    uint32_t acc_a[2], acc_b[2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int base = t_begin + (2 * w + half) * PER_HALF;
+      uint32_t x[PER_HALF];
+#pragma unroll
+      for (int u = 0; u < PER_HALF; ++u) x[u] = at(base + u);
+      auto codes = [&](int u) { return pair_codes<DT, CODE_BITS>(x[u], mn2, scale_lo, scale_hi, inv_lo, inv_hi, cap2); };
+      if (KB == 0) {
+        uint32_t even = 0u - magic_sum(MAGIC, 4, 4), odd = even;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          even = gather(even, codes(2 * u), 4 * u);
+          odd = gather(odd, codes(2 * u + 1), 4 * u);
+        }
+        acc_a[half] = (even & 0x33333333u) | ((odd << 2) & 0xCCCCCCCCu);
+        acc_b[half] = ((even >> 2) & 0x33333333u) | (odd & 0xCCCCCCCCu);
+      } else {
+        uint32_t acc = 0u - magic_sum(MAGIC, PER_HALF, PB);
+#pragma unroll
+        for (int u = 0; u < PER_HALF; ++u) acc = gather(acc, codes(u), PB * u);
+        acc_a[half] = acc;
+        acc_b[half] = 0;
+      }
+    }
+    word_at(a.values, row, w) = __byte_perm(acc_a[0], acc_a[1], 0x5410);
+    word_at(a.values, row + 1, w) = __byte_perm(acc_a[0], acc_a[1], 0x7632);
+    if (KB == 0) {
+      if (slot_lo >= 0) word_at(a.high, o * a.promoted + slot_lo, w) = __byte_perm(acc_b[0], acc_b[1], 0x5410);
+      if (slot_hi >= 0) word_at(a.high, o * a.promoted + slot_hi, w) = __byte_perm(acc_b[0], acc_b[1], 0x7632);
+    }
+  }
+}
+
+template <int DT>
+void launch_columns(int kb, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
+  if (kb == 0) quantize_columns_kernel<DT, 0><<<grid, threads, 0, stream>>>(a);
+  else if (kb == 2) quantize_columns_kernel<DT, 2><<<grid, threads, 0, stream>>>(a);
+  else if (kb == 4) quantize_columns_kernel<DT, 4><<<grid, threads, 0, stream>>>(a);
+  else quantize_columns_kernel<DT, 8><<<grid, threads, 0, stream>>>(a);
+}
+
+bool is16(int dt) { return dt == DARTKV_F16 || dt == DARTKV_BF16; }
+bool fits_int(int64_t v) { return v < (1ll << 31); }
+
+}  // namespace
+
+// Groups along an axis whose columns lie next to each other (inner > 1, stride 1).  key_bits 0: mixed 2+2-bit keys.
+// Returns 1 when the launch was made, 0 when the shape is not one of this file, a negative code on a failed launch.
+int dartkv_quantize_columns_fast(const void* x, int dtype, int64_t outer, int64_t n, int64_t inner, int64_t so, int64_t sn,
+                                 int key_bits, int group, int md, uint8_t* values, uint8_t* high, const int32_t* indices,
+                                 int promoted, void* scale, void* zero, int32_t* nonfinite, cudaStream_t stream) {
+  const int plane_bits = key_bits == 0 ? 2 : key_bits;
+  if (!is16(dtype) || inner < 2 || inner % 2 || so % 2 || sn % 2 || (uintptr_t)x % 4 || (uintptr_t)values % 4 || (uintptr_t)high % 4)
+    return 0;
+  if ((int64_t)group * plane_bits % 32 || outer > 65535 || !fits_int(n + group) || !fits_int(inner)) return 0;
+  const int64_t groups = ceil_div64(n, group), slabs = ceil_div64(inner, kSlab);
+  if (slabs > 65535) return 0;
+  const int words = (int)((int64_t)group * plane_bits / 32);
+  const int splits = words % 4 == 0 ? 4 : words % 2 == 0 ? 2 : 1;
+  ColumnArgs a{reinterpret_cast<const uint16_t*>(x), so, sn, (int)n, (int)inner, group, (int)groups,
+               groups * (int64_t)words * 4, values, high, indices, promoted, md, scale, zero, nonfinite};
+  const dim3 grid((unsigned)groups, (unsigned)slabs, (unsigned)outer);
+  if (dtype == DARTKV_F16) launch_columns<DARTKV_F16>(key_bits, grid, 64 * splits, stream, a);
+  else launch_columns<DARTKV_BF16>(key_bits, grid, 64 * splits, stream, a);
+  DARTKV_LAUNCH_OK("quantize_columns_kernel");
+  return 1;
+}
+
+// ---------------------------------------------------------------------------- groups along contiguous elements
+namespace {
+
+// Eight elements per thread, group / 8 neighbouring lanes per group (a power of two up to a warp).
+template <int DT, int VB>
+__global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __restrict__ x, int64_t rows, int n, int64_t so,
+                                                            int group, int md, uint8_t* __restrict__ values, void* scale_out,
+                                                            void* zero_out, int32_t* nonfinite) {
+  using P = Pack16<DT>;
+  const int per_row = n / 8, lanes = group / 8;
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = id < rows * per_row;
+  const int64_t row = live ? id / per_row : 0;
+  const int k = live ? (int)(id - row * per_row) : 0;
+  const uint4 raw = *reinterpret_cast<const uint4*>(x + row * so + 8 * k);
+  const uint32_t v[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t mn2 = P::min2(P::min2(v[0], v[1]), P::min2(v[2], v[3])), mx2 = P::max2(P::max2(v[0], v[1]), P::max2(v[2], v[3]));
+  for (int off = 1; off < lanes; off <<= 1) {
+    mn2 = P::min2(mn2, __shfl_xor_sync(0xffffffffu, mn2, off));
+    mx2 = P::max2(mx2, __shfl_xor_sync(0xffffffffu, mx2, off));
+  }
+  if (!live) return;   // groups lie wholly inside or outside
+  const uint32_t mn1 = P::min2(mn2, mn2 >> 16), mx1 = P::max2(mx2, mx2 >> 16);
+  const float mn = P::lo(mn1), mx = P::lo(mx1);
+  constexpr float qmax = (float)((1 << VB) - 1);
+  const float scale = scale_of<DT>(mn, mx, qmax), inv = inverse_scale(scale);
+  const float s_q = DT == DARTKV_F16 && isinf(scale) ? 0.0f : scale;
+  const uint32_t mnp = (mn1 & 0xFFFFu) * 0x00010001u, cap2 = cap_pair<DT>(qmax, qmax);
+  constexpr int PAIRS = 8 / VB, GATHERS = 4 / PAIRS;     // pairs per gathered 16 bits, gathers per thread
+  constexpr uint32_t MAGIC = pair_magic<DT, VB>();
+  constexpr uint32_t LOMASK = VB == 2 ? 0x3333u : VB == 4 ? 0x0F0Fu : 0x00FFu;
+  uint32_t half_word[GATHERS];
+#pragma unroll
+  for (int g = 0; g < GATHERS; ++g) {
+    uint32_t acc = 0u - magic_sum(MAGIC, PAIRS, 2 * VB);
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) acc = gather(acc, pair_codes<DT, VB>(v[g * PAIRS + i], mnp, s_q, s_q, inv, inv, cap2), 2 * VB * i);
+    half_word[g] = (acc & LOMASK) | ((acc >> (16 - VB)) & (LOMASK << VB));
+  }
+  if (VB == 2) reinterpret_cast<uint16_t*>(values)[id] = (uint16_t)half_word[0];
+  else if (VB == 4) reinterpret_cast<uint32_t*>(values)[id] = half_word[0] | (half_word[GATHERS / 2] << 16);
+  else reinterpret_cast<uint2*>(values)[id] = make_uint2(half_word[0] | (half_word[GATHERS > 1] << 16),
+                                                         half_word[GATHERS / 2] | (half_word[GATHERS - 1] << 16));
+  if (k % lanes == 0) {
+    if (nonfinite && !(isfinite(mn) && isfinite(mx))) *nonfinite = 1;
+    const int64_t g = row * (per_row / lanes) + k / lanes;
+    store_f(scale_out, md, g, scale);
+    store_f(zero_out, md, g, mn);
+  }
+}
+
+template <int DT>
+void launch_rows(int bits, unsigned blocks, cudaStream_t stream, const void* x_, int64_t rows, int n, int64_t so, int group, int md,
+                 uint8_t* values, void* scale, void* zero, int32_t* nonfinite) {
+  const uint16_t* x = reinterpret_cast<const uint16_t*>(x_);
+  if (bits == 2) quantize_rows_kernel<DT, 2><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
+  else if (bits == 4) quantize_rows_kernel<DT, 4><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
+  else quantize_rows_kernel<DT, 8><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
+}
+
+}  // namespace
+
+// Whole groups of 8..256 contiguous elements (a power of two); return value as above.
+int dartkv_quantize_rows_fast(const void* x, int dtype, int64_t rows, int64_t n, int64_t so, int bits, int group, int md,
+                              uint8_t* values, void* scale, void* zero, int32_t* nonfinite, cudaStream_t stream) {
+  if (!is16(dtype) || group < 8 || group > 256 || (group & (group - 1)) || n % group || so % 8 || (uintptr_t)x % 16 ||
+      (uintptr_t)values % 8 || !fits_int(n))
+    return 0;
+  const int64_t blocks = ceil_div64(rows * (n / 8), 256);
+  if (!fits_int(blocks)) return 0;
+  if (dtype == DARTKV_F16) launch_rows<DARTKV_F16>(bits, (unsigned)blocks, stream, x, rows, (int)n, so, group, md, values, scale, zero, nonfinite);
+  else launch_rows<DARTKV_BF16>(bits, (unsigned)blocks, stream, x, rows, (int)n, so, group, md, values, scale, zero, nonfinite);
+  DARTKV_LAUNCH_OK("quantize_rows_kernel");
+  return 1;
+}
+
+// ---------------------------------------------------------------------------- channel scores and selection
+namespace {
+
+constexpr int kScoreSplits = 16;
+
+// Promoted channels of one (batch, head): sum |k| per channel in double (exact for 16-bit data, in any order), scores
+// rounded to the data dtype, rank by (score descending, channel ascending).  One block of 16 token splits x 64 channel
+// pairs; scores (optional) are written too.
+template <int DT>
+__global__ void __launch_bounds__(64 * kScoreSplits) score_select_kernel(const uint16_t* __restrict__ keys, int64_t tokens, int d,
+                                                                         int64_t sbh, int64_t st, int count,
+                                                                         uint16_t* scores, int32_t* indices) {
+  using P = Pack16<DT>;
+  __shared__ double s_sum[kScoreSplits][2][64];
+  __shared__ uint32_t s_key[128];
+  const int p = threadIdx.x & 63, split = threadIdx.x >> 6;
+  const int64_t r = blockIdx.x;
+  double lo = 0.0, hi = 0.0;
+  if (2 * p < d) {
+    const uint16_t* col = keys + r * sbh + 2 * p;
+#pragma unroll 8
+    for (int64_t t = split; t < tokens; t += kScoreSplits) {
+      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(col + t * st));
+      lo += (double)fabsf(P::lo(v));
+      hi += (double)fabsf(P::hi(v));
+    }
+  }
+  s_sum[split][0][p] = lo;
+  s_sum[split][1][p] = hi;
+  __syncthreads();
+  const int c = threadIdx.x;
+  uint32_t key = 0;
+  if (c < d) {
+    double sum = 0.0;
+#pragma unroll
+    for (int s = 0; s < kScoreSplits; ++s) sum += s_sum[s][c & 1][c >> 1];
+    const uint16_t bits = P::bits(__fdiv_rn((float)sum, (float)tokens));
+    if (scores) scores[r * d + c] = bits;
+    // scores are non-negative 16-bit floats: their bit patterns order like integers
+    key = ((uint32_t)bits << 7) | (uint32_t)(127 - c);
+    s_key[c] = key;
+  }
+  if (indices == nullptr) return;
+  __syncthreads();
+  if (c < d) {
+    int rank = 0;
+    for (int o = 0; o < d; ++o) rank += s_key[o] > key;
+    if (rank < count) indices[r * count + rank] = c;
+  }
+}
+
+}  // namespace
+
+// keys [bh][tokens][d] with strides; scores and indices may be null.  Return value as above.
+int dartkv_score_select_fast(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t d, int64_t sbh, int64_t st,
+                             int count, void* scores, int32_t* indices, cudaStream_t stream) {
+  if (!is16(dtype) || d > 128 || d % 2 || sbh % 2 || st % 2 || (uintptr_t)keys % 4 || !fits_int(bh)) return 0;
+  const uint16_t* k = reinterpret_cast<const uint16_t*>(keys);
+  uint16_t* s = reinterpret_cast<uint16_t*>(scores);
+  if (dtype == DARTKV_F16) score_select_kernel<DARTKV_F16><<<(unsigned)bh, 64 * kScoreSplits, 0, stream>>>(k, tokens, (int)d, sbh, st, count, s, indices);
+  else score_select_kernel<DARTKV_BF16><<<(unsigned)bh, 64 * kScoreSplits, 0, stream>>>(k, tokens, (int)d, sbh, st, count, s, indices);
+  DARTKV_LAUNCH_OK("score_select_kernel");
+  return 1;
+}
+
+// ---------------------------------------------------------------------------- dequantization
+namespace {
+
+struct RestoreArgs {
+  const uint8_t *values, *high;
+  const int32_t* indices;
+  int promoted;
+  const void *scale, *zero;
+  int n, inner, group, groups, flavour;
+  int64_t packed_bytes, so, sn;
+  void* out;
+};
+
+template <int MD>
+__device__ __forceinline__ float meta16(const void* p, int64_t i) { return load_f(p, MD, i); }
+
+template <int OUT>
+__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) { return Pack16<OUT>::pack(hi, lo); }
+
+// Groups along a strided axis: a thread restores the tokens of one code word for two neighbouring columns.
+// grid (words / 4, slab of columns, outer), 256 threads = 64 column pairs x 4 words.  BITS 0: mixed keys.
+template <int MD, int OUT, int BITS>
+__global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_constant__ RestoreArgs a) {
+  constexpr int PB = BITS == 0 ? 2 : BITS, TOK = 32 / PB;
+  constexpr uint32_t MASK = (1u << PB) - 1u;
+  __shared__ int s_slot[BITS == 0 ? kSlab : 1];
+  const int64_t o = blockIdx.z;
+  if (BITS == 0) {
+    for (int i = threadIdx.x; i < kSlab; i += blockDim.x) s_slot[i] = -1;
+    __syncthreads();
+    for (int k = threadIdx.x; k < a.promoted; k += blockDim.x) {
+      const int c = a.indices[o * a.promoted + k] - (int)blockIdx.y * kSlab;
+      if (c >= 0 && c < kSlab) s_slot[c] = k;
+    }
+    __syncthreads();
+  }
+  const int p = threadIdx.x & 63, w = blockIdx.x * 4 + (threadIdx.x >> 6);
+  const int c0 = blockIdx.y * kSlab + 2 * p, t0 = w * TOK;
+  if (c0 >= a.inner || t0 >= a.n) return;
+  const int g = t0 / a.group;
+  const int64_t row = o * a.inner + c0;
+  uint32_t code[2], high[2] = {0, 0};
+  float s[2], z[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    code[i] = reinterpret_cast<const uint32_t*>(a.values + (row + i) * a.packed_bytes)[w];
+    if (BITS == 0) {
+      const int slot = s_slot[2 * p + i];
+      if (slot >= 0) high[i] = reinterpret_cast<const uint32_t*>(a.high + (o * a.promoted + slot) * a.packed_bytes)[w];
+    }
+    s[i] = meta16<MD>(a.scale, (row + i) * a.groups + g);
+    z[i] = meta16<MD>(a.zero, (row + i) * a.groups + g);
+  }
+  uint32_t* out = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(a.out) + o * a.so + (int64_t)t0 * a.sn + c0);
+#pragma unroll
+  for (int u = 0; u < TOK; ++u) {
+    if (t0 + u >= a.n) break;
+    float v[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint32_t q = (code[i] >> (PB * u)) & MASK;
+      if (BITS == 0) q |= ((high[i] >> (PB * u)) & MASK) << 2;
+      v[i] = affine_restore((float)q, s[i], z[i], MD, OUT, a.flavour);
+    }
+    *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + (int64_t)u * a.sn) = pack_pair<OUT>(v[0], v[1]);
+  }
+}
+
+// Groups along contiguous elements: a thread restores eight of them.
+template <int MD, int OUT, int BITS>
+__global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant__ RestoreArgs a, int64_t total) {
+  constexpr uint32_t MASK = (1u << BITS) - 1u;
+  const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= total) return;
+  const int per_row = a.n / 8;
+  const int64_t row = id / per_row;
+  const int k = (int)(id - row * per_row), g = 8 * k / a.group;
+  uint64_t codes;
+  if (BITS == 2) codes = reinterpret_cast<const uint16_t*>(a.values)[id];
+  else if (BITS == 4) codes = reinterpret_cast<const uint32_t*>(a.values)[id];
+  else codes = reinterpret_cast<const uint64_t*>(a.values)[id];
+  const float s = meta16<MD>(a.scale, row * a.groups + g), z = meta16<MD>(a.zero, row * a.groups + g);
+  uint32_t v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float lo = affine_restore((float)((uint32_t)(codes >> (BITS * 2 * i)) & MASK), s, z, MD, OUT, a.flavour);
+    const float hi = affine_restore((float)((uint32_t)(codes >> (BITS * (2 * i + 1))) & MASK), s, z, MD, OUT, a.flavour);
+    v[i] = pack_pair<OUT>(lo, hi);
+  }
+  reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + row * a.so)[k] = make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+template <int MD, int OUT>
+void launch_restore(bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a, int64_t total) {
+  if (columns) {
+    if (bits == 0) restore_columns_kernel<MD, OUT, 0><<<grid, 256, 0, stream>>>(a);
+    else if (bits == 2) restore_columns_kernel<MD, OUT, 2><<<grid, 256, 0, stream>>>(a);
+    else if (bits == 4) restore_columns_kernel<MD, OUT, 4><<<grid, 256, 0, stream>>>(a);
+    else restore_columns_kernel<MD, OUT, 8><<<grid, 256, 0, stream>>>(a);
+  } else {
+    if (bits == 2) restore_rows_kernel<MD, OUT, 2><<<grid, 256, 0, stream>>>(a, total);
+    else if (bits == 4) restore_rows_kernel<MD, OUT, 4><<<grid, 256, 0, stream>>>(a, total);
+    else restore_rows_kernel<MD, OUT, 8><<<grid, 256, 0, stream>>>(a, total);
+  }
+}
+void launch_restore_typed(int md, int out_dtype, bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a,
+                          int64_t total) {
+  if (md == DARTKV_F16 && out_dtype == DARTKV_F16) launch_restore<DARTKV_F16, DARTKV_F16>(columns, bits, grid, stream, a, total);
+  else if (md == DARTKV_F16) launch_restore<DARTKV_F16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
+  else if (out_dtype == DARTKV_F16) launch_restore<DARTKV_BF16, DARTKV_F16>(columns, bits, grid, stream, a, total);
+  else launch_restore<DARTKV_BF16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
+}
+
+}  // namespace
+
+// Inverse of dartkv_quantize_columns_fast; return value as above.
+int dartkv_restore_columns_fast(const uint8_t* values, const uint8_t* high, const int32_t* indices, int promoted,
+                                const void* scale, const void* zero, int md, int64_t outer, int64_t n, int64_t inner,
+                                int key_bits, int group, int flavour, void* out, int out_dtype, int64_t so, int64_t sn,
+                                cudaStream_t stream) {
+  const int plane_bits = key_bits == 0 ? 2 : key_bits;
+  if (!is16(md) || !is16(out_dtype) || inner < 2 || inner % 2 || so % 2 || sn % 2 || (uintptr_t)out % 4 || (uintptr_t)values % 4 ||
+      (uintptr_t)high % 4 || (int64_t)group * plane_bits % 32 || outer > 65535 || !fits_int(n + group) || !fits_int(inner))
+    return 0;
+  const int64_t groups = ceil_div64(n, group), words = groups * (int64_t)group * plane_bits / 32, slabs = ceil_div64(inner, kSlab);
+  if (slabs > 65535) return 0;
+  RestoreArgs a{values, high, indices, promoted, scale, zero, (int)n, (int)inner, group, (int)groups, flavour, words * 4, so, sn, out};
+  const dim3 grid((unsigned)ceil_div64(words, 4), (unsigned)slabs, (unsigned)outer);
+  launch_restore_typed(md, out_dtype, true, key_bits, grid, stream, a, 0);
+  DARTKV_LAUNCH_OK("restore_columns_kernel");
+  return 1;
+}
+
+// Inverse of dartkv_quantize_rows_fast (any group that is a multiple of eight); return value as above.
+int dartkv_restore_rows_fast(const uint8_t* values, const void* scale, const void* zero, int md, int64_t rows, int64_t n, int bits,
+                             int group, int flavour, void* out, int out_dtype, int64_t so, cudaStream_t stream) {
+  if (!is16(md) || !is16(out_dtype) || n % group || group % 8 || so % 8 || (uintptr_t)out % 16 || (uintptr_t)values % 8 || !fits_int(n))
+    return 0;
+  const int64_t total = rows * (n / 8), blocks = ceil_div64(total, 256);
+  if (!fits_int(blocks)) return 0;
+  RestoreArgs a{values, nullptr, nullptr, 0, scale, zero, (int)n, 1, group, (int)(n / group), flavour, 0, so, 1, out};
+  launch_restore_typed(md, out_dtype, false, bits, dim3((unsigned)blocks), stream, a, total);
+  DARTKV_LAUNCH_OK("restore_rows_kernel");
+  return 1;
+}

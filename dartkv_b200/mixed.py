@@ -201,9 +201,25 @@ def quantize_key_mixed(
     device = require_cuda(key_states)
     keys = key_states.detach().contiguous()
     batch, heads, tokens, head_dim = keys.shape
-    if indices is None:
+    count = promoted_count(head_dim, promote_ratio) if 0.0 <= promote_ratio <= 1.0 else -1
+    # magnitude selection with something to select runs in the quantizer's own call, without mask and int64 indices
+    select_here = indices is None and strategy == "magnitude" and 0 < count < head_dim
+    if indices is None and not select_here:
         _, indices = select_key_channels(keys, promote_ratio, strategy=strategy)
-    idx32 = indices.to(device=device, dtype=torch.int32).contiguous()
+    idx32 = None if select_here else indices.to(device=device, dtype=torch.int32).contiguous()
+    made = _lib.HOST.quantize_mixed(keys, group_size, count, _lib.DTYPE_CODE[meta_dtype], idx32, int(check_finite))
+    if made is False:
+        raise ValueError("key_states must contain finite values")
+    if type(made) is int:
+        check(made)
+    if made is not None:
+        low, high, idx32, scale, zero = made
+        return MixedQuantizedKey(
+            low_values=low, high_values=high, channel_indices=idx32, scale=scale, zero_point=zero,
+            original_shape=(batch, heads, tokens, head_dim), padded_tokens=-(-tokens // group_size) * group_size,
+            group_size=group_size, low_bits=2, promote_bits=promote_bits, output_dtype=keys.dtype)
+    if select_here:
+        idx32 = select_key_channels(keys, promote_ratio, strategy=strategy)[1].to(torch.int32).contiguous()
     promoted = idx32.shape[-1]
     groups = (tokens + group_size - 1) // group_size
     packed = (group_size + 3) // 4

@@ -195,6 +195,18 @@ def quantize(
     vpb = 8 // bits
     packed_dim = ((padded_dim + vpb - 1) // vpb) * vpb
     moved_shape = tuple(s for i, s in enumerate(original_shape) if i != axis)
+    made = _lib.HOST.quantize(data, bits, group_size, axis, _lib.DTYPE_CODE[meta_dtype],
+                              _lib.DIV_TRUE if division == "true" else _lib.DIV_RECIPROCAL, int(check_finite))
+    if made is False:
+        raise ValueError("quantize expects all values to be finite")
+    if type(made) is int:
+        check(made)
+    if made is not None:
+        values, scale, zero = made
+        return QuantizedTensor(
+            values=values, scale=scale, zero_point=zero, original_shape=original_shape, original_dim=n,
+            padded_dim=padded_dim, packed_dim=packed_dim, group_size=group_size, bits=bits, output_dtype=data.dtype,
+            axis=axis)
     values = torch.empty((*moved_shape, packed_dim // vpb), dtype=torch.uint8, device=device)
     scale = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)
     zero = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)

@@ -82,6 +82,10 @@ int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, int64_t token
  * scores per row, ordered by (score descending, channel ascending); indices int32 [bh, count]. */
 int dartkv_select_channels(const void* scores, int dtype, int64_t bh, int64_t head_dim, int count,
                            int32_t* indices, void* stream);
+/* Both for the 'magnitude' strategy, in one launch for 16-bit keys of up to 128 channels (scores: scratch of
+ * [bh, D] values of `dtype` for the other shapes). */
+int dartkv_promote_channels(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t head_dim, int64_t stride_bh,
+                            int64_t stride_token, int count, void* scores, int32_t* indices, void* stream);
 /* Replaces quantize_key_mixed (src/dart/mixed.py:166-244) for given promoted channels.
  * low [bh, D, G, ceil(Gk/4)], high [bh, K, G, ceil(Gk/4)], scale/zero [bh, D, G]. */
 int dartkv_quantize_key_mixed(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t head_dim,
@@ -202,6 +206,9 @@ int dartkv_cache_append_device_planned(const dartkv_cache_desc* desc, const dart
  * src/dart/cache.py:192-199); side 0 = keys, 1 = values. */
 int dartkv_cache_materialize(const dartkv_cache_desc* desc, int side, int32_t t0, int32_t t1, int flavour,
                              void* out, int out_dtype, void* stream);
+/* Keys and values of the same tokens in one launch. */
+int dartkv_cache_materialize_both(const dartkv_cache_desc* desc, int32_t t0, int32_t t1, int flavour, void* out_k,
+                                  void* out_v, int out_dtype, void* stream);
 
 /* ------------------------------------------------------------------ fused decode attention
  * Replaces fused_dart_attention (src/dart/fused_attention.py:654-771) and, numerically,
