@@ -15,7 +15,8 @@
 
 #include "common.cuh"
 
-#define GEN_THREADS 128
+#define GEN_THREADS 256
+#define GEN_WARPS (GEN_THREADS / 32)
 #define GEN_TILE 32
 #define GEN_MAX_REP 16
 #define GEN_MAX_D 256
@@ -49,21 +50,29 @@ struct GenericArgs {
   const int32_t* row_start;   // optional [batch] first live token of every batch row
 };
 
-__global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cache_desc d, GenericArgs a) {
+// One block per (batch, kv head) and run of tokens, in tiles of 32 tokens.  Keys: lane = token, the channels are dealt
+// out to the warps, so the codes of a channel are one short coalesced read, its scale and the query are broadcasts and
+// a dot product needs no shuffles; the warps' partial logits meet in shared memory.  Values: thread = channel, the
+// tile's tokens split over the remaining threads.  Nothing dequantized is staged.  Latency is what counts here (small
+// fp32 caches): loads of several channels / tokens are in flight together, and a call is cut into tiles until every SM
+// has a block.  [1,8,256,128] fp32, 2-bit: 94 us with one serial dot product per thread and staged tiles, now 8 us (B200).
+template <int REP>
+__global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __grid_constant__ dartkv_cache_desc d,
+                                                                     const __grid_constant__ GenericArgs a) {
   extern __shared__ float smem[];
-  const int D = d.head_dim, DP = D + 1;
-  const int rep = a.query_heads / d.kv_heads;
-  float* s_q = smem;                              // [rep][D]
-  float* s_tile = s_q + rep * D;                  // [GEN_TILE][D+1]
-  float* s_p = s_tile + GEN_TILE * DP;            // [rep][GEN_TILE]
-  float* s_alpha = s_p + rep * GEN_TILE;          // [rep]
-  float* s_m = s_alpha + rep;                     // [rep]
-  float* s_l = s_m + rep;                         // [rep]
-  int* s_slot = reinterpret_cast<int*>(s_l + rep);// [D]
+  const int D = d.head_dim;
+  const int rep = a.query_heads / d.kv_heads;            // at most REP
+  float* s_q = smem;                                     // [D][REP]: a channel's heads together
+  float* s_part = s_q + D * REP;                         // [warp][REP][32] partial logits, then [split][REP][D] sums
+  float* s_p = s_part + GEN_WARPS * REP * GEN_TILE;      // [32][REP] probabilities of the tile
+  float* s_alpha = s_p + GEN_TILE * REP;                 // [REP]
+  float* s_m = s_alpha + REP;
+  float* s_l = s_m + REP;
+  int* s_slot = reinterpret_cast<int*>(s_l + REP);       // [D]
 
   const int bh = blockIdx.x, split = blockIdx.y;
   const int b = bh / d.kv_heads, h = bh % d.kv_heads;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int seen = d.state[0], pages = d.state[1], k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
   const int end = a.tok_end < 0 ? seen : min(a.tok_end, seen);
   // tok_begin < 0: start where the tensor-core kernel stops (last full page packed on both sides)
@@ -74,16 +83,16 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cach
   // left padding: the tokens before the row's first live one get no weight (a split wholly before it stays empty)
   const int lo = a.row_start ? max(first, a.row_start[b]) : first;
 
-  for (int i = tid; i < rep * D; i += GEN_THREADS) {
-    int r = i / D, c = i % D;
-    s_q[i] = load_f(a.q, a.q_dt, ((int64_t)b * a.query_heads + h * rep + r) * D + c);
+  for (int i = tid; i < D * REP; i += GEN_THREADS) {
+    const int r = i % REP, c = i / REP;
+    s_q[i] = r < rep ? load_f(a.q, a.q_dt, ((int64_t)b * a.query_heads + h * rep + r) * D + c) : 0.0f;
   }
-  if (tid < rep) { s_m[tid] = -INFINITY; s_l[tid] = 0.0f; }
-  float acc[GEN_MAX_REP][GEN_MAX_D / GEN_THREADS];
+  if (tid < REP) { s_m[tid] = -INFINITY; s_l[tid] = 0.0f; }
+  // values: this thread's channel and share of the tile's tokens (D is at most the block)
+  const int vsplits = GEN_THREADS / D, vsplit = tid / D, vc = tid % D;
+  float acc[REP];
 #pragma unroll
-  for (int r = 0; r < GEN_MAX_REP; ++r)
-#pragma unroll
-    for (int k = 0; k < GEN_MAX_D / GEN_THREADS; ++k) acc[r][k] = 0.0f;
+  for (int r = 0; r < REP; ++r) acc[r] = 0.0f;
   __syncthreads();
 
   // A packed value segment [vs, ve) (page_size tokens from sink_tokens on, the last one ending at the packed end)
@@ -100,14 +109,14 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cach
   int t = lo;
   while (t < hi) {
     // ---- locate the key segment that holds token t
-    int seg_end, kind, page_first = 0, page_n = 0;
+    int seg_end, kind, page_first = 0, page_n = 1;
     int key_flavour = a.flavour;
     const uint8_t* page = nullptr;
     if (t < sink_filled) {
       kind = 0; seg_end = min(hi, sink_filled);
     } else if (t < k_end) {
       kind = 1;
-      int pg = gen_find_page(d, pages, t);
+      const int pg = d.regular_pages ? (t - d.sink_tokens) / d.page_size : gen_find_page(d, pages, t);
       page_first = d.page_start[pg];
       page_n = d.page_tokens[pg];
       seg_end = min(hi, page_first + page_n);
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cach
         __syncthreads();
         const int32_t* idx = reinterpret_cast<const int32_t*>(page + d.key_off_index);
         for (int k = tid; k < d.promoted; k += GEN_THREADS) {
-          int c = idx[k];
+          const int c = idx[k];
           if (c >= 0 && c < D) s_slot[c] = k;
         }
         __syncthreads();
@@ -133,86 +142,101 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cach
     } else {
       kind = 2; seg_end = hi;
     }
+    const bool mixed = d.key_mode == DARTKV_MIXED_PAGE;
+    const int Gk = d.key_group, G = ceil_div(page_n, Gk), bits = mixed ? 2 : d.key_bits, vpb = 8 / bits;
+    const int plane = ceil_div(Gk, 4);                                    // mixed: bytes of one group's plane
+    const int row_bytes = mixed ? G * plane : ceil_div(G * Gk, vpb);
     for (int tile0 = t; tile0 < seg_end; tile0 += GEN_TILE) {
       const int nt = min(GEN_TILE, seg_end - tile0);
-      // ---- K tile, dequantized to the cache dtype
-      for (int i = tid; i < nt * D; i += GEN_THREADS) {
-        int tt = i / D, c = i % D, tok = tile0 + tt;
-        float v;
-        if (kind == 0) v = load_f(d.k_sink, d.dtype, ((int64_t)bh * d.sink_tokens + tok) * D + c);
-        else if (kind == 2) v = load_f(d.k_ring, d.dtype, ((int64_t)bh * d.ring_tokens + (tok % d.ring_tokens)) * D + c);
-        else {
-          const int Gk = d.key_group, G = ceil_div(page_n, Gk), j = tok - page_first, g = j / Gk;
-          float s = load_f(page + d.key_off_scale, d.md_dtype, c * G + g);
-          float z = load_f(page + d.key_off_zero, d.md_dtype, c * G + g);
-          uint32_t code;
-          if (d.key_mode == DARTKV_MIXED_PAGE) {
-            const int pb = ceil_div(Gk, 4), jj = j % Gk, slot = s_slot[c];
-            code = (page[(c * G + g) * pb + jj / 4] >> ((jj % 4) * 2)) & 3u;
-            if (slot >= 0) code |= ((page[d.key_off_high + (slot * G + g) * pb + jj / 4] >> ((jj % 4) * 2)) & 3u) << 2;
-          } else {
-            const int bits = d.key_bits, vpb = 8 / bits, row_bytes = ceil_div(G * Gk, vpb);
-            code = (page[(int64_t)c * row_bytes + j / vpb] >> ((j % vpb) * bits)) & ((1u << bits) - 1u);
+      // ---- partial logits of this warp's channels (lanes past the tile repeat its last token)
+      float dot[REP];
+#pragma unroll
+      for (int r = 0; r < REP; ++r) dot[r] = 0.0f;
+      const int tok = tile0 + min(lane, nt - 1);
+      auto add = [&](int c, float k) {
+#pragma unroll
+        for (int r = 0; r < REP; ++r) dot[r] = fmaf(s_q[c * REP + r], k, dot[r]);
+      };
+      if (kind == 1) {
+        const int j = tok - page_first, g = j / Gk;
+        const int at = mixed ? g * plane + (j - g * Gk) / 4 : j / vpb;
+        const int shift = mixed ? ((j - g * Gk) % 4) * 2 : (j % vpb) * bits;
+        const uint32_t mask = (1u << bits) - 1u;
+        const uint8_t *scale = page + d.key_off_scale, *zero = page + d.key_off_zero;
+#pragma unroll 8
+        for (int c = warp; c < D; c += GEN_WARPS) {
+          uint32_t code = (page[c * row_bytes + at] >> shift) & mask;
+          const float s = load_f(scale, d.md_dtype, c * G + g), z = load_f(zero, d.md_dtype, c * G + g);
+          if (mixed && s_slot[c] >= 0) code |= ((page[d.key_off_high + s_slot[c] * row_bytes + at] >> shift) & 3u) << 2;
+          add(c, affine_restore((float)code, s, z, d.md_dtype, d.dtype, key_flavour));
+        }
+      } else {
+        const void* rows = kind == 0 ? d.k_sink : d.k_ring;
+        const int64_t row = kind == 0 ? (int64_t)bh * d.sink_tokens + tok : (int64_t)bh * d.ring_tokens + tok % d.ring_tokens;
+#pragma unroll 8
+        for (int c = warp; c < D; c += GEN_WARPS) add(c, load_f(rows, d.dtype, row * D + c));
+      }
+#pragma unroll
+      for (int r = 0; r < REP; ++r) s_part[(warp * REP + r) * GEN_TILE + lane] = dot[r];
+      __syncthreads();
+      // ---- online softmax state, a warp per query head
+      for (int r = warp; r < rep; r += GEN_WARPS) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < GEN_WARPS; ++w) v += s_part[(w * REP + r) * GEN_TILE + lane];
+        v = lane < nt ? v * a.scale : -INFINITY;
+        float mx = v;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const float m_old = s_m[r], m_new = fmaxf(m_old, mx);
+        const float e = expf(v - m_new);
+        float sum = e;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        s_p[lane * REP + r] = e;
+        __syncwarp();
+        if (lane == 0) {
+          const float alpha = expf(m_old - m_new);
+          s_alpha[r] = alpha;
+          s_m[r] = m_new;
+          s_l[r] = s_l[r] * alpha + sum;
+        }
+      }
+      __syncthreads();
+      // ---- values
+      if (vsplit < vsplits) {
+#pragma unroll
+        for (int r = 0; r < REP; ++r) acc[r] *= r < rep ? s_alpha[r] : 0.0f;
+        const int vbits = d.value_bits, per = 8 / vbits, vg = vc / d.value_group;
+        const uint32_t vmask = (1u << vbits) - 1u;
+        auto weigh = [&](int tt, float v) {
+#pragma unroll
+          for (int r = 0; r < REP; ++r) acc[r] = fmaf(r < rep ? s_p[tt * REP + r] : 0.0f, v, acc[r]);
+        };
+        if (tile0 >= sink_filled && tile0 + nt <= v_end) {
+#pragma unroll 8
+          for (int tt = vsplit; tt < nt; tt += vsplits) {
+            const int64_t row = (int64_t)bh * d.max_value_tokens + (tile0 + tt - d.sink_tokens);
+            const uint32_t code = (d.v_codes[row * d.value_row_bytes + vc / per] >> ((vc % per) * vbits)) & vmask;
+            const float s = load_f(d.v_meta, d.md_dtype, (row * 2 + 0) * d.value_groups + vg);
+            const float z = load_f(d.v_meta, d.md_dtype, (row * 2 + 1) * d.value_groups + vg);
+            weigh(tt, affine_restore((float)code, s, z, d.md_dtype, d.dtype, value_flavour(tile0 + tt)));
           }
-          v = affine_restore((float)code, s, z, d.md_dtype, d.dtype, key_flavour);
-        }
-        s_tile[tt * DP + c] = v;
-      }
-      __syncthreads();
-      // ---- logits
-      for (int i = tid; i < rep * nt; i += GEN_THREADS) {
-        int r = i / nt, tt = i % nt;
-        const float* qr = s_q + r * D;
-        const float* kr = s_tile + tt * DP;
-        float dot = 0.0f;
-        for (int c = 0; c < D; ++c) dot = fmaf(qr[c], kr[c], dot);
-        s_p[r * GEN_TILE + tt] = dot * a.scale;
-      }
-      __syncthreads();
-      // ---- online softmax state per query head
-      if (tid < rep) {
-        float* pr = s_p + tid * GEN_TILE;
-        float mx = -INFINITY;
-        for (int tt = 0; tt < nt; ++tt) mx = fmaxf(mx, pr[tt]);
-        float m_old = s_m[tid], m_new = fmaxf(m_old, mx);
-        float alpha = expf(m_old - m_new);
-        float sum = 0.0f;
-        for (int tt = 0; tt < nt; ++tt) { float p = expf(pr[tt] - m_new); pr[tt] = p; sum += p; }
-        s_alpha[tid] = alpha;
-        s_m[tid] = m_new;
-        s_l[tid] = s_l[tid] * alpha + sum;
-      }
-      __syncthreads();
-      // ---- V tile
-      for (int i = tid; i < nt * D; i += GEN_THREADS) {
-        int tt = i / D, c = i % D, tok = tile0 + tt;
-        float v;
-        if (tok < sink_filled) v = load_f(d.v_sink, d.dtype, ((int64_t)bh * d.sink_tokens + tok) * D + c);
-        else if (tok >= v_end) v = load_f(d.v_ring, d.dtype, ((int64_t)bh * d.ring_tokens + (tok % d.ring_tokens)) * D + c);
-        else {
-          int64_t row = (int64_t)bh * d.max_value_tokens + (tok - d.sink_tokens);
-          const int bits = d.value_bits, vpb = 8 / bits, g = c / d.value_group;
-          uint32_t code = (d.v_codes[row * d.value_row_bytes + c / vpb] >> ((c % vpb) * bits)) & ((1u << bits) - 1u);
-          float s = load_f(d.v_meta, d.md_dtype, (row * 2 + 0) * d.value_groups + g);
-          float z = load_f(d.v_meta, d.md_dtype, (row * 2 + 1) * d.value_groups + g);
-          v = affine_restore((float)code, s, z, d.md_dtype, d.dtype, value_flavour(tok));
-        }
-        s_tile[tt * DP + c] = v;
-      }
-      __syncthreads();
-      // ---- accumulate
-#pragma unroll
-      for (int k = 0; k < GEN_MAX_D / GEN_THREADS; ++k) {
-        int c = tid + k * GEN_THREADS;
-        if (c < D) {
-#pragma unroll
-          for (int r = 0; r < GEN_MAX_REP; ++r) {
-            if (r < rep) {
-              float sum = 0.0f;
-              const float* pr = s_p + r * GEN_TILE;
-              for (int tt = 0; tt < nt; ++tt) sum = fmaf(pr[tt], s_tile[tt * DP + c], sum);
-              acc[r][k] = acc[r][k] * s_alpha[r] + sum;
+        } else {
+#pragma unroll 4
+          for (int tt = vsplit; tt < nt; tt += vsplits) {
+            const int vt = tile0 + tt;
+            float v;
+            if (vt < sink_filled) v = load_f(d.v_sink, d.dtype, ((int64_t)bh * d.sink_tokens + vt) * D + vc);
+            else if (vt >= v_end) v = load_f(d.v_ring, d.dtype, ((int64_t)bh * d.ring_tokens + (vt % d.ring_tokens)) * D + vc);
+            else {
+              const int64_t row = (int64_t)bh * d.max_value_tokens + (vt - d.sink_tokens);
+              const uint32_t code = (d.v_codes[row * d.value_row_bytes + vc / per] >> ((vc % per) * vbits)) & vmask;
+              const float s = load_f(d.v_meta, d.md_dtype, (row * 2 + 0) * d.value_groups + vg);
+              const float z = load_f(d.v_meta, d.md_dtype, (row * 2 + 1) * d.value_groups + vg);
+              v = affine_restore((float)code, s, z, d.md_dtype, d.dtype, value_flavour(vt));
             }
+            weigh(tt, v);
           }
         }
       }
@@ -221,19 +245,33 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(dartkv_cach
     t = seg_end;
   }
 
+  // the token shares of a channel meet in shared memory
+  if (vsplits > 1) {
+    if (vsplit < vsplits)
+#pragma unroll
+      for (int r = 0; r < REP; ++r) s_part[(vsplit * REP + r) * D + vc] = acc[r];
+    __syncthreads();
+    if (vsplit == 0)
+#pragma unroll
+      for (int r = 0; r < REP; ++r) {
+        acc[r] = 0.0f;
+        for (int s = 0; s < vsplits; ++s) acc[r] += s_part[(s * REP + r) * D + vc];
+      }
+  }
   const int slot = a.split_base + split;
 #pragma unroll
-  for (int r = 0; r < GEN_MAX_REP; ++r) {
+  for (int r = 0; r < REP; ++r) {
     if (r < rep) {
-      int64_t row = ((int64_t)b * a.query_heads + h * rep + r) * a.total_splits + slot;
+      const int64_t row = ((int64_t)b * a.query_heads + h * rep + r) * a.total_splits + slot;
       if (tid == 0) { a.part_m[row] = s_m[r]; a.part_l[row] = s_l[r]; }
-#pragma unroll
-      for (int k = 0; k < GEN_MAX_D / GEN_THREADS; ++k) {
-        int c = tid + k * GEN_THREADS;
-        if (c < D) a.part_acc[row * D + c] = acc[r][k];
-      }
+      if (vsplit == 0) a.part_acc[row * D + vc] = acc[r];
     }
   }
+}
+
+// shared memory of decode_generic_kernel<REP>; the sums of up to GEN_THREADS channels reuse the partial logits
+static size_t generic_smem(int D, int rep) {
+  return ((size_t)D * rep + (size_t)GEN_WARPS * rep * GEN_TILE + (size_t)GEN_TILE * rep + 3 * rep) * sizeof(float) + (size_t)D * sizeof(int);
 }
 
 // one block per (batch, query head): combine split partials, normalize, cast
@@ -252,6 +290,10 @@ __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   return v;
 }
 
+constexpr int kFewSplits = 17;          // slots of a row on the tensor-core layouts
+constexpr int kMaxGenericSplits = 128;  // keeps the merge of the generic layout short
+constexpr int kManyThreads = 512;       // block of the merge where a row has more slots than kFewSplits
+
 __global__ void decode_merge_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
                                     const float* __restrict__ part_acc, int total_splits, int D, void* out, int out_dt,
                                     int stream_blocks, int64_t units, int quads, int query_heads, int kv_heads,
@@ -267,28 +309,69 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
     splits = 2 + dartkv_block_of_unit(bh * quads + quads - 1, stream_blocks, units) -
              dartkv_block_of_unit(bh * quads, stream_blocks, units);
   }
-  part_m += row * (total_splits - splits);   // rows are total_splits slots apart, the loops below index row * splits
-  part_l += row * (total_splits - splits);
-  part_acc += row * (total_splits - splits) * D;
-  float m = -INFINITY;
-  for (int s = 0; s < splits; ++s) m = fmaxf(m, part_m[row * splits + s]);
-  float l = 0.0f;
-  for (int s = 0; s < splits; ++s) {
-    float ms = part_m[row * splits + s];
-    if (ms != -INFINITY) l += part_l[row * splits + s] * expf(ms - m);
-  }
-  float inv = 1.0f / fmaxf(l, 1e-20f);
+  part_m += row * total_splits;
+  part_l += row * total_splits;
+  part_acc += row * total_splits * D;
   const int64_t out_row = blockIdx.x;
   const int64_t peer_row = (int64_t)(peers.dst_row_begin + out_row / query_heads) * peers.dst_heads_total +
                            peers.dst_head_begin + out_row % query_heads;
-  for (int c = threadIdx.x; c < D; c += blockDim.x) {
-    float acc = 0.0f;
-    for (int s = 0; s < splits; ++s) {
-      float ms = part_m[row * splits + s];
-      if (ms != -INFINITY) acc += part_acc[(row * splits + s) * D + c] * expf(ms - m);
+  auto deliver = [&](int c, float v) {
+    store_f(out, out_dt, out_row * D + c, v);
+    for (int p = 0; p < peers.world_size; ++p) store_f(peers.out[p], out_dt, peer_row * D + c, v);
+  };
+  const int lane = threadIdx.x & 31;
+  if (splits <= kFewSplits) {
+    // the partials of a channel are requested before the weights are known: one memory latency instead of three
+    for (int c0 = 0; c0 < D; c0 += blockDim.x) {   // every thread takes part in the shuffles
+      const int c = c0 + threadIdx.x;
+      float v[kFewSplits];
+#pragma unroll
+      for (int s = 0; s < kFewSplits; ++s) v[s] = s < splits && c < D ? part_acc[s * D + c] : 0.0f;
+      const float ms = lane < splits ? part_m[lane] : -INFINITY, ls = lane < splits ? part_l[lane] : 0.0f;
+      float m = ms;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      const float w = ms != -INFINITY ? expf(ms - m) : 0.0f;
+      float l = ls * w;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+      float acc = 0.0f;
+#pragma unroll
+      for (int s = 0; s < kFewSplits; ++s) {
+        const float ws = __shfl_sync(0xffffffffu, w, s);
+        if (ws != 0.0f) acc = fmaf(v[s], ws, acc);   // an empty split's sums may be anything
+      }
+      if (c < D) deliver(c, acc * (1.0f / fmaxf(l, 1e-20f)));
     }
-    store_f(out, out_dt, out_row * D + c, acc * inv);
-    for (int p = 0; p < peers.world_size; ++p) store_f(peers.out[p], out_dt, peer_row * D + c, acc * inv);
+  } else {
+    // many splits: warps of equal channels take every `groups`-th split
+    extern __shared__ float s_sum[];   // [groups][D]
+    const int groups = blockDim.x / D, group = threadIdx.x / D, c = threadIdx.x % D;
+    float m = -INFINITY;
+    for (int s = lane; s < splits; s += 32) m = fmaxf(m, part_m[s]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    float l = 0.0f;
+    for (int s = lane; s < splits; s += 32) {
+      const float ms = part_m[s];
+      if (ms != -INFINITY) l += part_l[s] * expf(ms - m);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+    float acc = 0.0f;
+    if (group < groups) {
+#pragma unroll 8
+      for (int s = group; s < splits; s += groups) {
+        const float ms = part_m[s], v = part_acc[s * D + c];
+        if (ms != -INFINITY) acc = fmaf(v, expf(ms - m), acc);
+      }
+      s_sum[group * D + c] = acc;
+    }
+    __syncthreads();
+    if (group == 0) {
+      for (int g = 1; g < groups; ++g) acc += s_sum[g * D + c];
+      deliver(c, acc * (1.0f / fmaxf(l, 1e-20f)));
+    }
   }
   if (peers.world_size > 1) {
     // the block's peer stores are ordered before the barrier; one cumulative system-scope fence after it makes
@@ -374,6 +457,11 @@ extern "C" int dartkv_decode_split_override(const char* spec) {
   return DARTKV_OK;
 }
 
+// Splits of the generic kernel: four blocks per SM where the tokens allow tiles for them.
+static int generic_splits_for(int bh, int tokens) {
+  return min(min(max(1, (148 * 4 + bh - 1) / bh), kMaxGenericSplits), max(1, (tokens + GEN_TILE - 1) / GEN_TILE));
+}
+
 static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens) {
   DecodeLayout L{};
   const int bh = d->batch * d->kv_heads;
@@ -436,9 +524,7 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
       }
     }
   } else {
-    int max_splits = max(1, (tokens + 63) / 64);
-    int want = max(1, (148 * 4 + bh - 1) / bh);
-    L.generic_splits = min(want, max_splits);
+    L.generic_splits = generic_splits_for(bh, tokens);
     int chunk = (tokens + L.generic_splits - 1) / L.generic_splits;
     L.generic_chunk = max(GEN_TILE, (chunk + GEN_TILE - 1) / GEN_TILE * GEN_TILE);
     L.generic_splits = max(1, (tokens + L.generic_chunk - 1) / L.generic_chunk);
@@ -465,11 +551,11 @@ extern "C" int64_t dartkv_decode_workspace_bytes(const dartkv_cache_desc* d, int
     }
   // The generic layout may serve any smaller token count (and is what a tensor-core cache falls back to for other
   // query dtypes).  Its split count is not monotonic in the token count, because the chunk is rounded up to whole
-  // tiles, but it never exceeds min(blocks wanted, tokens / 64 rounded up): rounding the chunk up only lowers it.
+  // tiles, but it never exceeds generic_splits_for(): rounding the chunk up only lowers it.
   {
     const int bh = d->batch * d->kv_heads;
     DecodeLayout L{};
-    L.total_splits = min(max(1, (148 * 4 + bh - 1) / bh), max(1, (max_tokens + 63) / 64));
+    L.total_splits = generic_splits_for(bh, max_tokens);
     best = max(best, layout_bytes(d, query_heads, L));
   }
   return best;
@@ -530,23 +616,26 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
         part_l, part_acc, status, row_start, stream);
     if (rc) return rc;
   } else {
-    size_t smem = ((size_t)rep * D + (size_t)GEN_TILE * (D + 1) + (size_t)rep * GEN_TILE + 3 * rep) * sizeof(float) +
-                  (size_t)D * sizeof(int);
     GenericArgs a;
     a.q = query; a.q_dt = q_dtype; a.query_heads = query_heads; a.flavour = flavour; a.scale = scale;
     a.total_splits = L.total_splits; a.part_m = part_m; a.part_l = part_l; a.part_acc = part_acc;
     a.tok_begin = 0; a.tok_end = -1; a.chunk = L.generic_chunk; a.split_base = 0;
     a.row_start = row_start;
-    if (smem > 48 * 1024)
-      DARTKV_CUDA_OK(cudaFuncSetAttribute(decode_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     DARTKV_REQUIRE(L.generic_splits <= 65535, "too many splits");
-    decode_generic_kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
+    const int padded_rep = rep <= 1 ? 1 : rep <= 2 ? 2 : rep <= 4 ? 4 : rep <= 8 ? 8 : 16;
+    const size_t smem = generic_smem(D, padded_rep);
+    const auto kernel = padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
+                      : padded_rep == 4 ? decode_generic_kernel<4> : padded_rep == 8 ? decode_generic_kernel<8> : decode_generic_kernel<16>;
+    if (smem > 48 * 1024) DARTKV_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
     DARTKV_LAUNCH_OK("decode_generic_kernel");
   }
   {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)((int64_t)d->batch * query_heads));
-    config.blockDim = dim3(128);
+    const bool few = L.total_splits <= kFewSplits;
+    config.blockDim = dim3(few ? min(256, (D + 31) / 32 * 32) : kManyThreads);
+    config.dynamicSmemBytes = few ? 0 : (size_t)(kManyThreads / D) * D * sizeof(float);
     config.stream = stream;
     cudaLaunchAttribute attribute = {};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
