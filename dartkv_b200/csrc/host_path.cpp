@@ -6,7 +6,8 @@
 //
 // Every function answers "not for me" (kSlowPath / None) for anything out of the ordinary -- other devices, odd
 // strides, wrong shapes, pools that have to grow -- before it launches anything; the Python code then takes its
-// full path, which also raises the errors.
+// full path, which also raises the errors.  HANDLE_TH_ERRORS turns a C++ exception (out of memory, a tensor without
+// storage) into a Python one at every entry.
 
 #include <Python.h>
 
@@ -14,6 +15,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/dartkv_b200.h"
@@ -39,6 +41,7 @@ void* stream_of(const at::Tensor& t) { return (void*)c10::cuda::getCurrentCUDASt
 
 // append(keys, values, desc, lifecycle_config, lifecycle_state, plan, nonfinite) -> return code or kSlowPath
 PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 7) { PyErr_SetString(PyExc_TypeError, "append takes 7 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) return PyLong_FromLong(kSlowPath);
   const at::Tensor& k = THPVariable_Unpack(args[0]);
@@ -71,11 +74,13 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                 plan, stream);
   Py_END_ALLOW_THREADS
   return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // decode(query, desc, workspace, workspace_bytes, query_heads, tokens, scale, flavour, row_start | None)
 //   -> output tensor shaped like the query ([B,Hq,D] or [B,Hq,1,D]), a negative return code, or None (slow path)
 PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 9) { PyErr_SetString(PyExc_TypeError, "decode takes 9 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   const at::Tensor& q = THPVariable_Unpack(args[0]);
@@ -114,6 +119,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_END_ALLOW_THREADS
   if (rc != 0) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
 }
 
 at::ScalarType scalar_type(int code) {
@@ -124,6 +130,7 @@ at::ScalarType scalar_type(int code) {
 // Python side, with the descriptor's pointers set; None when the device is not the current one.  Only the state words
 // and the finite-input flag start at zero (one fill for both); everything else is written before it is read.
 PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 4) { PyErr_SetString(PyExc_TypeError, "allocate takes 4 arguments"); return nullptr; }
   auto* d = static_cast<dartkv_cache_desc*>(PyLong_AsVoidPtr(args[0]));
   const long device = PyLong_AsLong(args[1]), pages = PyLong_AsLong(args[2]), rows = PyLong_AsLong(args[3]);
@@ -156,6 +163,7 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
   } catch (const c10::OutOfMemoryError&) {
     Py_RETURN_NONE;   // the Python path allocates the same pools and raises torch's own error
   }
+  END_HANDLE_TH_ERRORS
 }
 
 // Finite-input flag of a synchronous call: one pinned word per thread that the kernels write through its device
@@ -212,6 +220,7 @@ bool dense_here(const at::Tensor& t) { return t.is_contiguous() && on_current_de
 
 // quantize(data, bits, group, axis, metadata dtype code, division, check) -> (values, scale, zero); data contiguous
 PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 7) { PyErr_SetString(PyExc_TypeError, "quantize takes 7 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   const at::Tensor& x = THPVariable_Unpack(args[0]);
@@ -241,11 +250,13 @@ PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int rc = dartkv_quantize(x.data_ptr(), code, outer, len, inner, len * inner, inner, 1, bits, (int)group, md, division,
                                  (uint8_t*)values.data_ptr(), scale.data_ptr(), zero.data_ptr(), flag, stream);
   return finish(tensors({values, scale, zero}), rc, flag, stream);
+  END_HANDLE_TH_ERRORS
 }
 
 // quantize_mixed(keys, group, promoted count, metadata dtype code, indices | None, check)
 //   -> (low, high, indices, scale, zero); keys [B,H,T,D] contiguous, indices int32 contiguous
 PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 6) { PyErr_SetString(PyExc_TypeError, "quantize_mixed takes 6 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   const at::Tensor& k = THPVariable_Unpack(args[0]);
@@ -284,6 +295,7 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
                                  promoted ? (const int32_t*)index.data_ptr() : nullptr, (int)promoted, md, (uint8_t*)low.data_ptr(),
                                  promoted ? (uint8_t*)high.data_ptr() : nullptr, scale.data_ptr(), zero.data_ptr(), flag, stream);
   return finish(tensors({low, high, index, scale, zero}), rc, flag, stream);
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {
