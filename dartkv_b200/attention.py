@@ -32,6 +32,7 @@ def dense_attention(query: torch.Tensor, keys: torch.Tensor, values: torch.Tenso
 def streamed_dart_attention(query: torch.Tensor, cache: DartKVCache, *, scale: Optional[float] = None) -> torch.Tensor:
     """Attend to the packed pages without materializing the cache (reference attention.py:32-87)."""
 
+    from . import _lib
     from .fused_attention import decode_attention
 
     if query.ndim != 4:
@@ -48,10 +49,16 @@ def streamed_dart_attention(query: torch.Tensor, cache: DartKVCache, *, scale: O
         return decode_attention(query[:, :, 0], cache, scale=scale).unsqueeze(2)
     # Several query tokens (no mask between them, like the reference): the tokens of a query head attend to the
     # same KV head, so t tokens x rep query heads are served by ONE launch as t * rep query heads of that KV head.
-    # The tensor-core kernels take up to 4 of them per KV head, the generic kernel up to 16.
+    # One kernel takes 8 to 64 of them per KV head for most packed geometries, the other tensor-core kernels up to 4, the
+    # generic kernel up to 16.  Up to 8 (two passes of the four-row kernels), and on short caches, a token's result is
+    # bit for bit that of a call with this token alone; the many-row kernel adds in another order.
     rep = query.shape[1] // kv_heads
     per_launch = max(1, 16 // rep)
-    if rep <= 4 and _tensor_core_plan(cache, query.dtype, kv_heads * rep * max(1, 4 // rep)):
+    rows = cache.decode_rows_limit(query.dtype, _lib.DEQUANT_PER_OP, cache.seen_tokens)
+    if rep <= rows and rep * tokens > 8:
+        passes = -(-tokens // (rows // rep))
+        per_launch = -(-tokens // passes)
+    elif rep <= 4 and _tensor_core_plan(cache, query.dtype, kv_heads * rep * max(1, 4 // rep)):
         per_launch = max(1, 4 // rep)
     outputs = []
     for first in range(0, tokens, per_launch):

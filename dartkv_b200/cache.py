@@ -144,7 +144,7 @@ class DartKVCache:
         self._device: Optional[torch.device] = None
         self._desc: Optional[CacheDesc] = None
         self._pools: dict = {}
-        self._workspace: Optional[torch.Tensor] = None
+        self._workspaces: dict = {}     # split-K scratch by query heads
         self._page_table_cache: dict = {}
         self._page_run_cache: dict = {}
         self._forced_indices: Optional[torch.Tensor] = None
@@ -155,7 +155,7 @@ class DartKVCache:
         self._c_state = _lib.LifecycleStateC()
         # what the native host path needs of this cache, as plain integers (see _bind_native)
         self._append_args: Optional[tuple] = None
-        self._decode_args: Optional[tuple] = None
+        self._decode_args: dict = {}    # by query heads
 
     def _bind_native(self) -> None:
         """Addresses for the native append path: descriptor, lifecycle structs (their fields change in place, the
@@ -163,7 +163,7 @@ class DartKVCache:
 
         cfg = self.config
         address = ctypes.addressof
-        self._decode_args = None
+        self._decode_args = {}
         self._append_args = None
         if cfg.promote_ratio <= 0.0 or cfg.channel_selection == "magnitude":
             self._append_args = (address(self._desc), address(self._c_cfg), address(self._c_state), address(self._plan),
@@ -278,7 +278,7 @@ class DartKVCache:
         for name in ("k_sink", "v_sink", "k_ring", "v_ring", "k_pages", "v_codes", "v_meta", "page_start",
                      "page_tokens", "state"):
             setattr(d, name, old[name].data_ptr())
-        self._workspace = None
+        self._workspaces = {}
         self._bind_native()
 
     # ------------------------------------------------------------------ append / update
@@ -736,7 +736,7 @@ class DartKVCache:
             for name in ("k_sink", "v_sink", "k_ring", "v_ring", "k_pages", "v_codes", "v_meta", "page_start",
                          "page_tokens", "state"):
                 setattr(self._desc, name, self._pools[name].data_ptr())
-            self._workspace = None
+            self._workspaces = {}
             self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
@@ -765,7 +765,7 @@ class DartKVCache:
                 setattr(self._desc, name, self._pools[name].data_ptr())
         self._desc.batch = int(indices.numel())
         self._shape = (self._desc.batch, self._shape[1], self._shape[2])
-        self._workspace = None
+        self._workspaces = {}
         self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
@@ -809,21 +809,21 @@ class DartKVCache:
         d = self._desc
         capacity = self.config.sink_tokens + max(d.max_value_tokens, d.max_key_pages * self.config.page_size) \
             + d.ring_tokens
-        key = (query_heads, capacity)
-        if self._workspace is None or self._workspace[0] != key:
+        entry = self._workspaces.get(query_heads)
+        if entry is None or entry[0] != capacity:
             nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), query_heads, capacity)
             with device_guard(self._device):
                 buf = torch.empty(max(16, nbytes), dtype=torch.uint8, device=self._device)
                 buf[:16].zero_()        # status word and counters; the partials need no initial value
-            self._workspace = (key, buf)
-        self._decode_args = (ctypes.addressof(d), self._workspace[1].data_ptr(), self._workspace[1].numel(), query_heads)
-        return self._workspace[1], capacity
+            self._workspaces[query_heads] = entry = (capacity, buf)
+            self._decode_args[query_heads] = (ctypes.addressof(d), buf.data_ptr(), buf.numel(), query_heads)
+        return entry[1], capacity
 
     def decode_native(self, query: torch.Tensor, scale: Optional[float], flavour: int, row_start: Optional[torch.Tensor]):
         """One decode call through the native host path: the output shaped like ``query``, or ``None`` when the call
-        is not an ordinary one (first call on this cache, other shapes or devices, wide query groups)."""
+        is not an ordinary one (first call on this cache, other shapes or devices, query groups no kernel takes at once)."""
 
-        args = self._decode_args
+        args = self._decode_args.get(query.shape[1])
         if args is None:
             return None
         out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,
@@ -835,12 +835,20 @@ class DartKVCache:
     def decode_status(self) -> int:
         """0 unless a decode kernel gave up on a bounded wait for an async copy (synchronizes)."""
 
-        if self._workspace is None:
-            return 0
+        worst = 0
         status = ctypes.c_int(0)
-        with device_guard(self._device):
-            check(LIB.dartkv_decode_status(ptr(self._workspace[1]), ctypes.byref(status), stream_ptr(self._device)))
-        return status.value
+        for _, workspace in self._workspaces.values():
+            with device_guard(self._device):
+                check(LIB.dartkv_decode_status(ptr(workspace), ctypes.byref(status), stream_ptr(self._device)))
+            worst = max(worst, status.value)
+        return worst
+
+    def decode_rows_limit(self, dtype: torch.dtype, flavour: int, tokens: int) -> int:
+        """Query rows per KV head that one tensor-core call over `tokens` tokens should take when there are more than four: 8..64,
+        or 0 when no kernel takes more than four."""
+
+        code = _lib.DTYPE_CODE.get(dtype)
+        return 0 if code is None else LIB.dartkv_decode_rows_limit(ctypes.byref(self._desc), code, flavour, tokens)
 
     @property
     def descriptor(self) -> CacheDesc:

@@ -296,7 +296,7 @@ constexpr int kManyThreads = 512;       // block of the merge where a row has mo
 
 __global__ void decode_merge_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
                                     const float* __restrict__ part_acc, int total_splits, int D, void* out, int out_dt,
-                                    int stream_blocks, int64_t units, int quads, int query_heads, int kv_heads,
+                                    int stream_blocks, int64_t units, int quads, int query_heads, int kv_heads, int row_groups,
                                     dartkv_peer_scatter peers, int* status, unsigned int* done_counter) {
   // launched with programmatic stream serialization: the grid may become resident while the kernel before it
   // drains, and waits here until that kernel's memory is visible
@@ -304,8 +304,9 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
   int64_t row = blockIdx.x;
   int splits = total_splits;
   if (stream_blocks > 0) {
-    const int rep = query_heads / kv_heads;
-    const int64_t bh = (row / query_heads) * kv_heads + (row % query_heads) / rep;
+    // the work rows of the split are (batch, KV head, group of the head's query rows)
+    const int rep = query_heads / kv_heads, group_rows = (rep + row_groups - 1) / row_groups, head = (int)(row % query_heads);
+    const int64_t bh = ((row / query_heads) * kv_heads + head / rep) * row_groups + head % rep / group_rows;
     splits = 2 + dartkv_block_of_unit(bh * quads + quads - 1, stream_blocks, units) -
              dartkv_block_of_unit(bh * quads, stream_blocks, units);
   }
@@ -406,6 +407,7 @@ struct DecodeLayout {
   int quads, stream_blocks;            // tensor-core layouts: four-page units per (batch, kv head), stream blocks
   long long units;
   int total_splits;
+  int row_groups;                      // groups of query rows per KV head that are work rows of their own (layout 4)
 };
 
 int dartkv_decode_fast_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
@@ -420,7 +422,12 @@ int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, 
                               cudaStream_t stream);
 
 int dartkv_decode_wide_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
-int dartkv_decode_wide_blocks_per_sm(const dartkv_cache_desc* d);
+int dartkv_decode_wide_blocks_per_sm(const dartkv_cache_desc* d, int q_dtype, int rep, int flavour);
+int dartkv_decode_rows_supported(const dartkv_cache_desc* d, int q_dtype, int rep, int flavour);
+int dartkv_decode_rows_groups(int rep);
+int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int query_heads, float scale, int flavour, int quads,
+                              int stream_blocks, long long units, int total_splits, float* part_m, float* part_l, float* part_acc,
+                              int* status, const int32_t* row_start, cudaStream_t stream);
 int dartkv_decode_wide_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
                               int flavour, int quads, int stream_blocks, long long units, int total_splits,
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
@@ -462,16 +469,29 @@ static int generic_splits_for(int bh, int tokens) {
   return min(min(max(1, (148 * 4 + bh - 1) / bh), kMaxGenericSplits), max(1, (tokens + GEN_TILE - 1) / GEN_TILE));
 }
 
-static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens) {
+// rows_call: the call came through dartkv_decode_attention_rows, the only one that runs more than four query rows per
+// KV head on the tensor cores
+static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens,
+                                  bool rows_call = false) {
   DecodeLayout L{};
-  const int bh = d->batch * d->kv_heads;
-  L.fast = 0;
+  const int rep = query_heads / d->kv_heads;
+  int bh = d->batch * d->kv_heads;
+  L.row_groups = 1;
+  L.fast = rows_call && rep > 4 && dartkv_decode_rows_supported(d, q_dtype, rep, flavour) ? 4 : 0;
+  if (L.fast == 4) {
+    L.row_groups = dartkv_decode_rows_groups(rep);
+    bh *= L.row_groups;   // at most eight
+  }
   if (flavour == DARTKV_DEQUANT_PER_OP && dartkv_decode_fast_supported(d, q_dtype, query_heads)) L.fast = 1;
   if (flavour == DARTKV_DEQUANT_FUSED && dartkv_decode_fused32_supported(d, q_dtype, query_heads)) L.fast = 2;
   // every other packed geometry with 128-token pages and head_dim 128, and the fp32 flavour of all of them
   if (!L.fast && flavour != DARTKV_DEQUANT_FUSED && dartkv_decode_wide_supported(d, q_dtype, query_heads)) L.fast = 3;
   // the tensor-core kernels index (row, four-page unit) pairs with 32 bits
-  if (L.fast && (long long)bh * ((max(1, (tokens - d->sink_tokens) / d->page_size) + 3) / 4) >= (1ll << 31)) L.fast = 0;
+  if (L.fast && (long long)bh * ((max(1, (tokens - d->sink_tokens) / d->page_size) + 3) / 4) >= (1ll << 31)) {
+    L.fast = 0;
+    L.row_groups = 1;
+    bh = d->batch * d->kv_heads;
+  }
   if (L.fast) {
     // One unit = four consecutive pages of a (batch, kv head) (a block hands them to its four warp pairs).  The
     // units of all rows are dealt out evenly to `stream_blocks` blocks.  Two families of splits are compared with a
@@ -485,8 +505,8 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
-    const int resident = (L.fast == 3 ? dartkv_decode_wide_blocks_per_sm(d) : 2) * dartkv_sm_count();
-    const double block_fixed = 1.75, dense_cost = 2.0;
+    const int resident = (L.fast == 3 ? dartkv_decode_wide_blocks_per_sm(d, q_dtype, rep, flavour) : 2) * dartkv_sm_count();
+    const double block_fixed = 1.75, dense_cost = L.fast == 4 ? 4.0 : 2.0;
     int best_pieces = 1;
     double best_cost = 1e30;
     for (int q = max(1, (L.quads + 15) / 16); q <= L.quads; ++q) {
@@ -546,7 +566,7 @@ extern "C" int64_t dartkv_decode_workspace_bytes(const dartkv_cache_desc* d, int
     for (int flavour = 0; flavour < 3; ++flavour) {
       DecodeLayout L = decode_layout(d, dt, query_heads, flavour, max_tokens);
       // the tensor-core layouts use at most 16 stream slots + 1 dense slot per row whatever the token count
-      if (L.fast) L.total_splits = 17;
+      if (L.fast || dartkv_decode_rows_supported(d, dt, query_heads / d->kv_heads, flavour)) L.total_splits = max(L.total_splits, 17);
       best = max(best, layout_bytes(d, query_heads, L));
     }
   // The generic layout may serve any smaller token count (and is what a tensor-core cache falls back to for other
@@ -589,7 +609,7 @@ extern "C" int dartkv_decode_status(const void* workspace, int* status_out, void
 static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads,
                                  float scale, int flavour, int tokens, void* workspace, int64_t workspace_bytes,
                                  void* out, const dartkv_peer_scatter* peers, const int32_t* row_start,
-                                 void* stream_) {
+                                 void* stream_, bool rows_call = false) {
   DARTKV_REQUIRE(d != nullptr, "null descriptor");
   DARTKV_REQUIRE(query && out && workspace, "decode_attention received a null pointer");
   DARTKV_REQUIRE(dartkv_valid_dtype(q_dtype), "query must be f32, f16 or bf16");
@@ -597,10 +617,10 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   DARTKV_REQUIRE(tokens > 0, "cache is empty");
   DARTKV_REQUIRE(flavour >= DARTKV_DEQUANT_PER_OP && flavour <= DARTKV_DEQUANT_FUSED, "unknown dequant flavour %d", flavour);
   const int rep = query_heads / d->kv_heads;
-  DARTKV_REQUIRE(rep <= GEN_MAX_REP, "at most %d query heads per KV head are supported", GEN_MAX_REP);
+  DecodeLayout L = decode_layout(d, q_dtype, query_heads, flavour, tokens, rows_call);
+  DARTKV_REQUIRE(rep <= GEN_MAX_REP || L.fast == 4, "at most %d query heads per KV head are supported", GEN_MAX_REP);
   DARTKV_REQUIRE(d->head_dim <= GEN_MAX_D, "decode attention supports head_dim up to %d", GEN_MAX_D);
   cudaStream_t stream = (cudaStream_t)stream_;
-  DecodeLayout L = decode_layout(d, q_dtype, query_heads, flavour, tokens);
   const int64_t rows = (int64_t)d->batch * query_heads * L.total_splits;
   DARTKV_REQUIRE(workspace_bytes >= layout_bytes(d, query_heads, L), "decode workspace too small: need %lld bytes",
                  (long long)layout_bytes(d, query_heads, L));
@@ -610,7 +630,11 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   float* part_acc = part_l + rows;
   const int bh = d->batch * d->kv_heads;
   const int D = d->head_dim;
-  if (L.fast) {
+  if (L.fast == 4) {
+    int rc = dartkv_decode_rows_launch(d, query, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units, L.total_splits, part_m,
+                                       part_l, part_acc, status, row_start, stream);
+    if (rc) return rc;
+  } else if (L.fast) {
     int rc = (L.fast == 3 ? dartkv_decode_wide_launch : L.fast == 2 ? dartkv_decode_fused32_launch : dartkv_decode_fast_launch)(
         d, query, q_dtype, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units, L.total_splits, part_m,
         part_l, part_acc, status, row_start, stream);
@@ -646,7 +670,7 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     unsigned int* done_counter = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(workspace) + 4);
     DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, decode_merge_kernel, (const float*)part_m, (const float*)part_l,
                                       (const float*)part_acc, L.total_splits, D, out, q_dtype,
-                                      L.fast ? L.stream_blocks : 0, (int64_t)L.units, L.quads, query_heads, d->kv_heads,
+                                      L.fast ? L.stream_blocks : 0, (int64_t)L.units, L.quads, query_heads, d->kv_heads, L.row_groups,
                                       peers ? *peers : none, status, done_counter));
   }
   DARTKV_LAUNCH_OK("decode_merge_kernel");
@@ -666,6 +690,26 @@ extern "C" int dartkv_decode_attention_padded(const dartkv_cache_desc* d, const 
                                               void* out, void* stream) {
   return decode_attention_impl(d, query, q_dtype, query_heads, scale, flavour, tokens, workspace, workspace_bytes, out,
                                nullptr, row_start, stream);
+}
+
+// Below this many tokens passes of four rows stay: they read little twice, and every token's result is bit for bit that
+// of a call with this token alone, which many-row blocks with their own order of sums do not give.
+constexpr int kRowsMinTokens = 1024;
+
+extern "C" int dartkv_decode_rows_limit(const dartkv_cache_desc* d, int q_dtype, int flavour, int tokens) {
+  if (!d || tokens < kRowsMinTokens || !dartkv_decode_rows_supported(d, q_dtype, 64, flavour)) return 0;
+  // as many as keep the partials of a call (17 slots per row) within 64 MiB, in steps of a row group
+  const int64_t row_bytes = 17 * (2 + (int64_t)d->head_dim) * sizeof(float) * d->batch * d->kv_heads;
+  const int64_t fit = ((int64_t)64 << 20) / row_bytes / 8 * 8;
+  return fit < 8 ? 8 : fit > 64 ? 64 : (int)fit;
+}
+
+extern "C" int dartkv_decode_attention_rows(const dartkv_cache_desc* d, const void* query, int q_dtype,
+                                            int query_heads, float scale, int flavour, int tokens,
+                                            const int32_t* row_start, void* workspace, int64_t workspace_bytes,
+                                            void* out, void* stream) {
+  return decode_attention_impl(d, query, q_dtype, query_heads, scale, flavour, tokens, workspace, workspace_bytes, out,
+                               nullptr, row_start, stream, true);
 }
 
 extern "C" int dartkv_decode_attention_scatter(const dartkv_cache_desc* d, const void* query, int q_dtype,

@@ -70,12 +70,13 @@ __device__ __forceinline__ float restore16(float code, float scale, float zero, 
 // (Kitty lifecycle) take one warp per token, four channels per lane, fp32 math.
 // BS: the kernel's block-level shared struct (needs slot_map[128], merge_m / merge_l [kWarps][4])
 // MD: metadata dtype of the packed tokens (the tensor-core kernels for 2-bit pages only take MD = DT)
-template <int DT, int MD = DT, class BS>
-__device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& bs, float* warp_out, int bh) {
+// ROW_GROUPS: the block takes query rows head0 .. head0 + 3 of a KV head that has more than four
+template <int DT, int MD = DT, bool ROW_GROUPS = false, class BS>
+__device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& bs, float* warp_out, int bh, int head0 = 0) {
   using H = Half2Ops<DT>;
   using HM = Half2Ops<MD>;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rep = a.query_heads / d.kv_heads;
+  const int all_rows = a.query_heads / d.kv_heads, rep = ROW_GROUPS ? min(all_rows - head0, 4) : all_rows;
   const int seen = d.state[0], pages = d.state[1], k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
   const int fast_end = fast_range_end(d.sink_tokens, d.page_size, k_end, v_end, sink_filled);
   const int b = bh / d.kv_heads, h = bh % d.kv_heads;
@@ -84,7 +85,7 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      q[r][i] = r < rep ? load_f(a.q, d.dtype, ((int64_t)b * a.query_heads + h * rep + r) * 128 + lane * 4 + i) : 0.0f;
+      q[r][i] = r < rep ? load_f(a.q, d.dtype, ((int64_t)b * a.query_heads + h * all_rows + (ROW_GROUPS ? head0 : 0) + r) * 128 + lane * 4 + i) : 0.0f;
   float m[4], l[4], acc[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -108,7 +109,7 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
 #pragma unroll
     for (int j = 0; j < 2; ++j)
       qb[ks][j] = g < rep ? *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(a.q) +
-                                ((int64_t)b * a.query_heads + h * rep + g) * 128 + 16 * ks + 8 * j + 2 * c)
+                                ((int64_t)b * a.query_heads + h * all_rows + (ROW_GROUPS ? head0 : 0) + g) * 128 + 16 * ks + 8 * j + 2 * c)
                           : 0u;
   int tile_counter = 0;
   float* ptab = warp_out + 4096 + warp * 64;   // this warp's [16 tokens][4 heads] probabilities, beyond the merge buffer
@@ -316,12 +317,12 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 }
 
 // Block merge of the eight warp states: thread = (channel, head parity); partials leave in natural-log units.
-template <class BS>
+template <bool ROW_GROUPS = false, class BS>
 __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, const float* warp_out, int b, int hkv, int rep,
-                                            int slot) {
+                                            int slot, int head0 = 0) {
   const int tid = threadIdx.x;
   const int ch = tid & 127;
-  for (int r = tid >> 7; r < rep; r += kThreads / 128) {
+  for (int r = tid >> 7; r < (ROW_GROUPS ? min(rep - head0, 4) : rep); r += kThreads / 128) {
     float m = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) m = fmaxf(m, bs.merge_m[w][r]);
@@ -335,7 +336,7 @@ __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, con
         acc += warp_out[(w * 4 + r) * 128 + ch] * wgt;
       }
     }
-    const int64_t row = ((int64_t)b * a.query_heads + hkv * rep + r) * a.total_splits + slot;
+    const int64_t row = ((int64_t)b * a.query_heads + hkv * rep + (ROW_GROUPS ? head0 : 0) + r) * a.total_splits + slot;
     if (ch == 0) {
       a.part_m[row] = m == -INFINITY ? -INFINITY : m * 0.6931471805599453f;
       a.part_l[row] = l;

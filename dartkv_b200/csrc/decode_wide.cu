@@ -545,6 +545,12 @@ static WideKernel wide_variant(int dtype, int md, bool fp32) {
 
 }  // namespace
 
+// decode_rows.cu takes the geometries of this file that it can (one key group per page, keys of 2 and 4 bits)
+int dartkv_decode_rows_supported(const dartkv_cache_desc* d, int q_dtype, int rep, int flavour);
+int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int query_heads, float scale, int flavour, int quads,
+                              int stream_blocks, long long units, int total_splits, float* part_m, float* part_l, float* part_acc,
+                              int* status, const int32_t* row_start, cudaStream_t stream);
+
 int dartkv_decode_wide_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads) {
   if (d->head_dim != 128 || d->page_size != 128 || !d->regular_pages) return 0;
   if (d->dtype != DARTKV_F16 && d->dtype != DARTKV_BF16) return 0;
@@ -562,7 +568,8 @@ int dartkv_decode_wide_supported(const dartkv_cache_desc* d, int q_dtype, int qu
 }
 
 // resident blocks per SM (1 or 2): the work split counts on it
-int dartkv_decode_wide_blocks_per_sm(const dartkv_cache_desc* d) {
+int dartkv_decode_wide_blocks_per_sm(const dartkv_cache_desc* d, int q_dtype, int rep, int flavour) {
+  if (dartkv_decode_rows_supported(d, q_dtype, rep, flavour)) return 2;
   return 2 * (wide_smem_bytes(wide_geometry(d)) + 1024) <= 228 * 1024 ? 2 : 1;
 }
 
@@ -570,7 +577,9 @@ int dartkv_decode_wide_launch(const dartkv_cache_desc* d, const void* query, int
                               int flavour, int quads, int stream_blocks, long long units, int total_splits,
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                               cudaStream_t stream) {
-  (void)q_dtype;
+  if (dartkv_decode_rows_supported(d, q_dtype, query_heads / d->kv_heads, flavour))
+    return dartkv_decode_rows_launch(d, query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l,
+                                     part_acc, status, row_start, stream);
   FastArgs a{query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l, part_acc, status,
              row_start};
   const WideGeom w = wide_geometry(d);

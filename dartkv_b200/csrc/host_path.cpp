@@ -96,8 +96,10 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int code = dtype_code(q.scalar_type());
   if ((dims != 3 && dims != 4) || code < 0 || !on_current_device(q) || q.size(0) != desc->batch ||
       q.size(1) != query_heads || q.size(dims - 1) != desc->head_dim || (dims == 4 && q.size(2) != 1) ||
-      query_heads % desc->kv_heads != 0 || query_heads / desc->kv_heads > 4 || tokens < 1)
+      query_heads % desc->kv_heads != 0 || tokens < 1)
     Py_RETURN_NONE;
+  const long rep = query_heads / desc->kv_heads;
+  if (rep > 4 && rep > dartkv_decode_rows_limit(desc, code, (int)flavour, (int)tokens)) Py_RETURN_NONE;
   const int32_t* row_start = nullptr;
   if (args[8] != Py_None) {
     if (!THPVariable_Check(args[8])) Py_RETURN_NONE;
@@ -114,7 +116,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   void* stream = stream_of(q);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = dartkv_decode_attention_padded(desc, qp, code, (int)query_heads, (float)scale, (int)flavour, (int)tokens, row_start,
+  rc = (rep > 4 ? dartkv_decode_attention_rows : dartkv_decode_attention_padded)(desc, qp, code, (int)query_heads, (float)scale, (int)flavour, (int)tokens, row_start,
                                       workspace, workspace_bytes, op, stream);
   Py_END_ALLOW_THREADS
   if (rc != 0) return PyLong_FromLong(rc);

@@ -62,10 +62,11 @@ def decode_attention(query: torch.Tensor, cache: DartKVCache, *, scale: Optional
         if row_start.shape != (batch,):
             raise ValueError("row_start must have shape [batch]")
         row_start = row_start.to(device=q.device, dtype=torch.int32).contiguous()
-    if rep > 4 and peer_gather is None and _grouped_heads_pay_off(cache, q.dtype, kv_heads, flavour, seen):
-        # The tensor-core kernels take up to four query heads per KV head.  Wider groups (5..16 heads per KV head)
-        # are served four heads at a time: every pass streams the packed pages again, which is still far cheaper
-        # than the CUDA-core kernel that would otherwise take the whole group.
+    rows = cache.decode_rows_limit(q.dtype, flavour, seen) if rep > 4 and peer_gather is None else 0
+    if rep > max(4, rows) and peer_gather is None and _grouped_heads_pay_off(cache, q.dtype, kv_heads, flavour, seen):
+        # Most tensor-core kernels take up to four query heads per KV head.  Where none takes the whole group, wider
+        # groups are served four heads at a time: every pass streams the packed pages again, which is still far
+        # cheaper than the CUDA-core kernel that would otherwise take the group.
         grouped = q.view(batch, kv_heads, rep, head_dim)
         result = out if out is not None else torch.empty_like(q)
         result_view = result.view(batch, kv_heads, rep, head_dim)
@@ -86,9 +87,10 @@ def decode_attention(query: torch.Tensor, cache: DartKVCache, *, scale: Optional
                 ctypes.byref(cache.descriptor), ptr(q), _lib.DTYPE_CODE[q.dtype], q.shape[1], float(factor), flavour,
                 seen, ptr(workspace), workspace.numel(), ptr(out), ctypes.byref(peers), stream_ptr(device)))
         return gathered
-    if row_start is not None:
+    if row_start is not None or rep > 4:
         with device_guard(device):
-            check(LIB.dartkv_decode_attention_padded(
+            call = LIB.dartkv_decode_attention_rows if rep > 4 else LIB.dartkv_decode_attention_padded
+            check(call(
                 ctypes.byref(cache.descriptor), ptr(q), _lib.DTYPE_CODE[q.dtype], q.shape[1], float(factor), flavour,
                 seen, ptr(row_start), ptr(workspace), workspace.numel(), ptr(out), stream_ptr(device)))
         return out

@@ -257,6 +257,16 @@ int dartkv_decode_attention_padded(const dartkv_cache_desc* desc, const void* qu
                                    float scale, int flavour, int tokens, const int32_t* row_start, void* workspace,
                                    int64_t workspace_bytes, void* out, void* stream);
 
+/* Decode attention for more than four query rows per KV head in one launch (several query tokens of a head at once,
+ * wide query groups): `query` and `out` are [batch, query_heads, head_dim] with query_heads / kv_heads up to
+ * dartkv_decode_rows_limit(); wider calls and other geometries run as in dartkv_decode_attention_padded. */
+int dartkv_decode_attention_rows(const dartkv_cache_desc* desc, const void* query, int q_dtype, int query_heads,
+                                 float scale, int flavour, int tokens, const int32_t* row_start, void* workspace,
+                                 int64_t workspace_bytes, void* out, void* stream);
+/* Query rows per KV head that one call of dartkv_decode_attention_rows should take at most, 8..64 (its scratch grows
+ * with them); 0 when the geometry is not one it speeds up, or the cache holds few tokens. */
+int dartkv_decode_rows_limit(const dartkv_cache_desc* desc, int q_dtype, int flavour, int tokens);
+
 /* Decode attention for callers that cannot hand over scratch memory.  No counterpart in the
  * reference: this exists for hosts embedding the library where device allocation is off limits at
  * the call site -- a serving loop whose memory pool is sized and frozen at start-up, a plugin
