@@ -481,6 +481,7 @@ template <int DT, int KBITS, int VBITS>
 __global__ void __launch_bounds__(kThreads, 4) append_step_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                   const __grid_constant__ StepArgs a) {
   __shared__ KeySmem sm;
+  follow_previous();
   // read through the pointer where it is needed: the plan's numbers are not kept in registers across the page code
   const dartkv_append_plan& plan = a.device_plan ? *a.device_plan : a.plan;
   // grid: (kv head, batch row, page and role): no division to find any of them
@@ -535,7 +536,7 @@ int launch_step(const dartkv_cache_desc& d, StepArgs a, int blocks, int roles, c
   const int key_bits = d.key_mode == DARTKV_MIXED_PAGE ? 0 : d.key_bits;
   const StepKernel kernel = d.dtype == DARTKV_F16 ? step_variant_k<DARTKV_F16>(key_bits, d.value_bits)
                                                   : step_variant_k<DARTKV_BF16>(key_bits, d.value_bits);
-  kernel<<<dim3(d.kv_heads, d.batch, blocks * roles), kThreads, 0, stream>>>(d, a);
+  DARTKV_CUDA_OK(launch_following(kernel, dim3(d.kv_heads, d.batch, blocks * roles), dim3(kThreads), 0, stream, d, a));
   DARTKV_LAUNCH_OK("append_step_kernel");
   return DARTKV_OK;
 }

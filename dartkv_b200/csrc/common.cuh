@@ -115,4 +115,32 @@ __host__ __device__ __forceinline__ int dartkv_block_of_unit(int64_t x, int bloc
   return (int)j;
 }
 
+// ---------------------------------------------------------------------------- overlapped launches
+// An append of one page or token is a few microseconds of kernel, so the gap before it counts.  It is launched with
+// programmatic stream serialization: the grid is set up while the one before it runs.  follow_previous() is the first
+// statement of such a kernel: it waits until the grids before it have ended and their memory is visible (nothing may be
+// read or written before it), and lets the grid after it be set up once every block of this one has started.
+// B200: [16,8,4096,128] appended 128 tokens at a time 347 -> 328 us, 48 generation steps 1,052 -> 1,026 us, one bulk
+// append 74.6 -> 73.3 us.  The decode kernels are launched plainly: in the same form they were 1-4 % slower.
+__device__ __forceinline__ void follow_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+static inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                           const Args&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
 static inline int dartkv_gcd(int a, int b) { while (b) { int t = a % b; a = b; b = t; } return a; }
