@@ -144,7 +144,10 @@ class DartKVCache:
         self._device: Optional[torch.device] = None
         self._desc: Optional[CacheDesc] = None
         self._pools: dict = {}
-        self._workspaces: dict = {}     # split-K scratch by query heads
+        # split-K scratch: the newest buffer serves every call it is large enough for; outgrown ones stay alive for the
+        # CUDA graphs that hold their address (each at most half of the next one)
+        self._scratch: List[torch.Tensor] = []
+        self._workspaces: dict = {}     # (capacity, buffer) by query heads
         self._page_table_cache: dict = {}
         self._page_run_cache: dict = {}
         self._forced_indices: Optional[torch.Tensor] = None
@@ -278,7 +281,7 @@ class DartKVCache:
         for name in ("k_sink", "v_sink", "k_ring", "v_ring", "k_pages", "v_codes", "v_meta", "page_start",
                      "page_tokens", "state"):
             setattr(d, name, old[name].data_ptr())
-        self._workspaces = {}
+        self._workspaces, self._scratch = {}, []
         self._bind_native()
 
     # ------------------------------------------------------------------ append / update
@@ -736,7 +739,7 @@ class DartKVCache:
             for name in ("k_sink", "v_sink", "k_ring", "v_ring", "k_pages", "v_codes", "v_meta", "page_start",
                          "page_tokens", "state"):
                 setattr(self._desc, name, self._pools[name].data_ptr())
-            self._workspaces = {}
+            self._workspaces, self._scratch = {}, []
             self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
@@ -765,7 +768,7 @@ class DartKVCache:
                 setattr(self._desc, name, self._pools[name].data_ptr())
         self._desc.batch = int(indices.numel())
         self._shape = (self._desc.batch, self._shape[1], self._shape[2])
-        self._workspaces = {}
+        self._workspaces, self._scratch = {}, []
         self._bind_native()
         self._layout_version += 1
         self._invalidate_page_descriptors()
@@ -812,9 +815,12 @@ class DartKVCache:
         entry = self._workspaces.get(query_heads)
         if entry is None or entry[0] != capacity:
             nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), query_heads, capacity)
-            with device_guard(self._device):
-                buf = torch.empty(max(16, nbytes), dtype=torch.uint8, device=self._device)
-                buf[:16].zero_()        # status word and counters; the partials need no initial value
+            if not self._scratch or self._scratch[-1].numel() < nbytes:
+                size = max(16, nbytes, 2 * self._scratch[-1].numel() if self._scratch else 0)
+                with device_guard(self._device):
+                    self._scratch.append(torch.empty(size, dtype=torch.uint8, device=self._device))
+                    self._scratch[-1][:16].zero_()   # status word and counters; the partials need no initial value
+            buf = self._scratch[-1]
             self._workspaces[query_heads] = entry = (capacity, buf)
             self._decode_args[query_heads] = (ctypes.addressof(d), buf.data_ptr(), buf.numel(), query_heads)
         return entry[1], capacity
@@ -837,7 +843,7 @@ class DartKVCache:
 
         worst = 0
         status = ctypes.c_int(0)
-        for _, workspace in self._workspaces.values():
+        for workspace in self._scratch:
             with device_guard(self._device):
                 check(LIB.dartkv_decode_status(ptr(workspace), ctypes.byref(status), stream_ptr(self._device)))
             worst = max(worst, status.value)

@@ -89,3 +89,11 @@ def test_tokens_packed_on_one_side_only():
     cache, oracle = build(torch.float16, torch.float16, 1, 2, 32 + 8 * 128 + 40 + 30, seed=7, bits=4, local_tokens=1,
                           value_local_tokens=128, chunks=[32 + 8 * 128 + 40] + [1] * 30)
     check(cache, oracle, torch.float16, 8, 4)
+
+
+def test_scratch_of_calls_of_many_widths_is_shared():
+    cache, oracle = build(torch.bfloat16, torch.bfloat16, 2, 2, 32 + 8 * 128 + 5, seed=8, promote_ratio=0.25)
+    for queries in (1, 3, 5, 9, 2, 12, 16, 1, 16):
+        check(cache, oracle, torch.bfloat16, 8, queries)
+    largest = cache.decode_workspace(2 * 64)[0].numel()
+    assert sum(buffer.numel() for buffer in cache._scratch) <= 2 * largest
