@@ -161,8 +161,8 @@ class DartKVCache:
         self._decode_args: dict = {}    # by query heads
 
     def _bind_native(self) -> None:
-        """Addresses for the native append path: descriptor, lifecycle structs (their fields change in place, the
-        structs stay where they are) and the finite-input flag."""
+        """What the native append path needs: addresses of the descriptor, of the lifecycle structs (their fields change
+        in place, the structs stay where they are) and of the finite-input flag, and the device these pools are on."""
 
         cfg = self.config
         address = ctypes.addressof
@@ -170,7 +170,7 @@ class DartKVCache:
         self._append_args = None
         if cfg.promote_ratio <= 0.0 or cfg.channel_selection == "magnitude":
             self._append_args = (address(self._desc), address(self._c_cfg), address(self._c_state), address(self._plan),
-                                 self._pools["nonfinite"].data_ptr())
+                                 self._pools["nonfinite"].data_ptr(), self._device.index)
 
     def _set_c_state(self, state) -> None:
         mine = self._c_state
@@ -833,7 +833,7 @@ class DartKVCache:
         if args is None:
             return None
         out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,
-                               flavour, row_start)
+                               flavour, row_start, self._device.index)
         if type(out) is int:
             check(out)
         return out

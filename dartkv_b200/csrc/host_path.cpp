@@ -37,12 +37,18 @@ bool on_current_device(const at::Tensor& t) {
   return t.is_cuda() && t.device().index() == c10::cuda::current_device();
 }
 
+// Device index of the cache's pools: the last argument of append() and decode().  A caller that leaves it out vouches
+// that the tensors are on the cache's device.
+long device_argument(PyObject* const* args, Py_ssize_t n, Py_ssize_t at, const at::Tensor& t) {
+  return n > at ? PyLong_AsLong(args[at]) : (long)t.device().index();
+}
+
 void* stream_of(const at::Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
-// append(keys, values, desc, lifecycle_config, lifecycle_state, plan, nonfinite) -> return code or kSlowPath
+// append(keys, values, desc, lifecycle_config, lifecycle_state, plan, nonfinite[, device]) -> return code or kSlowPath
 PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 7) { PyErr_SetString(PyExc_TypeError, "append takes 7 arguments"); return nullptr; }
+  if (n != 7 && n != 8) { PyErr_SetString(PyExc_TypeError, "append takes 7 or 8 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0]) || !THPVariable_Check(args[1])) return PyLong_FromLong(kSlowPath);
   const at::Tensor& k = THPVariable_Unpack(args[0]);
   const at::Tensor& v = THPVariable_Unpack(args[1]);
@@ -51,9 +57,11 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
   auto* state = static_cast<dartkv_lifecycle_state*>(PyLong_AsVoidPtr(args[4]));
   auto* plan = static_cast<dartkv_append_plan*>(PyLong_AsVoidPtr(args[5]));
   auto* nonfinite = static_cast<int32_t*>(PyLong_AsVoidPtr(args[6]));
+  const long device = device_argument(args, n, 7, k);
   if (PyErr_Occurred()) return nullptr;
   if (k.dim() != 4 || v.dim() != 4 || k.sizes() != v.sizes() || k.scalar_type() != v.scalar_type() ||
-      dtype_code(k.scalar_type()) != desc->dtype || !on_current_device(k) || v.device() != k.device() ||
+      dtype_code(k.scalar_type()) != desc->dtype || !on_current_device(k) || k.device().index() != device ||
+      v.device() != k.device() ||
       k.size(0) != desc->batch || k.size(1) != desc->kv_heads || k.size(3) != desc->head_dim || k.size(2) < 1 ||
       k.size(2) > 32768)
     return PyLong_FromLong(kSlowPath);
@@ -77,11 +85,11 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// decode(query, desc, workspace, workspace_bytes, query_heads, tokens, scale, flavour, row_start | None)
+// decode(query, desc, workspace, workspace_bytes, query_heads, tokens, scale, flavour, row_start | None[, device])
 //   -> output tensor shaped like the query ([B,Hq,D] or [B,Hq,1,D]), a negative return code, or None (slow path)
 PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 9) { PyErr_SetString(PyExc_TypeError, "decode takes 9 arguments"); return nullptr; }
+  if (n != 9 && n != 10) { PyErr_SetString(PyExc_TypeError, "decode takes 9 or 10 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   const at::Tensor& q = THPVariable_Unpack(args[0]);
   auto* desc = static_cast<const dartkv_cache_desc*>(PyLong_AsVoidPtr(args[1]));
@@ -91,11 +99,12 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const long tokens = PyLong_AsLong(args[5]);
   const double scale = PyFloat_AsDouble(args[6]);
   const long flavour = PyLong_AsLong(args[7]);
+  const long device = device_argument(args, n, 9, q);
   if (PyErr_Occurred()) return nullptr;
   const int64_t dims = q.dim();
   const int code = dtype_code(q.scalar_type());
-  if ((dims != 3 && dims != 4) || code < 0 || !on_current_device(q) || q.size(0) != desc->batch ||
-      q.size(1) != query_heads || q.size(dims - 1) != desc->head_dim || (dims == 4 && q.size(2) != 1) ||
+  if ((dims != 3 && dims != 4) || code < 0 || !on_current_device(q) || q.device().index() != device ||
+      q.size(0) != desc->batch || q.size(1) != query_heads || q.size(dims - 1) != desc->head_dim || (dims == 4 && q.size(2) != 1) ||
       query_heads % desc->kv_heads != 0 || tokens < 1)
     Py_RETURN_NONE;
   const long rep = query_heads / desc->kv_heads;

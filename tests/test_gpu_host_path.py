@@ -1,0 +1,47 @@
+"""What the native host path leaves to the Python code, and what it keeps between calls."""
+
+import pytest
+import torch
+
+import dartkv_b200 as dart
+from dartkv_b200 import _lib
+from dartkv_b200.synthetic import make_kvq
+
+pytestmark = pytest.mark.gpu
+
+
+def build(tokens=32 + 3 * 128 + 5, batch=2, heads=2, dtype=torch.bfloat16, seed=1, **cfg):
+    keys, values, _ = make_kvq(seed, batch, heads, tokens + 1, 128, query_heads=heads, dtype=dtype, outlier_fraction=0.05)
+    base = dict(bits=2, page_size=128, key_group_size=128, value_group_size=64, sink_tokens=32, hold_partial_pages=True,
+                promote_ratio=0.25, metadata_dtype=dtype)
+    base.update(cfg)
+    cache = dart.DartKVCache(dart.DartKVCacheConfig(**base))
+    keys, values = keys.cuda(), values.cuda()
+    cache.append(keys[:, :, :tokens], values[:, :, :tokens])
+    return cache, keys[:, :, tokens:], values[:, :, tokens:]
+
+
+def test_tensors_on_another_device_than_the_pools_are_left_to_the_checks():
+    # a second GPU is not needed: the binding is told that the pools are on one
+    cache, keys, values = build()
+    query = torch.randn(2, 8, 1, 128, device="cuda", dtype=torch.bfloat16)
+    dart.fused_dart_attention(query, cache)
+    state = [getattr(cache._c_state, name) for name, _ in cache._c_state._fields_]
+    launches = _lib.LIB.dartkv_launch_count()
+    *addresses, device = cache._append_args
+    assert device == cache._device.index
+    assert _lib.HOST.append(keys, values, *addresses, device + 1) == _lib.HOST.SLOW_PATH
+    arguments = cache._decode_args[8]
+    assert _lib.HOST.decode(query, *arguments, cache.seen_tokens, 0.1, 0, None, device + 1) is None
+    assert [getattr(cache._c_state, name) for name, _ in cache._c_state._fields_] == state
+    # the public calls: the Python checks find the tensors on another device than the cache says
+    cache._device = torch.device("cuda", device + 1)
+    cache._bind_native()
+    cache._decode_args[8] = arguments
+    with pytest.raises(ValueError):
+        cache.append(keys, values)
+    with pytest.raises(ValueError):
+        dart.fused_dart_attention(query, cache)
+    with pytest.raises(ValueError):
+        dart.decode_attention(query[:, :, 0], cache)
+    assert _lib.LIB.dartkv_launch_count() == launches
