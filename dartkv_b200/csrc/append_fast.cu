@@ -237,36 +237,36 @@ __device__ __forceinline__ bool key_page(const dartkv_cache_desc& d, const RowSo
         score_lo = score((float)e_lo);
         score_hi = score((float)e_hi);
       }
-      // Rank by (score descending, channel ascending).  The 128 x 128 comparisons go as 16 squares of 32 channels
-      // against 32 others, two squares per warp, lane = channel, two others per packed comparison; a channel with
-      // the same score counts if it comes first, i.e. against the next smaller number instead of the score.
-      if (tq == 0) sm.score[p] = score_lo | (score_hi << 16);
+      // Rank by (score descending, channel ascending).  Scores are non-negative 16-bit floats, so their bit patterns
+      // order like integers with NaN above everything: each channel has a rank of its own whatever the keys hold.  The
+      // 128 x 128 comparisons go as 16 squares of 32 channels against 32 others, two squares per warp, lane = channel,
+      // two others per subtraction: bit 15 of (other | 0x8000) - than is set where other >= than (than is at most
+      // 0x8000, so the halves do not borrow from each other), and the 2 x 16 bits of a square are counted at once.  A
+      // channel with the same score counts if it comes first, i.e. against the score itself instead of the next number.
+      if (tq == 0) sm.score[p] = score_lo | (score_hi << 16) | 0x80008000u;
       __syncthreads();
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int mine = warp >> 1, others = 2 * (warp & 1) + i;     // blocks of 32 channels
-        const uint32_t bits = reinterpret_cast<const uint16_t*>(sm.score)[32 * mine + lane];
-        const uint32_t above = bits * 0x00010001u, from = (bits == 0 ? 0x8001u : bits - 1u) * 0x00010001u;
-        uint32_t count = 0;
+        const uint32_t bits = reinterpret_cast<const uint16_t*>(sm.score)[32 * mine + lane] & 0x7FFFu;
+        const uint32_t from = bits * 0x00010001u, above = from + 0x00010001u;
+        uint32_t flags = 0;
+        auto compare = [&](uint32_t other, uint32_t than) { flags = (flags >> 1) | ((other - than) & 0x80008000u); };
         const uint4* o4 = reinterpret_cast<const uint4*>(sm.score) + 4 * others;
         if (others != mine) {
           const uint32_t than = others < mine ? from : above;
 #pragma unroll
           for (int r4 = 0; r4 < 4; ++r4) {
             const uint4 o = o4[r4];
-            count = P::count_greater(P::count_greater(count, o.x, than), o.y, than);
-            count = P::count_greater(P::count_greater(count, o.z, than), o.w, than);
+            compare(o.x, than); compare(o.y, than); compare(o.z, than); compare(o.w, than);
           }
         } else {   // others 2r and 2r + 1 of the channel's own block come before it, after it, or on both sides
           const uint32_t both = lane & 1 ? (from & 0xFFFFu) | (above & 0xFFFF0000u) : above;
 #pragma unroll
-          for (int r = 0; r < 16; ++r) {
-            const uint32_t o = sm.score[16 * others + r];
-            count = P::count_greater(count, o, r < lane >> 1 ? from : (r == lane >> 1 ? both : above));
-          }
+          for (int r = 0; r < 16; ++r) compare(sm.score[16 * others + r], r < lane >> 1 ? from : (r == lane >> 1 ? both : above));
         }
-        sm.rank[others][32 * mine + lane] = (int)(P::lo(count) + P::hi(count));
+        sm.rank[others][32 * mine + lane] = __popc(flags);
       }
       __syncthreads();
       int rank_lo, rank_hi;

@@ -62,10 +62,6 @@ template <> struct Pack16<DARTKV_BF16> {
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
-  // count + (1.0 in each half where a > b)
-  static __device__ __forceinline__ uint32_t count_greater(uint32_t count, uint32_t a, uint32_t b) {
-    uint32_t d; asm("set.gt.bf16x2.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return add(count, d);
-  }
   static __device__ __forceinline__ float lo(uint32_t v) { return __uint_as_float(v << 16); }
   static __device__ __forceinline__ float hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
   static __device__ __forceinline__ uint32_t pack(float hi_v, float lo_v) {
@@ -98,9 +94,6 @@ template <> struct Pack16<DARTKV_F16> {
   }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
-  }
-  static __device__ __forceinline__ uint32_t count_greater(uint32_t count, uint32_t a, uint32_t b) {
-    uint32_t d; asm("set.gt.f16x2.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return add(count, d);
   }
   static __device__ __forceinline__ float lo(uint32_t v) { return __half2float(__ushort_as_half((uint16_t)(v & 0xFFFFu))); }
   static __device__ __forceinline__ float hi(uint32_t v) { return __half2float(__ushort_as_half((uint16_t)(v >> 16))); }
