@@ -332,15 +332,17 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
       float m = ms;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-      const float w = ms != -INFINITY ? expf(ms - m) : 0.0f;
-      float l = ls * w;
+      const bool live = ms != -INFINITY;   // the sums of an empty split may be anything
+      const float w = live ? expf(ms - m) : 0.0f;
+      float l = live ? ls * w : 0.0f;
+      const uint32_t lives = __ballot_sync(0xffffffffu, live);
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
       float acc = 0.0f;
 #pragma unroll
       for (int s = 0; s < kFewSplits; ++s) {
         const float ws = __shfl_sync(0xffffffffu, w, s);
-        if (ws != 0.0f) acc = fmaf(v[s], ws, acc);   // an empty split's sums may be anything
+        if ((lives >> s) & 1u) acc = fmaf(v[s], ws, acc);   // Inf and NaN count even where the weight is zero
       }
       if (c < D) deliver(c, acc * (1.0f / fmaxf(l, 1e-20f)));
     }
