@@ -189,14 +189,15 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __gri
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
         const float m_old = s_m[r], m_new = fmaxf(m_old, mx);
-        const float e = expf(v - m_new);
+        const float m_ref = m_new == -INFINITY ? 0.0f : m_new;   // every logit so far -Inf or NaN: the former weigh nothing
+        const float e = expf(v - m_ref);
         float sum = e;
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
         s_p[lane * REP + r] = e;
         __syncwarp();
         if (lane == 0) {
-          const float alpha = expf(m_old - m_new);
+          const float alpha = expf(m_old - m_ref);
           s_alpha[r] = alpha;
           s_m[r] = m_new;
           s_l[r] = s_l[r] * alpha + sum;
@@ -263,7 +264,8 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __gri
   for (int r = 0; r < REP; ++r) {
     if (r < rep) {
       const int64_t row = ((int64_t)b * a.query_heads + h * rep + r) * a.total_splits + slot;
-      if (tid == 0) { a.part_m[row] = s_m[r]; a.part_l[row] = s_l[r]; }
+      // a NaN logit does not show in the maximum: the merge must not take a split of nothing else for an empty one
+      if (tid == 0) { a.part_m[row] = s_l[r] == s_l[r] ? s_m[r] : s_l[r]; a.part_l[row] = s_l[r]; }
       if (vsplit == 0) a.part_acc[row * D + vc] = acc[r];
     }
   }

@@ -22,8 +22,9 @@ def make(dtype, cfg, keys, values):
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("dtype,cfg", CONFIGS)
 def test_a_value_whose_weight_underflows_still_counts(dtype, cfg, bad):
-    # the sink tokens' logits are 0, the others' 12 * sqrt(128): their weight is zero in fp32, and zero * bad is NaN
-    keys, values = torch.ones(1, 2, 32 + 4 * 128 + 3, 128), torch.ones(1, 2, 32 + 4 * 128 + 3, 128)
+    # the sink tokens' logits are 0, the others' 12 * sqrt(128): their weight is zero in fp32, and zero * bad is NaN.
+    # No token follows the full pages, so the sinks are a split of their own under every kernel
+    keys, values = torch.ones(1, 2, 32 + 3 * 128, 128), torch.ones(1, 2, 32 + 3 * 128, 128)
     keys[:, :, :32] = 0
     values[:, 1, 7, 5] = bad
     cache = make(dtype, cfg, keys, values)
@@ -33,3 +34,27 @@ def test_a_value_whose_weight_underflows_still_counts(dtype, cfg, bad):
         assert out[:, 4:, :, 5].isnan().all()
         out[:, 4:, :, 5] = 1.0
         assert torch.allclose(out, torch.ones_like(out), atol=1e-2)
+
+
+@pytest.mark.parametrize("tokens", [[0, 32], [3, 4], [32 + 4 * 128, 32 + 4 * 128 + 3], [32 + 4 * 128 + 2, 32 + 4 * 128 + 3]])
+def test_nan_keys_of_the_cuda_core_kernel(tokens):
+    # dense tokens, wherever the splits are cut: runs of NaN logits only, and single ones
+    gen = torch.Generator().manual_seed(2)
+    keys, values = torch.randn(1, 2, 32 + 4 * 128 + 3, 128, generator=gen), torch.randn(1, 2, 32 + 4 * 128 + 3, 128, generator=gen)
+    keys[:, 1, tokens[0]:tokens[1], 9] = float("nan")
+    cache = make(*CONFIGS[0], keys, values)
+    query = torch.randn(1, 8, 1, 128, generator=gen).cuda()
+    out = dart.fused_dart_attention(query, cache)
+    assert out[:, 4:].isnan().all() and out[:, :4].isfinite().all()
+
+
+def test_infinitely_small_logits_weigh_nothing():
+    gen = torch.Generator().manual_seed(3)
+    keys, values = torch.randn(1, 1, 32 + 2 * 128 + 3, 128, generator=gen), torch.randn(1, 1, 32 + 2 * 128 + 3, 128, generator=gen)
+    query = torch.rand(1, 2, 1, 128, generator=gen).cuda() + 0.5
+    keys[:, :, :32, 4] = float("-inf")      # a whole split
+    keys[:, :, -1, 4] = float("-inf")       # one token of another
+    cache = make(*CONFIGS[0], keys, values)
+    k, v = cache.get()
+    ref = torch.softmax(query.double() @ k.double().transpose(2, 3) * 128 ** -0.5, -1) @ v.double()
+    assert (dart.fused_dart_attention(query, cache).double() - ref).abs().max() < 1e-5
