@@ -47,6 +47,7 @@ __device__ __forceinline__ float inverse_scale(float scale) {
 template <int DT> struct Pack16;
 template <> struct Pack16<DARTKV_BF16> {
   static constexpr uint32_t kMagic = 0x43004300u;   // 128.0 | 128.0
+  static constexpr uint32_t kInfinity = 0x7F807F80u;
   static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b) {
     uint32_t d; asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
@@ -58,6 +59,9 @@ template <> struct Pack16<DARTKV_BF16> {
   }
   static __device__ __forceinline__ uint32_t cap2(uint32_t a, uint32_t b) {   // a NaN becomes the cap
     uint32_t d; asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
+  static __device__ __forceinline__ uint32_t floor2(uint32_t a, uint32_t b) {
+    uint32_t d; asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
@@ -80,6 +84,7 @@ template <> struct Pack16<DARTKV_BF16> {
 };
 template <> struct Pack16<DARTKV_F16> {
   static constexpr uint32_t kMagic = 0x64006400u;   // 1024.0 | 1024.0
+  static constexpr uint32_t kInfinity = 0x7C007C00u;
   static __device__ __forceinline__ uint32_t sub(uint32_t a, uint32_t b) {
     uint32_t d; asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
@@ -91,6 +96,9 @@ template <> struct Pack16<DARTKV_F16> {
   }
   static __device__ __forceinline__ uint32_t cap2(uint32_t a, uint32_t b) {
     uint32_t d; asm("min.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
+  }
+  static __device__ __forceinline__ uint32_t floor2(uint32_t a, uint32_t b) {
+    uint32_t d; asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
   }
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {
     uint32_t d; asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b)); return d;
@@ -110,6 +118,13 @@ template <> struct Pack16<DARTKV_F16> {
   static __device__ __forceinline__ uint16_t bits(float v) { return __half_as_ushort(__float2half_rn(v)); }
 };
 
+
+// whether an element of the pair is Inf or NaN
+template <int DT>
+__device__ __forceinline__ bool pair_nonfinite(uint32_t v) {
+  constexpr uint32_t kUnit = DT == DARTKV_BF16 ? 0x00800080u : 0x04000400u;   // one step of the exponent
+  return ((v & 0x7FFF7FFFu) + kUnit) & 0x80008000u;
+}
 
 // magic exponents in the codes of a pair (none where scalar rint produced them)
 template <int DT, int BITS>

@@ -62,11 +62,24 @@ __global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_cons
   }
   s_mn[split][p] = mn2;
   s_mx[split][p] = mx2;
-  __syncthreads();
-  for (int s = 0; s < splits; ++s) { mn2 = P::min2(mn2, s_mn[s][p]); mx2 = P::max2(mx2, s_mx[s][p]); }
+  const bool odd = pair_nonfinite<DT>(mn2) || pair_nonfinite<DT>(mx2);
+  if (odd && live && a.nonfinite) *a.nonfinite = 1;
+  const bool odd_block = __syncthreads_or(odd);
+  if (odd_block) {   // Inf or NaN in the block's groups: minimum and maximum leave the NaNs out, like quantize.cu
+    mn2 = P::kInfinity; mx2 = P::kInfinity | 0x80008000u;
+    for (int j = 0; j < tok; ++j) {
+      const uint32_t v = at(t_begin + j);
+      mn2 = P::cap2(mn2, v);
+      mx2 = P::floor2(mx2, v);
+    }
+    __syncthreads();
+    s_mn[split][p] = mn2;
+    s_mx[split][p] = mx2;
+    __syncthreads();
+  }
+  for (int s = 0; s < splits; ++s) { mn2 = P::cap2(mn2, s_mn[s][p]); mx2 = P::floor2(mx2, s_mx[s][p]); }
   if (!live) return;
   const float mn_lo = P::lo(mn2), mn_hi = P::hi(mn2), mx_lo = P::lo(mx2), mx_hi = P::hi(mx2);
-  if (a.nonfinite && !(isfinite(mn_lo) && isfinite(mn_hi) && isfinite(mx_lo) && isfinite(mx_hi))) *a.nonfinite = 1;
   const int slot_lo = KB == 0 ? s_slot[2 * p] : -1, slot_hi = KB == 0 ? s_slot[2 * p + 1] : -1;
   const float qmax_lo = KB == 0 ? (slot_lo >= 0 ? 15.0f : 3.0f) : (float)((1 << CODE_BITS) - 1);
   const float qmax_hi = KB == 0 ? (slot_hi >= 0 ? 15.0f : 3.0f) : (float)((1 << CODE_BITS) - 1);
@@ -78,15 +91,36 @@ __global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_cons
     store_f(a.zero, a.md, row * a.groups + g, mn_lo);
     store_f(a.zero, a.md, (row + 1) * a.groups + g, mn_hi);
   }
-  const float inv_lo = inverse_scale(scale_lo), inv_hi = inverse_scale(scale_hi);
-  if (DT == DARTKV_F16) {
-    scale_lo = isinf(scale_lo) ? 0.0f : scale_lo;
-    scale_hi = isinf(scale_hi) ? 0.0f : scale_hi;
-  }
-  const uint32_t cap2 = cap_pair<DT>(qmax_lo, qmax_hi);
   auto word_at = [&](uint8_t* plane, int64_t r, int w) -> uint32_t& {
     return reinterpret_cast<uint32_t*>(plane + r * a.packed_bytes + (int64_t)g * words * 4)[split * mine + w];
   };
+  if (odd_block || isinf(scale_lo) || isinf(scale_hi)) {
+    // element by element: the packed arithmetic would give a NaN quotient (Inf / Inf too) the largest code, not code 0
+    constexpr uint32_t MASK = (1u << PB) - 1u;
+#pragma unroll 1
+    for (int w = 0; w < mine; ++w) {
+      uint32_t low[2] = {0, 0}, high[2] = {0, 0};
+#pragma unroll 1
+      for (int u = 0; u < 2 * PER_HALF; ++u) {
+        const uint32_t v = at(t_begin + w * 2 * PER_HALF + u);
+        const uint32_t code[2] = {group_code(P::lo(v), mn_lo, scale_lo, qmax_lo, DT), group_code(P::hi(v), mn_hi, scale_hi, qmax_hi, DT)};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          low[i] |= (code[i] & MASK) << (PB * u);
+          if (KB == 0) high[i] |= (code[i] >> 2) << (PB * u);
+        }
+      }
+      word_at(a.values, row, w) = low[0];
+      word_at(a.values, row + 1, w) = low[1];
+      if (KB == 0) {
+        if (slot_lo >= 0) word_at(a.high, o * a.promoted + slot_lo, w) = high[0];
+        if (slot_hi >= 0) word_at(a.high, o * a.promoted + slot_hi, w) = high[1];
+      }
+    }
+    return;
+  }
+  const float inv_lo = inverse_scale(scale_lo), inv_hi = inverse_scale(scale_hi);
+  const uint32_t cap2 = cap_pair<DT>(qmax_lo, qmax_hi);
 #pragma unroll 1
   for (int w = 0; w < mine; ++w) {
     uint32_t acc_a[2], acc_b[2];
@@ -179,12 +213,21 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
     mn2 = P::min2(mn2, __shfl_xor_sync(0xffffffffu, mn2, off));
     mx2 = P::max2(mx2, __shfl_xor_sync(0xffffffffu, mx2, off));
   }
+  const bool odd = pair_nonfinite<DT>(mn2) || pair_nonfinite<DT>(mx2), odd_warp = __any_sync(0xffffffffu, odd);
+  if (odd_warp) {   // Inf or NaN in the warp's groups: minimum and maximum leave the NaNs out, like quantize.cu
+    mn2 = P::kInfinity; mx2 = P::kInfinity | 0x80008000u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { mn2 = P::cap2(mn2, v[i]); mx2 = P::floor2(mx2, v[i]); }
+    for (int off = 1; off < lanes; off <<= 1) {
+      mn2 = P::cap2(mn2, __shfl_xor_sync(0xffffffffu, mn2, off));
+      mx2 = P::floor2(mx2, __shfl_xor_sync(0xffffffffu, mx2, off));
+    }
+  }
   if (!live) return;   // groups lie wholly inside or outside
-  const uint32_t mn1 = P::min2(mn2, mn2 >> 16), mx1 = P::max2(mx2, mx2 >> 16);
+  const uint32_t mn1 = P::cap2(mn2, mn2 >> 16), mx1 = P::floor2(mx2, mx2 >> 16);
   const float mn = P::lo(mn1), mx = P::lo(mx1);
   constexpr float qmax = (float)((1 << VB) - 1);
   const float scale = scale_of<DT>(mn, mx, qmax), inv = inverse_scale(scale);
-  const float s_q = DT == DARTKV_F16 && isinf(scale) ? 0.0f : scale;
   const uint32_t mnp = (mn1 & 0xFFFFu) * 0x00010001u, cap2 = cap_pair<DT>(qmax, qmax);
   constexpr int PAIRS = 8 / VB, GATHERS = 4 / PAIRS;     // pairs per gathered 16 bits, gathers per thread
   constexpr uint32_t MAGIC = pair_magic<DT, VB>();
@@ -194,15 +237,26 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
   for (int g = 0; g < GATHERS; ++g) {
     uint32_t acc = 0u - magic_sum(MAGIC, PAIRS, 2 * VB);
 #pragma unroll
-    for (int i = 0; i < PAIRS; ++i) acc = gather(acc, pair_codes<DT, VB>(v[g * PAIRS + i], mnp, s_q, s_q, inv, inv, cap2), 2 * VB * i);
+    for (int i = 0; i < PAIRS; ++i) acc = gather(acc, pair_codes<DT, VB>(v[g * PAIRS + i], mnp, scale, scale, inv, inv, cap2), 2 * VB * i);
     half_word[g] = (acc & LOMASK) | ((acc >> (16 - VB)) & (LOMASK << VB));
+  }
+  if (odd_warp || isinf(scale)) {
+    // element by element: the packed arithmetic gives a NaN quotient (Inf / Inf too) the largest code, not code 0
+    uint64_t codes = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      codes |= (uint64_t)group_code(P::lo(v[i]), mn, scale, qmax, DT) << (2 * i * VB);
+      codes |= (uint64_t)group_code(P::hi(v[i]), mn, scale, qmax, DT) << ((2 * i + 1) * VB);
+    }
+#pragma unroll
+    for (int g = 0; g < GATHERS; ++g) half_word[g] = (uint32_t)(codes >> (16 * g)) & 0xFFFFu;
   }
   if (VB == 2) reinterpret_cast<uint16_t*>(values)[id] = (uint16_t)half_word[0];
   else if (VB == 4) reinterpret_cast<uint32_t*>(values)[id] = half_word[0] | (half_word[GATHERS / 2] << 16);
   else reinterpret_cast<uint2*>(values)[id] = make_uint2(half_word[0] | (half_word[GATHERS > 1] << 16),
                                                          half_word[GATHERS / 2] | (half_word[GATHERS - 1] << 16));
   if (k % lanes == 0) {
-    if (nonfinite && !(isfinite(mn) && isfinite(mx))) *nonfinite = 1;
+    if (nonfinite && odd) *nonfinite = 1;
     const int64_t g = row * (per_row / lanes) + k / lanes;
     store_f(scale_out, md, g, scale);
     store_f(zero_out, md, g, mn);
