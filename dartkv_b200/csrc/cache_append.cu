@@ -126,7 +126,7 @@ __global__ void key_pages_kernel(dartkv_cache_desc d, TokenSource src, int first
       for (int c = threadIdx.x; c < D; c += blockDim.x) {
         float mine = s_score[c];
         int rank = 0;
-        for (int o = 0; o < D; ++o) rank += (s_score[o] > mine) || (s_score[o] == mine && o < c);
+        for (int o = 0; o < D; ++o) rank += ranks_before(s_score[o], o, mine, c);
         if (rank < K) { s_slot[c] = rank; idx_field[rank] = c; }
       }
     }

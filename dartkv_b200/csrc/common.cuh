@@ -84,6 +84,14 @@ __device__ __forceinline__ float group_scale(float mn, float mx, float qmax, int
   return rnd_rt(__fdiv_rn(range, qmax), dt);
 }
 
+// Order of the promoted channels: score descending, channel ascending, NaN above every number like torch.topk has it.
+// A strict order whatever the scores are, so that every channel gets a rank of its own.
+__device__ __forceinline__ bool ranks_before(float score, int channel, float than, int than_channel) {
+  const bool nan = score != score, than_nan = than != than;
+  if (nan || than_nan) return nan && (!than_nan || channel < than_channel);
+  return score > than || (score == than && channel < than_channel);
+}
+
 // code of one element: clamp(rint(rnd(rnd(x - min) / scale)), 0, qmax)
 __device__ __forceinline__ uint32_t group_code(float x, float mn, float scale, float qmax, int dt) {
   float shifted = rnd_rt(__fsub_rn(x, mn), dt);

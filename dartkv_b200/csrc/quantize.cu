@@ -320,7 +320,7 @@ extern "C" int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, in
   return DARTKV_OK;
 }
 
-// rank by (score descending, channel ascending); one block per row
+// rank by (score descending, channel ascending), NaN first; one block per row
 __global__ void select_channels_kernel(const void* __restrict__ scores, int dt, int64_t d, int count,
                                        int32_t* __restrict__ indices) {
   extern __shared__ float s_score[];
@@ -330,10 +330,7 @@ __global__ void select_channels_kernel(const void* __restrict__ scores, int dt, 
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     float mine = s_score[c];
     int rank = 0;
-    for (int o = 0; o < d; ++o) {
-      float other = s_score[o];
-      rank += (other > mine) || (other == mine && o < c);
-    }
+    for (int o = 0; o < d; ++o) rank += ranks_before(s_score[o], o, mine, c);
     if (rank < count) indices[r * count + rank] = c;
   }
 }

@@ -14,8 +14,12 @@ def expected_ranks(keys):
     """[..., T, D] -> channels in rank order, from the score's bit pattern (exact sum, divided and rounded to the dtype)."""
 
     scores = (keys.double().abs().sum(-2).float() / keys.shape[-2]).to(keys.dtype)
-    bits = scores.view(torch.int16).numpy().astype(np.int64)
-    bits[np.isnan(scores.float().numpy())] = 0x7FFF
+    return order(scores)
+
+
+def order(scores):
+    bits = scores.view(torch.int32 if scores.dtype == torch.float32 else torch.int16).numpy().astype(np.int64)
+    bits[scores.isnan().numpy()] = 0x7FFFFFFF
     return np.argsort(-bits, axis=-1, kind="stable")
 
 
@@ -51,3 +55,30 @@ def test_pages_rank_each_channel_once(kind, ratio, dtype):
     assert len(indices) == 2
     for page, got in enumerate(indices):
         assert np.array_equal(got, ranks[:, :, page, :got.shape[-1]])
+
+
+@pytest.mark.parametrize("kind", ["ties", "nan_channel", "nan_row", "some_nan", "inf"])
+def test_general_page_kernel_ranks_each_channel_once(kind):
+    keys = special_keys(kind, torch.float32, 1)[..., :100].contiguous()
+    cache = dart.DartKVCache(dart.DartKVCacheConfig(bits=2, page_size=128, key_group_size=128, value_group_size=50, sink_tokens=0,
+                                                    hold_partial_pages=True, promote_ratio=0.25))
+    cache.append(keys.cuda(), torch.zeros_like(keys).cuda())
+    (key, _), = cache.iter_segments()
+    assert np.array_equal(key.channel_indices.cpu().numpy(), expected_ranks(keys)[..., :key.channel_indices.shape[-1]])
+
+
+@pytest.mark.parametrize("dtype,head_dim", [(torch.float32, 128), (torch.bfloat16, 128), (torch.bfloat16, 130), (torch.float16, 63)])
+@pytest.mark.parametrize("kind", ["ties", "nan_channel", "nan_row", "some_nan", "inf"])
+def test_functional_selection_ranks_each_channel_once(dtype, head_dim, kind):
+    keys = special_keys(kind, dtype, 1)
+    keys = torch.cat([keys, keys[..., :2]], -1)[..., :head_dim].contiguous()
+    ranks = expected_ranks(keys)
+    mask, indices = dart.select_key_channels(keys.cuda(), 0.25)
+    assert np.array_equal(indices.cpu().numpy(), ranks[..., :indices.shape[-1]])
+    assert np.array_equal(mask.sum(-1).cpu().numpy(), np.full((2, 3), indices.shape[-1]))
+    mixed = dart.quantize_key_mixed(keys.cuda(), group_size=128, promote_ratio=0.25, check_finite=False)
+    assert torch.equal(mixed.channel_indices.long(), indices)
+    # the variance of such keys is NaN for whole rows; the oracle of its other scores is elsewhere
+    _, indices = dart.select_key_channels(keys.cuda(), 0.25, strategy="variance")
+    assert indices.min() >= 0 and indices.max() < head_dim
+    assert all(len(set(row.tolist())) == len(row) for row in indices.flatten(0, 1).cpu())
