@@ -624,6 +624,8 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   DecodeLayout L = decode_layout(d, q_dtype, query_heads, flavour, tokens, rows_call);
   DARTKV_REQUIRE(rep <= GEN_MAX_REP || L.fast == 4, "at most %d query heads per KV head are supported", GEN_MAX_REP);
   DARTKV_REQUIRE(d->head_dim <= GEN_MAX_D, "decode attention supports head_dim up to %d", GEN_MAX_D);
+  // the dense-token blocks of the tensor-core kernels read the query two channels at a time
+  DARTKV_REQUIRE(!L.fast || (uintptr_t)query % 4 == 0, "the query must be 4-byte aligned");
   cudaStream_t stream = (cudaStream_t)stream_;
   const int64_t rows = (int64_t)d->batch * query_heads * L.total_splits;
   DARTKV_REQUIRE(workspace_bytes >= layout_bytes(d, query_heads, L), "decode workspace too small: need %lld bytes",

@@ -118,7 +118,10 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
       Py_RETURN_NONE;
     row_start = r.data_ptr<int32_t>();
   }
-  at::Tensor dense = q.is_contiguous() ? at::Tensor() : q.detach().contiguous();
+  // the kernels read the query two channels at a time: a 16-bit view from an odd element on is copied too
+  at::Tensor dense;
+  if (!q.is_contiguous()) dense = q.detach().contiguous();
+  else if ((uintptr_t)q.data_ptr() % 4) dense = q.detach().clone();
   const void* qp = dense.defined() ? dense.data_ptr() : q.data_ptr();
   at::Tensor out = at::empty(q.sizes(), q.options().requires_grad(false).memory_format(at::MemoryFormat::Contiguous));
   void* op = out.data_ptr();

@@ -55,6 +55,8 @@ def decode_attention(query: torch.Tensor, cache: DartKVCache, *, scale: Optional
     if device != cache._device:
         raise ValueError("query and cache must be on the same device")
     q = query.contiguous()
+    if q.data_ptr() % 4:
+        q = q.clone()           # a 16-bit view from an odd element on: the kernels read two channels at a time
     rep = q.shape[1] // kv_heads
     if row_start is not None:
         if peer_gather is not None:

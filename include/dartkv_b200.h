@@ -214,7 +214,8 @@ int dartkv_cache_materialize_both(const dartkv_cache_desc* desc, int32_t t0, int
  * Replaces fused_dart_attention (src/dart/fused_attention.py:654-771) and, numerically,
  * streamed_dart_attention (src/dart/attention.py:32-87): one query token per (batch, query head),
  * GQA by contiguous head groups, split-K over the token range with a cross-split merge.
- * query/out [B,Hq,D] (q_dtype, contiguous).
+ * query/out [B,Hq,D] (q_dtype, contiguous; the query 4-byte aligned where a tensor-core kernel serves the call,
+ * else -1 is returned).
  * workspace: split-K scratch of at least dartkv_decode_workspace_bytes(desc, Hq, max_tokens) bytes
  * for any call with tokens <= max_tokens; zero it once after allocating (its first word is a status
  * word that a kernel sets if a bounded wait on an async copy ran out).

@@ -119,3 +119,16 @@ def test_workspace_bound_covers_every_smaller_token_count(kwargs):
                     info = plan(d, q_dtype, hq, flavour, tokens)
                     worst = max(worst, 16 + batch * hq * info.total_splits * (2 + 128) * 4)
             assert have >= worst, (kwargs, batch, heads, capacity, have, worst)
+
+
+@pytest.mark.parametrize("kwargs,flavour", [(dict(), _lib.DEQUANT_PER_OP), (dict(), _lib.DEQUANT_FUSED), (dict(), _lib.DEQUANT_FP32),
+                                            (dict(value_bits=4, key_bits=4, promoted=0), _lib.DEQUANT_PER_OP)])
+def test_a_query_from_an_odd_element_on_is_refused_before_any_launch(kwargs, flavour):
+    d = make_desc(1, 2, **kwargs)
+    query, workspace, out = 0x20000002, 0x30000000, 0x40000000       # never dereferenced
+    for call, rep in ((LIB.dartkv_decode_attention, 4), (LIB.dartkv_decode_attention_padded, 4), (LIB.dartkv_decode_attention_rows, 8)):
+        if rep > 4 and flavour != _lib.DEQUANT_PER_OP:
+            continue
+        padding = [] if call is LIB.dartkv_decode_attention else [None]
+        args = [ctypes.byref(d), query, _lib.BF16, 2 * rep, 0.1, flavour, 5000, *padding, workspace, 1 << 40, out, None]
+        assert call(*args) == _lib.EINVAL and "aligned" in _lib.last_error()

@@ -45,3 +45,18 @@ def test_tensors_on_another_device_than_the_pools_are_left_to_the_checks():
     with pytest.raises(ValueError):
         dart.decode_attention(query[:, :, 0], cache)
     assert _lib.LIB.dartkv_launch_count() == launches
+
+
+@pytest.mark.parametrize("rep", [1, 4, 5])
+@pytest.mark.parametrize("flavour", [dart.DEQUANT_PER_OP, dart.DEQUANT_FUSED])
+def test_a_query_from_an_odd_element_on(flavour, rep):
+    cache, _, _ = build(tokens=32 + 9 * 128 + 5)
+    query = torch.randn(2, 2 * rep, 1, 128, device="cuda").bfloat16()
+    ref = dart.fused_dart_attention(query, cache, flavour=flavour)
+    odd = torch.empty(query.numel() + 1, device="cuda", dtype=query.dtype)[1:].view(query.shape)
+    odd.copy_(query)
+    assert odd.data_ptr() % 4 == 2
+    for call in range(2):       # the native path, then the Python one
+        if call:
+            cache._decode_args = {}
+        assert torch.equal(dart.fused_dart_attention(odd, cache, flavour=flavour), ref)
