@@ -36,7 +36,8 @@ __device__ void materialize_tokens(const dartkv_cache_desc& d, int bh, int side,
                                    void* out, int out_dt, int* s_slot) {
   const int D = d.head_dim, pairs = (D + 1) / 2, threads = blockDim.x;
   const int sink_filled = d.state[4], packed_end = side == 0 ? d.state[2] : d.state[3];
-  const bool wide = D % 2 == 0;                        // two channels are one aligned store
+  // two channels are one store where the rows and the output (any element-aligned pointer) allow it
+  const bool wide = D % 2 == 0 && (uintptr_t)out % (out_dt == DARTKV_F32 ? 8 : 4) == 0;
   auto put = [&](int t, int c, float a, float b) {
     const int64_t at = (row0 + t) * D + c;
     if (wide && out_dt == DARTKV_F32) reinterpret_cast<float2*>(out)[at / 2] = make_float2(a, b);
