@@ -142,7 +142,8 @@ __device__ void materialize_tokens(const dartkv_cache_desc& d, int bh, int side,
 constexpr int kTileTokens = 32, kTileThreads = 128, kSpan = 128, kSpanThreads = 256;
 
 struct MaterializeArgs {
-  int side0, t0, t1, flavour, out_dt;
+  int side0, t0, t1, flavour, out_dt;   // t0, t1: the tokens of the launch
+  int out_first, out_tokens;            // first token and row count of the output per (batch, head)
   void *out_k, *out_v;
 };
 
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(kTileThreads) materialize_kernel(const __grid_
                                                                    const __grid_constant__ MaterializeArgs a) {
   extern __shared__ int s_slot[];
   const int bh = blockIdx.x, side = a.side0 + blockIdx.z, first = a.t0 + blockIdx.y * kTileTokens;
-  materialize_tokens(d, bh, side, first, min(a.t1, first + kTileTokens), (int64_t)bh * (a.t1 - a.t0) - a.t0, a.flavour,
+  materialize_tokens(d, bh, side, first, min(a.t1, first + kTileTokens), (int64_t)bh * a.out_tokens - a.out_first, a.flavour,
                      side == 0 ? a.out_k : a.out_v, a.out_dt, s_slot);
 }
 
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(kSpanThreads) materialize_spans_kernel(const _
   const int lo = max(a.t0, span_lo), hi = min(a.t1, span_hi);
   if (lo >= hi) return;
   const int packed_hi = span == 0 ? lo : min(hi, max(lo, side == 0 ? d.state[2] : d.state[3]));
-  const int64_t row0 = (int64_t)bh * (a.t1 - a.t0) - a.t0;
+  const int64_t row0 = (int64_t)bh * a.out_tokens - a.out_first;
   uint16_t* out = reinterpret_cast<uint16_t*>(side == 0 ? a.out_k : a.out_v);
   if (lo < packed_hi && side == 1) {
     uint16_t* rows = out + row0 * D;
@@ -287,27 +288,32 @@ bool span_shapes(const dartkv_cache_desc* d, const void* out_k, const void* out_
          (uintptr_t)d->v_codes % 8 == 0;
 }
 
+constexpr int kMaxGridY = 65535;   // spans or tiles of one launch; longer ranges go in pieces
+
 int launch_materialize(const dartkv_cache_desc* d, int side, int sides, int t0, int t1, int flavour, void* out_k, void* out_v,
                        int out_dtype, cudaStream_t stream) {
-  MaterializeArgs a{side, t0, t1, flavour, out_dtype, out_k, out_v};
+  MaterializeArgs a{side, t0, t1, flavour, out_dtype, t0, t1 - t0, out_k, out_v};
   const unsigned bh = d->batch * d->kv_heads;
   const size_t smem = d->head_dim * sizeof(int);
   if (span_shapes(d, out_k, out_v, out_dtype)) {
     auto span_of = [&](int t) { return t < d->sink_tokens ? 0 : 1 + (t - d->sink_tokens) / kSpan; };
-    const int first = span_of(t0), spans = span_of(t1 - 1) - first + 1;
-    DARTKV_REQUIRE(spans <= 65535, "materialize at most %d tokens per call", 65534 * kSpan);
-    const dim3 grid(bh, spans, sides);
-    if (d->md_dtype == DARTKV_F16 && d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-    else if (d->md_dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-    else if (d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_BF16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-    else materialize_spans_kernel<DARTKV_BF16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-    DARTKV_LAUNCH_OK("materialize_spans_kernel");
+    const int end = span_of(t1 - 1) + 1;
+    for (int first = span_of(t0); first < end; first += kMaxGridY) {
+      const dim3 grid(bh, min(end - first, kMaxGridY), sides);
+      if (d->md_dtype == DARTKV_F16 && d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
+      else if (d->md_dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
+      else if (d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_BF16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
+      else materialize_spans_kernel<DARTKV_BF16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
+      DARTKV_LAUNCH_OK("materialize_spans_kernel");
+    }
     return DARTKV_OK;
   }
-  const int tiles = ceil_div(t1 - t0, kTileTokens);
-  DARTKV_REQUIRE(tiles <= 65535, "materialize at most %d tokens per call", 65535 * kTileTokens);
-  materialize_kernel<<<dim3(bh, tiles, sides), kTileThreads, smem, stream>>>(*d, a);
-  DARTKV_LAUNCH_OK("materialize_kernel");
+  for (int64_t first = t0; first < t1; first += (int64_t)kMaxGridY * kTileTokens) {
+    a.t0 = (int)first;
+    a.t1 = (int)min((int64_t)t1, first + (int64_t)kMaxGridY * kTileTokens);
+    materialize_kernel<<<dim3(bh, ceil_div(a.t1 - a.t0, kTileTokens), sides), kTileThreads, smem, stream>>>(*d, a);
+    DARTKV_LAUNCH_OK("materialize_kernel");
+  }
   return DARTKV_OK;
 }
 
