@@ -530,7 +530,7 @@ StepKernel step_variant_k(int key_bits, int value_bits) {
 }
 
 int launch_step(const dartkv_cache_desc& d, StepArgs a, int blocks, int roles, cudaStream_t stream) {
-  DARTKV_REQUIRE(blocks * roles <= 65535, "too many pages in one append (limit 32767)");
+  DARTKV_REQUIRE(blocks * roles <= 65535, "too many pages in one append (limit 65535)");
   DARTKV_REQUIRE(d.batch <= 65535, "batch above 65535");
   a.roles = roles;
   const int key_bits = d.key_mode == DARTKV_MIXED_PAGE ? 0 : d.key_bits;
@@ -570,13 +570,14 @@ static StepArgs step_args(const dartkv_cache_desc* d, const dartkv_append_plan* 
   return a;
 }
 
-// Whether one launch can do the whole step: the value rows are those of the key pages, and no page but the first
-// reads the ring (a local window longer than a page leaves more than a page waiting there).
+// Whether one launch can do the whole step: the value rows are those of the key pages, no page but the first
+// reads the ring (a local window longer than a page leaves more than a page waiting there), and keys and values of all
+// pages fit the grid's 65,535 layers together.
 int dartkv_append_fast_whole_step(const dartkv_append_plan* p) {
   const bool same_rows = p->num_pages == 0 ? p->value_end <= p->value_begin
                                            : p->value_begin == p->page_token_start &&
                                                  p->value_end == p->page_token_start + p->num_pages * kP;
-  return same_rows && (p->num_pages <= 1 || p->page_token_start + kP >= p->chunk_start);
+  return same_rows && p->num_pages <= 65535 / 2 && (p->num_pages <= 1 || p->page_token_start + kP >= p->chunk_start);
 }
 
 int dartkv_append_fast_step(const dartkv_cache_desc* d, const dartkv_append_plan* p, const void* keys, const void* values,

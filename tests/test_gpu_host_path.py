@@ -60,3 +60,23 @@ def test_a_query_from_an_odd_element_on(flavour, rep):
         if call:
             cache._decode_args = {}
         assert torch.equal(dart.fused_dart_attention(odd, cache, flavour=flavour), ref)
+
+
+def test_one_step_of_more_pages_than_a_shared_grid_holds():
+    # the C entry point takes chunks that the Python side would cut: 32,768 pages, each of them the same tokens
+    import ctypes
+
+    pages = 32768
+    gen = torch.Generator().manual_seed(4)
+    keys, values = (torch.randn(1, 1, 1, 128, generator=gen).bfloat16().cuda() for _ in range(2))
+    cache = dart.DartKVCache(dart.DartKVCacheConfig(bits=2, page_size=128, key_group_size=128, value_group_size=64, sink_tokens=0,
+                                                    hold_partial_pages=True, promote_ratio=0.25), max_tokens=(pages + 1) * 128)
+    cache.append(keys.expand(-1, -1, 128, -1), values.expand(-1, -1, 128, -1))
+    _lib.check(_lib.LIB.dartkv_cache_append_step(
+        ctypes.byref(cache.descriptor), ctypes.byref(cache._c_cfg), ctypes.byref(cache._c_state), keys.data_ptr(), values.data_ptr(),
+        pages * 128, 0, 0, 0, None, cache._pools["nonfinite"].data_ptr(), ctypes.byref(cache._plan),
+        torch.cuda.current_stream().cuda_stream))
+    assert cache._pools["state"][:4].tolist() == [(pages + 1) * 128, pages + 1] + [(pages + 1) * 128] * 2
+    for name, rows in (("k_pages", pages + 1), ("v_codes", (pages + 1) * 128), ("v_meta", (pages + 1) * 128)):
+        pool = cache._pools[name][0, 0, :rows].flatten(1)
+        assert torch.equal(pool, pool[:1].expand_as(pool))
