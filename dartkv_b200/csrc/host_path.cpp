@@ -290,12 +290,11 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (index.scalar_type() != at::kInt || !dense_here(index)) Py_RETURN_NONE;
   } else {
     index = at::empty({b, h, count}, options.dtype(at::kInt));
-    at::Tensor scores;
-    // the one-launch selection takes 16-bit keys of an even number of channels up to 128 and needs no score buffer
-    if (code == DARTKV_F32 || d > 128 || d % 2 || (uintptr_t)k.data_ptr() % 4 || b * h > INT32_MAX)
-      scores = at::empty({b, h, d}, options);
-    rc = dartkv_promote_channels(k.data_ptr(), code, b * h, t, d, t * d, d, (int)count,
-                                 scores.defined() ? scores.data_ptr() : index.data_ptr(), (int32_t*)index.data_ptr(), stream);
+    auto promote = [&](void* scores) {
+      return dartkv_promote_channels(k.data_ptr(), code, b * h, t, d, t * d, d, (int)count, scores, (int32_t*)index.data_ptr(), stream);
+    };
+    rc = promote(nullptr);   // enough where one launch does it
+    if (rc == DARTKV_ELIMIT) rc = promote(at::empty({b, h, d}, options).data_ptr());
     if (rc) return PyLong_FromLong(rc);
   }
   const int64_t promoted = index.size(-1);

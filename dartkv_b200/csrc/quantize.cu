@@ -356,10 +356,14 @@ extern "C" int dartkv_promote_channels(const void* keys, int dtype, int64_t bh, 
   DARTKV_REQUIRE(tokens > 0 && head_dim > 0 && head_dim <= 8192, "bad key_states extents");
   DARTKV_REQUIRE(count >= 0 && count <= head_dim, "count must be in [0, head_dim]");
   if (bh == 0 || count == 0) return DARTKV_OK;
-  DARTKV_REQUIRE(keys && scores && indices, "promote_channels received a null pointer");
+  DARTKV_REQUIRE(keys && indices, "promote_channels received a null pointer");
   const int made = dartkv_score_select_fast(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, count, nullptr, indices,
                                             (cudaStream_t)stream);
   if (made) return made > 0 ? DARTKV_OK : made;
+  if (!scores) {
+    dartkv_set_error("promote_channels needs a score buffer for this shape");
+    return DARTKV_ELIMIT;
+  }
   const int rc = dartkv_channel_scores(keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, DARTKV_SCORE_MAGNITUDE, scores, stream);
   return rc ? rc : dartkv_select_channels(scores, dtype, bh, head_dim, count, indices, stream);
 }

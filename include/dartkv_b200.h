@@ -82,8 +82,8 @@ int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, int64_t token
  * scores per row, ordered by (score descending, channel ascending); indices int32 [bh, count]. */
 int dartkv_select_channels(const void* scores, int dtype, int64_t bh, int64_t head_dim, int count,
                            int32_t* indices, void* stream);
-/* Both for the 'magnitude' strategy, in one launch for 16-bit keys of up to 128 channels (scores: scratch of
- * [bh, D] values of `dtype` for the other shapes). */
+/* Both for the 'magnitude' strategy, in one launch for 16-bit keys of up to 128 channels, which needs no scores.  The
+ * other shapes need scratch of [bh, D] values of `dtype` there; with scores == NULL they return -3, nothing launched. */
 int dartkv_promote_channels(const void* keys, int dtype, int64_t bh, int64_t tokens, int64_t head_dim, int64_t stride_bh,
                             int64_t stride_token, int count, void* scores, int32_t* indices, void* stream);
 /* Replaces quantize_key_mixed (src/dart/mixed.py:166-244) for given promoted channels.
