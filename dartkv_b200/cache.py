@@ -144,10 +144,9 @@ class DartKVCache:
         self._device: Optional[torch.device] = None
         self._desc: Optional[CacheDesc] = None
         self._pools: dict = {}
-        # split-K scratch: the newest buffer serves every call it is large enough for; outgrown ones stay alive for the
-        # CUDA graphs that hold their address (each at most half of the next one)
+        # split-K scratch (see decode_workspace); a buffer stays until the pools grow, CUDA graphs hold its address
         self._scratch: List[torch.Tensor] = []
-        self._workspaces: dict = {}     # (capacity, buffer) by query heads
+        self._workspaces: dict = {}     # (capacity, buffer) by (head count of the class, stream)
         self._page_table_cache: dict = {}
         self._page_run_cache: dict = {}
         self._forced_indices: Optional[torch.Tensor] = None
@@ -158,7 +157,7 @@ class DartKVCache:
         self._c_state = _lib.LifecycleStateC()
         # what the native host path needs of this cache, as plain integers (see _bind_native)
         self._append_args: Optional[tuple] = None
-        self._decode_args: dict = {}    # by query heads
+        self._decode_args: dict = {}    # by (query heads, stream)
 
     def _bind_native(self) -> None:
         """What the native append path needs: addresses of the descriptor, of the lifecycle structs (their fields change
@@ -807,29 +806,47 @@ class DartKVCache:
 
     # ------------------------------------------------------------------ attention support
     def decode_workspace(self, query_heads: int) -> Tuple[torch.Tensor, int]:
-        """Split-K scratch for the decode kernel and the token capacity it was sized for."""
+        """Split-K scratch for the decode kernel and the token capacity it was sized for.
+
+        Calls that may overlap on the GPU must not share scratch.  Each stream has its own, and so has each number of
+        query heads per KV head up to four; wider calls on a stream share a buffer up to the next power of two.  A call
+        under graph capture takes scratch that exists (call this method before the capture) and shares it, on every
+        replay, with the stream on which it was made; capturing without any allocates it in the graph's memory.
+        """
 
         d = self._desc
         capacity = self.config.sink_tokens + max(d.max_value_tokens, d.max_key_pages * self.config.page_size) \
             + d.ring_tokens
-        entry = self._workspaces.get(query_heads)
+        rows = -(-query_heads // d.kv_heads)
+        heads = d.kv_heads * (rows if rows <= 4 else 1 << (rows - 1).bit_length())
+        stream = stream_ptr(self._device)
+        entry = self._workspaces.get((heads, stream))
         if entry is None or entry[0] != capacity:
-            nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), query_heads, capacity)
-            if not self._scratch or self._scratch[-1].numel() < nbytes:
-                size = max(16, nbytes, 2 * self._scratch[-1].numel() if self._scratch else 0)
-                with device_guard(self._device):
-                    self._scratch.append(torch.empty(size, dtype=torch.uint8, device=self._device))
-                    self._scratch[-1][:16].zero_()   # status word and counters; the partials need no initial value
-            buf = self._scratch[-1]
-            self._workspaces[query_heads] = entry = (capacity, buf)
-            self._decode_args[query_heads] = (ctypes.addressof(d), buf.data_ptr(), buf.numel(), query_heads)
-        return entry[1], capacity
+            owner = stream
+            if torch.cuda.is_current_stream_capturing():
+                owner = None         # by nobody outside captures: the graph's memory is only filled by a replay
+                made = [e for (h, _), e in self._workspaces.items() if h == heads and e[0] == capacity]
+                if made:
+                    return made[-1][1], capacity
+            nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), heads, capacity)
+            with device_guard(self._device):
+                buf = torch.empty(max(16, nbytes), dtype=torch.uint8, device=self._device)
+                buf[:16].zero_()     # status word and counters; the partials need no initial value
+            self._scratch.append(buf)
+            self._workspaces[heads, owner] = entry = (capacity, buf)
+            if owner is None:
+                return buf, capacity
+        buf = entry[1]
+        self._decode_args[query_heads, stream] = (ctypes.addressof(d), buf.data_ptr(), buf.numel(), query_heads)
+        return buf, capacity
 
     def decode_native(self, query: torch.Tensor, scale: Optional[float], flavour: int, row_start: Optional[torch.Tensor]):
         """One decode call through the native host path: the output shaped like ``query``, or ``None`` when the call
         is not an ordinary one (first call on this cache, other shapes or devices, query groups no kernel takes at once)."""
 
-        args = self._decode_args.get(query.shape[1])
+        if self._desc is None or query.device != self._device:
+            return None
+        args = self._decode_args.get((query.shape[1], stream_ptr(self._device)))
         if args is None:
             return None
         out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,

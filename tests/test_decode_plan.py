@@ -132,3 +132,14 @@ def test_a_query_from_an_odd_element_on_is_refused_before_any_launch(kwargs, fla
         padding = [] if call is LIB.dartkv_decode_attention else [None]
         args = [ctypes.byref(d), query, _lib.BF16, 2 * rep, 0.1, flavour, 5000, *padding, workspace, 1 << 40, out, None]
         assert call(*args) == _lib.EINVAL and "aligned" in _lib.last_error()
+
+
+def test_the_scratch_of_a_class_of_widths_serves_every_width_in_it():
+    # calls of 5..8, 9..16, ... query heads per KV head share the buffer of the widest
+    for kwargs in (dict(), dict(value_bits=4, key_bits=4, promoted=0), dict(value_group=32), dict(dtype=_lib.F32)):
+        for (batch, heads), capacity in itertools.product([(1, 1), (2, 8), (128, 8)], [300, 3000, 40000]):
+            d = make_desc(batch, heads, **kwargs)
+            for low, high in ((5, 8), (9, 16), (17, 32), (33, 64)):
+                most = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), high * heads, capacity)
+                assert all(LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), rep * heads, capacity) <= most
+                           for rep in range(low, high))

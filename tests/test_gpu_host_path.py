@@ -10,12 +10,12 @@ from dartkv_b200.synthetic import make_kvq
 pytestmark = pytest.mark.gpu
 
 
-def build(tokens=32 + 3 * 128 + 5, batch=2, heads=2, dtype=torch.bfloat16, seed=1, **cfg):
+def build(tokens=32 + 3 * 128 + 5, batch=2, heads=2, dtype=torch.bfloat16, seed=1, max_tokens=None, **cfg):
     keys, values, _ = make_kvq(seed, batch, heads, tokens + 1, 128, query_heads=heads, dtype=dtype, outlier_fraction=0.05)
     base = dict(bits=2, page_size=128, key_group_size=128, value_group_size=64, sink_tokens=32, hold_partial_pages=True,
                 promote_ratio=0.25, metadata_dtype=dtype)
     base.update(cfg)
-    cache = dart.DartKVCache(dart.DartKVCacheConfig(**base))
+    cache = dart.DartKVCache(dart.DartKVCacheConfig(**base), max_tokens=max_tokens)
     keys, values = keys.cuda(), values.cuda()
     cache.append(keys[:, :, :tokens], values[:, :, :tokens])
     return cache, keys[:, :, tokens:], values[:, :, tokens:]
@@ -31,13 +31,14 @@ def test_tensors_on_another_device_than_the_pools_are_left_to_the_checks():
     *addresses, device = cache._append_args
     assert device == cache._device.index
     assert _lib.HOST.append(keys, values, *addresses, device + 1) == _lib.HOST.SLOW_PATH
-    arguments = cache._decode_args[8]
+    key = 8, torch.cuda.current_stream().cuda_stream
+    arguments = cache._decode_args[key]
     assert _lib.HOST.decode(query, *arguments, cache.seen_tokens, 0.1, 0, None, device + 1) is None
     assert [getattr(cache._c_state, name) for name, _ in cache._c_state._fields_] == state
     # the public calls: the Python checks find the tensors on another device than the cache says
     cache._device = torch.device("cuda", device + 1)
     cache._bind_native()
-    cache._decode_args[8] = arguments
+    cache._decode_args[key] = arguments
     with pytest.raises(ValueError):
         cache.append(keys, values)
     with pytest.raises(ValueError):
@@ -80,3 +81,52 @@ def test_one_step_of_more_pages_than_a_shared_grid_holds():
     for name, rows in (("k_pages", pages + 1), ("v_codes", (pages + 1) * 128), ("v_meta", (pages + 1) * 128)):
         pool = cache._pools[name][0, 0, :rows].flatten(1)
         assert torch.equal(pool, pool[:1].expand_as(pool))
+
+
+def test_calls_that_may_overlap_have_scratch_of_their_own():
+    cache, _, _ = build(tokens=32 + 9 * 128 + 5)
+    query = torch.randn(2, 2 * 16, 1, 128, device="cuda").bfloat16()
+    reps = (1, 2, 3, 4, 5, 8, 9, 16)
+    ref = {rep: dart.fused_dart_attention(query[:, :2 * rep], cache) for rep in reps}
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    ranges = {}
+    for stream in streams:
+        with torch.cuda.stream(stream):
+            for rep in reps:
+                assert torch.equal(dart.fused_dart_attention(query[:, :2 * rep], cache), ref[rep])
+                buffer = cache.decode_workspace(2 * rep)[0]
+                ranges[min(rep, 4) if rep <= 4 else 8 if rep <= 8 else 16, stream] = (buffer.data_ptr(), buffer.numel())
+                # what the native path is given is that buffer
+                assert cache._decode_args[2 * rep, stream.cuda_stream][1] == buffer.data_ptr()
+    spans = sorted(ranges.values())
+    assert len(spans) == 2 * 6 and all(a + n <= b for (a, n), (b, _) in zip(spans, spans[1:]))
+    held = len(cache._scratch)
+    for _ in range(3):          # nothing is made again
+        for stream in streams:
+            with torch.cuda.stream(stream):
+                dart.fused_dart_attention(query[:, :8], cache)
+    assert len(cache._scratch) == held and cache.decode_status() == 0
+
+
+@pytest.mark.parametrize("before", [True, False])
+def test_captured_calls_take_scratch_that_exists(before):
+    cache, _, _ = build(max_tokens=4096)
+    query = torch.randn(2, 8, 1, 128, device="cuda").bfloat16()
+    other, _, _ = build()
+    ref = dart.fused_dart_attention(query, other)      # kernel attributes are set outside the capture
+    made = cache.decode_workspace(8)[0].data_ptr() if before else None
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        capturing = torch.cuda.current_stream().cuda_stream
+        out = dart.fused_dart_attention(query, cache)
+    assert len(cache._scratch) == 1 and (8, capturing) not in cache._decode_args
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, ref)
+    # an eager call does not take the graph's memory
+    assert torch.equal(dart.fused_dart_attention(query, cache), ref)
+    assert len(cache._scratch) == (1 if before else 2)
+    if before:
+        assert cache._scratch[0].data_ptr() == made
