@@ -830,8 +830,7 @@ class DartKVCache:
                     return made[-1][1], capacity
             nbytes = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), heads, capacity)
             with device_guard(self._device):
-                buf = torch.empty(max(16, nbytes), dtype=torch.uint8, device=self._device)
-                buf[:16].zero_()     # status word and counters; the partials need no initial value
+                buf = _lib.HOST.scratch(max(16, nbytes), self._device.index)
             self._scratch.append(buf)
             self._workspaces[heads, owner] = entry = (capacity, buf)
             if owner is None:
@@ -842,13 +841,21 @@ class DartKVCache:
 
     def decode_native(self, query: torch.Tensor, scale: Optional[float], flavour: int, row_start: Optional[torch.Tensor]):
         """One decode call through the native host path: the output shaped like ``query``, or ``None`` when the call
-        is not an ordinary one (first call on this cache, other shapes or devices, query groups no kernel takes at once)."""
+        is not an ordinary one (other shapes or devices, query groups no kernel takes at once)."""
 
         if self._desc is None or query.device != self._device:
             return None
-        args = self._decode_args.get((query.shape[1], stream_ptr(self._device)))
-        if args is None:
-            return None
+        key = query.shape[1], stream_ptr(self._device)
+        args = self._decode_args.get(key)
+        if args is None:            # the first call of this width on this stream: make its scratch
+            rep, rest = divmod(key[0], self._desc.kv_heads)
+            if rest or rep == 0 or not self._life.seen or (
+                    rep > 4 and rep > self.decode_rows_limit(query.dtype, flavour, self._life.seen)):
+                return None
+            self.decode_workspace(key[0])
+            args = self._decode_args.get(key)
+            if args is None:        # under capture
+                return None
         out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,
                                flavour, row_start, self._device.index)
         if type(out) is int:

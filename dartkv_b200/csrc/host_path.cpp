@@ -180,6 +180,25 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// scratch(bytes, device_index): decode scratch with its first 16 bytes (status word and counters) zero, the rest as it
+// comes; None when the device is not the current one.
+PyObject* scratch(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 2) { PyErr_SetString(PyExc_TypeError, "scratch takes 2 arguments"); return nullptr; }
+  const int64_t bytes = PyLong_AsLongLong(args[0]);
+  const long device = PyLong_AsLong(args[1]);
+  if (PyErr_Occurred()) return nullptr;
+  if (bytes < 16 || device != c10::cuda::current_device()) Py_RETURN_NONE;
+  at::Tensor buffer = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
+  const cudaError_t err = cudaMemsetAsync(buffer.data_ptr(), 0, 16, (cudaStream_t)stream_of(buffer));
+  if (err != cudaSuccess) {
+    PyErr_Format(PyExc_RuntimeError, "CUDA error while clearing decode scratch: %s", cudaGetErrorString(err));
+    return nullptr;
+  }
+  return THPVariable_Wrap(std::move(buffer));
+  END_HANDLE_TH_ERRORS
+}
+
 // Finite-input flag of a synchronous call: one pinned word per thread that the kernels write through its device
 // mapping.  Such a call ends with a wait for its own stream anyway; the word saves the fill kernel before it and the
 // copy after it.
@@ -315,6 +334,7 @@ PyMethodDef methods[] = {
     {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "group-wise quantizer"},
     {"quantize_mixed", (PyCFunction)(void (*)(void))quantize_mixed, METH_FASTCALL, "mixed key quantizer"},
     {"allocate", (PyCFunction)(void (*)(void))allocate, METH_FASTCALL, "the pools of a new cache"},
+    {"scratch", (PyCFunction)(void (*)(void))scratch, METH_FASTCALL, "decode scratch"},
     {"append", (PyCFunction)(void (*)(void))append, METH_FASTCALL, "one append step of a cache"},
     {"decode", (PyCFunction)(void (*)(void))decode, METH_FASTCALL, "one decode attention call on a cache"},
     {nullptr, nullptr, 0, nullptr}};

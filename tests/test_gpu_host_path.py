@@ -130,3 +130,21 @@ def test_captured_calls_take_scratch_that_exists(before):
     assert len(cache._scratch) == (1 if before else 2)
     if before:
         assert cache._scratch[0].data_ptr() == made
+
+
+def test_the_first_call_on_a_cache_is_native():
+    cache, keys, values = build()
+    query = torch.randn(2, 8, 1, 128, device="cuda").bfloat16()
+    for change in (lambda: None, lambda: cache.append(keys, values), lambda: cache.reorder_batch([1, 0]),
+                   lambda: cache._ensure_capacity(2 * cache._desc.max_key_pages, cache._desc.max_value_tokens)):
+        change()
+        launches = _lib.LIB.dartkv_launch_count()
+        first = cache.decode_native(query, None, _lib.DEQUANT_PER_OP, None)
+        assert first is not None and _lib.LIB.dartkv_launch_count() == launches + 2
+        assert torch.equal(cache.decode_native(query, None, _lib.DEQUANT_PER_OP, None), first)
+        assert torch.equal(dart.decode_attention(query[:, :, 0], cache, out=torch.empty_like(first[:, :, 0])), first[:, :, 0])
+    # calls that the Python code refuses or serves otherwise make no scratch
+    made = len(cache._scratch)
+    for odd in (query[:, :7], query[:1], query.cpu(), torch.randn(2, 2 * 40, 1, 128, device="cuda").bfloat16()):
+        assert cache.decode_native(odd, None, _lib.DEQUANT_PER_OP, None) is None
+    assert len(cache._scratch) <= made + 1
