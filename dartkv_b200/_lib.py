@@ -115,7 +115,7 @@ def _load() -> ctypes.CDLL:
     if not os.path.exists(LIB_PATH):
         raise ImportError(
             f"{LIB_PATH} is missing: the CUDA library has not been built. Build it with "
-            "`python -m dartkv_b200.build` (needs nvcc; cross-compiles for sm_100a without a GPU)."
+            "`python dartkv_b200/build.py` (needs nvcc; cross-compiles for sm_100a without a GPU)."
         )
     lib = ctypes.CDLL(LIB_PATH)
     lib.dartkv_last_error.restype = c_char_p
@@ -168,9 +168,12 @@ def _load_host():
     """The per-call host path (``csrc/host_path.cpp``): append and decode without ctypes in between."""
 
     if not os.path.exists(HOST_PATH):
-        raise ImportError(f"{HOST_PATH} is missing: build it with `python -m dartkv_b200.build`")
-    from . import _dartkv_host
-
+        raise ImportError(f"{HOST_PATH} is missing: build it with `python dartkv_b200/build.py`")
+    try:
+        from . import _dartkv_host
+    except ImportError as error:
+        raise ImportError(f"{HOST_PATH} does not load ({error}); if it was built against another torch or Python, run "
+                          "`python dartkv_b200/build.py` again") from error
     return _dartkv_host
 
 

@@ -18,6 +18,7 @@ CSRC = os.path.join(PACKAGE_DIR, "csrc")
 LIB_PATH = os.path.join(PACKAGE_DIR, "libdartkv_b200.so")
 HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
 HOST_PATH = os.path.join(PACKAGE_DIR, "_dartkv_host.so")
+HOST_STAMP = os.path.join(PACKAGE_DIR, "build", "host_path.stamp")   # what the extension was built against
 SOURCES = ("quantize.cu", "quantize_fast.cu", "cache_append.cu", "append_fast.cu", "materialize.cu", "decode_attention.cu", "decode_fast.cu", "decode_fused32.cu",
            "decode_wide.cu", "decode_rows.cu")
 NVCC_FLAGS = (
@@ -42,12 +43,28 @@ def _stale(sources) -> bool:
     return any(os.path.exists(p) and os.path.getmtime(p) > built for p in deps)
 
 
+def _host_abi() -> str:
+    """The C++ side of the installed torch and Python: an extension built against another one must not be loaded."""
+
+    import torch
+
+    return f"torch {torch.__version__} cxx11 {int(torch._C._GLIBCXX_USE_CXX11_ABI)} python {sys.version_info[:2]}"
+
+
+def _host_stale() -> bool:
+    if not (os.path.exists(HOST_PATH) and os.path.exists(HOST_STAMP)):
+        return True
+    header = os.path.join(PACKAGE_DIR, "..", "include", "dartkv_b200.h")
+    if any(os.path.getmtime(p) > os.path.getmtime(HOST_PATH) for p in (HOST_SOURCE, header)):
+        return True
+    with open(HOST_STAMP) as stamp:
+        return stamp.read() != _host_abi()
+
+
 def _start_host_build(force: bool):
     """Start compiling the CPython extension (``None`` when it is up to date)."""
 
-    header = os.path.join(PACKAGE_DIR, "..", "include", "dartkv_b200.h")
-    if not force and os.path.exists(HOST_PATH) and all(
-            os.path.getmtime(p) <= os.path.getmtime(HOST_PATH) for p in (HOST_SOURCE, header)):
+    if not force and not _host_stale():
         return None
     import torch
     from torch.utils import cpp_extension
@@ -71,6 +88,8 @@ def _finish_host_build(proc) -> None:
     subprocess.run(["g++", "-shared", "-o", HOST_PATH, os.path.join(PACKAGE_DIR, "build", "host_path.o"), f"-L{PACKAGE_DIR}",
                     "-ldartkv_b200", "-Wl,-rpath,$ORIGIN", *libraries, "-ltorch_python", "-ltorch", "-ltorch_cpu",
                     "-lc10", "-lc10_cuda", "-lcudart"], check=True)
+    with open(HOST_STAMP, "w") as stamp:
+        stamp.write(_host_abi())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
