@@ -143,3 +143,12 @@ def test_the_scratch_of_a_class_of_widths_serves_every_width_in_it():
                 most = LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), high * heads, capacity)
                 assert all(LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), rep * heads, capacity) <= most
                            for rep in range(low, high))
+
+
+def test_cuda_core_plans_give_every_sm_blocks_where_there_are_tiles():
+    for (batch, heads), tokens in itertools.product([(1, 1), (1, 2), (1, 8), (4, 8), (37, 8)], [31, 1000, 32768, 131072]):
+        info = plan(make_desc(batch, heads, dtype=_lib.F32), _lib.F32, 4 * heads, _lib.DEQUANT_PER_OP, tokens)
+        rows, tiles = batch * heads, -(-tokens // 32)
+        assert info.kernel == 0 and info.total_splits == info.generic_splits <= tiles
+        # rounding a split up to whole tiles costs at most half of the blocks
+        assert rows * info.generic_splits >= min(rows * tiles, 2 * 148)
