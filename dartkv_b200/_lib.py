@@ -29,7 +29,7 @@ EXPORTS = (
     "dartkv_last_error", "dartkv_version", "dartkv_launch_count", "dartkv_pack", "dartkv_unpack", "dartkv_quantize", "dartkv_dequantize",
     "dartkv_channel_scores", "dartkv_select_channels", "dartkv_promote_channels", "dartkv_quantize_key_mixed", "dartkv_dequantize_key_mixed",
     "dartkv_cache_geometry", "dartkv_cache_append", "dartkv_cache_materialize", "dartkv_cache_materialize_both", "dartkv_decode_workspace_bytes",
-    "dartkv_decode_attention", "dartkv_decode_plan", "dartkv_decode_status", "dartkv_builtin_scratch_bytes",
+    "dartkv_decode_attention", "dartkv_decode_plan", "dartkv_decode_plan_rows", "dartkv_decode_status", "dartkv_builtin_scratch_bytes",
     "dartkv_decode_attention_builtin_scratch", "dartkv_shard_range", "dartkv_decode_split_override",
     "dartkv_lifecycle_plan", "dartkv_cache_append_step", "dartkv_decode_attention_scatter",
     "dartkv_decode_attention_padded", "dartkv_decode_attention_rows", "dartkv_decode_rows_limit", "dartkv_cache_append_device_planned",
@@ -145,6 +145,7 @@ def _load() -> ctypes.CDLL:
                                                     POINTER(PeerScatter), p]
     lib.dartkv_decode_status.argtypes = [p, POINTER(c_int), p]
     lib.dartkv_decode_plan.argtypes = [POINTER(CacheDesc), i32, i32, i32, i32, POINTER(DecodePlanInfo)]
+    lib.dartkv_decode_plan_rows.argtypes = lib.dartkv_decode_plan.argtypes
     lib.dartkv_builtin_scratch_bytes.restype = c_int64
     lib.dartkv_decode_split_override.argtypes = [c_char_p]
     lib.dartkv_lifecycle_plan.argtypes = [POINTER(LifecycleConfig), POINTER(LifecycleStateC), i32, POINTER(AppendPlan)]

@@ -586,14 +586,14 @@ extern "C" int64_t dartkv_decode_workspace_bytes(const dartkv_cache_desc* d, int
   return best;
 }
 
-extern "C" int dartkv_decode_plan(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens,
-                                  dartkv_decode_plan_info* out) {
+static int decode_plan_impl(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens, bool rows_call,
+                            dartkv_decode_plan_info* out) {
   DARTKV_REQUIRE(d != nullptr && out != nullptr, "decode_plan received a null pointer");
   DARTKV_REQUIRE(dartkv_valid_dtype(q_dtype), "query must be f32, f16 or bf16");
   DARTKV_REQUIRE(query_heads > 0 && query_heads % d->kv_heads == 0, "query heads must be divisible by cache KV heads");
   DARTKV_REQUIRE(tokens > 0, "cache is empty");
   DARTKV_REQUIRE(flavour >= DARTKV_DEQUANT_PER_OP && flavour <= DARTKV_DEQUANT_FUSED, "unknown dequant flavour %d", flavour);
-  const DecodeLayout L = decode_layout(d, q_dtype, query_heads, flavour, tokens);
+  const DecodeLayout L = decode_layout(d, q_dtype, query_heads, flavour, tokens, rows_call);
   out->kernel = L.fast;
   out->quads = L.fast ? L.quads : 0;
   out->stream_blocks = L.fast ? L.stream_blocks : 0;
@@ -602,6 +602,16 @@ extern "C" int dartkv_decode_plan(const dartkv_cache_desc* d, int q_dtype, int q
   out->generic_splits = L.fast ? 0 : L.generic_splits;
   out->generic_chunk = L.fast ? 0 : L.generic_chunk;
   return DARTKV_OK;
+}
+
+extern "C" int dartkv_decode_plan(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens,
+                                  dartkv_decode_plan_info* out) {
+  return decode_plan_impl(d, q_dtype, query_heads, flavour, tokens, false, out);
+}
+
+extern "C" int dartkv_decode_plan_rows(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens,
+                                       dartkv_decode_plan_info* out) {
+  return decode_plan_impl(d, q_dtype, query_heads, flavour, tokens, true, out);
 }
 
 extern "C" int dartkv_decode_status(const void* workspace, int* status_out, void* stream) {

@@ -227,9 +227,10 @@ int dartkv_decode_attention(const dartkv_cache_desc* desc, const void* query, in
                             void* out, void* stream);
 /* How dartkv_decode_attention would split a call; host arithmetic only, nothing is launched (no counterpart in
  * the reference: it exists so that integrators and tests can see the plan).  kernel: 0 generic, 1 tensor-core
- * per-op flavour (2-bit pages), 2 tensor-core unrounded flavour (2-bit pages), 3 tensor-core kernel for every
- * other packed geometry and the fp32 flavour.  On the tensor-core layouts one unit is four consecutive pages
- * of a (batch, kv head) row; block j of `stream_blocks` owns units [j*units/stream_blocks, (j+1)*units/stream_blocks)
+ * per-op flavour (2-bit pages), 2 tensor-core unrounded flavour (2-bit pages), 3 tensor-core kernels for every
+ * other packed geometry and the fp32 flavour, 4 (dartkv_decode_plan_rows only) tensor-core kernel for more than four
+ * query rows per KV head.  On the tensor-core layouts one unit is four consecutive pages of a row, i.e. of a
+ * (batch, kv head), under kernel 4 of one of the ceil(rows per KV head / 8) groups of its query rows; block j of `stream_blocks` owns units [j*units/stream_blocks, (j+1)*units/stream_blocks)
  * and every row is touched by at most total_splits - 1 of them (plus its dense-token block). */
 typedef struct {
   int32_t kernel;
@@ -242,6 +243,9 @@ typedef struct {
 } dartkv_decode_plan_info;
 int dartkv_decode_plan(const dartkv_cache_desc* desc, int q_dtype, int query_heads, int flavour, int tokens,
                        dartkv_decode_plan_info* out);
+/* The same for dartkv_decode_attention_rows. */
+int dartkv_decode_plan_rows(const dartkv_cache_desc* desc, int q_dtype, int query_heads, int flavour, int tokens,
+                            dartkv_decode_plan_info* out);
 /* Testing / debugging knob (no counterpart in the reference): force the family of work splits of the tensor-core
  * layouts for this process: "aligned", "unaligned", "unaligned:<blocks>", or NULL / "" for the cost model.  The
  * environment variable DARTKV_DECODE_SPLIT gives the initial value (read once).  Not thread-safe. */

@@ -152,3 +152,31 @@ def test_cuda_core_plans_give_every_sm_blocks_where_there_are_tiles():
         assert info.kernel == 0 and info.total_splits == info.generic_splits <= tiles
         # rounding a split up to whole tiles costs at most half of the blocks
         assert rows * info.generic_splits >= min(rows * tiles, 2 * 148)
+
+
+@pytest.mark.parametrize("split", [None, "aligned", "unaligned", "unaligned:7"])
+def test_many_row_plans_stay_inside_their_partial_slots(split, decode_split):
+    decode_split(split)
+    info = DecodePlanInfo()
+    for (batch, heads), tokens in itertools.product([(1, 1), (2, 8), (37, 8), (128, 8)], [1024, 1183, 8192, 32768 + 77, 131072]):
+        d = make_desc(batch, heads)
+        for rep in (5, 7, 8, 9, 16, 17, 20, 31, 33, 49, 57, 64):
+            assert plan(d, _lib.BF16, rep * heads, _lib.DEQUANT_PER_OP, tokens).kernel == 0      # the ordinary entry point
+            check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, rep * heads, _lib.DEQUANT_PER_OP, tokens, ctypes.byref(info)))
+            groups = -(-rep // 8)
+            rows = batch * heads * groups
+            assert info.kernel == 4 and info.quads == ((tokens - 32) // 128 + 3) // 4 and info.units == rows * info.quads
+            assert 1 <= info.stream_blocks <= info.units and 2 <= info.total_splits <= 17
+            sample = range(rows) if rows <= 64 else (0, 1, rows // 3, rows // 2, rows - 2, rows - 1)
+            for row in sample:
+                first = block_of_unit(row * info.quads, info.stream_blocks, info.units)
+                last = block_of_unit(row * info.quads + info.quads - 1, info.stream_blocks, info.units)
+                assert 1 + (last - first + 1) <= info.total_splits
+            need = 16 + batch * rep * heads * info.total_splits * (2 + 128) * 4
+            assert LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), rep * heads, tokens) >= need
+        # up to four rows, and what the many-row kernel does not take, run as through the ordinary entry point
+        for hq, flavour in ((4 * heads, _lib.DEQUANT_PER_OP), (4 * heads, _lib.DEQUANT_FUSED), (8 * heads, _lib.DEQUANT_FUSED),
+                            (8 * heads, _lib.DEQUANT_FP32), (65 * heads, _lib.DEQUANT_PER_OP)):
+            check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, hq, flavour, tokens, ctypes.byref(info)))
+            ordinary = plan(d, _lib.BF16, hq, flavour, tokens)
+            assert bytes(info) == bytes(ordinary)
