@@ -30,6 +30,9 @@ def special_keys(kind, dtype, pages):
         keys = (torch.randint(1, 3, (2, 3, 1, 128), generator=gen) * torch.ones(128 * pages, 1)).to(dtype)
     if kind == "zero":
         keys.zero_()
+    if kind == "wide":          # magnitudes far apart: more bits than a double holds in bf16
+        scale = torch.exp2(torch.randint(-14, 14, keys.shape, generator=gen).float() * (4 if dtype == torch.bfloat16 else 0.5))
+        keys = (keys.float() * scale).to(dtype)
     if kind == "nan_channel":   # one NaN: its channel ranks first
         keys[:, :, 5::128, 77] = float("nan")
     if kind == "nan_row":       # every score NaN
@@ -44,7 +47,7 @@ def special_keys(kind, dtype, pages):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("ratio", [0.25, 0.01, 0.9])
-@pytest.mark.parametrize("kind", ["ties", "zero", "nan_channel", "nan_row", "some_nan", "inf"])
+@pytest.mark.parametrize("kind", ["ties", "zero", "wide", "nan_channel", "nan_row", "some_nan", "inf"])
 def test_pages_rank_each_channel_once(kind, ratio, dtype):
     keys = special_keys(kind, dtype, 2)
     ranks = expected_ranks(keys.unflatten(2, (2, 128)))
@@ -68,7 +71,7 @@ def test_general_page_kernel_ranks_each_channel_once(kind):
 
 
 @pytest.mark.parametrize("dtype,head_dim", [(torch.float32, 128), (torch.bfloat16, 128), (torch.bfloat16, 130), (torch.float16, 63)])
-@pytest.mark.parametrize("kind", ["ties", "nan_channel", "nan_row", "some_nan", "inf"])
+@pytest.mark.parametrize("kind", ["ties", "zero", "wide", "nan_channel", "nan_row", "some_nan", "inf"])
 def test_functional_selection_ranks_each_channel_once(dtype, head_dim, kind):
     keys = special_keys(kind, dtype, 1)
     keys = torch.cat([keys, keys[..., :2]], -1)[..., :head_dim].contiguous()
@@ -78,7 +81,7 @@ def test_functional_selection_ranks_each_channel_once(dtype, head_dim, kind):
     assert np.array_equal(mask.sum(-1).cpu().numpy(), np.full((2, 3), indices.shape[-1]))
     mixed = dart.quantize_key_mixed(keys.cuda(), group_size=128, promote_ratio=0.25, check_finite=False)
     assert torch.equal(mixed.channel_indices.long(), indices)
-    # the variance of such keys is NaN for whole rows; the oracle of its other scores is elsewhere
+    # variance scores of such keys are NaN for whole rows: any order, but every channel once
     _, indices = dart.select_key_channels(keys.cuda(), 0.25, strategy="variance")
     assert indices.min() >= 0 and indices.max() < head_dim
     assert all(len(set(row.tolist())) == len(row) for row in indices.flatten(0, 1).cpu())

@@ -148,3 +148,34 @@ def test_the_first_call_on_a_cache_is_native():
     for odd in (query[:, :7], query[:1], query.cpu(), torch.randn(2, 2 * 40, 1, 128, device="cuda").bfloat16()):
         assert cache.decode_native(odd, None, _lib.DEQUANT_PER_OP, None) is None
     assert len(cache._scratch) <= made + 1
+
+
+LAYOUTS = {"contiguous": lambda t: t.contiguous(), "projection": lambda t: t.transpose(1, 2).contiguous().transpose(1, 2),
+           "wide_rows": lambda t: torch.cat([t, t], -1)[..., :128], "every_other": lambda t: torch.stack([t, -t], -1)[..., 0],
+           "same_batch": lambda t: t[:1].contiguous().expand(t.shape[0], -1, -1, -1),
+           "odd_start": lambda t: torch.cat([t.new_zeros(3), t.flatten()])[3:].view(t.shape)}
+
+
+@pytest.mark.parametrize("keys_as", sorted(LAYOUTS))
+@pytest.mark.parametrize("values_as", sorted(LAYOUTS))
+def test_layouts_of_keys_and_values(keys_as, values_as):
+    # whatever the strides of the two tensors, the pools get the bytes of contiguous ones
+    gen = torch.Generator().manual_seed(6)
+    base = torch.randn(2, 2, 2, 32 + 3 * 128 + 41, 128, generator=gen).bfloat16().cuda()
+    base[:, 1] = base[:, :1].squeeze(1) if "same_batch" in (keys_as, values_as) else base[:, 1]
+    caches = [dart.DartKVCache(dart.DartKVCacheConfig(bits=2, page_size=128, key_group_size=128, value_group_size=64, sink_tokens=32,
+                                                      hold_partial_pages=True, promote_ratio=0.25, metadata_dtype=torch.bfloat16))
+              for _ in range(2)]
+    start = 0
+    for chunk in (300, 1, 1, 40, 1, 114):
+        keys, values = base[0, :, :, start:start + chunk], base[1, :, :, start:start + chunk]
+        caches[0].append(keys.contiguous(), values.contiguous())
+        caches[1].append(LAYOUTS[keys_as](keys), LAYOUTS[values_as](values))
+        start += chunk
+    assert start == base.shape[3]
+    for (k0, v0), (k1, v1) in zip(*(cache.iter_segments() for cache in caches)):
+        for a, b in ((k0, k1), (v0, v1)):
+            names = ("values", "low_values", "high_values", "channel_indices", "scale", "zero_point")
+            fields = [("", a, b)] if isinstance(a, torch.Tensor) else [(n, getattr(a, n), getattr(b, n)) for n in names if hasattr(a, n)]
+            for name, x, y in fields:
+                assert torch.equal(x, y), name
