@@ -33,20 +33,7 @@
 
 namespace {
 
-// timing experiments only (a library built with these computes garbage)
-#if defined(PEROP_SKIP_MMA)
-#define PEROP_MMA(acc, a0, a1, a2, a3, b0, b1) ((acc)[0] += __uint_as_float((a0) ^ (a1) ^ (a2) ^ (a3) ^ (b0) ^ (b1)))
-#else
-#define PEROP_MMA(acc, a0, a1, a2, a3, b0, b1) HO::mma(acc, a0, a1, a2, a3, b0, b1)
-#endif
-
-#ifndef PEROP_QK_UNROLL
-#define PEROP_QK_UNROLL 8
-#endif
-#ifndef PEROP_PV_UNROLL
-#define PEROP_PV_UNROLL 4
-#endif
-constexpr int kQkUnroll = PEROP_QK_UNROLL, kPvUnroll = PEROP_PV_UNROLL;
+constexpr int kQkUnroll = 8, kPvUnroll = 4;
 
 struct PairSmem {
   uint8_t stage[2][kStageBytes];
@@ -99,7 +86,6 @@ __device__ __forceinline__ void page_half(const int HF, const int pair, const in
   for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
     for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
-#if !defined(PEROP_SKIP_QK)
   const int my_prom_steps = (prom_steps + 1 - HF) >> 1;   // promoted steps with the parity of this warp
   for (int i = 0; i < my_prom_steps; ++i) {
     const int s0 = 8 * (2 * i + HF) + c, s1 = s0 + 4;
@@ -118,18 +104,13 @@ __device__ __forceinline__ void page_half(const int HF, const int pair, const in
     const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_thread + o0.y);
     const uint32_t b1 = *reinterpret_cast<const uint32_t*>(q_thread + o1.y);
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) PEROP_MMA(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+    for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
   }
 #pragma unroll kQkUnroll
   for (int i = my_prom_steps; i < 8; ++i) {
     const int s0 = 8 * (2 * i + HF) + c, s1 = s0 + 4;
-#if defined(PEROP_SKIP_KPAR)
-    const uint4 a0 = make_uint4(cc.mask[0], cc.mask[1], cc.magic[0], cc.magic[1]), a1 = a0;
-    const uint2 o0 = make_uint2(cc.magic[2], 32u * s0), o1 = make_uint2(cc.magic[2], 32u * s1);
-#else
     const uint4 a0 = ps.kpar_a[s0], a1 = ps.kpar_a[s1];
     const uint2 o0 = ps.kpar_b[s0], o1 = ps.kpar_b[s1];
-#endif
     const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0.y);
     const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1.y);
     uint32_t r0[8], r1[8];
@@ -140,9 +121,8 @@ __device__ __forceinline__ void page_half(const int HF, const int pair, const in
     const uint32_t b0 = *reinterpret_cast<const uint32_t*>(q_thread + o0.y);
     const uint32_t b1 = *reinterpret_cast<const uint32_t*>(q_thread + o1.y);
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) PEROP_MMA(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+    for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
   }
-#endif   // PEROP_SKIP_QK
 
   // ---- exchange: this warp goes on with the tokens of m-tiles 2HF and 2HF+1 (codes 4HF .. 4HF+3 of every packed
   // half-word), so it hands its partial logits of the other two m-tiles to its partner and takes the partner's
@@ -262,7 +242,6 @@ __device__ __forceinline__ void page_half(const int HF, const int pair, const in
     cast_registers<DT, OUT>(r_lo);
     cast_registers<DT, OUT>(r_hi);
   };
-#if !defined(PEROP_SKIP_PV)
 #pragma unroll kPvUnroll
   for (int s = 0; s < 4; ++s) {
     uint32_t r0_lo[8], r0_hi[8], r1_lo[8], r1_hi[8];
@@ -270,9 +249,8 @@ __device__ __forceinline__ void page_half(const int HF, const int pair, const in
     token_pair(32 * s + tok_a + 16, r1_lo, r1_hi);     // local tokens 16s + 2c + 8, 16s + 2c + 9: a + 16, a + 24
     const uint32_t b0 = pb[8 * s], b1 = pb[8 * s + 4];
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt) PEROP_MMA(o_acc[mt], r0_lo[mt], r0_hi[mt], r1_lo[mt], r1_hi[mt], b0, b1);
+    for (int mt = 0; mt < 8; ++mt) HO::mma(o_acc[mt], r0_lo[mt], r0_hi[mt], r1_lo[mt], r1_hi[mt], b0, b1);
   }
-#endif   // PEROP_SKIP_PV
 }
 
 // GN: value groups per token (1 or 2).  KP: promoted channels per page when that is a multiple of eight known to
@@ -386,7 +364,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
       // ---- per-page setup: each warp orders the channels (promoted slots first) into its own copy, then
       // fills the per-position constants of the contraction steps it owns (steps 2i + hf); nothing of this is
       // shared with the other warp of the pair
-#if !defined(PEROP_SKIP_SETUP)
       {
         uint8_t* order = ps.order[hf];
         uint8_t* flag = ps.is_promoted[hf];
@@ -425,7 +402,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
           ps.kpar_b[p] = make_uint2(H::mul(ss, H::neg_magic(2)), 32u * ch);
         }
       }
-#endif
       __syncwarp();
 
       page_half<DT, OUT, GN, KP>(hf, pair, lane, d, ps, blob, ps.prob[hf], ps.prob[hf ^ 1], q_thread, cc, K, prom_steps, scale2, g, c, jp,

@@ -115,9 +115,6 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
   float* ptab = warp_out + 4096 + warp * 64;   // this warp's [16 tokens][4 heads] probabilities, beyond the merge buffer
   // segments: [0, sink_filled) then [fast_end, seen) cut at key page boundaries
   int t = a.row_start ? min(max(a.row_start[b], 0), seen) : 0;
-#ifdef DENSE_SKIP
-  t = seen;
-#endif
   while (t < seen) {
     if (t >= sink_filled && t < fast_end) { t = fast_end; continue; }
     int seg_end, kind;

@@ -28,14 +28,7 @@
 
 namespace {
 
-#ifndef FUSED_QK_UNROLL
-#define FUSED_QK_UNROLL 16
-#endif
-#ifndef FUSED_PV_UNROLL
-#define FUSED_PV_UNROLL 4
-#endif
-
-constexpr int kQkUnroll = FUSED_QK_UNROLL, kPvUnroll = FUSED_PV_UNROLL;
+constexpr int kQkUnroll = 16, kPvUnroll = 4;
 constexpr int kUStride = 36;   // 32-bit words per group of 8 local tokens in a warp's weight table (4 pad)
 
 struct FusedPairSmem {
@@ -121,7 +114,6 @@ __device__ __forceinline__ void fused_page_half(const int HF, const int tb, cons
   {
     const uint8_t* low_thread = blob + 4 * g + 32 * c;                               // + 256 * step (+128)
     const uint8_t* w_thread = reinterpret_cast<const uint8_t*>(ps.w_low[tb]) + 8 * c + 4 * (g >> 2);   // + 64 * step (+32)
-#ifndef FUSED_SKIP_QK
 #pragma unroll kQkUnroll
     for (int ks = 0; ks < 16; ++ks) {
       uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + 256 * ks);
@@ -154,7 +146,6 @@ __device__ __forceinline__ void fused_page_half(const int HF, const int tb, cons
         mma_f16(s_odd[mt], a0, a1, a2, a3, l0, l1);   // same codes against the dropped part of the weights
       }
     }
-#endif
   }
 
   // ---- online softmax for head c over this warp's 64 tokens (this thread: 8 of them)
@@ -270,7 +261,6 @@ __device__ __forceinline__ void fused_page_half(const int HF, const int tb, cons
     const uint32_t sel_v = (g >> 2) ? 0x7632u : 0x5410u;
     const uint8_t* vthread = blob + kOffVCodes + 32 * (4 * HF + c) + 4 * wi;   // + 512 * ks (+256 for the second token)
     const uint32_t* uthread = utab + c * 4 + (g >> 1);                         // + kUStride * ks (+16 for the second)
-#ifndef FUSED_SKIP_PV
 #pragma unroll kPvUnroll
     for (int ks = 0; ks < 8; ++ks) {
       const uint32_t x0 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 512 * ks),
@@ -285,7 +275,6 @@ __device__ __forceinline__ void fused_page_half(const int HF, const int tb, cons
       mma_f16(st.o_acc[2], x0 & 0x03000300u, y0 & 0x00030003u, x1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
       mma_f16(st.o_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u, b0, b1);
     }
-#endif
   }
 }
 
@@ -411,7 +400,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
 
       // ---- per-page setup by the 64 threads of the pair: thread tp owns channels 2tp, 2tp+1
       float f = 1.0f, f_inv = 1.0f;
-#ifndef FUSED_SKIP_SETUP
       {
         const uint32_t* kscale2 = reinterpret_cast<const uint32_t*>(blob + d.key_off_scale);
         const uint32_t* kzero2 = reinterpret_cast<const uint32_t*>(blob + d.key_off_zero);
@@ -461,7 +449,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
           ps.w_high_lo[stage][lane] = wl;
         }
       }
-#endif
       // the only meeting point of the pair per page: the tables of this page are complete and both warps are done
       // with the page before, whose stage can take the page after this one
       pair_barrier(pair);
