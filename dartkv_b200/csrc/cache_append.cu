@@ -90,8 +90,8 @@ __global__ void copy_dense_kernel(dartkv_cache_desc d, dartkv_append_plan p, con
 __global__ void key_pages_kernel(dartkv_cache_desc d, TokenSource src, int first_slot, int num_pages,
                                  int page_token_start, int last_page_tokens, const int32_t* __restrict__ indices,
                                  int32_t* nonfinite) {
-  extern __shared__ float s_mem[];
-  float* s_score = s_mem;
+  extern __shared__ uint32_t s_mem[];
+  uint32_t* s_key = s_mem;
   int* s_slot = reinterpret_cast<int*>(s_mem + d.head_dim);
   const int bh = blockIdx.x, pg = blockIdx.y;
   const int D = d.head_dim, P = d.page_size, Gk = d.key_group;
@@ -120,13 +120,13 @@ __global__ void key_pages_kernel(dartkv_cache_desc d, TokenSource src, int first
       for (int c = threadIdx.x; c < D; c += blockDim.x) {
         double sum = 0.0;
         for (int j = 0; j < n; ++j) sum += (double)fabsf(src.get(bh, t0 + j, c));
-        s_score[c] = rnd_rt(__fdiv_rn((float)sum, (float)n), d.dtype);
+        s_key[c] = rank_key(rnd_rt(__fdiv_rn((float)sum, (float)n), d.dtype));
       }
       __syncthreads();
       for (int c = threadIdx.x; c < D; c += blockDim.x) {
-        float mine = s_score[c];
+        const uint32_t mine = s_key[c];
         int rank = 0;
-        for (int o = 0; o < D; ++o) rank += ranks_before(s_score[o], o, mine, c);
+        for (int o = 0; o < D; ++o) rank += ranks_before(s_key[o], o, mine, c);
         if (rank < K) { s_slot[c] = rank; idx_field[rank] = c; }
       }
     }

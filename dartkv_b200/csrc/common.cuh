@@ -85,11 +85,15 @@ __device__ __forceinline__ float group_scale(float mn, float mx, float qmax, int
 }
 
 // Order of the promoted channels: score descending, channel ascending, NaN above every number like torch.topk has it.
-// A strict order whatever the scores are, so that every channel gets a rank of its own.
-__device__ __forceinline__ bool ranks_before(float score, int channel, float than, int than_channel) {
-  const bool nan = score != score, than_nan = than != than;
-  if (nan || than_nan) return nan && (!than_nan || channel < than_channel);
-  return score > than || (score == than && channel < than_channel);
+// The key of a score orders like the score itself and is the same for all NaNs, so the order is a strict one whatever
+// the scores are and every channel gets a rank of its own.
+__device__ __forceinline__ uint32_t rank_key(float score) {
+  if (score != score) return 0xFFFFFFFEu;
+  const uint32_t bits = __float_as_uint(score + 0.0f);   // -0 and +0 are one score
+  return bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+}
+__device__ __forceinline__ bool ranks_before(uint32_t key, int channel, uint32_t than, int than_channel) {
+  return key + (uint32_t)(channel < than_channel) > than;
 }
 
 // code of one element: clamp(rint(rnd(rnd(x - min) / scale)), 0, qmax)

@@ -272,9 +272,9 @@ extern "C" int dartkv_dequantize(const uint8_t* values, const void* scale, const
 }
 
 // ---------------------------------------------------------------------------- channel scores / selection
-// Sums run in double: for 16-bit inputs the sum of |k| over a page is then exact, so the score
-// does not depend on summation order (the reference accumulates in fp32, whose last-bit noise
-// only matters at exact rounding boundaries).
+// Sums run in double: exact for fp16 and for bf16 magnitudes within 2^37 of each other, otherwise (and for fp32) with an
+// error far below the fp32 rounding that follows, so the score does not depend on summation order but at exact rounding
+// boundaries (the reference accumulates in fp32, with last-bit noise at more of them).
 __global__ void channel_scores_kernel(const void* __restrict__ keys, int dt, int64_t bh, int64_t tokens, int64_t d,
                                       int64_t sbh, int64_t st, int strategy, void* scores) {
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,14 +323,14 @@ extern "C" int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, in
 // rank by (score descending, channel ascending), NaN first; one block per row
 __global__ void select_channels_kernel(const void* __restrict__ scores, int dt, int64_t d, int count,
                                        int32_t* __restrict__ indices) {
-  extern __shared__ float s_score[];
+  extern __shared__ uint32_t s_key[];
   int64_t r = blockIdx.x;
-  for (int c = threadIdx.x; c < d; c += blockDim.x) s_score[c] = load_f(scores, dt, r * d + c);
+  for (int c = threadIdx.x; c < d; c += blockDim.x) s_key[c] = rank_key(load_f(scores, dt, r * d + c));
   __syncthreads();
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    float mine = s_score[c];
+    const uint32_t mine = s_key[c];
     int rank = 0;
-    for (int o = 0; o < d; ++o) rank += ranks_before(s_score[o], o, mine, c);
+    for (int o = 0; o < d; ++o) rank += ranks_before(s_key[o], o, mine, c);
     if (rank < count) indices[r * count + rank] = c;
   }
 }
