@@ -157,7 +157,8 @@ class DartKVCache:
         self._c_state = _lib.LifecycleStateC()
         # what the native host path needs of this cache, as plain integers (see _bind_native)
         self._append_args: Optional[tuple] = None
-        self._decode_args: dict = {}    # by (query heads, stream)
+        # by (query heads, stream); by query heads alone the arguments and stream of the last native call
+        self._decode_args: dict = {}
 
     def _bind_native(self) -> None:
         """What the native append path needs: addresses of the descriptor, of the lifecycle structs (their fields change
@@ -843,23 +844,36 @@ class DartKVCache:
         """One decode call through the native host path: the output shaped like ``query``, or ``None`` when the call
         is not an ordinary one (other shapes or devices, query groups no kernel takes at once)."""
 
-        if self._desc is None or query.device != self._device:
+        heads, tokens = query.shape[1], self._life.seen
+        if scale is None and self._shape is not None:
+            scale = self._shape[2] ** -0.5
+        last = self._decode_args.get(heads)
+        if last is not None:        # the stream of the last call of this width: no more to look up
+            args, stream = last
+            out = _lib.HOST.decode(query, *args, tokens, scale, flavour, row_start, self._device.index, stream)
+            if out is not None:
+                if type(out) is int:
+                    check(out)
+                return out
+        if self._desc is None or query.device != self._device or not tokens:
             return None
-        key = query.shape[1], stream_ptr(self._device)
-        args = self._decode_args.get(key)
+        stream = stream_ptr(self._device)
+        if last is not None and last[1] == stream:
+            return None
+        args = self._decode_args.get((heads, stream))
         if args is None:            # the first call of this width on this stream: make its scratch
-            rep, rest = divmod(key[0], self._desc.kv_heads)
-            if rest or rep == 0 or not self._life.seen or (
-                    rep > 4 and rep > self.decode_rows_limit(query.dtype, flavour, self._life.seen)):
+            rep, rest = divmod(heads, self._desc.kv_heads)
+            if rest or rep == 0 or (rep > 4 and rep > self.decode_rows_limit(query.dtype, flavour, tokens)):
                 return None
-            self.decode_workspace(key[0])
-            args = self._decode_args.get(key)
+            self.decode_workspace(heads)
+            args = self._decode_args.get((heads, stream))
             if args is None:        # under capture
                 return None
-        out = _lib.HOST.decode(query, *args, self._life.seen, scale if scale is not None else self._shape[2] ** -0.5,
-                               flavour, row_start, self._device.index)
+        out = _lib.HOST.decode(query, *args, tokens, scale, flavour, row_start, self._device.index, stream)
         if type(out) is int:
             check(out)
+        if out is not None:
+            self._decode_args[heads] = args, stream
         return out
 
     def decode_status(self) -> int:

@@ -85,11 +85,12 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// decode(query, desc, workspace, workspace_bytes, query_heads, tokens, scale, flavour, row_start | None[, device])
+// decode(query, desc, workspace, workspace_bytes, query_heads, tokens, scale, flavour, row_start | None[, device[, stream]])
 //   -> output tensor shaped like the query ([B,Hq,D] or [B,Hq,1,D]), a negative return code, or None (slow path)
+// stream: the one the workspace belongs to; a call on another stream is not for this workspace.
 PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 9 && n != 10) { PyErr_SetString(PyExc_TypeError, "decode takes 9 or 10 arguments"); return nullptr; }
+  if (n < 9 || n > 11) { PyErr_SetString(PyExc_TypeError, "decode takes 9 to 11 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   const at::Tensor& q = THPVariable_Unpack(args[0]);
   auto* desc = static_cast<const dartkv_cache_desc*>(PyLong_AsVoidPtr(args[1]));
@@ -100,6 +101,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const double scale = PyFloat_AsDouble(args[6]);
   const long flavour = PyLong_AsLong(args[7]);
   const long device = device_argument(args, n, 9, q);
+  const void* owner = n > 10 ? PyLong_AsVoidPtr(args[10]) : nullptr;
   if (PyErr_Occurred()) return nullptr;
   const int64_t dims = q.dim();
   const int code = dtype_code(q.scalar_type());
@@ -107,6 +109,8 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
       q.size(0) != desc->batch || q.size(1) != query_heads || q.size(dims - 1) != desc->head_dim || (dims == 4 && q.size(2) != 1) ||
       query_heads % desc->kv_heads != 0 || tokens < 1)
     Py_RETURN_NONE;
+  void* stream = stream_of(q);
+  if (n > 10 && stream != owner) Py_RETURN_NONE;
   const long rep = query_heads / desc->kv_heads;
   if (rep > 4 && rep > dartkv_decode_rows_limit(desc, code, (int)flavour, (int)tokens)) Py_RETURN_NONE;
   const int32_t* row_start = nullptr;
@@ -125,7 +129,6 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const void* qp = dense.defined() ? dense.data_ptr() : q.data_ptr();
   at::Tensor out = at::empty(q.sizes(), q.options().requires_grad(false).memory_format(at::MemoryFormat::Contiguous));
   void* op = out.data_ptr();
-  void* stream = stream_of(q);
   int rc;
   Py_BEGIN_ALLOW_THREADS
   rc = (rep > 4 ? dartkv_decode_attention_rows : dartkv_decode_attention_padded)(desc, qp, code, (int)query_heads, (float)scale, (int)flavour, (int)tokens, row_start,
