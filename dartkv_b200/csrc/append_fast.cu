@@ -476,7 +476,8 @@ struct StepArgs {
   int copies;                              // the step's dense rows and metadata are written here
 };
 
-// KBITS as in key_page().  Three blocks per SM: 24 warps whose loads (32 words per thread) are all in flight at once.
+// KBITS as in key_page().  Four blocks per SM (64 registers, 42 KB of shared memory each): 32 warps, every block's page
+// in flight as asynchronous copies.
 template <int DT, int KBITS, int VBITS>
 __global__ void __launch_bounds__(kThreads, 4) append_step_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                   const __grid_constant__ StepArgs a) {

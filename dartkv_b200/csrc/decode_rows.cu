@@ -6,8 +6,9 @@
 // are split into groups of equal size; a group is a row of work like a (batch, KV head) pair, so all of them run in
 // one launch and find each other's pages in L2.
 //
-// What bounds it: instruction issue, as in decode_fast.cu (three packed operations per operand register).  What the
-// layout is for:
+// What bounds it: as in decode_fast.cu, the dependent phases of a page (order, table, logits, softmax, P.V) at four warps
+// per scheduler, here with instruction fetch as the largest stall; time moves with the number of instructions (three
+// packed operations per operand register).  What the layout is for:
 //   * keys: a register pairs two CHANNELS of one token (the contraction direction).  The half-words of two channel
 //     rows are put side by side with one prmt, after which every register is one logic op plus the packed arithmetic
 //     with the two channels' scales side by side.  Register u of a thread is token 16g + 8*HF + u, the same for 2-bit

@@ -545,7 +545,15 @@ static WideKernel wide_variant(int dtype, int md, bool fp32) {
 
 }  // namespace
 
-// decode_rows.cu takes the geometries of this file that it can (one key group per page, keys of 2 and 4 bits)
+// decode_rows.cu takes the geometries of this file that it can (one key group per page, keys of 2 and 4 bits), at every
+// size: of a call among others it is the faster one or even (32 heads on 8; us here / there, B200):
+//   batch x tokens                1 x 300      4 x 1,500    8 x 6,001    32 x 1,500
+//   4-bit fp16                    16.5 / 14.4  18.5 / 16.0  49 / 31      52 / 37
+//   the same, fp32 flavour        18.0 / 18.5  20.5 / 18.5  54 / 39      56 / 44
+//   2+2-bit keys, 8-bit values    20.5 / 16.5  22.6 / 16.5  64 / 37      66 / 43
+//   2+2-bit, value groups of 16   18.5 / 14.4  20.5 / 16.0  54 / 33      57 / 39
+//   2+2-bit, fp32 flavour         18.5 / 18.5  21.4 / 18.5  60 / 41      62 / 45
+// A call whose code is not in the caches yet is up to 2 us (fp32 flavour: 4-8 us) slower there below some 1,500 tokens.
 int dartkv_decode_rows_supported(const dartkv_cache_desc* d, int q_dtype, int rep, int flavour);
 int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int query_heads, float scale, int flavour, int quads,
                               int stream_blocks, long long units, int total_splits, float* part_m, float* part_l, float* part_acc,

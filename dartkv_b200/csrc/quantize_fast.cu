@@ -293,8 +293,10 @@ namespace {
 
 constexpr int kScoreSplits = 16;
 
-// Promoted channels of one (batch, head): sum |k| per channel in double (exact for 16-bit data, in any order), scores
-// rounded to the data dtype, rank by (score descending, channel ascending).  One block of 16 token splits x 64 channel
+// Promoted channels of one (batch, head): sum |k| per channel in double, scores rounded to the data dtype, rank by (score
+// descending, channel ascending).  In fp16 the sum is exact in any order.  bf16 values can be further apart than a double
+// has bits; the error is then some 2^-50 of the sum, which changes the score only where the sum lies that close to a
+// boundary of the fp32 rounding that follows.  One block of 16 token splits x 64 channel
 // pairs; scores (optional) are written too.
 template <int DT>
 __global__ void __launch_bounds__(64 * kScoreSplits) score_select_kernel(const uint16_t* __restrict__ keys, int64_t tokens, int d,
