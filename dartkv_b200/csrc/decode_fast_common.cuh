@@ -313,6 +313,25 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   return d;
 }
 
+// The query of a KV head's group as 16-bit values, the heads of a channel side by side (zero for absent heads), by one warp.
+__device__ __forceinline__ void store_query_compact(uint2* query, const void* q, int64_t first_row, int rep, int lane) {
+  uint2 v[4];   // [head]: channels 4 * lane .. + 3
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    v[r] = make_uint2(0u, 0u);
+    if (r < rep) {   // the query is 4-byte aligned, no more
+      const uint32_t* at = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(q) + (first_row + r) * 128) + 2 * lane;
+      v[r] = make_uint2(at[0], at[1]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t sel = i & 1 ? 0x7632u : 0x5410u;
+    query[4 * lane + i] = i < 2 ? make_uint2(prmt(v[0].x, v[1].x, sel), prmt(v[2].x, v[3].x, sel))
+                                : make_uint2(prmt(v[0].y, v[1].y, sel), prmt(v[2].y, v[3].y, sel));
+  }
+}
+
 // Block merge of the eight warp states: thread = (channel, head parity); partials leave in natural-log units.
 template <bool ROW_GROUPS = false, class BS>
 __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, const float* warp_out, int b, int hkv, int rep,

@@ -28,28 +28,32 @@
 
 namespace {
 
-constexpr int kQkUnroll = 16, kPvUnroll = 4;
-constexpr int kUStride = 36;   // 32-bit words per group of 8 local tokens in a warp's weight table (4 pad)
+constexpr int kUStride = 132;   // 32-bit words per head of a warp's weight table: 128 tokens, 4 pad
 
-struct FusedPairSmem {
-  uint8_t stage[2][kStageBytes];
-  // per-page tables, double-buffered like the stages so that one warp of the pair may set up the next page while
-  // the other still reads this page's
-  uint2 w_low[2][128];           // per channel: fp16 q*s*f of heads (0,1) and (2,3)
-  uint2 w_high[2][32];           // per promoted slot: fp16 4*q*s*f of its channel, zero past the last slot
-  uint2 w_high_lo[2][32];        // what the fp16 rounding of w_high dropped, as fp16: the high plane carries most of a
-                                 // promoted (outlier) channel's magnitude, so its weights get a second term
-  uint32_t u[2][8 * kUStride];   // per warp: [local token][head] = fp16 p*s*fv of (value group 0 | group 1 << 16)
-  float bias_part[2][2][4];      // [table][warp]: partial sum_ch q*z per head
-  uint64_t bar[2];
+// what a warp needs beside a staged page
+union FusedScratch {
+  struct {
+    uint2 w_low[128];      // per channel: fp16 q*s*f of heads (0,1) and (2,3)
+    uint2 w_high[32];      // per promoted slot: fp16 4*q*s*f of its channel, zero past the last slot
+    uint2 w_high_lo[32];   // what the fp16 rounding of w_high dropped, as fp16: the high plane carries most of a
+                           // promoted (outlier) channel's magnitude, so its weights get a second term
+  };
+  // takes their place after the logits: [head][token] = fp16 p*s*fv of (value group 0 | group 1 << 16)
+  uint32_t u[4 * kUStride];
+};
+
+struct FusedWarpSmem {
+  uint8_t keys[kPageBytesK];
+  uint8_t values[kStageBytes - kPageBytesK];   // codes, then scales and zero points
+  FusedScratch scratch;
+  uint64_t k_bar, v_bar;
 };
 
 struct FusedBlockSmem {
-  float qf[128][4];              // [channel][head] query as fp32 (zero for absent heads)
+  uint2 query[128];              // [channel]: the 16-bit query values of the four heads (zero for absent heads)
   float merge_m[kWarps][4];
   float merge_l[kWarps][4];
   int slot_map[128];
-  float q_absmax;
 };
 
 template <int DT>
@@ -89,212 +93,314 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// per-warp running state of the online softmax and the output accumulators
-struct WarpState {
-  float o_acc[4][4];   // [m-tile][c-reg], in units of 4^p * 2^-24 / fv_run
-  float m_run, l_run;  // head c, log2 domain
-  float zs[2];         // this thread's share of sum_t p * z for (head c, value group j)
+// One page, as one warp works on it.  DT: dtype of the cache and the query; MD: dtype of the scales and zero points.
+// GN: value groups per token (1 or 2).  KP: promoted channels per page when that is a multiple of eight known to
+// the host (0, 8, 16, 24, 32), else -1 (read from the descriptor).
+template <int DT, int MD, int GN, int KP>
+struct FusedWork {
+  static constexpr int kQkUnroll = 16, kPvUnroll = 4;   // 64 x 32,768 tokens: 382 us; with 4 and 4 386, with 2 and 2 396
+  const dartkv_cache_desc& d;
+  const uint2* query;
+  float scale2;
+  int lane, g, c, K, prom_steps;
+  uint32_t sel_w, mask_u;
+  float q_absmax;
+  float o_acc[4][4];           // [m-tile][c-reg], in units of 4^p * 2^-24 / fv_run
+  float m_run, l_run;          // head c, log2 domain
+  float zs[2];                 // this thread's share of sum_t p * z for (head c, value group j)
   float fv_run, fv_inv_run;
-};
+  float bias, f_inv;           // of the page in work
 
-// One warp's share of a staged page.  HF: which four codes of every 16-bit half this warp owns;
-// GN: value groups per token (1 or 2).
-template <int DT, int GN>
-__device__ __forceinline__ void fused_page_half(const int HF, const int tb, const dartkv_cache_desc& d, FusedPairSmem& ps, const uint8_t* blob,
-                                                uint32_t* utab, int prom_steps, float scale2, float f_inv, int g, int c,
-                                                uint32_t sel_w, uint32_t mask_u, int mask_below, WarpState& st) {
-  // ---- logits: S[token pair][(head, j')] over the doubled contraction (channel, j).  Row g of m-tile mt
-  // reads code position 2mt, row g+8 position 2mt+1.
-  // Even and odd contraction steps use separate accumulators so consecutive MMAs are independent.
-  float s_acc[2][4], s_odd[2][4];
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s_acc[mt][i] = s_odd[mt][i] = 0.0f;
-  {
-    const uint8_t* low_thread = blob + 4 * g + 32 * c;                               // + 256 * step (+128)
-    const uint8_t* w_thread = reinterpret_cast<const uint8_t*>(ps.w_low[tb]) + 8 * c + 4 * (g >> 2);   // + 64 * step (+32)
-#pragma unroll kQkUnroll
-    for (int ks = 0; ks < 16; ++ks) {
-      uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + 256 * ks);
-      uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + 256 * ks + 128);
-      w0 >>= 8 * HF; w1 >>= 8 * HF;   // HF is a run-time value: one copy of this code serves both warps of a pair
-      const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(w_thread + 64 * ks), 0u, sel_w);
-      const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(w_thread + 64 * ks + 32), 0u, sel_w);
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-        mma_f16((ks & 1) ? s_odd[mt] : s_acc[mt], w0 & (0x00030003u << (4 * mt)), w0 & (0x000C000Cu << (4 * mt)),
-                w1 & (0x00030003u << (4 * mt)), w1 & (0x000C000Cu << (4 * mt)), b0, b1);
-    }
-    // high plane of the promoted slots
-    const uint8_t* high_thread = blob + d.key_off_high + 4 * g + 32 * c;
-    const uint8_t* wh_thread = reinterpret_cast<const uint8_t*>(ps.w_high[tb]) + 8 * c + 4 * (g >> 2);
-    const uint8_t* wl_thread = reinterpret_cast<const uint8_t*>(ps.w_high_lo[tb]) + 8 * c + 4 * (g >> 2);
-    for (int ks = 0; ks < prom_steps; ++ks) {
-      uint32_t w0 = *reinterpret_cast<const uint32_t*>(high_thread + 256 * ks);
-      uint32_t w1 = *reinterpret_cast<const uint32_t*>(high_thread + 256 * ks + 128);
-      w0 >>= 8 * HF; w1 >>= 8 * HF;   // HF is a run-time value: one copy of this code serves both warps of a pair
-      const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(wh_thread + 64 * ks), 0u, sel_w);
-      const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(wh_thread + 64 * ks + 32), 0u, sel_w);
-      const uint32_t l0 = prmt(*reinterpret_cast<const uint32_t*>(wl_thread + 64 * ks), 0u, sel_w);
-      const uint32_t l1 = prmt(*reinterpret_cast<const uint32_t*>(wl_thread + 64 * ks + 32), 0u, sel_w);
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        const uint32_t a0 = w0 & (0x00030003u << (4 * mt)), a1 = w0 & (0x000C000Cu << (4 * mt));
-        const uint32_t a2 = w1 & (0x00030003u << (4 * mt)), a3 = w1 & (0x000C000Cu << (4 * mt));
-        mma_f16(s_acc[mt], a0, a1, a2, a3, b0, b1);
-        mma_f16(s_odd[mt], a0, a1, a2, a3, l0, l1);   // same codes against the dropped part of the weights
-      }
-    }
+  __device__ __forceinline__ FusedWork(const dartkv_cache_desc& desc, const uint2* query_table, float scale, int lane_)
+      : d(desc), query(query_table), scale2(scale * kLog2e), lane(lane_), g(lane_ >> 2), c(lane_ & 3) {
+    K = KP >= 0 ? KP : (d.key_mode == DARTKV_MIXED_PAGE ? d.promoted : 0);
+    prom_steps = (K + 7) >> 3;
+    // weight operand: column n = g is (head g >> 1, j' = g & 1); the 32-bit word read holds the fp16 weights of the
+    // head pair g >> 2.  Take the head's half into half j' and zeros (from the second source) into the other.
+    const uint32_t head_bytes = ((g >> 1) & 1) ? 0x32u : 0x10u;
+    sel_w = (g & 1) ? (0x0054u | (head_bytes << 8)) : (head_bytes | 0x5400u);
+    mask_u = (g & 1) ? 0xFFFF0000u : 0x0000FFFFu;
   }
 
-  // ---- online softmax for head c over this warp's 64 tokens (this thread: 8 of them)
-  const float bias = (ps.bias_part[tb][0][c] + ps.bias_part[tb][1][c]) * scale2;
-  float cm[4];   // scale2 / f * 2^(24 - 2p)
-  {
-    const float base = scale2 * f_inv;
-    cm[0] = base * 16777216.0f; cm[1] = base * 4194304.0f; cm[2] = base * 1048576.0f; cm[3] = base * 262144.0f;
+  __device__ __forceinline__ float4 query_of(int ch) const {
+    const uint2 x = query[ch];
+    float4 q;
+    md_pair_to_float<DT>(x.x, q.x, q.y);
+    md_pair_to_float<DT>(x.y, q.z, q.w);
+    return q;
   }
-  float mx = -INFINITY;
-  float s_sum[2][4];
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      s_sum[mt][i] = fmaf(s_acc[mt][i] + s_odd[mt][i], cm[2 * mt + (i >> 1)], bias);
-    }
-  if (mask_below > 0) {   // the page that holds the row's first live token: the tokens before it drop out
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (16 * g + 4 * HF + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_sum[mt][i] = -INFINITY;
-  }
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) mx = fmaxf(mx, s_sum[mt][i]);
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-  const float m_new = fmaxf(st.m_run, mx);
-  const float m_ref = m_new == -INFINITY ? 0.0f : m_new;   // nothing live yet: every weight below comes out zero
-  const float alpha = fast_exp2(st.m_run - m_ref);
-  st.m_run = m_new;
 
-  // value metadata of this thread's 8 tokens: token = 16g + 4HF + p + 8j', p = 2mt + (i >> 1), j' = i & 1
-  const uint8_t* vmeta = blob + kOffVMeta;
-  uint32_t meta_s[8], meta_z[8];   // GN == 2: (s0 | s1 << 16), (z0 | z1 << 16); GN == 1: s, z in the low half
-  uint32_t smax = 0;
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  // the query table is complete: its largest magnitude bounds the weights q*s
+  __device__ __forceinline__ void start_row() {
+    q_absmax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int tok = 16 * g + 4 * HF + 2 * mt + (i >> 1) + 8 * (i & 1);
-      const int k = 4 * mt + i;
-      if (GN == 2) {
-        const uint2 m = *reinterpret_cast<const uint2*>(vmeta + tok * 8);
-        meta_s[k] = m.x; meta_z[k] = m.y;
-        smax = max(smax, max(m.x & 0xFFFFu, m.x >> 16));
-      } else {
-        const uint32_t m = *reinterpret_cast<const uint32_t*>(vmeta + tok * 4);
-        meta_s[k] = m & 0xFFFFu; meta_z[k] = m >> 16;
-        smax = max(smax, m & 0xFFFFu);
-      }
+      const float4 q = query_of(32 * i + lane);
+      q_absmax = fmaxf(q_absmax, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
     }
-  // scales are positive finite 16-bit floats: their bit patterns order like the values
-  smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, 4));
-  smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, 8));
-  smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, 16));
-  float fv_page, fv_inv_page;
-  pow2_normaliser(md_to_float<DT>(smax), fv_page, fv_inv_page);
-  // the normaliser only ever shrinks, so accumulators are rescaled at most a handful of times per run
-  const bool shrink = fv_page < st.fv_run;
-  const float factor = shrink ? alpha * (fv_page * st.fv_inv_run) : alpha;
-  if (shrink) { st.fv_run = fv_page; st.fv_inv_run = fv_inv_page; }
-  const float fv = st.fv_run;
-
-  float psum = 0.0f, zs0 = 0.0f, zs1 = 0.0f;
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = 4 * mt + i;
-      const float p = fast_exp2(s_sum[mt][i] - m_ref);
-      psum += p;
-      const float pf = p * fv;
-      const int li = 2 * mt + (i >> 1) + 4 * (i & 1);   // local token inside this thread's 8: position + 4 j'
-      uint32_t packed;
-      if (GN == 2) {
-        float s0, s1, z0, z1;
-        md_pair_to_float<DT>(meta_s[k], s0, s1);
-        md_pair_to_float<DT>(meta_z[k], z0, z1);
-        zs0 = fmaf(p, z0, zs0);
-        zs1 = fmaf(p, z1, zs1);
-        packed = pack_f16x2(pf * s0, pf * s1);
-      } else {
-        const float s0 = md_to_float<DT>(meta_s[k]), z0 = md_to_float<DT>(meta_z[k]);
-        zs0 = fmaf(p, z0, zs0);
-        const float u = pf * s0;
-        packed = pack_f16x2(u, u);
-      }
-      utab[g * kUStride + li * 4 + c] = packed;
-    }
-  st.l_run = st.l_run * alpha + psum;
-  st.zs[0] = st.zs[0] * alpha + zs0;
-  st.zs[1] = st.zs[1] * alpha + (GN == 2 ? zs1 : zs0);
-  // the running maximum and the normaliser rarely move after the first pages
-  if (__any_sync(0xffffffffu, factor != 1.0f)) {
+    for (int off = 16; off > 0; off >>= 1) q_absmax = fmaxf(q_absmax, __shfl_xor_sync(0xffffffffu, q_absmax, off));
 #pragma unroll
     for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st.o_acc[mt][i] *= factor;
+      for (int i = 0; i < 4; ++i) o_acc[mt][i] = 0.0f;
+    m_run = -INFINITY; l_run = 0.0f; zs[0] = zs[1] = 0.0f;
+    fv_run = __uint_as_float(253u << 23); fv_inv_run = __uint_as_float(1u << 23);
   }
-  __syncwarp();
 
-  // ---- O[channel pair][(head, j')] += V^T U over the doubled contraction (token, j): lane row g reads the
-  // code words wi = g & 3 and wi + 4 of a token row and pairs their low (g < 4) or high (g >= 4) halves, so a
-  // register holds (channel 16wi + 8xy + u of group 0, the same channel + 64 of group 1).  Step ks covers the
-  // eight tokens 16ks + 4HF + {0..3} and + 8.
-  {
-    const int wi = g & 3;
-    const uint32_t sel_v = (g >> 2) ? 0x7632u : 0x5410u;
-    const uint8_t* vthread = blob + kOffVCodes + 32 * (4 * HF + c) + 4 * wi;   // + 512 * ks (+256 for the second token)
-    const uint32_t* uthread = utab + c * 4 + (g >> 1);                         // + kUStride * ks (+16 for the second)
-#pragma unroll kPvUnroll
-    for (int ks = 0; ks < 8; ++ks) {
-      const uint32_t x0 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 512 * ks),
-                               *reinterpret_cast<const uint32_t*>(vthread + 512 * ks + 16), sel_v);
-      const uint32_t x1 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 512 * ks + 256),
-                               *reinterpret_cast<const uint32_t*>(vthread + 512 * ks + 256 + 16), sel_v);
-      const uint32_t y0 = x0 >> 10, y1 = x1 >> 10;   // codes 5, 6, 7 at positions 0, 1, 2
-      const uint32_t b0 = uthread[kUStride * ks] & mask_u;
-      const uint32_t b1 = uthread[kUStride * ks + 16] & mask_u;
-      mma_f16(st.o_acc[0], x0 & 0x00030003u, x0 & 0x000C000Cu, x1 & 0x00030003u, x1 & 0x000C000Cu, b0, b1);
-      mma_f16(st.o_acc[1], x0 & 0x00300030u, x0 & 0x00C000C0u, x1 & 0x00300030u, x1 & 0x00C000C0u, b0, b1);
-      mma_f16(st.o_acc[2], x0 & 0x03000300u, y0 & 0x00030003u, x1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
-      mma_f16(st.o_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u, b0, b1);
+  // weights of the page's channels and promoted slots
+  __device__ __forceinline__ void fill_table(const uint8_t* keys, FusedScratch& ws) {
+    const uint32_t* kscale2 = reinterpret_cast<const uint32_t*>(keys + d.key_off_scale);
+    const uint32_t* kzero2 = reinterpret_cast<const uint32_t*>(keys + d.key_off_zero);
+    const uint32_t sc[2] = {kscale2[lane], kscale2[32 + lane]}, zp[2] = {kzero2[lane], kzero2[32 + lane]};
+    // scales are positive finite 16-bit floats: their bit patterns order like the values
+    const uint32_t smax = __reduce_max_sync(0xffffffffu, max(max(sc[0] & 0xFFFFu, sc[0] >> 16), max(sc[1] & 0xFFFFu, sc[1] >> 16)));
+    float f;
+    pow2_normaliser(4.0f * q_absmax * md_to_float<MD>(smax), f, f_inv);
+    float bz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {   // channels 2 * tp and 2 * tp + 1
+      const int tp = 32 * i + lane;
+      float s0, s1, z0, z1;
+      md_pair_to_float<MD>(sc[i], s0, s1);
+      md_pair_to_float<MD>(zp[i], z0, z1);
+      const float4 qa = query_of(2 * tp), qb = query_of(2 * tp + 1);
+      const float sa = s0 * f, sb = s1 * f;
+      *reinterpret_cast<uint4*>(&ws.w_low[2 * tp]) = make_uint4(pack_f16x2(qa.x * sa, qa.y * sa), pack_f16x2(qa.z * sa, qa.w * sa),
+                                                                pack_f16x2(qb.x * sb, qb.y * sb), pack_f16x2(qb.z * sb, qb.w * sb));
+      bz[0] += fmaf(qa.x, z0, qb.x * z1); bz[1] += fmaf(qa.y, z0, qb.y * z1);
+      bz[2] += fmaf(qa.z, z0, qb.z * z1); bz[3] += fmaf(qa.w, z0, qb.w * z1);
+    }
+    if (prom_steps > 0) {   // lane = slot
+      uint2 wh = make_uint2(0u, 0u), wl = make_uint2(0u, 0u);
+      if (lane < K) {
+        const int ch = reinterpret_cast<const int32_t*>(keys + d.key_off_index)[lane] & 127;
+        const float s4 = 4.0f * f * md_to_float<MD>(reinterpret_cast<const uint16_t*>(keys + d.key_off_scale)[ch]);
+        const float4 qh = query_of(ch);
+        const float e0 = qh.x * s4, e1 = qh.y * s4, e2 = qh.z * s4, e3 = qh.w * s4;
+        wh = make_uint2(pack_f16x2(e0, e1), pack_f16x2(e2, e3));
+        const float2 h01 = __half22float2(*reinterpret_cast<const __half2*>(&wh.x));
+        const float2 h23 = __half22float2(*reinterpret_cast<const __half2*>(&wh.y));
+        wl = make_uint2(pack_f16x2(e0 - h01.x, e1 - h01.y), pack_f16x2(e2 - h23.x, e3 - h23.y));
+      }
+      ws.w_high[lane] = wh;
+      ws.w_high_lo[lane] = wl;
+    }
+    // sum_ch q*z per head: four sums over 32 lanes in 6 shuffles, halving the number of sums a lane carries at the
+    // first two levels; head 2*up16 + up8 ends up in the lanes of that eighth
+    const bool up16 = lane & 16, up8 = lane & 8;
+    const float k0 = (up16 ? bz[2] : bz[0]) + __shfl_xor_sync(0xffffffffu, up16 ? bz[0] : bz[2], 16);
+    const float k1 = (up16 ? bz[3] : bz[1]) + __shfl_xor_sync(0xffffffffu, up16 ? bz[1] : bz[3], 16);
+    float k = (up8 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up8 ? k0 : k1, 8);
+    k += __shfl_xor_sync(0xffffffffu, k, 4);
+    k += __shfl_xor_sync(0xffffffffu, k, 2);
+    k += __shfl_xor_sync(0xffffffffu, k, 1);
+    bias = __shfl_sync(0xffffffffu, k, 8 * c) * scale2;
+  }
+
+  // logits S[token pair][(head, j')] over the doubled contraction (channel, j).  A thread reads the whole word g of a
+  // channel's code row (tokens 16g .. 16g+15); row g of m-tile mt is code u = 2mt of both halves, row g+8 u = 2mt + 1:
+  // u = 0..4 at positions 0..4 of the mantissa, 5..7 at positions 0..2 after a shift.
+  __device__ __forceinline__ void logits(const uint8_t* keys, const FusedScratch& ws, float (&s_acc)[4][4]) const {
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
+    const uint8_t* const low = keys + 4 * g + 32 * c;                          // + 256 * step (+128)
+    const int w_thread = 8 * c + 4 * (g >> 2);                                 // + 64 * step (+32)
+    const uint8_t* const w_low = reinterpret_cast<const uint8_t*>(ws.w_low) + w_thread;
+#pragma unroll kQkUnroll
+    for (int ks = 0; ks < 16; ++ks) {
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low + 256 * ks);
+      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low + 256 * ks + 128);
+      const uint32_t y0 = w0 >> 10, y1 = w1 >> 10;
+      const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(w_low + 64 * ks), 0u, sel_w);
+      const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(w_low + 64 * ks + 32), 0u, sel_w);
+      mma_f16(s_acc[0], w0 & 0x00030003u, w0 & 0x000C000Cu, w1 & 0x00030003u, w1 & 0x000C000Cu, b0, b1);
+      mma_f16(s_acc[1], w0 & 0x00300030u, w0 & 0x00C000C0u, w1 & 0x00300030u, w1 & 0x00C000C0u, b0, b1);
+      mma_f16(s_acc[2], w0 & 0x03000300u, y0 & 0x00030003u, w1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
+      mma_f16(s_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u, b0, b1);
+    }
+    // high plane of the promoted slots: the same codes against both terms of the weights
+    const uint8_t* const high = keys + d.key_off_high + 4 * g + 32 * c;
+    const uint8_t* const w_high = reinterpret_cast<const uint8_t*>(ws.w_high) + w_thread;
+    const uint8_t* const w_high_lo = reinterpret_cast<const uint8_t*>(ws.w_high_lo) + w_thread;
+    for (int ks = 0; ks < prom_steps; ++ks) {
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(high + 256 * ks);
+      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(high + 256 * ks + 128);
+      const uint32_t y0 = w0 >> 10, y1 = w1 >> 10;
+      const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(w_high + 64 * ks), 0u, sel_w);
+      const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(w_high + 64 * ks + 32), 0u, sel_w);
+      const uint32_t l0 = prmt(*reinterpret_cast<const uint32_t*>(w_high_lo + 64 * ks), 0u, sel_w);
+      const uint32_t l1 = prmt(*reinterpret_cast<const uint32_t*>(w_high_lo + 64 * ks + 32), 0u, sel_w);
+      auto both = [&](float (&s)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+        mma_f16(s, a0, a1, a2, a3, b0, b1);
+        mma_f16(s, a0, a1, a2, a3, l0, l1);
+      };
+      both(s_acc[0], w0 & 0x00030003u, w0 & 0x000C000Cu, w1 & 0x00030003u, w1 & 0x000C000Cu);
+      both(s_acc[1], w0 & 0x00300030u, w0 & 0x00C000C0u, w1 & 0x00300030u, w1 & 0x00C000C0u);
+      both(s_acc[2], w0 & 0x03000300u, y0 & 0x00030003u, w1 & 0x03000300u, y1 & 0x00030003u);
+      both(s_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u);
     }
   }
-}
 
-// GN: value groups per token (1 or 2).  KP: promoted channels per page when that is a multiple of eight known to
-// the host (0, 8, 16, 24, 32), else -1 (read from the descriptor).
-// DT: dtype of the cache and the query; MD: dtype of the scales and zero points
+  // online softmax for head c over the page (this thread: tokens 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1); the
+  // probabilities leave as weights p*s*fv.  wait_for_values() returns when the page's values have landed.
+  template <class Wait>
+  __device__ __forceinline__ void softmax(float (&s_acc)[4][4], int mask_below, FusedScratch& ws, Wait wait_for_values, const uint8_t* values) {
+    {
+      const float base = scale2 * f_inv * 16777216.0f;
+      const float cm[5] = {base, base * 0.25f, base * 0.0625f, base * 0.015625f, base * 0.00390625f};
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int u = 2 * mt + (i >> 1);
+          s_acc[mt][i] = fmaf(s_acc[mt][i], cm[u < 5 ? u : u - 5], bias);
+        }
+    }
+    if (mask_below > 0) {   // the page that holds the row's first live token: the tokens before it drop out
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (16 * g + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
+    }
+    float mx = -INFINITY;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mx = fmaxf(mx, s_acc[mt][i]);
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    const float m_new = fmaxf(m_run, mx);
+    const float m_ref = m_new == -INFINITY ? 0.0f : m_new;   // nothing live yet: every weight below comes out zero
+    const float alpha = fast_exp2(m_run - m_ref);
+    m_run = m_new;
+
+    // largest value scale of the page; the normaliser only ever shrinks, so accumulators are rescaled at most a handful
+    // of times per run
+    wait_for_values();
+    const uint8_t* const vmeta = values + kValueCodes;
+    uint32_t smax;
+    {
+      const uint4 m0 = reinterpret_cast<const uint4*>(vmeta)[lane];
+      if (GN == 2) {
+        const uint4 m1 = reinterpret_cast<const uint4*>(vmeta)[32 + lane];
+        smax = max(max(max(m0.x & 0xFFFFu, m0.x >> 16), max(m0.z & 0xFFFFu, m0.z >> 16)),
+                   max(max(m1.x & 0xFFFFu, m1.x >> 16), max(m1.z & 0xFFFFu, m1.z >> 16)));
+      } else {
+        smax = max(max(m0.x & 0xFFFFu, m0.y & 0xFFFFu), max(m0.z & 0xFFFFu, m0.w & 0xFFFFu));
+      }
+    }
+    smax = __reduce_max_sync(0xffffffffu, smax);
+    float fv_page, fv_inv_page;
+    pow2_normaliser(md_to_float<MD>(smax), fv_page, fv_inv_page);
+    const bool shrink = fv_page < fv_run;
+    const float factor = shrink ? alpha * (fv_page * fv_inv_run) : alpha;
+    if (shrink) { fv_run = fv_page; fv_inv_run = fv_inv_page; }
+    const float fv = fv_run;
+
+    float psum = 0.0f, zs0 = 0.0f, zs1 = 0.0f;
+    uint32_t* const row = &ws.u[c * kUStride + 16 * g];
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {   // tokens 16g + 4*k4 .. + 3
+      uint32_t packed[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int u = 4 * (k4 & 1) + k, j = k4 >> 1;
+        const float p = fast_exp2(s_acc[u >> 1][2 * (u & 1) + j] - m_ref);
+        psum += p;
+        const float pf = p * fv;
+        const int tok = 16 * g + 4 * k4 + k;
+        if (GN == 2) {
+          const uint2 m = *reinterpret_cast<const uint2*>(vmeta + tok * 8);   // (s0 | s1 << 16), (z0 | z1 << 16)
+          float s0, s1, z0, z1;
+          md_pair_to_float<MD>(m.x, s0, s1);
+          md_pair_to_float<MD>(m.y, z0, z1);
+          zs0 = fmaf(p, z0, zs0);
+          zs1 = fmaf(p, z1, zs1);
+          packed[k] = pack_f16x2(pf * s0, pf * s1);
+        } else {
+          float s0, z0;
+          md_pair_to_float<MD>(*reinterpret_cast<const uint32_t*>(vmeta + tok * 4), s0, z0);
+          zs0 = fmaf(p, z0, zs0);
+          const float w = pf * s0;
+          packed[k] = pack_f16x2(w, w);
+        }
+      }
+      *reinterpret_cast<uint4*>(row + 4 * k4) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+    l_run = l_run * alpha + psum;
+    zs[0] = zs[0] * alpha + zs0;
+    zs[1] = zs[1] * alpha + (GN == 2 ? zs1 : zs0);
+    // the running maximum and the normaliser rarely move after the first pages
+    if (__any_sync(0xffffffffu, factor != 1.0f)) {
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o_acc[mt][i] *= factor;
+    }
+  }
+
+  // O[channel pair][(head, j')] += V^T U over the doubled contraction (token, j): lane row g reads the
+  // code words wi = g & 3 and wi + 4 of a token row and pairs their low (g < 4) or high (g >= 4) halves, so a
+  // register holds (channel 16wi + 8xy + u of group 0, the same channel + 64 of group 1).  Step ks covers the
+  // eight tokens from 8ks on.
+  __device__ __forceinline__ void weigh_values(const uint8_t* values, const FusedScratch& ws) {
+    const int wi = g & 3;
+    const uint32_t sel_v = (g >> 2) ? 0x7632u : 0x5410u;
+    const uint8_t* const vthread = values + 32 * c + 4 * wi;               // + 256 * ks (+128 for the second token)
+    const uint32_t* const uthread = &ws.u[(g >> 1) * kUStride + c];        // + 8 * ks (+4 for the second token)
+#pragma unroll kPvUnroll
+    for (int ks = 0; ks < 16; ++ks) {
+      const uint32_t x0 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 256 * ks),
+                               *reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 16), sel_v);
+      const uint32_t x1 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 128),
+                               *reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 128 + 16), sel_v);
+      const uint32_t y0 = x0 >> 10, y1 = x1 >> 10;   // codes 5, 6, 7 at positions 0, 1, 2
+      const uint32_t b0 = uthread[8 * ks] & mask_u;
+      const uint32_t b1 = uthread[8 * ks + 4] & mask_u;
+      mma_f16(o_acc[0], x0 & 0x00030003u, x0 & 0x000C000Cu, x1 & 0x00030003u, x1 & 0x000C000Cu, b0, b1);
+      mma_f16(o_acc[1], x0 & 0x00300030u, x0 & 0x00C000C0u, x1 & 0x00300030u, x1 & 0x00C000C0u, b0, b1);
+      mma_f16(o_acc[2], x0 & 0x03000300u, y0 & 0x00030003u, x1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
+      mma_f16(o_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u, b0, b1);
+    }
+  }
+
+  // this warp's state for the merge: m_run and l_run of head c, accumulators [head][channel]
+  __device__ __forceinline__ void hand_over(float* acc) {
+#pragma unroll
+    for (int off = 4; off < 32; off <<= 1) {
+      l_run += __shfl_xor_sync(0xffffffffu, l_run, off);
+      zs[0] += __shfl_xor_sync(0xffffffffu, zs[0], off);
+      zs[1] += __shfl_xor_sync(0xffffffffu, zs[1], off);
+    }
+    const int wi = g & 3, xy = g >> 2;
+    const float unit = fv_inv_run * 16777216.0f;   // accumulators hold codes * 4^p * 2^-24 * fv
+    const float pos_scale[5] = {unit, unit * 0.25f, unit * 0.0625f, unit * 0.015625f, unit * 0.00390625f};
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int u = 2 * mt + (i >> 1), jp = i & 1;
+        acc[c * 128 + 64 * jp + 16 * wi + 8 * xy + u] = fmaf(o_acc[mt][i], pos_scale[u < 5 ? u : u - 5], zs[jp]);
+      }
+  }
+};
+
+// the work split of decode_fast_kernel
 template <int DT, int MD, int GN, int KP>
 __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cache_desc d, FastArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  FusedPairSmem* psm_all = reinterpret_cast<FusedPairSmem*>(smem_raw);
-  FusedBlockSmem& bs = *reinterpret_cast<FusedBlockSmem*>(smem_raw + sizeof(FusedPairSmem) * kPairs);
+  FusedBlockSmem& bs = *reinterpret_cast<FusedBlockSmem*>(smem_raw + sizeof(FusedWarpSmem) * kWarps);
   float* warp_out = reinterpret_cast<float*>(smem_raw);   // reused after the page loop: [warp][head][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, c = lane & 3;
   const int rep = a.query_heads / d.kv_heads;
 
   if ((int)blockIdx.x >= a.stream_blocks) {
-    // dense tokens of one (batch, kv head): partial slot 0.  These short blocks come last in launch order and fill
-    // the slots the stream blocks leave.
     const int bh = blockIdx.x - a.stream_blocks;
     dense_block<DT, MD>(d, a, bs, warp_out, bh);
     __syncthreads();
@@ -302,45 +408,34 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
     return;
   }
 
-  // ---- stream block: an even share of all (row, four-page unit) work, possibly spanning several rows
   const int sb = blockIdx.x;
   int unit = (int)((int64_t)sb * a.units / a.stream_blocks);   // the host keeps the unit count below 2^31
   const int unit_end = (int)((int64_t)(sb + 1) * a.units / a.stream_blocks);
-  const int pair = warp >> 1, hf = warp & 1;
-  FusedPairSmem& ps = psm_all[pair];
+  FusedWarpSmem& ws = reinterpret_cast<FusedWarpSmem*>(smem_raw)[warp];
   const int k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
   const int fast_end = fast_range_end(d.sink_tokens, d.page_size, k_end, v_end, sink_filled);
   const int total_pages = fast_end > d.sink_tokens ? (fast_end - d.sink_tokens) / 128 : 0;
-  const bool issuer = hf == 0 && lane == 0;
-  const int vmeta_page_bytes = 128 * 2 * d.value_groups * 2;
-  const uint32_t stage_tx = d.key_page_bytes + kValueCodes + vmeta_page_bytes;
+  constexpr int kMetaBytes = 128 * 2 * GN * 2;
   int bh = 0;
-  auto issue = [&](int pg, int stage) {
-    // one lane starts the three bulk copies of a page; the barrier completes when all bytes landed
-    mbar_expect_tx(&ps.bar[stage], stage_tx);
-    const int64_t vrow = (int64_t)bh * d.max_value_tokens + (int64_t)pg * 128;
-    bulk_copy_g2s(ps.stage[stage], d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes, d.key_page_bytes, &ps.bar[stage]);
-    bulk_copy_g2s(ps.stage[stage] + kOffVCodes, d.v_codes + vrow * 32, kValueCodes, &ps.bar[stage]);
-    bulk_copy_g2s(ps.stage[stage] + kOffVMeta,
-                  reinterpret_cast<const uint8_t*>(d.v_meta) + vrow * (2 * d.value_groups * 2), vmeta_page_bytes, &ps.bar[stage]);
+  auto issue_keys = [&](int pg) {
+    mbar_expect_tx(&ws.k_bar, d.key_page_bytes);
+    bulk_copy_g2s(ws.keys, d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes, d.key_page_bytes, &ws.k_bar);
   };
-  if (issuer) {
-    mbar_init(&ps.bar[0], 1);
-    mbar_init(&ps.bar[1], 1);
+  auto issue_values = [&](int pg) {
+    mbar_expect_tx(&ws.v_bar, kValueCodes + kMetaBytes);
+    const int64_t vrow = (int64_t)bh * d.max_value_tokens + (int64_t)pg * 128;
+    bulk_copy_g2s(ws.values, d.v_codes + vrow * 32, kValueCodes, &ws.v_bar);
+    bulk_copy_g2s(ws.values + kValueCodes, reinterpret_cast<const uint8_t*>(d.v_meta) + vrow * (4 * GN), kMetaBytes, &ws.v_bar);
+  };
+  if (lane == 0) {
+    mbar_init(&ws.k_bar, 1);
+    mbar_init(&ws.v_bar, 1);
     mbar_fence_init();
   }
-  __syncthreads();
-  const int K = KP >= 0 ? KP : (d.key_mode == DARTKV_MIXED_PAGE ? d.promoted : 0);
-  const int prom_steps = (K + 7) >> 3;
-  const float scale2 = a.scale * kLog2e;
-  // weight operand: column n = g is (head g >> 1, j' = g & 1); the 32-bit word read holds the fp16 weights of the
-  // head pair g >> 2.  Take the head's half into half j' and zeros (from the second source) into the other.
-  const uint32_t head_bytes = ((g >> 1) & 1) ? 0x32u : 0x10u;
-  const uint32_t sel_w = (g & 1) ? (0x0054u | (head_bytes << 8)) : (head_bytes | 0x5400u);
-  const uint32_t mask_u = (g & 1) ? 0xFFFF0000u : 0x0000FFFFu;
-  uint32_t* utab = ps.u[hf];
+  __syncwarp();
+  FusedWork<DT, MD, GN, KP> work(d, bs.query, a.scale, lane);
   bool ok = true;
-  int iter = 0;   // pages this pair has consumed so far: stage and barrier parity carry over from row to row
+  uint32_t parity = 0;   // of the pages this warp has consumed so far
 
   while (unit < unit_end) {
     bh = unit / a.quads;
@@ -352,145 +447,45 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
     const int p_begin = max(4 * quad_begin, row_first > d.sink_tokens ? (row_first - d.sink_tokens) >> 7 : 0);
     const int p_end = min(4 * (quad_begin + quad_count), total_pages);
 
-    // the first two pages of this pair are requested before anything else, so their latency overlaps the
-    // query load below
-    const int pg0 = p_begin + pair;
-    if (issuer) {
-      if (pg0 < p_end) issue(pg0, iter & 1);
-      if (pg0 + kPairs < p_end) issue(pg0 + kPairs, (iter + 1) & 1);
-    }
+    // this warp's first page is requested before anything else, so its latency overlaps the query load below
+    const int pg0 = p_begin + warp;
+    if (lane == 0 && pg0 < p_end) { issue_keys(pg0); issue_values(pg0); }
 
-    // query as fp32 and its largest magnitude (bounds the page weights q*s)
-    {
-      const int b = bh / d.kv_heads, hkv = bh % d.kv_heads;
-      float amax = 0.0f;
-      for (int i = tid; i < 4 * 128; i += kThreads) {
-        const int r = i >> 7, ch = i & 127;
-        float v = 0.0f;
-        if (r < rep)
-          v = md_to_float<DT>(reinterpret_cast<const uint16_t*>(a.q)[((int64_t)b * a.query_heads + hkv * rep + r) * 128 + ch]);
-        bs.qf[ch][r] = v;
-        amax = fmaxf(amax, fabsf(v));
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      if (lane == 0) bs.merge_m[warp][0] = amax;   // scratch use before the merge
-    }
+    const int b = bh / d.kv_heads, hkv = bh % d.kv_heads;
+    if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)b * a.query_heads + hkv * rep, rep, lane);
     __syncthreads();
-    if (tid == 0) {
-      float amax = 0.0f;
-      for (int w = 0; w < kWarps; ++w) amax = fmaxf(amax, bs.merge_m[w][0]);
-      bs.q_absmax = amax;
-    }
-    __syncthreads();
-    const float q_absmax = bs.q_absmax;
 
-    WarpState st;
-#pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) st.o_acc[mt][i] = 0.0f;
-    st.m_run = -INFINITY; st.l_run = 0.0f; st.zs[0] = st.zs[1] = 0.0f;
-    st.fv_run = __uint_as_float(253u << 23); st.fv_inv_run = __uint_as_float(1u << 23);
-    for (int pg = pg0; pg < p_end; pg += kPairs, ++iter) {
-      const int stage = iter & 1;
-      const uint32_t parity = (iter >> 1) & 1;
-      ok = mbar_wait(&ps.bar[stage], parity) && ok;
-      const uint8_t* blob = ps.stage[stage];
-
-      // ---- per-page setup by the 64 threads of the pair: thread tp owns channels 2tp, 2tp+1
-      float f = 1.0f, f_inv = 1.0f;
-      {
-        const uint32_t* kscale2 = reinterpret_cast<const uint32_t*>(blob + d.key_off_scale);
-        const uint32_t* kzero2 = reinterpret_cast<const uint32_t*>(blob + d.key_off_zero);
-        // largest key scale of the page (every warp computes it for itself: no exchange needed)
-        const uint2 sc4 = reinterpret_cast<const uint2*>(kscale2)[lane];   // channels 4*lane .. 4*lane+3
-        uint32_t smax = max(max(sc4.x & 0xFFFFu, sc4.x >> 16), max(sc4.y & 0xFFFFu, sc4.y >> 16));
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, off));
-        pow2_normaliser(4.0f * q_absmax * md_to_float<MD>(smax), f, f_inv);
-
-        const int tp = 32 * hf + lane;
-        float s0, s1, z0, z1;
-        md_pair_to_float<MD>(kscale2[tp], s0, s1);
-        md_pair_to_float<MD>(kzero2[tp], z0, z1);
-        const float4 qa = *reinterpret_cast<const float4*>(bs.qf[2 * tp]);
-        const float4 qb = *reinterpret_cast<const float4*>(bs.qf[2 * tp + 1]);
-        const float sa = s0 * f, sb = s1 * f;
-        ps.w_low[stage][2 * tp] = make_uint2(pack_f16x2(qa.x * sa, qa.y * sa), pack_f16x2(qa.z * sa, qa.w * sa));
-        ps.w_low[stage][2 * tp + 1] = make_uint2(pack_f16x2(qb.x * sb, qb.y * sb), pack_f16x2(qb.z * sb, qb.w * sb));
-        // sum_ch q*z per head, reduced over the warp
-        float bz[4] = {fmaf(qa.x, z0, qb.x * z1), fmaf(qa.y, z0, qb.y * z1), fmaf(qa.z, z0, qb.z * z1), fmaf(qa.w, z0, qb.w * z1)};
-        // four sums over 32 lanes in 6 shuffles: halve the number of sums a lane carries at the first two levels
-        {
-          const bool up16 = lane & 16, up8 = lane & 8;
-          const float k0 = (up16 ? bz[2] : bz[0]) + __shfl_xor_sync(0xffffffffu, up16 ? bz[0] : bz[2], 16);
-          const float k1 = (up16 ? bz[3] : bz[1]) + __shfl_xor_sync(0xffffffffu, up16 ? bz[1] : bz[3], 16);
-          float k = (up8 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up8 ? k0 : k1, 8);   // head 2*up16 + up8
-          k += __shfl_xor_sync(0xffffffffu, k, 4);
-          k += __shfl_xor_sync(0xffffffffu, k, 2);
-          k += __shfl_xor_sync(0xffffffffu, k, 1);
-          if ((lane & 7) == 0) ps.bias_part[stage][hf][lane >> 3] = k;
-        }
-        // promoted slots: warp 1 of the pair, lane = slot
-        if (hf == 1 && prom_steps > 0) {
-          uint2 wh = make_uint2(0u, 0u), wl = make_uint2(0u, 0u);
-          if (lane < K) {
-            const int ch = reinterpret_cast<const int32_t*>(blob + d.key_off_index)[lane] & 127;
-            const float s4 = 4.0f * f * md_to_float<MD>(reinterpret_cast<const uint16_t*>(blob + d.key_off_scale)[ch]);
-            const float4 qh = *reinterpret_cast<const float4*>(bs.qf[ch]);
-            const float e0 = qh.x * s4, e1 = qh.y * s4, e2 = qh.z * s4, e3 = qh.w * s4;
-            wh = make_uint2(pack_f16x2(e0, e1), pack_f16x2(e2, e3));
-            const float2 h01 = __half22float2(*reinterpret_cast<const __half2*>(&wh.x));
-            const float2 h23 = __half22float2(*reinterpret_cast<const __half2*>(&wh.y));
-            wl = make_uint2(pack_f16x2(e0 - h01.x, e1 - h01.y), pack_f16x2(e2 - h23.x, e3 - h23.y));
-          }
-          ps.w_high[stage][lane] = wh;
-          ps.w_high_lo[stage][lane] = wl;
-        }
-      }
-      // the only meeting point of the pair per page: the tables of this page are complete and both warps are done
-      // with the page before, whose stage can take the page after this one
-      pair_barrier(pair);
-      if (issuer && pg != pg0 && pg + kPairs < p_end) issue(pg + kPairs, stage ^ 1);
-
-      fused_page_half<MD, GN>(hf, stage, d, ps, blob, utab, prom_steps, scale2, f_inv, g, c, sel_w, mask_u,
-                              row_first - (d.sink_tokens + 128 * pg), st);
-
+    work.start_row();
+    for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
+      ok = mbar_wait(&ws.k_bar, parity) && ok;
+      work.fill_table(ws.keys, ws.scratch);
+      __syncwarp();
+      float s_acc[4][4];
+      work.logits(ws.keys, ws.scratch, s_acc);
+      __syncwarp();
+      // the keys are consumed: their buffer takes the next page's while the values are worked on
+      if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
+      work.softmax(s_acc, row_first - (d.sink_tokens + 128 * pg), ws.scratch, [&] { ok = mbar_wait(&ws.v_bar, parity) && ok; }, ws.values);
+      __syncwarp();
+      work.weigh_values(ws.values, ws.scratch);
+      __syncwarp();
+      if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
     }
 
-    // ---- hand the warp state to the block merge: sums over the lanes that share head c
-#pragma unroll
-    for (int off = 4; off < 32; off <<= 1) {
-      st.l_run += __shfl_xor_sync(0xffffffffu, st.l_run, off);
-      st.zs[0] += __shfl_xor_sync(0xffffffffu, st.zs[0], off);
-      st.zs[1] += __shfl_xor_sync(0xffffffffu, st.zs[1], off);
-    }
     __syncthreads();   // every warp is done with its stages: the staging memory becomes the merge buffer
-    if (g == 0) { bs.merge_m[warp][c] = st.m_run; bs.merge_l[warp][c] = st.l_run; }
-    {
-      const int wi = g & 3, xy = g >> 2;
-      const float unit = st.fv_inv_run * 16777216.0f;   // accumulators hold codes * 4^p * 2^-24 * fv
-      const float pos_scale[5] = {unit, unit * 0.25f, unit * 0.0625f, unit * 0.015625f, unit * 0.00390625f};
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int u = 2 * mt + (i >> 1), jp = i & 1;
-          const int p = u < 5 ? u : u - 5;
-          const int ch = 64 * jp + 16 * wi + 8 * xy + u;
-          warp_out[(warp * 4 + c) * 128 + ch] = fmaf(st.o_acc[mt][i], pos_scale[p], st.zs[jp]);
-        }
-    }
+    work.hand_over(warp_out + warp * 512);
+    if (lane < 4) { bs.merge_m[warp][lane] = work.m_run; bs.merge_l[warp][lane] = work.l_run; }
     __syncthreads();
     block_merge(a, bs, warp_out, bh / d.kv_heads, bh % d.kv_heads, rep,
                 1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
-    __syncthreads();   // the merge buffer is staging memory again, the query table may be overwritten
+    // the merge buffer is staging memory again, the query table may be overwritten
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
   }
   if (!ok && lane == 0) atomicExch(a.status, 1);
 }
 
-constexpr size_t kFusedSmemBytes = sizeof(FusedPairSmem) * kPairs + sizeof(FusedBlockSmem);
+constexpr size_t kFusedSmemBytes = sizeof(FusedWarpSmem) * kWarps + sizeof(FusedBlockSmem);
 
 }  // namespace
 
