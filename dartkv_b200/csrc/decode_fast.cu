@@ -27,7 +27,7 @@ namespace {
 struct WarpSmem {
   uint8_t keys[kPageBytesK];
   uint8_t values[kStageBytes - kPageBytesK];   // codes, then scales and zero points
-  PageScratch<4> scratch;
+  PageScratch scratch;
   uint64_t k_bar, v_bar;
 };
 
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
     mbar_fence_init();
   }
   __syncwarp();
-  PageWork<DT, OUT, GN, KP, 4> work(d, bs.q32, a.scale, lane, 0);
+  PageWork<DT, OUT, GN, KP> work(d, bs.q32, a.scale, lane);
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 

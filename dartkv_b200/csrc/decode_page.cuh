@@ -1,5 +1,5 @@
 // One page of the per-op rounded decode on tensor cores, as one warp works on it: contraction table, logits, online softmax,
-// P.V.  Shared by the kernels that give a warp whole pages and those that let several warps share a page's tokens.
+// P.V.
 //
 // Packed 2-bit codes are turned into exactly rounded 16-bit operands with one logic op and two packed fma/add per pair
 // (mma_utils.cuh) and fed straight into m16n8k16 MMAs; K and V are never materialized.  Keys: a register of the operand
@@ -11,22 +11,20 @@
 // of the four heads' probabilities, so one MMA accumulates both.
 //
 // Lane (g, c) = (lane >> 2, lane & 3).  A thread reads the whole 32-bit word g of a channel's code row, tokens 16g .. 16g+15;
-// register u pairs tokens 16g + u and 16g + u + 8, and two registers make an m-tile.  MT: m-tiles of this warp, 4 for the
-// whole page; with MT = 4 / S the S warps of a page take the registers u0 .. u0 + 2 MT - 1 each, u0 = 2 MT * part.
+// register u pairs tokens 16g + u and 16g + u + 8, and registers 2mt, 2mt + 1 are the row halves of m-tile mt.
 #pragma once
 
 #include "decode_fast_common.cuh"
 
 namespace {
 
-template <int MT> constexpr int kProbStride = 32 * MT + 8;   // 16-bit elements per (part, head) row of the probabilities
+constexpr int kProbStride = 136;   // 16-bit elements per (part, head) row of the probabilities: 128 tokens, 8 pad
 
 // what a warp needs beside a staged page; the probabilities take the table's place after the logits
-template <int MT>
 union PageScratch {
   // by contraction position: (s, s), (z, z), (-magic0*s, -magic1*s), (-magic2*s, byte offset of the channel's row)
   uint4 table[128];
-  uint16_t prob[2 * 4 * kProbStride<MT>];   // [hi/lo][head][local token]
+  uint16_t prob[2 * 4 * kProbStride];   // [hi/lo][head][local token]
 };
 
 // the dequantized registers of a code word, from the metadata dtype to the cache dtype (nothing when they agree)
@@ -47,7 +45,7 @@ __device__ __forceinline__ uint32_t high_twice(uint32_t x) { return prmt(x, x, 0
 // the host (0, 8, 16, 24, 32), else -1 (read from the descriptor): with the count fixed the logits loops have
 // constant trip counts and no per-position "is this slot promoted" test.
 // COMPACT: the query as 16-bit values [channel][head] instead of pre-shifted words [channel][2 * head + j'].
-template <int DT, int OUT, int GN, int KP, int MT, bool COMPACT = false>
+template <int DT, int OUT, int GN, int KP, bool COMPACT = false>
 struct PageWork {
   using H = Half2Ops<DT>;
   using HO = Half2Ops<OUT>;
@@ -59,17 +57,16 @@ struct PageWork {
   const dartkv_cache_desc& d;
   const uint8_t* q_thread;   // this thread's column of the query: + 32 * channel, COMPACT + 8 * channel
   float scale2;
-  int lane, g, c, K, prom_steps, u0;
+  int lane, g, c, K, prom_steps;
   bool gv;                   // this thread's sixteen channels are of value group 1
   float o_acc[8][4];         // [m-tile][c-reg]: channel 16g + mt + 8(i>>1), head 2(c&1) + (i&1), high (c<2) or low part of P
   float m_run, l_run;        // head c, log2 domain
 
-  __device__ __forceinline__ PageWork(const dartkv_cache_desc& desc, const void* query_table, float scale, int lane_, int part)
+  __device__ __forceinline__ PageWork(const dartkv_cache_desc& desc, const void* query_table, float scale, int lane_)
       : d(desc), scale2(scale * kLog2e), lane(lane_), g(lane_ >> 2), c(lane_ & 3) {
     cc.init();
     K = KP >= 0 ? KP : (d.key_mode == DARTKV_MIXED_PAGE ? d.promoted : 0);
     prom_steps = (K + 7) >> 3;
-    u0 = 2 * MT * part;
     gv = (16 * g) / d.value_group;
     q_thread = reinterpret_cast<const uint8_t*>(query_table) + (COMPACT ? 2 * (g >> 1) : 4 * g);
   }
@@ -90,7 +87,7 @@ struct PageWork {
   }
 
   // contraction table: the promoted slots first, then the other channels in order
-  __device__ __forceinline__ void fill_table(const uint8_t* keys, PageScratch<MT>& scratch) const {
+  __device__ __forceinline__ void fill_table(const uint8_t* keys, PageScratch& scratch) const {
     const uint16_t* kscale = reinterpret_cast<const uint16_t*>(keys + d.key_off_scale);
     const uint16_t* kzero = reinterpret_cast<const uint16_t*>(keys + d.key_off_zero);
     auto fill = [&](int pos, int ch) {
@@ -114,14 +111,13 @@ struct PageWork {
   }
 
   // logits S[token pair][(head, j')] over the doubled contraction (channel, j), eight positions per step
-  __device__ __forceinline__ void logits(const uint8_t* keys, const PageScratch<MT>& scratch, float (&s_acc)[MT][4]) const {
+  __device__ __forceinline__ void logits(const uint8_t* keys, const PageScratch& scratch, float (&s_acc)[4][4]) const {
     const uint8_t* const low_thread = keys + 4 * g;                                                     // + 32 * channel
     const uint32_t* const high_thread = reinterpret_cast<const uint32_t*>(keys + d.key_off_high) + g;   // + 8 * slot
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
-    auto own = [&](uint32_t w) { return MT == 4 ? w : w >> (2 * u0); };   // this warp's codes of both halves, from bit 0 on
 #pragma unroll kPromUnroll
     for (int i = 0; i < prom_steps; ++i) {
       const int s0 = 8 * i + c, s1 = s0 + 4;
@@ -132,14 +128,14 @@ struct PageWork {
       // with a promoted count that is a multiple of eight every position of a promoted step is a promoted slot
       const uint32_t h0 = (KP >= 0 || s0 < K) ? high_thread[s0 * 8] : 0u;
       const uint32_t h1 = (KP >= 0 || s1 < K) ? high_thread[s1 * 8] : 0u;
-      uint32_t r0[2 * MT], r1[2 * MT];
-      dequant_word4<DT>(cc, own(w0), own(h0), e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), r0);
-      dequant_word4<DT>(cc, own(w1), own(h1), e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), r1);
+      uint32_t r0[8], r1[8];
+      dequant_word4<DT>(cc, w0, h0, e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), r0);
+      dequant_word4<DT>(cc, w1, h1, e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), r1);
       cast_registers<DT, OUT>(r0);
       cast_registers<DT, OUT>(r1);
       const uint32_t b0 = query(o0), b1 = query(o1);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+      for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
     }
 #pragma unroll kQkUnroll
     for (int i = prom_steps; i < 16; ++i) {
@@ -148,34 +144,34 @@ struct PageWork {
       const uint32_t o0 = e0.w >> 16, o1 = e1.w >> 16;
       const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0);
       const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1);
-      uint32_t r0[2 * MT], r1[2 * MT];
-      dequant_word2<DT>(cc, own(w0), e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), low_twice(e0.w), r0);
-      dequant_word2<DT>(cc, own(w1), e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), low_twice(e1.w), r1);
+      uint32_t r0[8], r1[8];
+      dequant_word2<DT>(cc, w0, e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), low_twice(e0.w), r0);
+      dequant_word2<DT>(cc, w1, e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), low_twice(e1.w), r1);
       cast_registers<DT, OUT>(r0);
       cast_registers<DT, OUT>(r1);
       const uint32_t b0 = query(o0), b1 = query(o1);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+      for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
     }
   }
 
-  // online softmax for head c (this thread's tokens are 16g + u + 8j, u = u0 + 2mt + (i >> 1), j = i & 1); the
+  // online softmax for head c (this thread's tokens are 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1); the
   // probabilities go to the table with the pairs (u, u + 8) side by side.  mask_below: tokens before it drop out.
-  __device__ __forceinline__ void softmax(float (&s_acc)[MT][4], int mask_below, PageScratch<MT>& scratch) {
+  __device__ __forceinline__ void softmax(float (&s_acc)[4][4], int mask_below, PageScratch& scratch) {
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_acc[mt][i] *= scale2;
     if (mask_below > 0) {   // the page that holds the row's first live token
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+      for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (16 * g + u0 + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
+          if (16 * g + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
     }
     float mx = -INFINITY;
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+    for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) mx = fmaxf(mx, s_acc[mt][i]);
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
@@ -186,9 +182,9 @@ struct PageWork {
     const float alpha = fast_exp2(m_run - m_ref);
     m_run = m_new;
     float psum = 0.0f;
-    uint32_t hi[2 * MT], lo[2 * MT];
+    uint32_t hi[8], lo[8];
 #pragma unroll
-    for (int u = 0; u < 2 * MT; ++u) {
+    for (int u = 0; u < 8; ++u) {
       const float p0 = fast_exp2(s_acc[u >> 1][2 * (u & 1)] - m_ref), p1 = fast_exp2(s_acc[u >> 1][2 * (u & 1) + 1] - m_ref);
       psum += p0 + p1;
       hi[u] = pack16<OUT>(p0, p1);
@@ -196,17 +192,12 @@ struct PageWork {
       unpack16<OUT>(hi[u], h0, h1);
       lo[u] = pack16<OUT>(p0 - h0, p1 - h1);
     }
-    uint16_t* const row_hi = &scratch.prob[c * kProbStride<MT> + 4 * MT * g];
-    uint16_t* const row_lo = &scratch.prob[(4 + c) * kProbStride<MT> + 4 * MT * g];
-    if constexpr (MT == 1) {
-      *reinterpret_cast<uint2*>(row_hi) = make_uint2(hi[0], hi[1]);
-      *reinterpret_cast<uint2*>(row_lo) = make_uint2(lo[0], lo[1]);
-    } else {
+    uint4* const row_hi = reinterpret_cast<uint4*>(&scratch.prob[c * kProbStride + 16 * g]);
+    uint4* const row_lo = reinterpret_cast<uint4*>(&scratch.prob[(4 + c) * kProbStride + 16 * g]);
 #pragma unroll
-      for (int k = 0; k < MT / 2; ++k) {
-        reinterpret_cast<uint4*>(row_hi)[k] = make_uint4(hi[4 * k], hi[4 * k + 1], hi[4 * k + 2], hi[4 * k + 3]);
-        reinterpret_cast<uint4*>(row_lo)[k] = make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
-      }
+    for (int k = 0; k < 2; ++k) {
+      row_hi[k] = make_uint4(hi[4 * k], hi[4 * k + 1], hi[4 * k + 2], hi[4 * k + 3]);
+      row_lo[k] = make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
     }
     l_run = l_run * alpha + psum;
     // the running maximum rarely moves after the first pages: skip the rescale when no lane needs it.  This thread's
@@ -225,10 +216,10 @@ struct PageWork {
   // O[channel][(part, head)] += V^T P, 16 tokens per step.  The code words of two tokens are byte-interleaved (low halves
   // together: channels 0..7 of both tokens; high halves: channels 8..15), so that the packed dequantization sees token a in
   // the low half and token b in the high half.  m-tile mt, row g is channel 16g + mt, row g+8 channel 16g + 8 + mt.
-  __device__ __forceinline__ void weigh_values(const uint8_t* values, const PageScratch<MT>& scratch) {
+  __device__ __forceinline__ void weigh_values(const uint8_t* values, const PageScratch& scratch) {
     const uint32_t* vcodes = reinterpret_cast<const uint32_t*>(values) + g;   // word g of a token row: + 8 * token
     const uint8_t* vmeta = values + kValueCodes;
-    const uint32_t* pb = reinterpret_cast<const uint32_t*>(&scratch.prob[g * kProbStride<MT>]) + c;   // column n = g
+    const uint32_t* pb = reinterpret_cast<const uint32_t*>(&scratch.prob[g * kProbStride]) + c;   // column n = g
     // byte selectors that bring the scale (zero point) of this thread's value group of tokens a and b together
     const uint32_t sel_s = GN == 2 ? (gv ? 0x7632u : 0x5410u) : 0x5410u;
     const uint32_t sel_z = GN == 2 ? (gv ? 0x7632u : 0x5410u) : 0x7632u;
@@ -252,13 +243,11 @@ struct PageWork {
       cast_registers<DT, OUT>(r_lo);
       cast_registers<DT, OUT>(r_hi);
     };
-    // pair p of the warp's tokens (the order of the table) is token 16 * (p / 2 MT) + u0 + p % (2 MT) and the one eight on
-    auto token = [&](int p) { return 16 * (p / (2 * MT)) + u0 + p % (2 * MT); };
 #pragma unroll kPvUnroll
-    for (int s = 0; s < 2 * MT; ++s) {
+    for (int s = 0; s < 8; ++s) {
       uint32_t r0_lo[8], r0_hi[8], r1_lo[8], r1_hi[8];
-      token_pair(token(8 * s + c), r0_lo, r0_hi);         // contraction index 2c, 2c + 1
-      token_pair(token(8 * s + c + 4), r1_lo, r1_hi);     // contraction index 2c + 8, 2c + 9
+      token_pair(16 * s + c, r0_lo, r0_hi);         // contraction index 2c, 2c + 1
+      token_pair(16 * s + c + 4, r1_lo, r1_hi);     // contraction index 2c + 8, 2c + 9
       const uint32_t b0 = pb[8 * s], b1 = pb[8 * s + 4];
 #pragma unroll
       for (int mt = 0; mt < 8; ++mt) HO::mma(o_acc[mt], r0_lo[mt], r0_hi[mt], r1_lo[mt], r1_hi[mt], b0, b1);
