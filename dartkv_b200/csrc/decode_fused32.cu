@@ -46,7 +46,6 @@ struct FusedWarpSmem {
   uint8_t keys[kPageBytesK];
   uint8_t values[kStageBytes - kPageBytesK];   // codes, then scales and zero points
   FusedScratch scratch;
-  uint64_t k_bar, v_bar;
 };
 
 struct FusedBlockSmem {
@@ -54,6 +53,7 @@ struct FusedBlockSmem {
   float merge_m[kWarps][4];
   float merge_l[kWarps][4];
   int slot_map[128];
+  uint64_t k_bar[kWarps], v_bar[kWarps];   // not beside the staging memory, which becomes the merge buffer
 };
 
 template <int DT>
@@ -418,18 +418,18 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   constexpr int kMetaBytes = 128 * 2 * GN * 2;
   int bh = 0;
   auto issue_keys = [&](int pg) {
-    mbar_expect_tx(&ws.k_bar, d.key_page_bytes);
-    bulk_copy_g2s(ws.keys, d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes, d.key_page_bytes, &ws.k_bar);
+    mbar_expect_tx(&bs.k_bar[warp], d.key_page_bytes);
+    bulk_copy_g2s(ws.keys, d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes, d.key_page_bytes, &bs.k_bar[warp]);
   };
   auto issue_values = [&](int pg) {
-    mbar_expect_tx(&ws.v_bar, kValueCodes + kMetaBytes);
+    mbar_expect_tx(&bs.v_bar[warp], kValueCodes + kMetaBytes);
     const int64_t vrow = (int64_t)bh * d.max_value_tokens + (int64_t)pg * 128;
-    bulk_copy_g2s(ws.values, d.v_codes + vrow * 32, kValueCodes, &ws.v_bar);
-    bulk_copy_g2s(ws.values + kValueCodes, reinterpret_cast<const uint8_t*>(d.v_meta) + vrow * (4 * GN), kMetaBytes, &ws.v_bar);
+    bulk_copy_g2s(ws.values, d.v_codes + vrow * 32, kValueCodes, &bs.v_bar[warp]);
+    bulk_copy_g2s(ws.values + kValueCodes, reinterpret_cast<const uint8_t*>(d.v_meta) + vrow * (4 * GN), kMetaBytes, &bs.v_bar[warp]);
   };
   if (lane == 0) {
-    mbar_init(&ws.k_bar, 1);
-    mbar_init(&ws.v_bar, 1);
+    mbar_init(&bs.k_bar[warp], 1);
+    mbar_init(&bs.v_bar[warp], 1);
     mbar_fence_init();
   }
   __syncwarp();
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
 
     work.start_row();
     for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
-      ok = mbar_wait(&ws.k_bar, parity) && ok;
+      ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
       work.fill_table(ws.keys, ws.scratch);
       __syncwarp();
       float s_acc[4][4];
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
       __syncwarp();
       // the keys are consumed: their buffer takes the next page's while the values are worked on
       if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
-      work.softmax(s_acc, row_first - (d.sink_tokens + 128 * pg), ws.scratch, [&] { ok = mbar_wait(&ws.v_bar, parity) && ok; }, ws.values);
+      work.softmax(s_acc, row_first - (d.sink_tokens + 128 * pg), ws.scratch, [&] { ok = mbar_wait(&bs.v_bar[warp], parity) && ok; }, ws.values);
       __syncwarp();
       work.weigh_values(ws.values, ws.scratch);
       __syncwarp();
