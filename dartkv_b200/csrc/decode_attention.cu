@@ -13,6 +13,8 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "mma_utils.cuh"
 
@@ -49,6 +51,8 @@ struct GenericArgs {
   float* part_l;
   float* part_acc;
   const int32_t* row_start;   // optional [batch] first live token of every batch row
+  int cluster;                // decode_tiles_kernel: blocks of a (batch, kv head)
+  void* out;                  // and where their results go
 };
 
 // One block per (batch, kv head) and run of tokens, in tiles of 32 tokens.  Keys: lane = token, the channels are dealt
@@ -271,6 +275,264 @@ __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __gri
       if (vsplit == 0) a.part_acc[row * D + vc] = acc[r];
     }
   }
+}
+
+template <int MD> __device__ __forceinline__ float load_md(const void* p, int64_t i) {
+  if (MD == DARTKV_F16) return __half2float(reinterpret_cast<const __half*>(p)[i]);
+  if (MD == DARTKV_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
+  return reinterpret_cast<const float*>(p)[i];
+}
+
+// Uniform key pages: what decode_generic_kernel does, with the chain of memory latencies of a tile cut to two.  Every lane
+// finds the place of its own token (sink, page, dense tail), so a tile is not cut at segment edges; pages are found without
+// a search where there are at most 32; the metadata dtype is a template argument (loads behind a run-time choice of dtype
+// are not batched); the tile's values are requested with its keys.  The blocks of a (batch, KV head), a.cluster of them,
+// are a cluster that merges its results through distributed shared memory.
+template <int REP, int MD>
+__global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __grid_constant__ dartkv_cache_desc d,
+                                                                      const __grid_constant__ GenericArgs a) {
+  extern __shared__ float smem[];
+  const int D = d.head_dim;
+  const int rep = a.query_heads / d.kv_heads;            // at most REP
+  float* s_q = smem;                                     // [D][REP]
+  float* s_part = s_q + D * REP;                         // [warp][REP][32] partial logits, then [split][REP][D] sums
+  float* s_p = s_part + GEN_THREADS * REP;               // [32][REP] probabilities of the tile
+  float* s_alpha = s_p + GEN_TILE * REP;                 // [REP]
+  float* s_m = s_alpha + REP;
+  float* s_l = s_m + REP;
+  static_assert(GEN_WARPS * GEN_TILE <= GEN_THREADS, "partial logits and sums share memory");
+
+  const int split = blockIdx.x % a.cluster, bh = blockIdx.x / a.cluster;
+  const int b = bh / d.kv_heads, h = bh % d.kv_heads;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int seen = d.state[0], pages = d.state[1], k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
+  const int first = split * a.chunk;
+  const int hi = (int)min((int64_t)first + a.chunk, (int64_t)seen);
+  const int lo = a.row_start ? max(first, a.row_start[b]) : first;
+  // irregular pages, a page per lane where there are few; regular ones are computed
+  int my_first = 0, my_tokens = 0;
+  const bool by_lane = !d.regular_pages && pages <= 32;
+  if (by_lane && lane < pages) { my_first = d.page_start[lane]; my_tokens = d.page_tokens[lane]; }
+  for (int i = tid; i < D * REP; i += GEN_THREADS) {
+    const int r = i % REP, c = i / REP;
+    s_q[i] = r < rep ? load_f(a.q, a.q_dt, ((int64_t)b * a.query_heads + h * rep + r) * D + c) : 0.0f;
+  }
+  if (tid < REP) { s_m[tid] = -INFINITY; s_l[tid] = 0.0f; }
+  const int vsplits = GEN_THREADS / D, vsplit = tid / D, vc = tid % D;
+  float acc[REP];
+#pragma unroll
+  for (int r = 0; r < REP; ++r) acc[r] = 0.0f;
+  const int bits = d.key_bits, vpb = 8 / bits, vbits = d.value_bits, per = 8 / vbits, vg = vc / d.value_group;
+  const uint32_t mask = (1u << bits) - 1u, vmask = (1u << vbits) - 1u;
+  auto value_flavour = [&](int tok) -> int {             // see decode_generic_kernel
+    if (a.flavour == DARTKV_DEQUANT_PER_OP || d.regular_pages) return a.flavour;
+    const int vs = d.sink_tokens + (tok - d.sink_tokens) / d.page_size * d.page_size;
+    const int ve = min(v_end, vs + d.page_size);
+    if (vs >= k_end) return a.flavour;
+    const int pg = gen_find_page(d, pages, vs);
+    return d.page_start[pg] + d.page_tokens[pg] < ve ? DARTKV_DEQUANT_PER_OP : a.flavour;
+  };
+  __syncthreads();
+
+  for (int tile0 = lo; tile0 < hi; tile0 += GEN_TILE) {
+    const int nt = min(GEN_TILE, hi - tile0);
+    const int tok = tile0 + min(lane, nt - 1);           // lanes past the tile repeat its last token
+    // ---- the place of this lane's key
+    const bool packed = tok >= sink_filled && tok < k_end;
+    int page_first = 0, page_n = 1, pg = 0, key_flavour = a.flavour;
+    if (by_lane) {
+      for (int i = 0; i < pages; ++i) {
+        const int f = __shfl_sync(0xffffffffu, my_first, i), n = __shfl_sync(0xffffffffu, my_tokens, i);
+        if (f <= tok && tok < f + n) { page_first = f; page_n = n; pg = i; }
+      }
+    } else if (packed && d.regular_pages) {
+      pg = (tok - d.sink_tokens) / d.page_size;
+      page_first = d.sink_tokens + pg * d.page_size;
+      page_n = d.page_size;
+    } else if (packed) {
+      pg = gen_find_page(d, pages, tok);
+      page_first = d.page_start[pg];
+      page_n = d.page_tokens[pg];
+    }
+    const uint8_t* page = d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes;
+    if (a.flavour != DARTKV_DEQUANT_PER_OP && packed && page_first < v_end) {   // see decode_generic_kernel
+      const int next_value_edge = d.sink_tokens + ((page_first - d.sink_tokens) / d.page_size + 1) * d.page_size;
+      if (min(next_value_edge, v_end) < page_first + page_n) key_flavour = DARTKV_DEQUANT_PER_OP;
+    }
+    // ---- the tile's values are requested (the first kAhead of this thread's tokens)
+    constexpr int kAhead = REP <= 4 ? 16 : 8;
+    uint32_t v_code[kAhead];
+    float v_scale[kAhead], v_zero[kAhead];
+    auto value_packed = [&](int t) { return t >= sink_filled && t < v_end; };
+    auto dense_value = [&](int t) {
+      return t < sink_filled ? load_f(d.v_sink, d.dtype, ((int64_t)bh * d.sink_tokens + t) * D + vc)
+                             : load_f(d.v_ring, d.dtype, ((int64_t)bh * d.ring_tokens + (t % d.ring_tokens)) * D + vc);
+    };
+    auto value_row = [&](int t) { return (int64_t)bh * d.max_value_tokens + (t - d.sink_tokens); };
+    if (vsplit < vsplits) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int t = tile0 + vsplit + i * vsplits;
+        v_code[i] = 0; v_scale[i] = v_zero[i] = 0.0f;
+        if (t < tile0 + nt && value_packed(t)) {
+          const int64_t row = value_row(t);
+          v_code[i] = d.v_codes[row * d.value_row_bytes + vc / per];
+          v_scale[i] = load_md<MD>(d.v_meta, (row * 2 + 0) * d.value_groups + vg);
+          v_zero[i] = load_md<MD>(d.v_meta, (row * 2 + 1) * d.value_groups + vg);
+        }
+      }
+    }
+    // ---- partial logits of this warp's channels
+    float dot[REP];
+#pragma unroll
+    for (int r = 0; r < REP; ++r) dot[r] = 0.0f;
+    auto add = [&](int c, float k) {
+#pragma unroll
+      for (int r = 0; r < REP; ++r) dot[r] = fmaf(s_q[c * REP + r], k, dot[r]);
+    };
+    if (packed) {
+      const int j = tok - page_first, g = j / d.key_group, G = ceil_div(page_n, d.key_group);
+      const int row_bytes = ceil_div(G * d.key_group, vpb);
+      const uint8_t* codes = page + j / vpb;
+      const int shift = (j % vpb) * bits;
+      const uint8_t *scale = page + d.key_off_scale, *zero = page + d.key_off_zero;
+#pragma unroll 2
+      for (int c0 = warp; c0 < D; c0 += 8 * GEN_WARPS) {
+        uint32_t code[8];
+        float s[8], z[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int c = min(c0 + i * GEN_WARPS, D - 1);
+          code[i] = codes[c * row_bytes];
+          s[i] = load_md<MD>(scale, c * G + g);
+          z[i] = load_md<MD>(zero, c * G + g);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (c0 + i * GEN_WARPS < D)
+            add(c0 + i * GEN_WARPS, affine_restore((float)((code[i] >> shift) & mask), s[i], z[i], MD, d.dtype, key_flavour));
+      }
+    } else {
+      const void* rows = tok < sink_filled ? d.k_sink : d.k_ring;
+      const int64_t row = tok < sink_filled ? (int64_t)bh * d.sink_tokens + tok : (int64_t)bh * d.ring_tokens + tok % d.ring_tokens;
+      if (d.dtype == DARTKV_F32) {
+        const float* k = reinterpret_cast<const float*>(rows) + row * D;
+#pragma unroll 16
+        for (int c = warp; c < D; c += GEN_WARPS) add(c, k[c]);
+      } else {
+#pragma unroll 8
+        for (int c = warp; c < D; c += GEN_WARPS) add(c, load_f(rows, d.dtype, row * D + c));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < REP; ++r) s_part[(warp * REP + r) * GEN_TILE + lane] = dot[r];
+    __syncthreads();
+    // ---- online softmax state, a warp per query head
+    for (int r = warp; r < rep; r += GEN_WARPS) {
+      float v = 0.0f;
+#pragma unroll
+      for (int w = 0; w < GEN_WARPS; ++w) v += s_part[(w * REP + r) * GEN_TILE + lane];
+      v = lane < nt ? v * a.scale : -INFINITY;
+      float mx = v;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float m_old = s_m[r], m_new = fmaxf(m_old, mx);
+      const float m_ref = m_new == -INFINITY ? 0.0f : m_new;   // every logit so far -Inf or NaN: the former weigh nothing
+      const float e = expf(v - m_ref);
+      float sum = e;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      s_p[lane * REP + r] = e;
+      __syncwarp();
+      if (lane == 0) {
+        const float alpha = expf(m_old - m_ref);
+        s_alpha[r] = alpha;
+        s_m[r] = m_new;
+        s_l[r] = s_l[r] * alpha + sum;
+      }
+    }
+    __syncthreads();
+    // ---- values
+    if (vsplit < vsplits) {
+#pragma unroll
+      for (int r = 0; r < REP; ++r) acc[r] *= r < rep ? s_alpha[r] : 0.0f;
+      auto weigh = [&](int tt, float v) {
+#pragma unroll
+        for (int r = 0; r < REP; ++r) acc[r] = fmaf(r < rep ? s_p[tt * REP + r] : 0.0f, v, acc[r]);
+      };
+      const int vshift = (vc % per) * vbits;
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int tt = vsplit + i * vsplits;
+        if (tt < nt)
+          weigh(tt, value_packed(tile0 + tt) ? affine_restore((float)((v_code[i] >> vshift) & vmask), v_scale[i], v_zero[i], MD, d.dtype,
+                                                              value_flavour(tile0 + tt))
+                                             : dense_value(tile0 + tt));
+      }
+#pragma unroll 4
+      for (int tt = vsplit + kAhead * vsplits; tt < nt; tt += vsplits) {
+        const int t = tile0 + tt;
+        const int64_t row = value_row(t);
+        weigh(tt, value_packed(t) ? affine_restore((float)((d.v_codes[row * d.value_row_bytes + vc / per] >> vshift) & vmask),
+                                                   load_md<MD>(d.v_meta, (row * 2 + 0) * d.value_groups + vg),
+                                                   load_md<MD>(d.v_meta, (row * 2 + 1) * d.value_groups + vg), MD, d.dtype, value_flavour(t))
+                                  : dense_value(t));
+      }
+    }
+    __syncthreads();
+  }
+
+  // the token shares of a channel meet in shared memory
+  if (vsplit < vsplits)
+#pragma unroll
+    for (int r = 0; r < REP; ++r) s_part[(vsplit * REP + r) * D + vc] = acc[r];
+  __syncthreads();
+  if (vsplit == 0)
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      acc[r] = 0.0f;
+      for (int s = 0; s < vsplits; ++s) acc[r] += s_part[(s * REP + r) * D + vc];
+    }
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  if (vsplit == 0)
+#pragma unroll
+    for (int r = 0; r < REP; ++r) s_part[r * D + vc] = acc[r];   // nobody else reads these entries before the cluster meets
+  cluster.sync();
+  for (int i = split * GEN_THREADS + tid; i < rep * D; i += a.cluster * GEN_THREADS) {
+    const int r = i / D, c = i - r * D;
+    float m = -INFINITY, l = 0.0f, sum = 0.0f;
+    for (int k = 0; k < a.cluster; ++k) m = fmaxf(m, *cluster.map_shared_rank(&s_m[r], k));
+    for (int k = 0; k < a.cluster; ++k) {
+      const float mk = *cluster.map_shared_rank(&s_m[r], k), lk = *cluster.map_shared_rank(&s_l[r], k);
+      if (mk != -INFINITY || lk != lk) {   // a NaN logit does not show in the maximum
+        const float w = lk == lk ? expf(mk - m) : lk;
+        l = fmaf(lk, w, l);
+        sum = fmaf(*cluster.map_shared_rank(&s_part[r * D + c], k), w, sum);   // Inf and NaN count even where the weight is zero
+      }
+    }
+    store_f(a.out, a.q_dt, ((int64_t)b * a.query_heads + h * rep + r) * D + c, sum * (1.0f / fmaxf(l, 1e-20f)));
+  }
+  cluster.sync();   // no block leaves while another one reads its results
+}
+
+static size_t tiles_smem(int D, int rep) {
+  return ((size_t)D * rep + (size_t)GEN_THREADS * rep + (size_t)GEN_TILE * rep + 3 * rep) * sizeof(float);
+}
+
+using GenericKernel = void (*)(const dartkv_cache_desc, const GenericArgs);
+template <int MD>
+static GenericKernel tiles_variant_of(int rep) {
+  switch (rep) {
+    case 1: return decode_tiles_kernel<1, MD>;
+    case 2: return decode_tiles_kernel<2, MD>;
+    case 4: return decode_tiles_kernel<4, MD>;
+    case 8: return decode_tiles_kernel<8, MD>;
+    default: return decode_tiles_kernel<16, MD>;
+  }
+}
+static GenericKernel tiles_variant(int md, int rep) {
+  return md == DARTKV_F32 ? tiles_variant_of<DARTKV_F32>(rep) : md == DARTKV_F16 ? tiles_variant_of<DARTKV_F16>(rep) : tiles_variant_of<DARTKV_BF16>(rep);
 }
 
 // shared memory of decode_generic_kernel<REP>; the sums of up to GEN_THREADS channels reuse the partial logits
@@ -733,10 +995,33 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     a.row_start = row_start;
     DARTKV_REQUIRE(L.generic_splits <= 65535, "too many splits");
     const int padded_rep = rep <= 1 ? 1 : rep <= 2 ? 2 : rep <= 4 ? 4 : rep <= 8 ? 8 : 16;
-    const size_t smem = generic_smem(D, padded_rep);
-    const auto kernel = padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
+    // Uniform pages of few tiles: decode_tiles_kernel, whose blocks of a KV head are a cluster of the portable size at most
+    // and two of which fit an SM: [1,8,256,128] fp32, 2-bit 31.2 -> 21.0 us (23 with a merge launch of its own).  Calls of more
+    // blocks need the occupancy of decode_generic_kernel (four of 2,048 tokens 80 us there, 107 as tiles), and calls of
+    // more tiles gain nothing (two of 700 tokens, 64 channels: 18.7 us there, 19.5 as tiles).
+    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_splits <= 8 && !peers && bh * L.generic_splits <= 2 * dartkv_sm_count();
+    a.cluster = tiles ? L.generic_splits : 0;
+    a.out = out;
+    const size_t smem = tiles ? tiles_smem(D, padded_rep) : generic_smem(D, padded_rep);
+    const GenericKernel kernel = tiles ? tiles_variant(d->md_dtype, padded_rep) : padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
                       : padded_rep == 4 ? decode_generic_kernel<4> : padded_rep == 8 ? decode_generic_kernel<8> : decode_generic_kernel<16>;
     if (smem > 48 * 1024) DARTKV_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (a.cluster) {
+      cudaLaunchConfig_t config = {};
+      config.gridDim = dim3((unsigned)(bh * a.cluster));
+      config.blockDim = dim3(GEN_THREADS);
+      config.dynamicSmemBytes = smem;
+      config.stream = stream;
+      cudaLaunchAttribute attribute = {};
+      attribute.id = cudaLaunchAttributeClusterDimension;
+      attribute.val.clusterDim.x = a.cluster;
+      attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+      config.attrs = &attribute;
+      config.numAttrs = 1;
+      DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, kernel, *d, a));
+      DARTKV_LAUNCH_OK("decode_tiles_kernel");
+      return DARTKV_OK;
+    }
     kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
     DARTKV_LAUNCH_OK("decode_generic_kernel");
   }
