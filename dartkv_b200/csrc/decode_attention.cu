@@ -60,8 +60,8 @@ struct GenericArgs {
 // a dot product needs no shuffles; the warps' partial logits meet in shared memory.  Values: thread = channel, the
 // tile's tokens split over the remaining threads.  Nothing dequantized is staged.  Latency is what counts here (small
 // fp32 caches): loads of several channels / tokens are in flight together, and a call is cut into tiles until every SM
-// has a block.  [1,8,256,128] fp32, 2-bit: 98 us per call with one serial dot product per thread and staged tiles, now 31
-// us, of which this kernel is some 26 (B200).
+// has a block.  [1,8,256,128] fp32, 2-bit: 98 us per call with one serial dot product per thread and staged tiles, 31 us so
+// (B200; decode_tiles_kernel, which takes such small calls of uniform pages, 21).
 template <int REP>
 __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                      const __grid_constant__ GenericArgs a) {

@@ -15,7 +15,7 @@
 // operand register, address arithmetic, shifts; packed 16-bit arithmetic: two per register), and four warps per scheduler to
 // keep them so.  Time goes with the number of instructions.  Batch 128, 32,768 tokens: 1,143 us with two warps per page that
 // split the logits by channels, the rest by tokens, and met twice per page; 1,080 us with a warp per page, which fills
-// one table instead of two and exchanges nothing (B200).
+// one table instead of two and exchanges nothing (B200; 1,091 us with the barriers where the merge buffer cannot reach them).
 // Algorithmic HBM bytes per page and (batch, kv head): 10880.
 
 #include <atomic>
