@@ -3,10 +3,13 @@
 // keeps the kernels of quantize.cu, which handle one group (or element) per thread.
 //
 // All of these are bound by memory latency and by the few instructions per element, not by capacity: a group's tokens
-// are split over up to four threads per channel pair, loads run eight deep, codes gather in registers (quant_math.cuh)
+// are split over up to four threads per channel pair, and requested at once where they fit registers, codes gather in registers (quant_math.cuh)
 // and leave as whole words.  fp16 [8,8,1024,128], 2-bit + promoted keys / 2-bit values, a call among others: keys with the
-// selection 24.6 us, values 12.3, restoring either 10.3; all four calls with their checks and waits 102 us, 503 with one
+// selection 24.6 us, values 12.3, restoring either 10.3; all four calls with their checks and waits 103 us, 96 with the
+// tokens of a column group held in registers, several blocks per row for the scores and no 64-bit divisions; 503 with one
 // group or element per thread (B200).
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 #include "quant_math.cuh"
@@ -29,8 +32,10 @@ struct ColumnArgs {
 };
 
 // grid (group, slab of columns, outer); 64 threads per token split.  KB: 0 = mixed 2+2-bit keys, else the code width.
-template <int DT, int KB>
-__global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_constant__ ColumnArgs a) {
+// TOK: tokens of a thread where that is 8, 16 or 32 (groups of 32, 64 and 128): all are requested at once and kept in registers
+// between the search for minimum and maximum and the codes; 0 for other groups, which read them twice, eight at a time.
+template <int DT, int KB, int TOK>
+__global__ void __launch_bounds__(256, TOK == 32 ? 2 : 4) quantize_columns_kernel(const __grid_constant__ ColumnArgs a) {
   using P = Pack16<DT>;
   constexpr int PB = KB == 0 ? 2 : KB, CODE_BITS = KB == 0 ? 4 : KB;
   constexpr int PER_HALF = 16 / PB;
@@ -54,12 +59,25 @@ __global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_cons
   const uint16_t* col = a.x + o * a.so + (live ? c0 : 0);
   // the last group is padded by repeating the final element
   auto at = [&](int t) { return __ldg(reinterpret_cast<const uint32_t*>(col + (int64_t)min(t, a.n - 1) * a.sn)); };
-  uint32_t mn2 = at(t_begin), mx2 = mn2;
+  uint32_t held[TOK > 0 ? TOK : 1];
+  uint32_t mn2, mx2;
+  if constexpr (TOK > 0) {
+#pragma unroll
+    for (int j = 0; j < TOK; ++j) held[j] = at(t_begin + j);
+    mn2 = mx2 = held[0];
+#pragma unroll
+    for (int j = 1; j < TOK; ++j) {
+      mn2 = P::min2(mn2, held[j]);
+      mx2 = P::max2(mx2, held[j]);
+    }
+  } else {
+    mn2 = mx2 = at(t_begin);
 #pragma unroll 8
-  for (int j = 1; j < tok; ++j) {
-    const uint32_t v = at(t_begin + j);
-    mn2 = P::min2(mn2, v);
-    mx2 = P::max2(mx2, v);
+    for (int j = 1; j < tok; ++j) {
+      const uint32_t v = at(t_begin + j);
+      mn2 = P::min2(mn2, v);
+      mx2 = P::max2(mx2, v);
+    }
   }
   s_mn[split][p] = mn2;
   s_mx[split][p] = mx2;
@@ -122,15 +140,15 @@ __global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_cons
   }
   const float inv_lo = inverse_scale(scale_lo), inv_hi = inverse_scale(scale_hi);
   const uint32_t cap2 = cap_pair<DT>(qmax_lo, qmax_hi);
-#pragma unroll 1
-  for (int w = 0; w < mine; ++w) {
+#pragma unroll (TOK > 0 ? TOK / (2 * PER_HALF) : 1)
+  for (int w = 0; w < (TOK > 0 ? TOK / (2 * PER_HALF) : mine); ++w) {
     uint32_t acc_a[2], acc_b[2];
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int base = t_begin + (2 * w + half) * PER_HALF;
       uint32_t x[PER_HALF];
 #pragma unroll
-      for (int u = 0; u < PER_HALF; ++u) x[u] = at(base + u);
+      for (int u = 0; u < PER_HALF; ++u) x[u] = TOK > 0 ? held[(2 * w + half) * PER_HALF + u] : at(base + u);
       auto codes = [&](int u) { return pair_codes<DT, CODE_BITS>(x[u], mn2, scale_lo, scale_hi, inv_lo, inv_hi, cap2); };
       if (KB == 0) {
         uint32_t even = 0u - magic_sum(MAGIC, 4, 4), odd = even;
@@ -158,12 +176,19 @@ __global__ void __launch_bounds__(256) quantize_columns_kernel(const __grid_cons
   }
 }
 
+template <int DT, int KB>
+void launch_columns_of(int tok, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
+  if (tok == 32) quantize_columns_kernel<DT, KB, 32><<<grid, threads, 0, stream>>>(a);
+  else if (tok == 16) quantize_columns_kernel<DT, KB, 16><<<grid, threads, 0, stream>>>(a);
+  else if (tok == 8 && KB >= 4) quantize_columns_kernel<DT, KB, KB >= 4 ? 8 : 0><<<grid, threads, 0, stream>>>(a);
+  else quantize_columns_kernel<DT, KB, 0><<<grid, threads, 0, stream>>>(a);
+}
 template <int DT>
-void launch_columns(int kb, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
-  if (kb == 0) quantize_columns_kernel<DT, 0><<<grid, threads, 0, stream>>>(a);
-  else if (kb == 2) quantize_columns_kernel<DT, 2><<<grid, threads, 0, stream>>>(a);
-  else if (kb == 4) quantize_columns_kernel<DT, 4><<<grid, threads, 0, stream>>>(a);
-  else quantize_columns_kernel<DT, 8><<<grid, threads, 0, stream>>>(a);
+void launch_columns(int kb, int tok, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
+  if (kb == 0) launch_columns_of<DT, 0>(tok, grid, threads, stream, a);
+  else if (kb == 2) launch_columns_of<DT, 2>(tok, grid, threads, stream, a);
+  else if (kb == 4) launch_columns_of<DT, 4>(tok, grid, threads, stream, a);
+  else launch_columns_of<DT, 8>(tok, grid, threads, stream, a);
 }
 
 bool is16(int dt) { return dt == DARTKV_F16 || dt == DARTKV_BF16; }
@@ -187,8 +212,8 @@ int dartkv_quantize_columns_fast(const void* x, int dtype, int64_t outer, int64_
   ColumnArgs a{reinterpret_cast<const uint16_t*>(x), so, sn, (int)n, (int)inner, group, (int)groups,
                groups * (int64_t)words * 4, values, high, indices, promoted, md, scale, zero, nonfinite};
   const dim3 grid((unsigned)groups, (unsigned)slabs, (unsigned)outer);
-  if (dtype == DARTKV_F16) launch_columns<DARTKV_F16>(key_bits, grid, 64 * splits, stream, a);
-  else launch_columns<DARTKV_BF16>(key_bits, grid, 64 * splits, stream, a);
+  if (dtype == DARTKV_F16) launch_columns<DARTKV_F16>(key_bits, group / splits, grid, 64 * splits, stream, a);
+  else launch_columns<DARTKV_BF16>(key_bits, group / splits, grid, 64 * splits, stream, a);
   DARTKV_LAUNCH_OK("quantize_columns_kernel");
   return 1;
 }
@@ -202,12 +227,17 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
                                                             int group, int md, uint8_t* __restrict__ values, void* scale_out,
                                                             void* zero_out, int32_t* nonfinite) {
   using P = Pack16<DT>;
+  // the eighths of a row are numbered through all rows: whole groups in order, so neither the group's number nor this
+  // lane's place in it needs a division, and the row only where rows are not contiguous
   const int per_row = n / 8, lanes = group / 8;
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = id < rows * per_row;
-  const int64_t row = live ? id / per_row : 0;
-  const int k = live ? (int)(id - row * per_row) : 0;
-  const uint4 raw = *reinterpret_cast<const uint4*>(x + row * so + 8 * k);
+  int64_t at = live ? 8 * id : 0;
+  if (so != n && live) {
+    const int64_t row = id < (1ll << 31) ? (int64_t)((uint32_t)id / (uint32_t)per_row) : id / per_row;
+    at = row * so + 8 * (id - row * per_row);
+  }
+  const uint4 raw = *reinterpret_cast<const uint4*>(x + at);
   const uint32_t v[4] = {raw.x, raw.y, raw.z, raw.w};
   uint32_t mn2 = P::min2(P::min2(v[0], v[1]), P::min2(v[2], v[3])), mx2 = P::max2(P::max2(v[0], v[1]), P::max2(v[2], v[3]));
   for (int off = 1; off < lanes; off <<= 1) {
@@ -256,9 +286,9 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
   else if (VB == 4) reinterpret_cast<uint32_t*>(values)[id] = half_word[0] | (half_word[GATHERS / 2] << 16);
   else reinterpret_cast<uint2*>(values)[id] = make_uint2(half_word[0] | (half_word[GATHERS > 1] << 16),
                                                          half_word[GATHERS / 2] | (half_word[GATHERS - 1] << 16));
-  if (k % lanes == 0) {
+  if (((int)id & (lanes - 1)) == 0) {   // a power of two, which divides the eighths of a row
     if (nonfinite && odd) *nonfinite = 1;
-    const int64_t g = row * (per_row / lanes) + k / lanes;
+    const int64_t g = id >> (31 - __clz(lanes));
     store_f(scale_out, md, g, scale);
     store_f(zero_out, md, g, mn);
   }
@@ -292,27 +322,31 @@ int dartkv_quantize_rows_fast(const void* x, int dtype, int64_t rows, int64_t n,
 // ---------------------------------------------------------------------------- channel scores and selection
 namespace {
 
-constexpr int kScoreSplits = 16;
+constexpr int kScoreSplits = 16, kScoreBlocks = 8;
 
 // Promoted channels of one (batch, head): sum |k| per channel in double, scores rounded to the data dtype, rank by (score
 // descending, channel ascending).  In fp16 the sum is exact in any order.  bf16 values can be further apart than a double
 // has bits; the error is then some 2^-50 of the sum, which changes the score only where the sum lies that close to a
-// boundary of the fp32 rounding that follows.  One block of 16 token splits x 64 channel
-// pairs; scores (optional) are written too.
+// boundary of the fp32 rounding that follows.  A cluster of blocks, each of 16 token splits x 64
+// channel pairs, shares a row's tokens and meets in the first block's shared memory; scores (optional) are written too.
 template <int DT>
 __global__ void __launch_bounds__(64 * kScoreSplits) score_select_kernel(const uint16_t* __restrict__ keys, int64_t tokens, int d,
                                                                          int64_t sbh, int64_t st, int count,
                                                                          uint16_t* scores, int32_t* indices) {
   using P = Pack16<DT>;
   __shared__ double s_sum[kScoreSplits][2][64];
+  __shared__ double s_all[kScoreBlocks][128];   // the blocks' sums, in the first one
   __shared__ uint32_t s_key[128];
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int blocks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int p = threadIdx.x & 63, split = threadIdx.x >> 6;
-  const int64_t r = blockIdx.x;
+  const int64_t r = blockIdx.x / blocks;
   double lo = 0.0, hi = 0.0;
   if (2 * p < d) {
     const uint16_t* col = keys + r * sbh + 2 * p;
 #pragma unroll 8
-    for (int64_t t = split; t < tokens; t += kScoreSplits) {
+    for (int64_t t = rank * kScoreSplits + split; t < tokens; t += blocks * kScoreSplits) {
       const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(col + t * st));
       lo += (double)fabsf(P::lo(v));
       hi += (double)fabsf(P::hi(v));
@@ -323,10 +357,20 @@ __global__ void __launch_bounds__(64 * kScoreSplits) score_select_kernel(const u
   __syncthreads();
   const int c = threadIdx.x;
   uint32_t key = 0;
+  double sum = 0.0;
   if (c < d) {
-    double sum = 0.0;
 #pragma unroll
     for (int s = 0; s < kScoreSplits; ++s) sum += s_sum[s][c & 1][c >> 1];
+  }
+  if (blocks > 1) {
+    cluster.sync();   // every block of the cluster has started
+    if (c < d) *cluster.map_shared_rank(&s_all[rank][c], 0) = sum;
+    cluster.sync();
+    if (rank > 0) return;
+    sum = 0.0;
+    for (int k = 0; k < blocks && c < d; ++k) sum += s_all[k][c];
+  }
+  if (c < d) {
     const uint16_t bits = P::bits(__fdiv_rn((float)sum, (float)tokens));
     if (scores) scores[r * d + c] = bits;
     // scores are non-negative 16-bit floats: their bit patterns order like integers
@@ -350,8 +394,21 @@ int dartkv_score_select_fast(const void* keys, int dtype, int64_t bh, int64_t to
   if (!is16(dtype) || d > 128 || d % 2 || sbh % 2 || st % 2 || (uintptr_t)keys % 4 || !fits_int(bh)) return 0;
   const uint16_t* k = reinterpret_cast<const uint16_t*>(keys);
   uint16_t* s = reinterpret_cast<uint16_t*>(scores);
-  if (dtype == DARTKV_F16) score_select_kernel<DARTKV_F16><<<(unsigned)bh, 64 * kScoreSplits, 0, stream>>>(k, tokens, (int)d, sbh, st, count, s, indices);
-  else score_select_kernel<DARTKV_BF16><<<(unsigned)bh, 64 * kScoreSplits, 0, stream>>>(k, tokens, (int)d, sbh, st, count, s, indices);
+  // blocks per row: as many as the SMs hold at a time (two on each), with at least 64 tokens per block and no less
+  int blocks = 1;
+  while (blocks < kScoreBlocks && bh * blocks * 2 <= 296 && tokens >= 64 * blocks * 2) blocks *= 2;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(bh * blocks));
+  config.blockDim = dim3(64 * kScoreSplits);
+  config.stream = stream;
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = blocks;
+  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, dtype == DARTKV_F16 ? score_select_kernel<DARTKV_F16> : score_select_kernel<DARTKV_BF16>, k,
+                                    tokens, (int)d, sbh, st, count, s, indices));
   DARTKV_LAUNCH_OK("score_select_kernel");
   return 1;
 }
@@ -430,14 +487,25 @@ __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant
   constexpr uint32_t MASK = (1u << BITS) - 1u;
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= total) return;
-  const int per_row = a.n / 8;
-  const int64_t row = id / per_row;
-  const int k = (int)(id - row * per_row), g = 8 * k / a.group;
+  // whole groups follow one another through all rows; divisions in 32 bits where they do
+  const int eighths = a.group / 8;
+  int64_t at = 8 * id, g;
+  if (total < (1ll << 31)) {
+    g = (uint32_t)id / (uint32_t)eighths;
+    if (a.so != a.n) {
+      const uint32_t row = (uint32_t)id / (uint32_t)(a.n / 8);
+      at = row * a.so + 8 * ((uint32_t)id - row * (uint32_t)(a.n / 8));
+    }
+  } else {
+    const int64_t row = id / (a.n / 8);
+    g = id / eighths;
+    at = row * a.so + 8 * (id - row * (a.n / 8));
+  }
   uint64_t codes;
   if (BITS == 2) codes = reinterpret_cast<const uint16_t*>(a.values)[id];
   else if (BITS == 4) codes = reinterpret_cast<const uint32_t*>(a.values)[id];
   else codes = reinterpret_cast<const uint64_t*>(a.values)[id];
-  const float s = meta16<MD>(a.scale, row * a.groups + g), z = meta16<MD>(a.zero, row * a.groups + g);
+  const float s = meta16<MD>(a.scale, g), z = meta16<MD>(a.zero, g);
   uint32_t v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -445,7 +513,7 @@ __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant
     const float hi = affine_restore((float)((uint32_t)(codes >> (BITS * (2 * i + 1))) & MASK), s, z, MD, OUT, a.flavour);
     v[i] = pack_pair<OUT>(lo, hi);
   }
-  reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + row * a.so)[k] = make_uint4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + at) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
 template <int MD, int OUT>
