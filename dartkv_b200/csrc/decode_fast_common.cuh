@@ -63,6 +63,10 @@ __device__ __forceinline__ float restore16(float code, float scale, float zero, 
   return MD == DT ? md : rnd16<DT>(md);
 }
 
+// The maximum a state enters a merge with.  A NaN logit shows in the sum l but not in the maximum m, and the merges take a
+// state whose maximum is -Inf for an empty one: a state with a NaN goes by NaN.
+__device__ __forceinline__ float merge_maximum(float m, float l) { return l == l ? m : l; }
+
 // ------------------------------------------------------------------------------------------------
 // dense tokens (sink prefix, unpacked tail, and tokens packed on one side only).  Tokens whose key and value rows
 // are both dense go through 16-token tiles: logits by m16n8k16 MMAs straight from the rows, probabilities
@@ -89,7 +93,7 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
   float m[4], l[4], acc[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    m[r] = -INFINITY;
+    m[r] = -3.402823466e38f;   // the lowest finite number: logits of -Inf then weigh exp2(-Inf) = 0 against it, not exp2(NaN)
     l[r] = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[r][i] = 0.0f;
@@ -300,7 +304,7 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
   // hand the warp state to the block merge: acc in channel order
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    if (lane == 0) { bs.merge_m[warp][r] = m[r]; bs.merge_l[warp][r] = l[r]; }
+    if (lane == 0) { bs.merge_m[warp][r] = l[r] == 0.0f ? -INFINITY : merge_maximum(m[r], l[r]); bs.merge_l[warp][r] = l[r]; }
 #pragma unroll
     for (int i = 0; i < 4; ++i) warp_out[(warp * 4 + r) * 128 + lane * 4 + i] = acc[r][i];
   }
@@ -354,7 +358,7 @@ __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, con
     }
     const int64_t row = ((int64_t)b * a.query_heads + hkv * rep + (ROW_GROUPS ? head0 : 0) + r) * a.total_splits + slot;
     if (ch == 0) {
-      a.part_m[row] = m == -INFINITY ? -INFINITY : m * 0.6931471805599453f;
+      a.part_m[row] = merge_maximum(m == -INFINITY ? -INFINITY : m * 0.6931471805599453f, l);
       a.part_l[row] = l;
     }
     a.part_acc[row * 128 + ch] = acc;

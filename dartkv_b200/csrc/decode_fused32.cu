@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
 
     __syncthreads();   // every warp is done with its stages: the staging memory becomes the merge buffer
     work.hand_over(warp_out + warp * 512);
-    if (lane < 4) { bs.merge_m[warp][lane] = work.m_run; bs.merge_l[warp][lane] = work.l_run; }
+    if (lane < 4) { bs.merge_m[warp][lane] = merge_maximum(work.m_run, work.l_run); bs.merge_l[warp][lane] = work.l_run; }
     __syncthreads();
     block_merge(a, bs, warp_out, bh / d.kv_heads, bh % d.kv_heads, rep,
                 1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));

@@ -163,7 +163,7 @@ __device__ __forceinline__ void rows_merge(const FastArgs& a, const RowsSmem<R>&
     }
     const int64_t row = (first_row + r) * a.total_splits + slot;
     if (ch == 0) {
-      a.part_m[row] = m == -INFINITY ? -INFINITY : m * 0.6931471805599453f;
+      a.part_m[row] = merge_maximum(m == -INFINITY ? -INFINITY : m * 0.6931471805599453f, l);
       a.part_l[row] = l;
     }
     a.part_acc[row * 128 + ch] = acc;
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int row = 2 * c + e;
-      if (g == 0 && row < R) { bs.merge_m[warp][row] = m_run[e]; bs.merge_l[warp][row] = l_run[e]; }
+      if (g == 0 && row < R) { bs.merge_m[warp][row] = merge_maximum(m_run[e], l_run[e]); bs.merge_l[warp][row] = l_run[e]; }
 #pragma unroll
       for (int mt = 0; mt < 8; ++mt)
 #pragma unroll

@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_wide_kernel(dartkv_cache_d
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     __syncthreads();   // every warp is done streaming: its memory becomes the merge buffer
-    if (c == 0 && g < 4) { bs.merge_m[warp][g] = m_run; bs.merge_l[warp][g] = l_run; }
+    if (c == 0 && g < 4) { bs.merge_m[warp][g] = merge_maximum(m_run, l_run); bs.merge_l[warp][g] = l_run; }
     if (g < 4) {
 #pragma unroll
       for (int n = 0; n < 16; ++n) {
