@@ -52,7 +52,7 @@ struct GenericArgs {
   float* part_acc;
   const int32_t* row_start;   // optional [batch] first live token of every batch row
   int cluster;                // decode_tiles_kernel: blocks of a (batch, kv head)
-  void* out;                  // and where their results go
+  void* out;                  // and where their results go; null: to the partials, one per row
 };
 
 // One block per (batch, kv head) and run of tokens, in tiles of 32 tokens.  Keys: lane = token, the channels are dealt
@@ -511,7 +511,14 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
         sum = fmaf(*cluster.map_shared_rank(&s_part[r * D + c], k), w, sum);   // Inf and NaN count even where the weight is zero
       }
     }
-    store_f(a.out, a.q_dt, ((int64_t)b * a.query_heads + h * rep + r) * D + c, sum * (1.0f / fmaxf(l, 1e-20f)));
+    const float v = sum * (1.0f / fmaxf(l, 1e-20f));
+    const int64_t row = (int64_t)b * a.query_heads + h * rep + r;
+    if (a.out != nullptr) {
+      store_f(a.out, a.q_dt, row * D + c, v);
+    } else {   // the row's only partial: the merge kernel delivers the same numbers to the peers
+      a.part_acc[row * D + c] = v;
+      if (c == 0) { a.part_m[row] = 0.0f; a.part_l[row] = 1.0f; }
+    }
   }
   cluster.sync();   // no block leaves while another one reads its results
 }
@@ -999,9 +1006,9 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     // and two of which fit an SM: [1,8,256,128] fp32, 2-bit 31.2 -> 21.0 us (23 with a merge launch of its own).  Calls of more
     // blocks need the occupancy of decode_generic_kernel (four of 2,048 tokens 80 us there, 107 as tiles), and calls of
     // more tiles gain nothing (two of 700 tokens, 64 channels: 18.7 us there, 19.5 as tiles).
-    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_splits <= 8 && !peers && bh * L.generic_splits <= 2 * dartkv_sm_count();
+    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_splits <= 8 && bh * L.generic_splits <= 2 * dartkv_sm_count();
     a.cluster = tiles ? L.generic_splits : 0;
-    a.out = out;
+    a.out = peers ? nullptr : out;
     const size_t smem = tiles ? tiles_smem(D, padded_rep) : generic_smem(D, padded_rep);
     const GenericKernel kernel = tiles ? tiles_variant(d->md_dtype, padded_rep) : padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
                       : padded_rep == 4 ? decode_generic_kernel<4> : padded_rep == 8 ? decode_generic_kernel<8> : decode_generic_kernel<16>;
@@ -1020,10 +1027,12 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
       config.numAttrs = 1;
       DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, kernel, *d, a));
       DARTKV_LAUNCH_OK("decode_tiles_kernel");
-      return DARTKV_OK;
+      if (!peers) return DARTKV_OK;
+      L.total_splits = 1;
+    } else {
+      kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
+      DARTKV_LAUNCH_OK("decode_generic_kernel");
     }
-    kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
-    DARTKV_LAUNCH_OK("decode_generic_kernel");
   }
   {
     cudaLaunchConfig_t config = {};
