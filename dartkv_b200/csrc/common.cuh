@@ -11,6 +11,7 @@
 // ---------------------------------------------------------------------------- errors
 void dartkv_set_error(const char* fmt, ...);
 void dartkv_count_launch();
+int dartkv_sm_count();   // of the current device
 
 #define DARTKV_REQUIRE(cond, ...)          \
   do {                                     \

@@ -772,7 +772,7 @@ int dartkv_decode_wide_launch(const dartkv_cache_desc* d, const void* query, int
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                               cudaStream_t stream);
 
-static int dartkv_sm_count() {
+int dartkv_sm_count() {
   // per device: a process may drive GPUs of different sizes
   static std::atomic<int> cached[64];
   int device = 0, count = 0;

@@ -397,9 +397,11 @@ int dartkv_score_select_fast(const void* keys, int dtype, int64_t bh, int64_t to
   if (!is16(dtype) || d > 128 || d % 2 || sbh % 2 || st % 2 || (uintptr_t)keys % 4 || !fits_int(bh)) return 0;
   const uint16_t* k = reinterpret_cast<const uint16_t*>(keys);
   uint16_t* s = reinterpret_cast<uint16_t*>(scores);
-  // blocks per row: as many as the SMs hold at a time (two on each), with at least 64 tokens per block and no less
+  // blocks per row: as many as the SMs hold at a time (two on each; with twice as many [8,8,512,128] takes 34.0 us instead of
+  // 28.2, [8,8,4096,128] 68.4 instead of 65.1), with at least 128 tokens each ([4,8,512,128]: 25.2 us, with 64 tokens 27.1, one
+  // block a row 26.5; [4,8,1024,128]: 28.3, one block a row 30.8; whole quantize_key_mixed calls)
   int blocks = 1;
-  while (blocks < kScoreBlocks && bh * blocks * 2 <= 296 && tokens >= 64 * blocks * 2) blocks *= 2;
+  while (blocks < kScoreBlocks && bh * blocks * 2 <= 2 * dartkv_sm_count() && tokens >= 128 * blocks * 2) blocks *= 2;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)(bh * blocks));
   config.blockDim = dim3(64 * kScoreSplits);
