@@ -675,10 +675,12 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
 }
 
 // The merge of rows of few slots without peers: a warp per row, four channels a lane, eight rows a block.  Bound by latency;
-// a block per row with a channel per thread took the larger calls two waves of blocks and every thread seventeen predicated
-// loads: whole decode call of batch 128, 32,768 tokens 1,087 -> 1,079 us, batch 32, 8,192 tokens 93.1 -> 90.5, batch 24 of
-// 6,001 tokens in 4 bits 74.2 -> 69.9, 48 generation steps of two layers 1,027 -> 986 (B200).
-constexpr int kRowSlots = 5;
+// a block per row with a channel per thread takes the larger calls two waves of blocks and every thread seventeen predicated
+// loads: whole decode call of batch 128, 32,768 tokens 1,097 -> 1,089 us, batch 32, 8,192 tokens 94.3 -> 91.5, batch 24 of
+// 6,001 tokens in 4 bits 73.4 -> 69.4.  Eight slots: with room for five only, calls of six to eight slots (batch 1, 2,700 and
+// 3,300 tokens) take 14.3 us instead of 12.3; with room for seventeen, calls of two and three slots take 13.3 to 14.3 us
+// instead of 12.3 and calls of nine to seventeen gain nothing (B200).
+constexpr int kRowSlots = 8;   // the lanes of the reductions below
 __global__ void __launch_bounds__(256) decode_merge_rows_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
                                                                 const float* __restrict__ part_acc, int total_splits, int D, void* out,
                                                                 int out_dt, int stream_blocks, int64_t units, int quads, int query_heads,
