@@ -7,15 +7,16 @@
 // evenly to the stream blocks (aligned to rows, or one block per resident slot whose share may run from one
 // row into the next; the host chooses).  A warp of a block's eight takes every eighth page of the block's run by itself
 // (decode_page.cuh), from buffers of its own that bulk async copies fill, completion on an mbarrier: the keys' buffer is
-// refilled as soon as the logits are done, the values' after P.V.  The block merges the eight states when it leaves a row
+// refilled as soon as the logits are done, the values' after P.V.  Where blocks have one unit and an SM each, two warps share a
+// page, half of its tokens each.  The block merges the eight states when it leaves a row
 // and writes one partial per row it touched.  One more short block per row, launched after the stream blocks, handles the
 // dense tokens: the sink prefix and everything after the last page that is packed on both the key and the value side.
 //
 // What bounds it: two pipes that take a warp instruction every other cycle, each busy half of the time (logic: one LOP3 per
 // operand register, address arithmetic, shifts; packed 16-bit arithmetic: two per register), and four warps per scheduler to
-// keep them so.  Time goes with the number of instructions.  Batch 128, 32,768 tokens: 1,143 us with two warps per page that
-// split the logits by channels, the rest by tokens, and met twice per page; 1,080 us with a warp per page, which fills
-// one table instead of two and exchanges nothing (B200; 1,091 us with the barriers where the merge buffer cannot reach them).
+// keep them so.  Batch 128, 32,768 tokens: 1,144 us with two warps per page that split the logits by channels, the rest by
+// tokens, and met twice per page; 1,089 us with a warp per page, which fills one table instead of two and exchanges nothing
+// (B200; the instructions of a launch went from 3,340 to 3,287 per page).
 // Algorithmic HBM bytes per page and (batch, kv head): 10880.
 
 #include <atomic>
@@ -40,8 +41,8 @@ struct BlockSmem {
 
 // GN: value groups per token (1 or 2).  KP: promoted channels per page when that is a multiple of eight known to
 // the host (0, 8, 16, 24, 32), else -1 (read from the descriptor): with the count fixed the logits loops have
-// constant trip counts and no per-position "is this slot promoted" test.
-template <int DT, int OUT, int GN, int KP>
+// constant trip counts and no per-position "is this slot promoted" test.  FEW: one unit per block (see dartkv_few_pages).
+template <int DT, int OUT, int GN, int KP, bool FEW>
 __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_desc d, FastArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   BlockSmem& bs = *reinterpret_cast<BlockSmem*>(smem_raw + sizeof(WarpSmem) * kWarps);
@@ -110,21 +111,39 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
     __syncthreads();
 
     work.start_row();
-    for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
-      ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
-      work.fill_table(ws.keys, ws.scratch);
-      __syncwarp();
-      float s_acc[4][4];
-      work.logits(ws.keys, ws.scratch, s_acc);
-      __syncwarp();
-      // the keys are consumed: their buffer takes the next page's while the values are worked on
-      if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
-      work.softmax(s_acc, row_first - (d.sink_tokens + 128 * pg), ws.scratch);
-      __syncwarp();
-      ok = mbar_wait(&bs.v_bar[warp], parity) && ok;
-      work.weigh_values(ws.values, ws.scratch);
-      __syncwarp();
-      if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
+    if constexpr (FEW) {
+      // the block's only unit: warps w and w + 4 share page w, half of its tokens each
+      const int hf = warp >> 2, shared = warp & 3;
+      const WarpSmem& page = reinterpret_cast<const WarpSmem*>(smem_raw)[shared];
+      if (p_begin + shared < p_end) {
+        ok = mbar_wait(&bs.k_bar[shared], 0) && ok;
+        work.fill_table(page.keys, ws.scratch);
+        __syncwarp();
+        float s_acc[2][4];
+        work.template logits<2>(page.keys, ws.scratch, hf, s_acc);
+        __syncwarp();
+        work.template softmax<2>(s_acc, hf, row_first - (d.sink_tokens + 128 * (p_begin + shared)), ws.scratch);
+        __syncwarp();
+        ok = mbar_wait(&bs.v_bar[shared], 0) && ok;
+        work.template weigh_values<2>(page.values, ws.scratch, hf);
+      }
+    } else {
+      for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
+        ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
+        work.fill_table(ws.keys, ws.scratch);
+        __syncwarp();
+        float s_acc[4][4];
+        work.template logits<4>(ws.keys, ws.scratch, 0, s_acc);
+        __syncwarp();
+        // the keys are consumed: their buffer takes the next page's while the values are worked on
+        if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
+        work.template softmax<4>(s_acc, 0, row_first - (d.sink_tokens + 128 * pg), ws.scratch);
+        __syncwarp();
+        ok = mbar_wait(&bs.v_bar[warp], parity) && ok;
+        work.template weigh_values<4>(ws.values, ws.scratch, 0);
+        __syncwarp();
+        if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
+      }
     }
 
     __syncthreads();   // every warp is done with its stages: the staging memory becomes the merge buffer
@@ -160,37 +179,37 @@ int dartkv_decode_fast_supported(const dartkv_cache_desc* d, int q_dtype, int qu
 // every (metadata dtype, cache dtype, value groups, promoted count) variant of the kernel; a cache whose metadata
 // dtype differs from its dtype gets the promoted counts 0 and 32 specialized, the others read the count at run time
 using FastKernel = void (*)(dartkv_cache_desc, FastArgs);
-template <int DT, int GN>
+template <bool FEW, int DT, int GN>
 static FastKernel fast_variant_kp(int kp) {
   switch (kp) {
-    case 0: return decode_fast_kernel<DT, DT, GN, 0>;
-    case 8: return decode_fast_kernel<DT, DT, GN, 8>;
-    case 16: return decode_fast_kernel<DT, DT, GN, 16>;
-    case 24: return decode_fast_kernel<DT, DT, GN, 24>;
-    case 32: return decode_fast_kernel<DT, DT, GN, 32>;
-    default: return decode_fast_kernel<DT, DT, GN, -1>;
+    case 0: return decode_fast_kernel<DT, DT, GN, 0, FEW>;
+    case 8: return decode_fast_kernel<DT, DT, GN, 8, FEW>;
+    case 16: return decode_fast_kernel<DT, DT, GN, 16, FEW>;
+    case 24: return decode_fast_kernel<DT, DT, GN, 24, FEW>;
+    case 32: return decode_fast_kernel<DT, DT, GN, 32, FEW>;
+    default: return decode_fast_kernel<DT, DT, GN, -1, FEW>;
   }
 }
-template <int DT, int OUT, int GN>
+template <bool FEW, int DT, int OUT, int GN>
 static FastKernel mixed_variant_kp(int kp) {
   switch (kp) {
-    case 0: return decode_fast_kernel<DT, OUT, GN, 0>;
-    case 32: return decode_fast_kernel<DT, OUT, GN, 32>;
-    default: return decode_fast_kernel<DT, OUT, GN, -1>;
+    case 0: return decode_fast_kernel<DT, OUT, GN, 0, FEW>;
+    case 32: return decode_fast_kernel<DT, OUT, GN, 32, FEW>;
+    default: return decode_fast_kernel<DT, OUT, GN, -1, FEW>;
   }
 }
-static FastKernel fast_variant(int md, int dtype, int value_groups, int kp) {
+template <bool FEW>
+static FastKernel fast_variant_of(int md, int dtype, int value_groups, int kp) {
   if (md == dtype) {
-    if (dtype == DARTKV_BF16) return value_groups == 2 ? fast_variant_kp<DARTKV_BF16, 2>(kp) : fast_variant_kp<DARTKV_BF16, 1>(kp);
-    return value_groups == 2 ? fast_variant_kp<DARTKV_F16, 2>(kp) : fast_variant_kp<DARTKV_F16, 1>(kp);
+    if (dtype == DARTKV_BF16) return value_groups == 2 ? fast_variant_kp<FEW, DARTKV_BF16, 2>(kp) : fast_variant_kp<FEW, DARTKV_BF16, 1>(kp);
+    return value_groups == 2 ? fast_variant_kp<FEW, DARTKV_F16, 2>(kp) : fast_variant_kp<FEW, DARTKV_F16, 1>(kp);
   }
   if (md == DARTKV_F16)
-    return value_groups == 2 ? mixed_variant_kp<DARTKV_F16, DARTKV_BF16, 2>(kp) : mixed_variant_kp<DARTKV_F16, DARTKV_BF16, 1>(kp);
-  return value_groups == 2 ? mixed_variant_kp<DARTKV_BF16, DARTKV_F16, 2>(kp) : mixed_variant_kp<DARTKV_BF16, DARTKV_F16, 1>(kp);
+    return value_groups == 2 ? mixed_variant_kp<FEW, DARTKV_F16, DARTKV_BF16, 2>(kp) : mixed_variant_kp<FEW, DARTKV_F16, DARTKV_BF16, 1>(kp);
+  return value_groups == 2 ? mixed_variant_kp<FEW, DARTKV_BF16, DARTKV_F16, 2>(kp) : mixed_variant_kp<FEW, DARTKV_BF16, DARTKV_F16, 1>(kp);
 }
-static void launch_variant(int md, int dtype, int value_groups, int kp, dim3 grid, cudaStream_t stream,
-                           const dartkv_cache_desc& d, const FastArgs& a) {
-  fast_variant(md, dtype, value_groups, kp)<<<grid, kThreads, kSmemBytes, stream>>>(d, a);
+static FastKernel fast_variant(bool few, int md, int dtype, int value_groups, int kp) {
+  return few ? fast_variant_of<true>(md, dtype, value_groups, kp) : fast_variant_of<false>(md, dtype, value_groups, kp);
 }
 
 int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
@@ -201,25 +220,26 @@ int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int
   FastArgs a{query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l, part_acc, status,
              row_start};
   dim3 grid(stream_blocks + d->batch * d->kv_heads);
+  const bool few = dartkv_few_pages(units, stream_blocks);
   {
     // the shared-memory opt-in is per device and per kernel: ask once per device (the flags are atomic; two threads
     // that race on a device's first call both set the attribute, which is harmless)
-    static std::atomic<bool> ready[64];
+    static std::atomic<bool> ready[64][2];
     int device = 0;
     DARTKV_CUDA_OK(cudaGetDevice(&device));
-    if (device < 0 || device >= 64 || !ready[device].load(std::memory_order_acquire)) {
+    if (device < 0 || device >= 64 || !ready[device][few].load(std::memory_order_acquire)) {
       for (int md : {DARTKV_BF16, DARTKV_F16})
         for (int dt : {DARTKV_BF16, DARTKV_F16})
           for (int gn : {1, 2})
             for (int kp : {-1, 0, 8, 16, 24, 32})
-              DARTKV_CUDA_OK(cudaFuncSetAttribute(fast_variant(md, dt, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
+              DARTKV_CUDA_OK(cudaFuncSetAttribute(fast_variant(few, md, dt, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)kSmemBytes));
-      if (device >= 0 && device < 64) ready[device].store(true, std::memory_order_release);
+      if (device >= 0 && device < 64) ready[device][few].store(true, std::memory_order_release);
     }
   }
   const int promoted = d->key_mode == DARTKV_MIXED_PAGE ? d->promoted : 0;
   const int kp = (promoted % 8 == 0 && promoted <= 32) ? promoted : -1;
-  launch_variant(d->md_dtype, d->dtype, d->value_groups, kp, grid, stream, *d, a);
+  fast_variant(few, d->md_dtype, d->dtype, d->value_groups, kp)<<<grid, kThreads, kSmemBytes, stream>>>(*d, a);
   DARTKV_LAUNCH_OK("decode_fast_kernel");
   return DARTKV_OK;
 }

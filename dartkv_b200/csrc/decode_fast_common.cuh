@@ -43,6 +43,13 @@ struct FastArgs {
   const int32_t* row_start;
 };
 
+// Calls of the 2-bit kernels whose blocks have one unit each, four pages at most, and an SM each: a warp per page would leave
+// half the warps of a block idle and the call waiting for one warp's way through a page, so two warps share one.  Per-op flavour,
+// 32 heads on 8: 16 x 160 tokens 14.3 -> 12.3 us, 8 x 800 14.1 -> 12.9, 4 x 2,080 13.5 -> 13.1; unrounded 12.3 -> 10.3, 12.3 ->
+// 11.2, 11.8 -> 11.3.  Two blocks on an SM keep it busy, and the second table of a page costs: 4 x 4,128 tokens (256 blocks) 17.5
+// us, shared 18.4, 2 x 6,000 (192) 17.0 and 18.4 (B200).
+inline bool dartkv_few_pages(long long units, int stream_blocks) { return units == stream_blocks && stream_blocks <= dartkv_sm_count(); }
+
 __host__ __device__ __forceinline__ int fast_range_end(int sink_tokens, int page_size, int k_end, int v_end,
                                                        int sink_filled) {
   int packed = min(k_end, v_end);

@@ -200,12 +200,26 @@ struct FusedWork {
 
   // logits S[token pair][(head, j')] over the doubled contraction (channel, j).  A thread reads the whole word g of a
   // channel's code row (tokens 16g .. 16g+15); row g of m-tile mt is code u = 2mt of both halves, row g+8 u = 2mt + 1:
-  // u = 0..4 at positions 0..4 of the mantissa, 5..7 at positions 0..2 after a shift.
-  __device__ __forceinline__ void logits(const uint8_t* keys, const FusedScratch& ws, float (&s_acc)[4][4]) const {
+  // u = 0..4 at positions 0..4 of the mantissa, 5..7 at positions 0..2 after a shift.  MT: m-tiles, 4 for the whole page or 2
+  // for the half `hf` of it (u = 4hf .. 4hf + 3, at positions 0..3).
+  template <int MT>
+  __device__ __forceinline__ void logits(const uint8_t* keys, const FusedScratch& ws, int hf, float (&s_acc)[MT][4]) const {
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
+    const int shift = MT == 4 ? 0 : 8 * hf;
+    // the A operands of two code words, m-tile by m-tile
+    auto tiles = [&](uint32_t w0, uint32_t w1, auto multiply) {
+      w0 >>= shift; w1 >>= shift;
+      multiply(s_acc[0], w0 & 0x00030003u, w0 & 0x000C000Cu, w1 & 0x00030003u, w1 & 0x000C000Cu);
+      multiply(s_acc[1], w0 & 0x00300030u, w0 & 0x00C000C0u, w1 & 0x00300030u, w1 & 0x00C000C0u);
+      if constexpr (MT == 4) {
+        const uint32_t y0 = w0 >> 10, y1 = w1 >> 10;
+        multiply(s_acc[2], w0 & 0x03000300u, y0 & 0x00030003u, w1 & 0x03000300u, y1 & 0x00030003u);
+        multiply(s_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u);
+      }
+    };
     const uint8_t* const low = keys + 4 * g + 32 * c;                          // + 256 * step (+128)
     const int w_thread = 8 * c + 4 * (g >> 2);                                 // + 64 * step (+32)
     const uint8_t* const w_low = reinterpret_cast<const uint8_t*>(ws.w_low) + w_thread;
@@ -213,13 +227,9 @@ struct FusedWork {
     for (int ks = 0; ks < 16; ++ks) {
       const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low + 256 * ks);
       const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low + 256 * ks + 128);
-      const uint32_t y0 = w0 >> 10, y1 = w1 >> 10;
       const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(w_low + 64 * ks), 0u, sel_w);
       const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(w_low + 64 * ks + 32), 0u, sel_w);
-      mma_f16(s_acc[0], w0 & 0x00030003u, w0 & 0x000C000Cu, w1 & 0x00030003u, w1 & 0x000C000Cu, b0, b1);
-      mma_f16(s_acc[1], w0 & 0x00300030u, w0 & 0x00C000C0u, w1 & 0x00300030u, w1 & 0x00C000C0u, b0, b1);
-      mma_f16(s_acc[2], w0 & 0x03000300u, y0 & 0x00030003u, w1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
-      mma_f16(s_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u, b0, b1);
+      tiles(w0, w1, [&](float (&s)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) { mma_f16(s, a0, a1, a2, a3, b0, b1); });
     }
     // high plane of the promoted slots: the same codes against both terms of the weights
     const uint8_t* const high = keys + d.key_off_high + 4 * g + 32 * c;
@@ -228,31 +238,28 @@ struct FusedWork {
     for (int ks = 0; ks < prom_steps; ++ks) {
       const uint32_t w0 = *reinterpret_cast<const uint32_t*>(high + 256 * ks);
       const uint32_t w1 = *reinterpret_cast<const uint32_t*>(high + 256 * ks + 128);
-      const uint32_t y0 = w0 >> 10, y1 = w1 >> 10;
       const uint32_t b0 = prmt(*reinterpret_cast<const uint32_t*>(w_high + 64 * ks), 0u, sel_w);
       const uint32_t b1 = prmt(*reinterpret_cast<const uint32_t*>(w_high + 64 * ks + 32), 0u, sel_w);
       const uint32_t l0 = prmt(*reinterpret_cast<const uint32_t*>(w_high_lo + 64 * ks), 0u, sel_w);
       const uint32_t l1 = prmt(*reinterpret_cast<const uint32_t*>(w_high_lo + 64 * ks + 32), 0u, sel_w);
-      auto both = [&](float (&s)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+      tiles(w0, w1, [&](float (&s)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
         mma_f16(s, a0, a1, a2, a3, b0, b1);
         mma_f16(s, a0, a1, a2, a3, l0, l1);
-      };
-      both(s_acc[0], w0 & 0x00030003u, w0 & 0x000C000Cu, w1 & 0x00030003u, w1 & 0x000C000Cu);
-      both(s_acc[1], w0 & 0x00300030u, w0 & 0x00C000C0u, w1 & 0x00300030u, w1 & 0x00C000C0u);
-      both(s_acc[2], w0 & 0x03000300u, y0 & 0x00030003u, w1 & 0x03000300u, y1 & 0x00030003u);
-      both(s_acc[3], y0 & 0x000C000Cu, y0 & 0x00300030u, y1 & 0x000C000Cu, y1 & 0x00300030u);
+      });
     }
   }
 
-  // online softmax for head c over the page (this thread: tokens 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1); the
-  // probabilities leave as weights p*s*fv.  wait_for_values() returns when the page's values have landed.
-  template <class Wait>
-  __device__ __forceinline__ void softmax(float (&s_acc)[4][4], int mask_below, FusedScratch& ws, Wait wait_for_values, const uint8_t* values) {
+  // online softmax for head c over the page or half of it (this thread: tokens 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1, in
+  // a half + 4hf); the probabilities leave as weights p*s*fv.  wait_for_values() returns when the page's values have landed.
+  template <int MT, class Wait>
+  __device__ __forceinline__ void softmax(float (&s_acc)[MT][4], int hf, int mask_below, FusedScratch& ws, Wait wait_for_values,
+                                          const uint8_t* values) {
+    const int first = 16 * g + (MT == 4 ? 0 : 4 * hf);
     {
       const float base = scale2 * f_inv * 16777216.0f;
       const float cm[5] = {base, base * 0.25f, base * 0.0625f, base * 0.015625f, base * 0.00390625f};
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int u = 2 * mt + (i >> 1);
@@ -261,14 +268,14 @@ struct FusedWork {
     }
     if (mask_below > 0) {   // the page that holds the row's first live token: the tokens before it drop out
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (16 * g + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
+          if (first + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
     }
     float mx = -INFINITY;
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) mx = fmaxf(mx, s_acc[mt][i]);
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
@@ -303,17 +310,19 @@ struct FusedWork {
     const float fv = fv_run;
 
     float psum = 0.0f, zs0 = 0.0f, zs1 = 0.0f;
-    uint32_t* const row = &ws.u[c * kUStride + 16 * g];
+    constexpr int kQuads = MT / 2;   // fours of tokens on each side of j, eight tokens apart
+    uint32_t* const row = &ws.u[c * kUStride + first];
 #pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4) {   // tokens 16g + 4*k4 .. + 3
+    for (int k4 = 0; k4 < MT; ++k4) {   // tokens `first` + from .. + 3
+      const int from = kQuads == 2 ? 4 * k4 : 8 * k4;
       uint32_t packed[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int u = 4 * (k4 & 1) + k, j = k4 >> 1;
+        const int u = kQuads == 2 ? 4 * (k4 & 1) + k : k, j = k4 / kQuads;
         const float p = fast_exp2(s_acc[u >> 1][2 * (u & 1) + j] - m_ref);
         psum += p;
         const float pf = p * fv;
-        const int tok = 16 * g + 4 * k4 + k;
+        const int tok = first + from + k;
         if (GN == 2) {
           const uint2 m = *reinterpret_cast<const uint2*>(vmeta + tok * 8);   // (s0 | s1 << 16), (z0 | z1 << 16)
           float s0, s1, z0, z1;
@@ -330,7 +339,7 @@ struct FusedWork {
           packed[k] = pack_f16x2(w, w);
         }
       }
-      *reinterpret_cast<uint4*>(row + 4 * k4) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      *reinterpret_cast<uint4*>(row + from) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
     l_run = l_run * alpha + psum;
     zs[0] = zs[0] * alpha + zs0;
@@ -347,21 +356,24 @@ struct FusedWork {
   // O[channel pair][(head, j')] += V^T U over the doubled contraction (token, j): lane row g reads the
   // code words wi = g & 3 and wi + 4 of a token row and pairs their low (g < 4) or high (g >= 4) halves, so a
   // register holds (channel 16wi + 8xy + u of group 0, the same channel + 64 of group 1).  Step ks covers the
-  // eight tokens from 8ks on.
-  __device__ __forceinline__ void weigh_values(const uint8_t* values, const FusedScratch& ws) {
+  // eight tokens from 8ks on, in a half the tokens 16ks + 4hf .. + 3 and 16ks + 4hf + 8 .. + 11.
+  template <int MT>
+  __device__ __forceinline__ void weigh_values(const uint8_t* values, const FusedScratch& ws, int hf) {
+    constexpr int kStep = MT == 4 ? 8 : 16, kSecond = MT == 4 ? 4 : 8;   // tokens from step to step, to the second four
+    const int base = c + (MT == 4 ? 0 : 4 * hf);
     const int wi = g & 3;
     const uint32_t sel_v = (g >> 2) ? 0x7632u : 0x5410u;
-    const uint8_t* const vthread = values + 32 * c + 4 * wi;               // + 256 * ks (+128 for the second token)
-    const uint32_t* const uthread = &ws.u[(g >> 1) * kUStride + c];        // + 8 * ks (+4 for the second token)
+    const uint8_t* const vthread = values + 32 * base + 4 * wi;            // + 32 * tokens
+    const uint32_t* const uthread = &ws.u[(g >> 1) * kUStride + base];     // + tokens
 #pragma unroll kPvUnroll
-    for (int ks = 0; ks < 16; ++ks) {
-      const uint32_t x0 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 256 * ks),
-                               *reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 16), sel_v);
-      const uint32_t x1 = prmt(*reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 128),
-                               *reinterpret_cast<const uint32_t*>(vthread + 256 * ks + 128 + 16), sel_v);
+    for (int ks = 0; ks < 4 * MT; ++ks) {
+      const uint8_t* const va = vthread + 32 * kStep * ks;
+      const uint8_t* const vb = va + 32 * kSecond;
+      const uint32_t x0 = prmt(*reinterpret_cast<const uint32_t*>(va), *reinterpret_cast<const uint32_t*>(va + 16), sel_v);
+      const uint32_t x1 = prmt(*reinterpret_cast<const uint32_t*>(vb), *reinterpret_cast<const uint32_t*>(vb + 16), sel_v);
       const uint32_t y0 = x0 >> 10, y1 = x1 >> 10;   // codes 5, 6, 7 at positions 0, 1, 2
-      const uint32_t b0 = uthread[8 * ks] & mask_u;
-      const uint32_t b1 = uthread[8 * ks + 4] & mask_u;
+      const uint32_t b0 = uthread[kStep * ks] & mask_u;
+      const uint32_t b1 = uthread[kStep * ks + kSecond] & mask_u;
       mma_f16(o_acc[0], x0 & 0x00030003u, x0 & 0x000C000Cu, x1 & 0x00030003u, x1 & 0x000C000Cu, b0, b1);
       mma_f16(o_acc[1], x0 & 0x00300030u, x0 & 0x00C000C0u, x1 & 0x00300030u, x1 & 0x00C000C0u, b0, b1);
       mma_f16(o_acc[2], x0 & 0x03000300u, y0 & 0x00030003u, x1 & 0x03000300u, y1 & 0x00030003u, b0, b1);
@@ -390,8 +402,8 @@ struct FusedWork {
   }
 };
 
-// the work split of decode_fast_kernel
-template <int DT, int MD, int GN, int KP>
+// the work split of decode_fast_kernel, FEW included
+template <int DT, int MD, int GN, int KP, bool FEW>
 __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cache_desc d, FastArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   FusedBlockSmem& bs = *reinterpret_cast<FusedBlockSmem*>(smem_raw + sizeof(FusedWarpSmem) * kWarps);
@@ -456,20 +468,39 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
     __syncthreads();
 
     work.start_row();
-    for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
-      ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
-      work.fill_table(ws.keys, ws.scratch);
-      __syncwarp();
-      float s_acc[4][4];
-      work.logits(ws.keys, ws.scratch, s_acc);
-      __syncwarp();
-      // the keys are consumed: their buffer takes the next page's while the values are worked on
-      if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
-      work.softmax(s_acc, row_first - (d.sink_tokens + 128 * pg), ws.scratch, [&] { ok = mbar_wait(&bs.v_bar[warp], parity) && ok; }, ws.values);
-      __syncwarp();
-      work.weigh_values(ws.values, ws.scratch);
-      __syncwarp();
-      if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
+    if constexpr (FEW) {
+      // the block's only unit: warps w and w + 4 share page w, half of its tokens each
+      const int hf = warp >> 2, shared = warp & 3;
+      const FusedWarpSmem& page = reinterpret_cast<const FusedWarpSmem*>(smem_raw)[shared];
+      if (p_begin + shared < p_end) {
+        ok = mbar_wait(&bs.k_bar[shared], 0) && ok;
+        work.fill_table(page.keys, ws.scratch);
+        __syncwarp();
+        float s_acc[2][4];
+        work.template logits<2>(page.keys, ws.scratch, hf, s_acc);
+        __syncwarp();
+        work.template softmax<2>(s_acc, hf, row_first - (d.sink_tokens + 128 * (p_begin + shared)), ws.scratch,
+                                 [&] { ok = mbar_wait(&bs.v_bar[shared], 0) && ok; }, page.values);
+        __syncwarp();
+        work.template weigh_values<2>(page.values, ws.scratch, hf);
+      }
+    } else {
+      for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
+        ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
+        work.fill_table(ws.keys, ws.scratch);
+        __syncwarp();
+        float s_acc[4][4];
+        work.template logits<4>(ws.keys, ws.scratch, 0, s_acc);
+        __syncwarp();
+        // the keys are consumed: their buffer takes the next page's while the values are worked on
+        if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
+        work.template softmax<4>(s_acc, 0, row_first - (d.sink_tokens + 128 * pg), ws.scratch,
+                                 [&] { ok = mbar_wait(&bs.v_bar[warp], parity) && ok; }, ws.values);
+        __syncwarp();
+        work.template weigh_values<4>(ws.values, ws.scratch, 0);
+        __syncwarp();
+        if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
+      }
     }
 
     __syncthreads();   // every warp is done with its stages: the staging memory becomes the merge buffer
@@ -505,33 +536,38 @@ int dartkv_decode_fused32_supported(const dartkv_cache_desc* d, int q_dtype, int
 // every (cache dtype, metadata dtype, value groups, promoted count) variant of the kernel; a cache whose metadata
 // dtype differs from its dtype gets the promoted counts 0 and 32 specialized, the others read the count at run time
 using FusedKernel = void (*)(dartkv_cache_desc, FastArgs);
-template <int DT, int GN>
+template <bool FEW, int DT, int GN>
 static FusedKernel fused_variant_kp(int kp) {
   switch (kp) {
-    case 0: return decode_fused32_kernel<DT, DT, GN, 0>;
-    case 8: return decode_fused32_kernel<DT, DT, GN, 8>;
-    case 16: return decode_fused32_kernel<DT, DT, GN, 16>;
-    case 24: return decode_fused32_kernel<DT, DT, GN, 24>;
-    case 32: return decode_fused32_kernel<DT, DT, GN, 32>;
-    default: return decode_fused32_kernel<DT, DT, GN, -1>;
+    case 0: return decode_fused32_kernel<DT, DT, GN, 0, FEW>;
+    case 8: return decode_fused32_kernel<DT, DT, GN, 8, FEW>;
+    case 16: return decode_fused32_kernel<DT, DT, GN, 16, FEW>;
+    case 24: return decode_fused32_kernel<DT, DT, GN, 24, FEW>;
+    case 32: return decode_fused32_kernel<DT, DT, GN, 32, FEW>;
+    default: return decode_fused32_kernel<DT, DT, GN, -1, FEW>;
   }
 }
-template <int DT, int MD, int GN>
+template <bool FEW, int DT, int MD, int GN>
 static FusedKernel fused_mixed_kp(int kp) {
   switch (kp) {
-    case 0: return decode_fused32_kernel<DT, MD, GN, 0>;
-    case 32: return decode_fused32_kernel<DT, MD, GN, 32>;
-    default: return decode_fused32_kernel<DT, MD, GN, -1>;
+    case 0: return decode_fused32_kernel<DT, MD, GN, 0, FEW>;
+    case 32: return decode_fused32_kernel<DT, MD, GN, 32, FEW>;
+    default: return decode_fused32_kernel<DT, MD, GN, -1, FEW>;
   }
 }
-static FusedKernel fused_variant(int dtype, int md, int value_groups, int kp) {
+template <bool FEW>
+static FusedKernel fused_variant_of(int dtype, int md, int value_groups, int kp) {
   if (md == dtype) {
-    if (dtype == DARTKV_BF16) return value_groups == 2 ? fused_variant_kp<DARTKV_BF16, 2>(kp) : fused_variant_kp<DARTKV_BF16, 1>(kp);
-    return value_groups == 2 ? fused_variant_kp<DARTKV_F16, 2>(kp) : fused_variant_kp<DARTKV_F16, 1>(kp);
+    if (dtype == DARTKV_BF16) return value_groups == 2 ? fused_variant_kp<FEW, DARTKV_BF16, 2>(kp) : fused_variant_kp<FEW, DARTKV_BF16, 1>(kp);
+    return value_groups == 2 ? fused_variant_kp<FEW, DARTKV_F16, 2>(kp) : fused_variant_kp<FEW, DARTKV_F16, 1>(kp);
   }
   if (dtype == DARTKV_BF16)
-    return value_groups == 2 ? fused_mixed_kp<DARTKV_BF16, DARTKV_F16, 2>(kp) : fused_mixed_kp<DARTKV_BF16, DARTKV_F16, 1>(kp);
-  return value_groups == 2 ? fused_mixed_kp<DARTKV_F16, DARTKV_BF16, 2>(kp) : fused_mixed_kp<DARTKV_F16, DARTKV_BF16, 1>(kp);
+    return value_groups == 2 ? fused_mixed_kp<FEW, DARTKV_BF16, DARTKV_F16, 2>(kp) : fused_mixed_kp<FEW, DARTKV_BF16, DARTKV_F16, 1>(kp);
+  return value_groups == 2 ? fused_mixed_kp<FEW, DARTKV_F16, DARTKV_BF16, 2>(kp) : fused_mixed_kp<FEW, DARTKV_F16, DARTKV_BF16, 1>(kp);
+}
+
+static FusedKernel fused_variant(bool few, int dtype, int md, int value_groups, int kp) {
+  return few ? fused_variant_of<true>(dtype, md, value_groups, kp) : fused_variant_of<false>(dtype, md, value_groups, kp);
 }
 
 int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
@@ -542,25 +578,26 @@ int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, 
   FastArgs a{query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l, part_acc, status,
              row_start};
   dim3 grid(stream_blocks + d->batch * d->kv_heads);
+  const bool few = dartkv_few_pages(units, stream_blocks);
   {
     // the shared-memory opt-in is per device and per kernel: ask once per device (the flags are atomic; two threads
     // that race on a device's first call both set the attribute, which is harmless)
-    static std::atomic<bool> ready[64];
+    static std::atomic<bool> ready[64][2];
     int device = 0;
     DARTKV_CUDA_OK(cudaGetDevice(&device));
-    if (device < 0 || device >= 64 || !ready[device].load(std::memory_order_acquire)) {
+    if (device < 0 || device >= 64 || !ready[device][few].load(std::memory_order_acquire)) {
       for (int dt : {DARTKV_BF16, DARTKV_F16})
         for (int md : {DARTKV_BF16, DARTKV_F16})
           for (int gn : {1, 2})
             for (int kp : {-1, 0, 8, 16, 24, 32})
-              DARTKV_CUDA_OK(cudaFuncSetAttribute(fused_variant(dt, md, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
+              DARTKV_CUDA_OK(cudaFuncSetAttribute(fused_variant(few, dt, md, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)kFusedSmemBytes));
-      if (device >= 0 && device < 64) ready[device].store(true, std::memory_order_release);
+      if (device >= 0 && device < 64) ready[device][few].store(true, std::memory_order_release);
     }
   }
   const int promoted = d->key_mode == DARTKV_MIXED_PAGE ? d->promoted : 0;
   const int kp = (promoted % 8 == 0 && promoted <= 32) ? promoted : -1;
-  fused_variant(d->dtype, d->md_dtype, d->value_groups, kp)<<<grid, kThreads, kFusedSmemBytes, stream>>>(*d, a);
+  fused_variant(few, d->dtype, d->md_dtype, d->value_groups, kp)<<<grid, kThreads, kFusedSmemBytes, stream>>>(*d, a);
   DARTKV_LAUNCH_OK("decode_fused32_kernel");
   return DARTKV_OK;
 }

@@ -1,5 +1,5 @@
-// One page of the per-op rounded decode on tensor cores, as one warp works on it: contraction table, logits, online softmax,
-// P.V.
+// One page of the per-op rounded decode on tensor cores, as one warp works on it, or one of two warps on half of its tokens:
+// contraction table, logits, online softmax, P.V.
 //
 // Packed 2-bit codes are turned into exactly rounded 16-bit operands with one logic op and two packed fma/add per pair
 // (mma_utils.cuh) and fed straight into m16n8k16 MMAs; K and V are never materialized.  Keys: a register of the operand
@@ -50,8 +50,8 @@ struct PageWork {
   using H = Half2Ops<DT>;
   using HO = Half2Ops<OUT>;
   // Unrolling, for whole pages: longer bodies (12 and 8 steps) cost 5 us of instruction fetch on the first pages of a call,
-  // shorter ones expose shared-memory latency (batch 128, 32,768 tokens: 1,080 us; with single promoted steps 1,094, with
-  // single steps throughout 1,120, with two of P.V 1,103).
+  // shorter ones expose shared-memory latency (batch 128, 32,768 tokens: 1,089 us; with single promoted steps 1,107, with
+  // single steps throughout 1,116, with two of P.V 1,077, though with fp16 scales beside bf16 1,536 instead of 1,524).
   static constexpr int kPromUnroll = 4, kQkUnroll = 4, kPvUnroll = 1;
   CodeConsts<DT> cc;
   const dartkv_cache_desc& d;
@@ -110,12 +110,15 @@ struct PageWork {
     }
   }
 
-  // logits S[token pair][(head, j')] over the doubled contraction (channel, j), eight positions per step
-  __device__ __forceinline__ void logits(const uint8_t* keys, const PageScratch& scratch, float (&s_acc)[4][4]) const {
+  // logits S[token pair][(head, j')] over the doubled contraction (channel, j), eight positions per step.  MT: m-tiles, 4 for
+  // the whole page or 2 for the half `hf` of it (codes u = 4hf .. 4hf + 3 of each half of a word)
+  template <int MT>
+  __device__ __forceinline__ void logits(const uint8_t* keys, const PageScratch& scratch, int hf, float (&s_acc)[MT][4]) const {
     const uint8_t* const low_thread = keys + 4 * g;                                                     // + 32 * channel
     const uint32_t* const high_thread = reinterpret_cast<const uint32_t*>(keys + d.key_off_high) + g;   // + 8 * slot
+    const int shift = MT == 4 ? 0 : 8 * hf;
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
 #pragma unroll kPromUnroll
@@ -123,55 +126,57 @@ struct PageWork {
       const int s0 = 8 * i + c, s1 = s0 + 4;
       const uint4 e0 = scratch.table[s0], e1 = scratch.table[s1];
       const uint32_t o0 = e0.w >> 16, o1 = e1.w >> 16;
-      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0);
-      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1);
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0) >> shift;
+      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1) >> shift;
       // with a promoted count that is a multiple of eight every position of a promoted step is a promoted slot
-      const uint32_t h0 = (KP >= 0 || s0 < K) ? high_thread[s0 * 8] : 0u;
-      const uint32_t h1 = (KP >= 0 || s1 < K) ? high_thread[s1 * 8] : 0u;
-      uint32_t r0[8], r1[8];
+      const uint32_t h0 = (KP >= 0 || s0 < K) ? high_thread[s0 * 8] >> shift : 0u;
+      const uint32_t h1 = (KP >= 0 || s1 < K) ? high_thread[s1 * 8] >> shift : 0u;
+      uint32_t r0[2 * MT], r1[2 * MT];
       dequant_word4<DT>(cc, w0, h0, e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), r0);
       dequant_word4<DT>(cc, w1, h1, e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), r1);
       cast_registers<DT, OUT>(r0);
       cast_registers<DT, OUT>(r1);
       const uint32_t b0 = query(o0), b1 = query(o1);
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+      for (int mt = 0; mt < MT; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
     }
 #pragma unroll kQkUnroll
     for (int i = prom_steps; i < 16; ++i) {
       const int s0 = 8 * i + c, s1 = s0 + 4;
       const uint4 e0 = scratch.table[s0], e1 = scratch.table[s1];
       const uint32_t o0 = e0.w >> 16, o1 = e1.w >> 16;
-      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0);
-      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1);
-      uint32_t r0[8], r1[8];
+      const uint32_t w0 = *reinterpret_cast<const uint32_t*>(low_thread + o0) >> shift;
+      const uint32_t w1 = *reinterpret_cast<const uint32_t*>(low_thread + o1) >> shift;
+      uint32_t r0[2 * MT], r1[2 * MT];
       dequant_word2<DT>(cc, w0, e0.x, e0.y, low_twice(e0.z), high_twice(e0.z), low_twice(e0.w), r0);
       dequant_word2<DT>(cc, w1, e1.x, e1.y, low_twice(e1.z), high_twice(e1.z), low_twice(e1.w), r1);
       cast_registers<DT, OUT>(r0);
       cast_registers<DT, OUT>(r1);
       const uint32_t b0 = query(o0), b1 = query(o1);
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
+      for (int mt = 0; mt < MT; ++mt) HO::mma(s_acc[mt], r0[2 * mt], r0[2 * mt + 1], r1[2 * mt], r1[2 * mt + 1], b0, b1);
     }
   }
 
-  // online softmax for head c (this thread's tokens are 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1); the
+  // online softmax for head c (this thread's tokens are 16g + u + 8j, u = 2mt + (i >> 1), j = i & 1, in a half + 4hf); the
   // probabilities go to the table with the pairs (u, u + 8) side by side.  mask_below: tokens before it drop out.
-  __device__ __forceinline__ void softmax(float (&s_acc)[4][4], int mask_below, PageScratch& scratch) {
+  template <int MT>
+  __device__ __forceinline__ void softmax(float (&s_acc)[MT][4], int hf, int mask_below, PageScratch& scratch) {
+    const int first = 16 * g + (MT == 4 ? 0 : 4 * hf);
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_acc[mt][i] *= scale2;
     if (mask_below > 0) {   // the page that holds the row's first live token
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (16 * g + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
+          if (first + 2 * mt + (i >> 1) + 8 * (i & 1) < mask_below) s_acc[mt][i] = -INFINITY;
     }
     float mx = -INFINITY;
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int i = 0; i < 4; ++i) mx = fmaxf(mx, s_acc[mt][i]);
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
@@ -182,9 +187,9 @@ struct PageWork {
     const float alpha = fast_exp2(m_run - m_ref);
     m_run = m_new;
     float psum = 0.0f;
-    uint32_t hi[8], lo[8];
+    uint32_t hi[2 * MT], lo[2 * MT];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < 2 * MT; ++u) {
       const float p0 = fast_exp2(s_acc[u >> 1][2 * (u & 1)] - m_ref), p1 = fast_exp2(s_acc[u >> 1][2 * (u & 1) + 1] - m_ref);
       psum += p0 + p1;
       hi[u] = pack16<OUT>(p0, p1);
@@ -192,10 +197,10 @@ struct PageWork {
       unpack16<OUT>(hi[u], h0, h1);
       lo[u] = pack16<OUT>(p0 - h0, p1 - h1);
     }
-    uint4* const row_hi = reinterpret_cast<uint4*>(&scratch.prob[c * kProbStride + 16 * g]);
-    uint4* const row_lo = reinterpret_cast<uint4*>(&scratch.prob[(4 + c) * kProbStride + 16 * g]);
+    uint4* const row_hi = reinterpret_cast<uint4*>(&scratch.prob[c * kProbStride + 16 * g]) + (MT == 4 ? 0 : hf);
+    uint4* const row_lo = reinterpret_cast<uint4*>(&scratch.prob[(4 + c) * kProbStride + 16 * g]) + (MT == 4 ? 0 : hf);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < MT / 2; ++k) {
       row_hi[k] = make_uint4(hi[4 * k], hi[4 * k + 1], hi[4 * k + 2], hi[4 * k + 3]);
       row_lo[k] = make_uint4(lo[4 * k], lo[4 * k + 1], lo[4 * k + 2], lo[4 * k + 3]);
     }
@@ -213,13 +218,17 @@ struct PageWork {
     }
   }
 
-  // O[channel][(part, head)] += V^T P, 16 tokens per step.  The code words of two tokens are byte-interleaved (low halves
+  // O[channel][(part, head)] += V^T P, 16 tokens per step; in a half, whose tokens are 16s + 4hf .. + 3 and 8 more, of two
+  // s a step.  The code words of two tokens are byte-interleaved (low halves
   // together: channels 0..7 of both tokens; high halves: channels 8..15), so that the packed dequantization sees token a in
   // the low half and token b in the high half.  m-tile mt, row g is channel 16g + mt, row g+8 channel 16g + 8 + mt.
-  __device__ __forceinline__ void weigh_values(const uint8_t* values, const PageScratch& scratch) {
+  template <int MT>
+  __device__ __forceinline__ void weigh_values(const uint8_t* values, const PageScratch& scratch, int hf) {
+    constexpr int kStep = MT == 4 ? 16 : 32, kSecond = MT == 4 ? 4 : 16;   // tokens from step to step, to the second pair
+    const int base = c + (MT == 4 ? 0 : 4 * hf);
     const uint32_t* vcodes = reinterpret_cast<const uint32_t*>(values) + g;   // word g of a token row: + 8 * token
     const uint8_t* vmeta = values + kValueCodes;
-    const uint32_t* pb = reinterpret_cast<const uint32_t*>(&scratch.prob[g * kProbStride]) + c;   // column n = g
+    const uint32_t* pb = reinterpret_cast<const uint32_t*>(&scratch.prob[g * kProbStride]) + base;   // column n = g
     // byte selectors that bring the scale (zero point) of this thread's value group of tokens a and b together
     const uint32_t sel_s = GN == 2 ? (gv ? 0x7632u : 0x5410u) : 0x5410u;
     const uint32_t sel_z = GN == 2 ? (gv ? 0x7632u : 0x5410u) : 0x7632u;
@@ -244,11 +253,12 @@ struct PageWork {
       cast_registers<DT, OUT>(r_hi);
     };
 #pragma unroll kPvUnroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 0; s < 2 * MT; ++s) {
       uint32_t r0_lo[8], r0_hi[8], r1_lo[8], r1_hi[8];
-      token_pair(16 * s + c, r0_lo, r0_hi);         // contraction index 2c, 2c + 1
-      token_pair(16 * s + c + 4, r1_lo, r1_hi);     // contraction index 2c + 8, 2c + 9
-      const uint32_t b0 = pb[8 * s], b1 = pb[8 * s + 4];
+      token_pair(kStep * s + base, r0_lo, r0_hi);             // contraction index 2c, 2c + 1
+      token_pair(kStep * s + base + kSecond, r1_lo, r1_hi);   // contraction index 2c + 8, 2c + 9
+      // the pairs (t, t + 8) of sixteen tokens are eight words
+      const uint32_t b0 = pb[kStep / 2 * s], b1 = pb[kStep / 2 * s + (MT == 4 ? 4 : 8)];
 #pragma unroll
       for (int mt = 0; mt < 8; ++mt) HO::mma(o_acc[mt], r0_lo[mt], r0_hi[mt], r1_lo[mt], r1_hi[mt], b0, b1);
     }

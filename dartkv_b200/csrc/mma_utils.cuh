@@ -183,18 +183,19 @@ __device__ __forceinline__ uint32_t align_codes(uint32_t w, int code, int pos, i
 //   t = fma(m, s, -magic*s)   = round16(code * s)
 //   r = add(t, z)             = round16(round16(code * s) + z)
 // which is the reference's per-op rounding in the metadata dtype (src/dart/quantization.py:103-106).
-template <int DT>
+// N: codes of each half that are wanted, the first eight (all) or four.
+template <int DT, int N>
 __device__ __forceinline__ void dequant_word2(const CodeConsts<DT>& k, uint32_t w, uint32_t ss, uint32_t zz,
-                                              uint32_t ms0, uint32_t ms1, uint32_t ms2, uint32_t (&r)[8]) {
+                                              uint32_t ms0, uint32_t ms1, uint32_t ms2, uint32_t (&r)[N]) {
   using H = Half2Ops<DT>;
   constexpr int P0 = H::kFirstPos;
 #pragma unroll
-  for (int grp = 0; grp < 3; ++grp) {
+  for (int grp = 0; grp < (N + 2) / 3; ++grp) {
     const uint32_t x = align_codes(w, 3 * grp, P0);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int u = 3 * grp + j;
-      if (u < 8) {
+      if (u < N) {
         const uint32_t m = and_or(x, k.mask[j], k.magic[j]);
         const uint32_t ms = j == 0 ? ms0 : (j == 1 ? ms1 : ms2);
         r[u] = H::add(H::fma(m, ss, ms), zz);
@@ -204,13 +205,13 @@ __device__ __forceinline__ void dequant_word2(const CodeConsts<DT>& k, uint32_t 
 }
 
 // 4-bit codes split over a low-bit word and a high-bit word (promoted key channels): code = low | high << 2
-template <int DT>
+template <int DT, int N>
 __device__ __forceinline__ void dequant_word4(const CodeConsts<DT>& k, uint32_t wl, uint32_t wh, uint32_t ss,
-                                              uint32_t zz, uint32_t ms0, uint32_t ms1, uint32_t (&r)[8]) {
+                                              uint32_t zz, uint32_t ms0, uint32_t ms1, uint32_t (&r)[N]) {
   using H = Half2Ops<DT>;
   constexpr int P0 = H::kFirstPos;
 #pragma unroll
-  for (int grp = 0; grp < 4; ++grp) {
+  for (int grp = 0; grp < N / 2; ++grp) {
     const uint32_t xl = align_codes(wl, 2 * grp, P0);
     const uint32_t xh = align_codes(wh, 2 * grp, P0, 2);
 #pragma unroll
