@@ -681,8 +681,9 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
 // 3,300 tokens) take 14.3 us instead of 12.3; with room for seventeen, calls of two and three slots take 13.3 to 14.3 us
 // instead of 12.3 and calls of nine to seventeen gain nothing (B200).
 constexpr int kRowSlots = 8;   // the lanes of the reductions below
+constexpr int kRowDim = 128;   // channels of the tensor-core layouts
 __global__ void __launch_bounds__(256) decode_merge_rows_kernel(const float* __restrict__ part_m, const float* __restrict__ part_l,
-                                                                const float* __restrict__ part_acc, int total_splits, int D, void* out,
+                                                                const float* __restrict__ part_acc, int total_splits, void* out,
                                                                 int out_dt, int stream_blocks, int64_t units, int quads, int query_heads,
                                                                 int kv_heads, int row_groups, int rows) {
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -693,52 +694,42 @@ __global__ void __launch_bounds__(256) decode_merge_rows_kernel(const float* __r
                      dartkv_block_of_unit(bh * quads, stream_blocks, units);
   const int64_t base = (int64_t)row * total_splits;
   asm volatile("griddepcontrol.wait;" ::: "memory");   // see decode_merge_kernel
-  float4 v[kRowSlots];
-  auto load = [&](int c) {
+  const int c = 4 * lane;
+  float4 v[kRowSlots];   // requested before the weights are known
 #pragma unroll
-    for (int s = 0; s < kRowSlots; ++s) {
-      v[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (s < splits && c < D) {
-        const float2* at = reinterpret_cast<const float2*>(part_acc + (base + s) * D + c);   // 8-byte aligned
-        const float2 a = at[0], b = at[1];
-        v[s] = make_float4(a.x, a.y, b.x, b.y);
-      }
+  for (int s = 0; s < kRowSlots; ++s) {
+    v[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (s < splits) {
+      const float2* at = reinterpret_cast<const float2*>(part_acc + (base + s) * kRowDim + c);   // 8-byte aligned
+      const float2 a = at[0], b = at[1];
+      v[s] = make_float4(a.x, a.y, b.x, b.y);
     }
-  };
-  load(4 * lane);   // requested before the weights are known
+  }
   const float ms = lane < splits ? part_m[base + lane] : -INFINITY, ls = lane < splits ? part_l[base + lane] : 0.0f;
   float m = ms;
 #pragma unroll
-  for (int off = 4; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = kRowSlots / 2; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
   const bool live = ms != -INFINITY;   // the sums of an empty split may be anything
   const float w = live ? expf(ms - m) : 0.0f;
   float l = live ? ls * w : 0.0f;
 #pragma unroll
-  for (int off = 4; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+  for (int off = kRowSlots / 2; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
   const float norm = 1.0f / fmaxf(__shfl_sync(0xffffffffu, l, 0), 1e-20f);
   const uint32_t lives = __ballot_sync(0xffffffffu, live);
-  float ws[kRowSlots];
+  float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-  for (int s = 0; s < kRowSlots; ++s) ws[s] = __shfl_sync(0xffffffffu, w, s);
-  for (int c = 4 * lane; c < D; c += 128) {
-    if (c >= 128) load(c);
-    float r[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int s = 0; s < kRowSlots; ++s)
-      if ((lives >> s) & 1u) {   // Inf and NaN count even where the weight is zero
-        r[0] = fmaf(v[s].x, ws[s], r[0]); r[1] = fmaf(v[s].y, ws[s], r[1]);
-        r[2] = fmaf(v[s].z, ws[s], r[2]); r[3] = fmaf(v[s].w, ws[s], r[3]);
-      }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r[i] *= norm;
-    if (out_dt == DARTKV_F32) {
-      *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (int64_t)row * D + c) = make_float4(r[0], r[1], r[2], r[3]);
-    } else {
-      const uint2 x = out_dt == DARTKV_BF16 ? make_uint2(pack16<DARTKV_BF16>(r[0], r[1]), pack16<DARTKV_BF16>(r[2], r[3]))
-                                            : make_uint2(pack16<DARTKV_F16>(r[0], r[1]), pack16<DARTKV_F16>(r[2], r[3]));
-      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out) + (int64_t)row * D + c) = x;
+  for (int s = 0; s < kRowSlots; ++s) {
+    const float ws = __shfl_sync(0xffffffffu, w, s);
+    if ((lives >> s) & 1u) {   // Inf and NaN count even where the weight is zero
+      r[0] = fmaf(v[s].x, ws, r[0]); r[1] = fmaf(v[s].y, ws, r[1]);
+      r[2] = fmaf(v[s].z, ws, r[2]); r[3] = fmaf(v[s].w, ws, r[3]);
     }
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) r[i] *= norm;
+  const uint2 x = out_dt == DARTKV_BF16 ? make_uint2(pack16<DARTKV_BF16>(r[0], r[1]), pack16<DARTKV_BF16>(r[2], r[3]))
+                                        : make_uint2(pack16<DARTKV_F16>(r[0], r[1]), pack16<DARTKV_F16>(r[2], r[3]));
+  *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(out) + (int64_t)row * kRowDim + c) = x;
 }
 
 // ---------------------------------------------------------------------------- host side
@@ -836,15 +827,16 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     bh = d->batch * d->kv_heads;
   }
   if (L.fast) {
-    // One unit = four consecutive pages of a (batch, kv head) (a block hands them to its four warp pairs).  The
-    // units of all rows are dealt out evenly to `stream_blocks` blocks.  Two families of splits are compared with a
-    // cost model in units of one page per pair (a block costs its pages per pair plus 1.75 per row it touches:
-    // query load, first-page latency, merge of its eight warps; the dense block of a row about 2; blocks run in
-    // waves of two per SM; constants fitted to B200 timings):
+    // One unit = four consecutive pages of a (batch, kv head).  The units of all rows are dealt out evenly to
+    // `stream_blocks` blocks.  Two families of splits are compared with a cost model in units of a round of four pages
+    // (a block costs its rounds plus 1.75 per row it touches: query load, first-page latency, merge of its eight warps;
+    // the dense block of a row about 2; blocks run in waves of two per SM):
     //   aligned    rows * s blocks, s = 1..16 pieces per row;
     //   unaligned  one block per resident slot, a block may finish one row and start the next (at most 16 blocks
     //              touch a row); measured ~3 % slower per unit than aligned blocks, but it fills every slot when
     //              the rows do not (e.g. 256 rows on 296 slots: 9 % faster at context 32768).
+    // The constants were fitted to B200 timings of kernels that put two warps on each of a round's four pages, as
+    // decode_rows and decode_wide do.  The 2-bit kernels take eight pages a round; they have not been refitted to them.
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
@@ -1048,16 +1040,16 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     attribute.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    // few slots a row: a warp per row.  It reads and writes groups of four channels.
-    if (L.fast && L.total_splits <= kRowSlots && !peers && D % 4 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)part_acc % 8 == 0 &&
+    // few slots a row of a tensor-core layout (128 channels, 16 bits): a warp per row, which moves four channels at a time
+    if (L.fast && L.total_splits <= kRowSlots && !peers && (uintptr_t)out % 8 == 0 && (uintptr_t)part_acc % 8 == 0 &&
         rows / L.total_splits < (1ll << 31)) {
       const int out_rows = (int)(rows / L.total_splits);
       config.gridDim = dim3((out_rows + 7) / 8);
       config.blockDim = dim3(256);
       config.dynamicSmemBytes = 0;
       DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, decode_merge_rows_kernel, (const float*)part_m, (const float*)part_l,
-                                        (const float*)part_acc, L.total_splits, D, out, q_dtype, L.stream_blocks, (int64_t)L.units,
-                                        L.quads, query_heads, d->kv_heads, L.row_groups, out_rows));
+                                        (const float*)part_acc, L.total_splits, out, q_dtype, L.stream_blocks, (int64_t)L.units, L.quads,
+                                        query_heads, d->kv_heads, L.row_groups, out_rows));
       DARTKV_LAUNCH_OK("decode_merge_rows_kernel");
       return DARTKV_OK;
     }

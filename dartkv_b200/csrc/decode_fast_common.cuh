@@ -14,9 +14,6 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kPageBytesK = 5760;
 constexpr int kValueCodes = 4096;
 constexpr int kStageBytes = 10880;            // key blob (<= 5760) | value codes 4096 | value metadata (<= 1024)
-constexpr int kOffVCodes = kPageBytesK;       // 5760
-constexpr int kOffVMeta = kPageBytesK + kValueCodes;  // 9856
-constexpr int kPStride = 72;                  // 16-bit elements per (plane, head) row of a warp's probability tile
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ void pair_barrier(int pair) {
@@ -28,10 +25,10 @@ struct FastArgs {
   int query_heads;
   float scale;
   int flavour;
-  // Work split: one unit = four consecutive pages of one (batch, kv head) (one page per warp pair); the units of
-  // all (batch, kv head) rows, `quads` each, are dealt out evenly to `stream_blocks` blocks, so a block may finish
-  // one row and start the next.  Partial slot 0 of a row belongs to its dense-token block, slot 1 + k to the
-  // k-th stream block that touches the row.
+  // Work split: one unit = four consecutive pages of one (batch, kv head) (a round of the four warp pairs of decode_rows and
+  // decode_wide, half a round of the eight warps of the 2-bit kernels); the units of all (batch, kv head) rows, `quads` each,
+  // are dealt out evenly to `stream_blocks` blocks, so a block may finish one row and start the next.  Partial slot 0 of a row
+  // belongs to its dense-token block, slot 1 + k to the k-th stream block that touches the row.
   int quads, stream_blocks;
   long long units;
   int total_splits;

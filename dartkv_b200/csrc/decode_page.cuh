@@ -44,8 +44,7 @@ __device__ __forceinline__ uint32_t high_twice(uint32_t x) { return prmt(x, x, 0
 // GN: value groups per token (1 or 2).  KP: promoted channels per page when that is a multiple of eight known to
 // the host (0, 8, 16, 24, 32), else -1 (read from the descriptor): with the count fixed the logits loops have
 // constant trip counts and no per-position "is this slot promoted" test.
-// COMPACT: the query as 16-bit values [channel][head] instead of pre-shifted words [channel][2 * head + j'].
-template <int DT, int OUT, int GN, int KP, bool COMPACT = false>
+template <int DT, int OUT, int GN, int KP>
 struct PageWork {
   using H = Half2Ops<DT>;
   using HO = Half2Ops<OUT>;
@@ -55,7 +54,7 @@ struct PageWork {
   static constexpr int kPromUnroll = 4, kQkUnroll = 4, kPvUnroll = 1;
   CodeConsts<DT> cc;
   const dartkv_cache_desc& d;
-  const uint8_t* q_thread;   // this thread's column of the query: + 32 * channel, COMPACT + 8 * channel
+  const uint8_t* q_thread;   // this thread's column of the query: + 32 * channel
   float scale2;
   int lane, g, c, K, prom_steps;
   bool gv;                   // this thread's sixteen channels are of value group 1
@@ -68,13 +67,12 @@ struct PageWork {
     K = KP >= 0 ? KP : (d.key_mode == DARTKV_MIXED_PAGE ? d.promoted : 0);
     prom_steps = (K + 7) >> 3;
     gv = (16 * g) / d.value_group;
-    q_thread = reinterpret_cast<const uint8_t*>(query_table) + (COMPACT ? 2 * (g >> 1) : 4 * g);
+    q_thread = reinterpret_cast<const uint8_t*>(query_table) + 4 * g;
   }
 
   // column n = g of the query operand: head g >> 1 in half j' = g & 1, zero in the other; row32 = 32 * channel
   __device__ __forceinline__ uint32_t query(uint32_t row32) const {
-    if (!COMPACT) return *reinterpret_cast<const uint32_t*>(q_thread + row32);
-    return (uint32_t)*reinterpret_cast<const uint16_t*>(q_thread + (row32 >> 2)) << (16 * (g & 1));
+    return *reinterpret_cast<const uint32_t*>(q_thread + row32);
   }
 
   __device__ __forceinline__ void start_row() {

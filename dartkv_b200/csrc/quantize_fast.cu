@@ -32,8 +32,8 @@ struct ColumnArgs {
 };
 
 // grid (group, slab of columns, outer); 64 threads per token split.  KB: 0 = mixed 2+2-bit keys, else the code width.
-// TOK: tokens of a thread where that is 8, 16 or 32 (groups of 32, 64 and 128): all are requested at once and kept in registers
-// between the search for minimum and maximum and the codes; 0 for other groups, which read them twice, eight at a time.
+// TOK: tokens of a thread, which is the group over the token splits, where that is 8, 16 or 32: all are requested at once and
+// kept in registers between the search for minimum and maximum and the codes; 0 for other groups, which read them twice, eight at a time.
 template <int DT, int KB, int TOK>
 __global__ void __launch_bounds__(256, TOK == 32 ? 2 : 4) quantize_columns_kernel(const __grid_constant__ ColumnArgs a) {
   using P = Pack16<DT>;
