@@ -224,17 +224,18 @@ int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int
   {
     // the shared-memory opt-in is per device and per kernel: ask once per device (the flags are atomic; two threads
     // that race on a device's first call both set the attribute, which is harmless)
-    static std::atomic<bool> ready[64][2];
+    static std::atomic<bool> ready[64];
     int device = 0;
     DARTKV_CUDA_OK(cudaGetDevice(&device));
-    if (device < 0 || device >= 64 || !ready[device][few].load(std::memory_order_acquire)) {
+    if (device < 0 || device >= 64 || !ready[device].load(std::memory_order_acquire)) {
       for (int md : {DARTKV_BF16, DARTKV_F16})
         for (int dt : {DARTKV_BF16, DARTKV_F16})
           for (int gn : {1, 2})
             for (int kp : {-1, 0, 8, 16, 24, 32})
-              DARTKV_CUDA_OK(cudaFuncSetAttribute(fast_variant(few, md, dt, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)kSmemBytes));
-      if (device >= 0 && device < 64) ready[device][few].store(true, std::memory_order_release);
+              for (bool each : {false, true})   // the next call, of another length, may be under graph capture
+                DARTKV_CUDA_OK(cudaFuncSetAttribute(fast_variant(each, md, dt, gn, kp), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)kSmemBytes));
+      if (device >= 0 && device < 64) ready[device].store(true, std::memory_order_release);
     }
   }
   const int promoted = d->key_mode == DARTKV_MIXED_PAGE ? d->promoted : 0;
