@@ -61,7 +61,7 @@ struct GenericArgs {
 // tile's tokens split over the remaining threads.  Nothing dequantized is staged.  Latency is what counts here (small
 // fp32 caches): loads of several channels / tokens are in flight together, and a call is cut into tiles until every SM
 // has a block.  [1,8,256,128] fp32, 2-bit: 98 us per call with one serial dot product per thread and staged tiles, 31 us so
-// (B200; decode_tiles_kernel, which takes such small calls of uniform pages, 21).
+// (B200; decode_tiles_kernel, which takes such small calls of uniform pages, 16).
 template <int REP>
 __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                      const __grid_constant__ GenericArgs a) {
@@ -283,11 +283,11 @@ template <int MD> __device__ __forceinline__ float load_md(const void* p, int64_
   return reinterpret_cast<const float*>(p)[i];
 }
 
-// Uniform key pages: what decode_generic_kernel does, with the chain of memory latencies of a tile cut to two.  Every lane
-// finds the place of its own token (sink, page, dense tail), so a tile is not cut at segment edges; pages are found without
-// a search where there are at most 32; the metadata dtype is a template argument (loads behind a run-time choice of dtype
-// are not batched); the tile's values are requested with its keys.  The blocks of a (batch, KV head), a.cluster of them,
-// are a cluster that merges its results through distributed shared memory.
+// Uniform key pages of few tokens: what decode_generic_kernel does, one tile of 32 tokens per block, with the chain of memory
+// latencies cut to two.  Every lane finds the place of its own token (sink, page, dense tail), so a tile is not cut at segment
+// edges; pages are found without a search where there are at most 32; the metadata dtype is a template argument (loads behind a
+// run-time choice of dtype are not batched); the tile's values, packed or dense, are requested with its keys.  The blocks of a
+// (batch, KV head), a.cluster of them, are a cluster that merges its results through distributed shared memory.
 template <int REP, int MD>
 __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                       const __grid_constant__ GenericArgs a) {
@@ -297,8 +297,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
   float* s_q = smem;                                     // [D][REP]
   float* s_part = s_q + D * REP;                         // [warp][REP][32] partial logits, then [split][REP][D] sums
   float* s_p = s_part + GEN_THREADS * REP;               // [32][REP] probabilities of the tile
-  float* s_alpha = s_p + GEN_TILE * REP;                 // [REP]
-  float* s_m = s_alpha + REP;
+  float* s_m = s_p + GEN_TILE * REP;                     // [REP]
   float* s_l = s_m + REP;
   static_assert(GEN_WARPS * GEN_TILE <= GEN_THREADS, "partial logits and sums share memory");
 
@@ -306,9 +305,9 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
   const int b = bh / d.kv_heads, h = bh % d.kv_heads;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int seen = d.state[0], pages = d.state[1], k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
-  const int first = split * a.chunk;
-  const int hi = (int)min((int64_t)first + a.chunk, (int64_t)seen);
+  const int first = split * GEN_TILE;
   const int lo = a.row_start ? max(first, a.row_start[b]) : first;
+  const int nt = min(first + GEN_TILE, seen) - lo;       // tokens of this block, none or less where the row starts behind them
   // irregular pages, a page per lane where there are few; regular ones are computed
   int my_first = 0, my_tokens = 0;
   const bool by_lane = !d.regular_pages && pages <= 32;
@@ -334,9 +333,8 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
   };
   __syncthreads();
 
-  for (int tile0 = lo; tile0 < hi; tile0 += GEN_TILE) {
-    const int nt = min(GEN_TILE, hi - tile0);
-    const int tok = tile0 + min(lane, nt - 1);           // lanes past the tile repeat its last token
+  if (nt > 0) {
+    const int tok = lo + min(lane, nt - 1);              // lanes past the tile repeat its last token
     // ---- the place of this lane's key
     const bool packed = tok >= sink_filled && tok < k_end;
     int page_first = 0, page_n = 1, pg = 0, key_flavour = a.flavour;
@@ -359,29 +357,36 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
       const int next_value_edge = d.sink_tokens + ((page_first - d.sink_tokens) / d.page_size + 1) * d.page_size;
       if (min(next_value_edge, v_end) < page_first + page_n) key_flavour = DARTKV_DEQUANT_PER_OP;
     }
-    // ---- the tile's values are requested (the first kAhead of this thread's tokens)
+    // ---- the tile's values are requested, kAhead of this thread's tokens at a time, the first ones before the keys are
+    // waited for.  A dense value takes the scale's register.  One copy of this code serves all of a tile's tokens: instruction
+    // fetch is the longest stall of such a call.  Dense [1,8,20,256] fp32, one query row per KV head: 20.5 us with dense values
+    // loaded one by one behind the softmax, 21.2 with a second copy of the code for the first tokens, 16.4 so.  Sixteen ahead
+    // with more query rows: 16 rows of that shape 37.2 us instead of 33.1.
     constexpr int kAhead = REP <= 4 ? 16 : 8;
     uint32_t v_code[kAhead];
     float v_scale[kAhead], v_zero[kAhead];
     auto value_packed = [&](int t) { return t >= sink_filled && t < v_end; };
-    auto dense_value = [&](int t) {
-      return t < sink_filled ? load_f(d.v_sink, d.dtype, ((int64_t)bh * d.sink_tokens + t) * D + vc)
-                             : load_f(d.v_ring, d.dtype, ((int64_t)bh * d.ring_tokens + (t % d.ring_tokens)) * D + vc);
-    };
-    auto value_row = [&](int t) { return (int64_t)bh * d.max_value_tokens + (t - d.sink_tokens); };
-    if (vsplit < vsplits) {
+    auto request = [&](int base, auto dense) {
 #pragma unroll
       for (int i = 0; i < kAhead; ++i) {
-        const int t = tile0 + vsplit + i * vsplits;
+        const int tt = vsplit + (base + i) * vsplits, t = lo + tt;
         v_code[i] = 0; v_scale[i] = v_zero[i] = 0.0f;
-        if (t < tile0 + nt && value_packed(t)) {
-          const int64_t row = value_row(t);
+        if (tt < nt && value_packed(t)) {
+          const int64_t row = (int64_t)bh * d.max_value_tokens + (t - d.sink_tokens);
           v_code[i] = d.v_codes[row * d.value_row_bytes + vc / per];
           v_scale[i] = load_md<MD>(d.v_meta, (row * 2 + 0) * d.value_groups + vg);
           v_zero[i] = load_md<MD>(d.v_meta, (row * 2 + 1) * d.value_groups + vg);
+        } else if (tt < nt) {
+          v_scale[i] = t < sink_filled ? dense(d.v_sink, ((int64_t)bh * d.sink_tokens + t) * D + vc)
+                                       : dense(d.v_ring, ((int64_t)bh * d.ring_tokens + (t % d.ring_tokens)) * D + vc);
         }
       }
-    }
+    };
+    auto request_values = [&](int base) {
+      if (d.dtype == DARTKV_F32) request(base, [](const void* p, int64_t i) { return reinterpret_cast<const float*>(p)[i]; });
+      else request(base, [&](const void* p, int64_t i) { return load_f(p, d.dtype, i); });
+    };
+    if (vsplit < vsplits) request_values(0);
     // ---- partial logits of this warp's channels
     float dot[REP];
 #pragma unroll
@@ -427,56 +432,38 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
 #pragma unroll
     for (int r = 0; r < REP; ++r) s_part[(warp * REP + r) * GEN_TILE + lane] = dot[r];
     __syncthreads();
-    // ---- online softmax state, a warp per query head
+    // ---- softmax over the tile, a warp per query head
     for (int r = warp; r < rep; r += GEN_WARPS) {
       float v = 0.0f;
 #pragma unroll
       for (int w = 0; w < GEN_WARPS; ++w) v += s_part[(w * REP + r) * GEN_TILE + lane];
       v = lane < nt ? v * a.scale : -INFINITY;
-      float mx = v;
+      float m = v;
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_old = s_m[r], m_new = fmaxf(m_old, mx);
-      const float m_ref = m_new == -INFINITY ? 0.0f : m_new;   // every logit so far -Inf or NaN: the former weigh nothing
-      const float e = expf(v - m_ref);
+      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+      const float e = expf(v - (m == -INFINITY ? 0.0f : m));   // every logit -Inf or NaN: the former weigh nothing
       float sum = e;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
       s_p[lane * REP + r] = e;
-      __syncwarp();
-      if (lane == 0) {
-        const float alpha = expf(m_old - m_ref);
-        s_alpha[r] = alpha;
-        s_m[r] = m_new;
-        s_l[r] = s_l[r] * alpha + sum;
-      }
+      if (lane == 0) { s_m[r] = m; s_l[r] = sum; }
     }
     __syncthreads();
     // ---- values
     if (vsplit < vsplits) {
-#pragma unroll
-      for (int r = 0; r < REP; ++r) acc[r] *= r < rep ? s_alpha[r] : 0.0f;
-      auto weigh = [&](int tt, float v) {
-#pragma unroll
-        for (int r = 0; r < REP; ++r) acc[r] = fmaf(r < rep ? s_p[tt * REP + r] : 0.0f, v, acc[r]);
-      };
       const int vshift = (vc % per) * vbits;
+#pragma unroll 1
+      for (int base = 0; vsplit + base * vsplits < nt; base += kAhead) {
+        if (base > 0) request_values(base);
 #pragma unroll
-      for (int i = 0; i < kAhead; ++i) {
-        const int tt = vsplit + i * vsplits;
-        if (tt < nt)
-          weigh(tt, value_packed(tile0 + tt) ? affine_restore((float)((v_code[i] >> vshift) & vmask), v_scale[i], v_zero[i], MD, d.dtype,
-                                                              value_flavour(tile0 + tt))
-                                             : dense_value(tile0 + tt));
-      }
-#pragma unroll 4
-      for (int tt = vsplit + kAhead * vsplits; tt < nt; tt += vsplits) {
-        const int t = tile0 + tt;
-        const int64_t row = value_row(t);
-        weigh(tt, value_packed(t) ? affine_restore((float)((d.v_codes[row * d.value_row_bytes + vc / per] >> vshift) & vmask),
-                                                   load_md<MD>(d.v_meta, (row * 2 + 0) * d.value_groups + vg),
-                                                   load_md<MD>(d.v_meta, (row * 2 + 1) * d.value_groups + vg), MD, d.dtype, value_flavour(t))
-                                  : dense_value(t));
+        for (int i = 0; i < kAhead; ++i) {
+          const int tt = vsplit + (base + i) * vsplits, t = lo + tt;
+          if (tt >= nt) break;
+          const float v = value_packed(t) ? affine_restore((float)((v_code[i] >> vshift) & vmask), v_scale[i], v_zero[i], MD, d.dtype, value_flavour(t))
+                                          : v_scale[i];
+#pragma unroll
+          for (int r = 0; r < REP; ++r) acc[r] = fmaf(r < rep ? s_p[tt * REP + r] : 0.0f, v, acc[r]);
+        }
       }
     }
     __syncthreads();
@@ -492,12 +479,10 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
     for (int r = 0; r < REP; ++r) {
       acc[r] = 0.0f;
       for (int s = 0; s < vsplits; ++s) acc[r] += s_part[(s * REP + r) * D + vc];
+      s_part[r * D + vc] = acc[r];   // nobody else reads these entries before the cluster meets
     }
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
-  if (vsplit == 0)
-#pragma unroll
-    for (int r = 0; r < REP; ++r) s_part[r * D + vc] = acc[r];   // nobody else reads these entries before the cluster meets
   cluster.sync();
   for (int i = split * GEN_THREADS + tid; i < rep * D; i += a.cluster * GEN_THREADS) {
     const int r = i / D, c = i - r * D;
@@ -524,7 +509,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
 }
 
 static size_t tiles_smem(int D, int rep) {
-  return ((size_t)D * rep + (size_t)GEN_THREADS * rep + (size_t)GEN_TILE * rep + 3 * rep) * sizeof(float);
+  return ((size_t)D * rep + (size_t)GEN_THREADS * rep + (size_t)GEN_TILE * rep + 2 * rep) * sizeof(float);
 }
 
 using GenericKernel = void (*)(const dartkv_cache_desc, const GenericArgs);
@@ -996,11 +981,12 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     a.row_start = row_start;
     DARTKV_REQUIRE(L.generic_splits <= 65535, "too many splits");
     const int padded_rep = rep <= 1 ? 1 : rep <= 2 ? 2 : rep <= 4 ? 4 : rep <= 8 ? 8 : 16;
-    // Uniform pages of few tiles: decode_tiles_kernel, whose blocks of a KV head are a cluster of the portable size at most
-    // and two of which fit an SM: [1,8,256,128] fp32, 2-bit 31.2 -> 21.0 us (23 with a merge launch of its own).  Calls of more
-    // blocks need the occupancy of decode_generic_kernel (four of 2,048 tokens 80 us there, 107 as tiles), and calls of
-    // more tiles gain nothing (two of 700 tokens, 64 channels: 18.7 us there, 19.5 as tiles).
-    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_splits <= 8 && bh * L.generic_splits <= 2 * dartkv_sm_count();
+    // Uniform pages of up to eight tiles, a block each: decode_tiles_kernel, whose blocks of a KV head are a cluster (of the
+    // portable size) and two of which fit an SM.  [1,8,256,128] fp32, 2-bit: 31.2 us through decode_generic_kernel and a merge
+    // launch, 16.4 here (23 with a merge launch of its own).  More blocks than two per SM gain nothing or lose: 64 rows of 160 tokens (320 blocks) 22.6 us there and
+    // 24.6 as tiles with 64 channels, 32.8 and 30.8 with 128; 192 rows of 96 tokens (576 blocks) 24.6 and 42.8.
+    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_chunk == GEN_TILE && L.generic_splits <= 8 &&
+                       bh * L.generic_splits <= 2 * dartkv_sm_count();
     a.cluster = tiles ? L.generic_splits : 0;
     a.out = peers ? nullptr : out;
     const size_t smem = tiles ? tiles_smem(D, padded_rep) : generic_smem(D, padded_rep);
