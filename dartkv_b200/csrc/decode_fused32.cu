@@ -98,7 +98,8 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1,
 // the host (0, 8, 16, 24, 32), else -1 (read from the descriptor).
 template <int DT, int MD, int GN, int KP>
 struct FusedWork {
-  static constexpr int kQkUnroll = 16, kPvUnroll = 4;   // 64 x 32,768 tokens: 382 us; with 4 and 4 386, with 2 and 2 396
+  // 64 x 32,768 tokens: 382 us; with 4 and 4 386, with 2 and 2 396 (on one GPU; others give this version 392 to 414)
+  static constexpr int kQkUnroll = 16, kPvUnroll = 4;
   const dartkv_cache_desc& d;
   const uint2* query;
   float scale2;

@@ -24,10 +24,10 @@
 // Staging is by bulk copies on mbarriers, keys and values separately: with one buffer each (4-bit pages) the next
 // page's keys arrive during P.V and its values during the logits, two blocks per SM stay resident.
 //
-// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 75 us here (the query
+// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 70 us here (the query
 // rows in M instead of N needed 64 + 32 accumulators and spilled: 88 us).  Five query tokens on batch 8, 4,096 tokens,
 // 2-bit: 160 us as five passes of decode_fast.cu, 68 us here in one launch (16-row blocks, which spill: 92 us).  One
-// query token on the 2-bit pages of decode_fast.cu stays there: 1,091 us against 1,462 us at batch 128, 32,768 tokens.
+// query token on the 2-bit pages of decode_fast.cu stays there: 1,089 us against 1,462 us at batch 128, 32,768 tokens.
 
 #include <atomic>
 

@@ -3,11 +3,11 @@
 // keeps the kernels of quantize.cu, which handle one group (or element) per thread.
 //
 // All of these are bound by memory latency and by the few instructions per element, not by capacity: a group's tokens
-// are split over up to four threads per channel pair, and requested at once where they fit registers, codes gather in registers (quant_math.cuh)
-// and leave as whole words.  fp16 [8,8,1024,128], 2-bit + promoted keys / 2-bit values, a call among others: keys with the
-// selection 24.6 us, values 12.3, restoring either 10.3; all four calls with their checks and waits 103 us, 96 with the
-// tokens of a column group held in registers, several blocks per row for the scores and no 64-bit divisions; 503 with one
-// group or element per thread (B200).
+// are split over up to four threads per channel pair, and requested at once where they fit registers, codes gather in
+// registers (quant_math.cuh) and leave as whole words.  fp16 [8,8,1024,128], 2-bit + promoted keys in groups of 128 / 2-bit
+// values, a call of the Python API among others, with its allocations and the check of its input: keys with the selection
+// 33.7 us (36.7 with the tokens of a column group read twice), values 24.3, restoring them 10.7; all four calls with their
+// waits 92.5 us, 503 with one group or element per thread (B200).
 
 #include <cooperative_groups.h>
 
