@@ -983,7 +983,7 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     const int padded_rep = rep <= 1 ? 1 : rep <= 2 ? 2 : rep <= 4 ? 4 : rep <= 8 ? 8 : 16;
     // Uniform pages of up to eight tiles, a block each: decode_tiles_kernel, whose blocks of a KV head are a cluster (of the
     // portable size) and two of which fit an SM.  [1,8,256,128] fp32, 2-bit: 31.2 us through decode_generic_kernel and a merge
-    // launch, 16.4 here (23 with a merge launch of its own).  More blocks than two per SM gain nothing or lose: 64 rows of 160 tokens (320 blocks) 22.6 us there and
+    // launch, 16.4 here.  More blocks than two per SM gain nothing or lose: 64 rows of 160 tokens (320 blocks) 22.6 us there and
     // 24.6 as tiles with 64 channels, 32.8 and 30.8 with 128; 192 rows of 96 tokens (576 blocks) 24.6 and 42.8.
     const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_chunk == GEN_TILE && L.generic_splits <= 8 &&
                        bh * L.generic_splits <= 2 * dartkv_sm_count();
