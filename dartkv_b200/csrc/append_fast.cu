@@ -482,7 +482,7 @@ template <int DT, int KBITS, int VBITS>
 __global__ void __launch_bounds__(kThreads, 4) append_step_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                   const __grid_constant__ StepArgs a) {
   __shared__ KeySmem sm;
-  follow_previous();
+  wait_previous();
   // read through the pointer where it is needed: the plan's numbers are not kept in registers across the page code
   const dartkv_append_plan& plan = a.device_plan ? *a.device_plan : a.plan;
   // grid: (kv head, batch row, page and role): no division to find any of them

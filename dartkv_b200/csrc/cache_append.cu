@@ -69,6 +69,7 @@ constexpr int kCopyRows = 8;   // rows per block of the dense copy
 __global__ void copy_dense_kernel(dartkv_cache_desc d, dartkv_append_plan p, const void* keys, const void* values,
                                   int64_t sb, int64_t sh, int64_t st, int ring_first, int rows, int vector_ok,
                                   int32_t* nonfinite, const dartkv_append_plan* device_plan) {
+  wait_previous();
   if (device_plan) {
     p = *device_plan;
     const DenseRows r = dense_rows(p);
@@ -91,6 +92,7 @@ __global__ void key_pages_kernel(dartkv_cache_desc d, TokenSource src, int first
                                  int page_token_start, int last_page_tokens, const int32_t* __restrict__ indices,
                                  int32_t* nonfinite) {
   extern __shared__ uint32_t s_mem[];
+  wait_previous();
   uint32_t* s_key = s_mem;
   int* s_slot = reinterpret_cast<int*>(s_mem + d.head_dim);
   const int bh = blockIdx.x, pg = blockIdx.y;
@@ -214,6 +216,7 @@ __global__ void key_pages_kernel(dartkv_cache_desc d, TokenSource src, int first
 // One thread per (bh, token, unit); a token's groups run along head_dim.
 __global__ void value_rows_kernel(dartkv_cache_desc d, TokenSource src, int value_begin, int value_end, int unit,
                                   int units, int32_t* nonfinite) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int count = value_end - value_begin;
   int64_t total = (int64_t)d.batch * d.kv_heads * count * units;
@@ -280,6 +283,7 @@ __device__ __forceinline__ float page_key_element(const dartkv_cache_desc& d, co
 // re-quantization of src/dart/cache.py:427-439); grid (bh, token of the page)
 __global__ void page_to_ring_kernel(dartkv_cache_desc d, int slot_index, int page_token_start, int n) {
   extern __shared__ int s_slot[];
+  wait_previous();
   const int bh = blockIdx.x, j = blockIdx.y, D = d.head_dim;
   const uint8_t* page = d.k_pages + ((int64_t)bh * d.max_key_pages + slot_index) * d.key_page_bytes;
   if (d.key_mode == DARTKV_MIXED_PAGE) {
@@ -338,10 +342,12 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
   if (p.requantize_last_page) {
     DARTKV_REQUIRE(p.first_page > 0 && p.page_token_start - d.page_size >= 0, "nothing to re-quantize");
     const int slot = p.first_page - 1, start = p.page_token_start - d.page_size;
-    page_to_ring_kernel<<<dim3(bh, d.page_size), 128, d.head_dim * sizeof(int), stream>>>(d, slot, start, d.page_size);
+    DARTKV_CUDA_OK(launch_following(page_to_ring_kernel, dim3(bh, d.page_size), 128, d.head_dim * sizeof(int), stream, d, slot, start,
+                                    d.page_size));
     DARTKV_LAUNCH_OK("page_to_ring_kernel");
     TokenSource ring_only{nullptr, d.k_ring, 0, 0, 0, INT32_MAX, d.ring_tokens, d.head_dim, d.kv_heads, d.dtype};
-    key_pages_kernel<<<dim3(bh, 1), 128, page_smem, stream>>>(d, ring_only, slot, 1, start, d.page_size, indices, nullptr);
+    DARTKV_CUDA_OK(launch_following(key_pages_kernel, dim3(bh, 1), 128, page_smem, stream, d, ring_only, slot, 1, start, d.page_size,
+                                    indices, nullptr));
     DARTKV_LAUNCH_OK("key_pages_kernel (re-quantize)");
     // an explicit index list carries the re-quantized page first, one [promoted] row per (bh)
     if (indices) new_page_indices = indices + (int64_t)bh * d.promoted;
@@ -358,9 +364,8 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
     } else {
       TokenSource ks{keys, d.k_ring, stride_b, stride_h, stride_t, p.chunk_start, d.ring_tokens, d.head_dim, d.kv_heads, d.dtype};
       DARTKV_REQUIRE(p.num_pages <= 65535, "too many pages in one append (limit 65535)");
-      key_pages_kernel<<<dim3(bh, p.num_pages), 128, page_smem, stream>>>(d, ks, p.first_page, p.num_pages,
-                                                                         p.page_token_start, p.last_page_tokens,
-                                                                         new_page_indices, nonfinite);
+      DARTKV_CUDA_OK(launch_following(key_pages_kernel, dim3(bh, p.num_pages), 128, page_smem, stream, d, ks, p.first_page, p.num_pages,
+                                      p.page_token_start, p.last_page_tokens, new_page_indices, nonfinite));
       DARTKV_LAUNCH_OK("key_pages_kernel");
     }
   }
@@ -374,7 +379,8 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
       const int unit = d.value_group / dartkv_gcd(d.value_group, vpb) * vpb;
       const int units = ceil_div(d.value_groups * d.value_group, unit);
       int64_t threads = (int64_t)bh * (p.value_end - p.value_begin) * units;
-      value_rows_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, stream>>>(d, vs, p.value_begin, p.value_end, unit, units, nonfinite);
+      DARTKV_CUDA_OK(launch_following(value_rows_kernel, (unsigned)((threads + 127) / 128), 128, 0, stream, d, vs, p.value_begin,
+                                      p.value_end, unit, units, nonfinite));
       DARTKV_LAUNCH_OK("value_rows_kernel");
     }
   }
@@ -386,8 +392,8 @@ extern "C" int dartkv_cache_append(const dartkv_cache_desc* desc, const dartkv_a
     const int esize = dartkv_dtype_size(d.dtype);
     const int vector_ok = (d.head_dim * esize) % 16 == 0 && (stride_b * esize) % 16 == 0 && (stride_h * esize) % 16 == 0 &&
                           (stride_t * esize) % 16 == 0 && ((uintptr_t)keys | (uintptr_t)values) % 16 == 0;
-    copy_dense_kernel<<<dim3(rows > 0 ? bh : 1, row_blocks, rows > 0 ? 2 : 1), 128, 0, stream>>>(
-        d, p, keys, values, stride_b, stride_h, stride_t, ring_first, rows, vector_ok, nonfinite, nullptr);
+    DARTKV_CUDA_OK(launch_following(copy_dense_kernel, dim3(rows > 0 ? bh : 1, row_blocks, rows > 0 ? 2 : 1), 128, 0, stream, d, p, keys,
+                                    values, stride_b, stride_h, stride_t, ring_first, rows, vector_ok, nonfinite, nullptr));
     DARTKV_LAUNCH_OK("copy_dense_kernel");
   }
   return DARTKV_OK;
@@ -510,6 +516,7 @@ extern "C" int dartkv_cache_append_step(const dartkv_cache_desc* desc, const dar
 // (src/dart/cache.py:427-439) can only be the first append after a prompt, and the host, whose copy of the state
 // tells it so, sends that one through the host-planned path.
 __global__ void plan_append_kernel(dartkv_cache_desc d, dartkv_lifecycle_config cfg, int chunk_tokens) {
+  wait_previous();
   dartkv_lifecycle_state state{d.state[0], d.state[2], d.state[3], d.state[1]};
   dartkv_append_plan plan;
   lifecycle_core(cfg, state, chunk_tokens, plan);
@@ -544,7 +551,7 @@ extern "C" int dartkv_cache_append_device_planned(const dartkv_cache_desc* desc,
                  "device-planned appends need the geometry of the page kernels (head_dim 128, 16-bit data, 128-token "
                  "pages and key groups, aligned inputs)");
   const dartkv_append_plan* device_plan = reinterpret_cast<const dartkv_append_plan*>(d.state + 8);
-  plan_append_kernel<<<1, 1, 0, stream>>>(d, *cfg, chunk_tokens);
+  DARTKV_CUDA_OK(launch_following(plan_append_kernel, 1, 1, 0, stream, d, *cfg, chunk_tokens));
   DARTKV_LAUNCH_OK("plan_append_kernel");
   // lifecycles whose value rows are those of the key pages, at most one page waiting in the ring: one launch
   if (cfg->value_local_tokens == 0 && (cfg->local_tokens == 0 || chunk_tokens == 1))
@@ -559,8 +566,8 @@ extern "C" int dartkv_cache_append_device_planned(const dartkv_cache_desc* desc,
   const int esize = dartkv_dtype_size(d.dtype);
   const int vector_ok = (d.head_dim * esize) % 16 == 0 && (stride_b * esize) % 16 == 0 && (stride_h * esize) % 16 == 0 &&
                         (stride_t * esize) % 16 == 0;
-  copy_dense_kernel<<<dim3(bh, row_blocks, 2), 128, 0, stream>>>(d, most, keys, values, stride_b, stride_h, stride_t, 0, 0,
-                                                                 vector_ok, nonfinite, device_plan);
+  DARTKV_CUDA_OK(launch_following(copy_dense_kernel, dim3(bh, row_blocks, 2), 128, 0, stream, d, most, keys, values, stride_b, stride_h,
+                                  stride_t, 0, 0, vector_ok, nonfinite, device_plan));
   DARTKV_LAUNCH_OK("copy_dense_kernel");
   return DARTKV_OK;
 }

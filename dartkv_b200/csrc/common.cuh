@@ -129,31 +129,40 @@ __host__ __device__ __forceinline__ int dartkv_block_of_unit(int64_t x, int bloc
 }
 
 // ---------------------------------------------------------------------------- overlapped launches
-// An append of one page or token is a few microseconds of kernel, so the gap before it counts.  It is launched with
-// programmatic stream serialization: the grid is set up while the one before it runs.  follow_previous() is the first
-// statement of such a kernel: it waits until the grids before it have ended and their memory is visible (nothing may be
-// read or written before it), and lets the grid after it be set up once every block of this one has started.
-// B200: [16,8,4096,128] appended 128 tokens at a time 347 -> 328 us, 48 generation steps 1,052 -> 1,026 us, one bulk
-// append 74.6 -> 73.3 us.  The decode kernels are launched plainly: in the same form they were 1-4 % slower.
-__device__ __forceinline__ void follow_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// Every kernel is launched with programmatic stream serialization, and wait_previous() is the first statement of each (nothing
+// may be read or written before it): it returns once the grids before this one have ended and their memory is visible.  Calls
+// here are a few to some tens of microseconds of kernel, so the gap between two of them counts.  A plainly launched kernel
+// starts at a multiple of 1 or 2 us after the one before it: kernels that spin for 5, 7.3 and 11.1 us come every 8.2, 10.2 and
+// 14.3 us, so launched every 5.6, 7.9 and 11.7 us.  No kernel lets its successor in before it has ended
+// (griddepcontrol.launch_dependents): 48 generation steps of append, decode and merge take 997 us with an append step that does
+// and 822 us with one that does not; decode kernels that do are 1-4 % slower (B200).
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// cluster: blocks of a cluster, 0 for none
 template <class... Params, class... Args>
-static inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                           const Args&... args) {
+static inline cudaError_t launch_clusters(int cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                          const Args&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute = {};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  cudaLaunchAttribute attributes[2] = {};
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = cluster;
+  attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = cluster > 0 ? 2 : 1;
+  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  if (err != cudaSuccess) cudaGetLastError();   // reported by the caller, not left for the next one who asks
+  return err;
+}
+template <class... Params, class... Args>
+static inline cudaError_t launch_following(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                           const Args&... args) {
+  return launch_clusters(0, kernel, grid, block, smem, stream, args...);
 }
 
 static inline int dartkv_gcd(int a, int b) { while (b) { int t = a % b; a = b; b = t; } return a; }

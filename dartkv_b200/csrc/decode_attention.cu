@@ -66,6 +66,7 @@ template <int REP>
 __global__ void __launch_bounds__(GEN_THREADS) decode_generic_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                      const __grid_constant__ GenericArgs a) {
   extern __shared__ float smem[];
+  wait_previous();
   const int D = d.head_dim;
   const int rep = a.query_heads / d.kv_heads;            // at most REP
   float* s_q = smem;                                     // [D][REP]: a channel's heads together
@@ -292,6 +293,7 @@ template <int REP, int MD>
 __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                       const __grid_constant__ GenericArgs a) {
   extern __shared__ float smem[];
+  wait_previous();
   const int D = d.head_dim;
   const int rep = a.query_heads / d.kv_heads;            // at most REP
   float* s_q = smem;                                     // [D][REP]
@@ -555,9 +557,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_m, const floa
                                     const float* __restrict__ part_acc, int total_splits, int D, void* out, int out_dt,
                                     int stream_blocks, int64_t units, int quads, int query_heads, int kv_heads, int row_groups,
                                     dartkv_peer_scatter peers, int* status, unsigned int* done_counter) {
-  // launched with programmatic stream serialization: the grid may become resident while the kernel before it
-  // drains, and waits here until that kernel's memory is visible
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  wait_previous();
   int64_t row = blockIdx.x;
   int splits = total_splits;
   if (stream_blocks > 0) {
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) decode_merge_rows_kernel(const float* __r
   const int splits = 2 + dartkv_block_of_unit(bh * quads + quads - 1, stream_blocks, units) -
                      dartkv_block_of_unit(bh * quads, stream_blocks, units);
   const int64_t base = (int64_t)row * total_splits;
-  asm volatile("griddepcontrol.wait;" ::: "memory");   // see decode_merge_kernel
+  wait_previous();
   const int c = 4 * lane;
   float4 v[kRowSlots];   // requested before the weights are known
 #pragma unroll
@@ -994,57 +994,34 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
                       : padded_rep == 4 ? decode_generic_kernel<4> : padded_rep == 8 ? decode_generic_kernel<8> : decode_generic_kernel<16>;
     if (smem > 48 * 1024) DARTKV_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (a.cluster) {
-      cudaLaunchConfig_t config = {};
-      config.gridDim = dim3((unsigned)(bh * a.cluster));
-      config.blockDim = dim3(GEN_THREADS);
-      config.dynamicSmemBytes = smem;
-      config.stream = stream;
-      cudaLaunchAttribute attribute = {};
-      attribute.id = cudaLaunchAttributeClusterDimension;
-      attribute.val.clusterDim.x = a.cluster;
-      attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-      config.attrs = &attribute;
-      config.numAttrs = 1;
-      DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, kernel, *d, a));
+      DARTKV_CUDA_OK(launch_clusters(a.cluster, kernel, dim3((unsigned)(bh * a.cluster)), dim3(GEN_THREADS), smem, stream, *d, a));
       DARTKV_LAUNCH_OK("decode_tiles_kernel");
       if (!peers) return DARTKV_OK;
       L.total_splits = 1;
     } else {
-      kernel<<<dim3(bh, L.generic_splits), GEN_THREADS, smem, stream>>>(*d, a);
+      DARTKV_CUDA_OK(launch_following(kernel, dim3(bh, L.generic_splits), GEN_THREADS, smem, stream, *d, a));
       DARTKV_LAUNCH_OK("decode_generic_kernel");
     }
   }
   {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((unsigned)((int64_t)d->batch * query_heads));
     const bool few = L.total_splits <= kFewSplits;
-    config.blockDim = dim3(few ? min(256, (D + 31) / 32 * 32) : kManyThreads);
-    config.dynamicSmemBytes = few ? 0 : (size_t)(kManyThreads / D) * D * sizeof(float);
-    config.stream = stream;
-    cudaLaunchAttribute attribute = {};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
     // few slots a row of a tensor-core layout (128 channels, 16 bits): a warp per row, which moves four channels at a time
     if (L.fast && L.total_splits <= kRowSlots && !peers && (uintptr_t)out % 8 == 0 && (uintptr_t)part_acc % 8 == 0 &&
         rows / L.total_splits < (1ll << 31)) {
       const int out_rows = (int)(rows / L.total_splits);
-      config.gridDim = dim3((out_rows + 7) / 8);
-      config.blockDim = dim3(256);
-      config.dynamicSmemBytes = 0;
-      DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, decode_merge_rows_kernel, (const float*)part_m, (const float*)part_l,
-                                        (const float*)part_acc, L.total_splits, out, q_dtype, L.stream_blocks, (int64_t)L.units, L.quads,
-                                        query_heads, d->kv_heads, L.row_groups, out_rows));
+      DARTKV_CUDA_OK(launch_following(decode_merge_rows_kernel, dim3((out_rows + 7) / 8), dim3(256), 0, stream, part_m, part_l, part_acc,
+                                      L.total_splits, out, q_dtype, L.stream_blocks, L.units, L.quads, query_heads, d->kv_heads,
+                                      L.row_groups, out_rows));
       DARTKV_LAUNCH_OK("decode_merge_rows_kernel");
       return DARTKV_OK;
     }
     dartkv_peer_scatter none{};
     unsigned int* done_counter = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(workspace) + 4);
-    DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, decode_merge_kernel, (const float*)part_m, (const float*)part_l,
-                                      (const float*)part_acc, L.total_splits, D, out, q_dtype,
-                                      L.fast ? L.stream_blocks : 0, (int64_t)L.units, L.quads, query_heads, d->kv_heads, L.row_groups,
-                                      peers ? *peers : none, status, done_counter));
+    DARTKV_CUDA_OK(launch_following(decode_merge_kernel, dim3((unsigned)((int64_t)d->batch * query_heads)),
+                                    dim3(few ? min(256, (D + 31) / 32 * 32) : kManyThreads),
+                                    few ? 0 : (size_t)(kManyThreads / D) * D * sizeof(float), stream, part_m, part_l, part_acc,
+                                    L.total_splits, D, out, q_dtype, L.fast ? L.stream_blocks : 0, L.units, L.quads, query_heads,
+                                    d->kv_heads, L.row_groups, peers ? *peers : none, status, done_counter));
   }
   DARTKV_LAUNCH_OK("decode_merge_kernel");
   return DARTKV_OK;

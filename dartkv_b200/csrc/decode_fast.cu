@@ -45,6 +45,7 @@ struct BlockSmem {
 template <int DT, int OUT, int GN, int KP, bool FEW>
 __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_desc d, FastArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
+  wait_previous();
   BlockSmem& bs = *reinterpret_cast<BlockSmem*>(smem_raw + sizeof(WarpSmem) * kWarps);
   float* warp_out = reinterpret_cast<float*>(smem_raw);   // reused after the page loop: [warp][head][128]
 
@@ -240,7 +241,8 @@ int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int
   }
   const int promoted = d->key_mode == DARTKV_MIXED_PAGE ? d->promoted : 0;
   const int kp = (promoted % 8 == 0 && promoted <= 32) ? promoted : -1;
-  fast_variant(few, d->md_dtype, d->dtype, d->value_groups, kp)<<<grid, kThreads, kSmemBytes, stream>>>(*d, a);
+  DARTKV_CUDA_OK(launch_following(fast_variant(few, d->md_dtype, d->dtype, d->value_groups, kp), grid, kThreads, kSmemBytes, stream, *d,
+                                  a));
   DARTKV_LAUNCH_OK("decode_fast_kernel");
   return DARTKV_OK;
 }

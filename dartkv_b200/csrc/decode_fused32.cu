@@ -407,6 +407,7 @@ struct FusedWork {
 template <int DT, int MD, int GN, int KP, bool FEW>
 __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cache_desc d, FastArgs a) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
+  wait_previous();
   FusedBlockSmem& bs = *reinterpret_cast<FusedBlockSmem*>(smem_raw + sizeof(FusedWarpSmem) * kWarps);
   float* warp_out = reinterpret_cast<float*>(smem_raw);   // reused after the page loop: [warp][head][128]
 
@@ -599,7 +600,8 @@ int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, 
   }
   const int promoted = d->key_mode == DARTKV_MIXED_PAGE ? d->promoted : 0;
   const int kp = (promoted % 8 == 0 && promoted <= 32) ? promoted : -1;
-  fused_variant(few, d->dtype, d->md_dtype, d->value_groups, kp)<<<grid, kThreads, kFusedSmemBytes, stream>>>(*d, a);
+  DARTKV_CUDA_OK(launch_following(fused_variant(few, d->dtype, d->md_dtype, d->value_groups, kp), grid, kThreads, kFusedSmemBytes,
+                                  stream, *d, a));
   DARTKV_LAUNCH_OK("decode_fused32_kernel");
   return DARTKV_OK;
 }

@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
   using HO = Half2Ops<DT>;
   using Affine = PairAffine<MD, DT, FP32>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
+  wait_previous();
   RowsSmem<R>& bs = *reinterpret_cast<RowsSmem<R>*>(smem_raw);
   uint8_t* q_table = smem_raw + (sizeof(RowsSmem<R>) + 127) / 128 * 128;   // [channel] rows of w.key_row bytes: 8 columns
   uint8_t* pair_base = q_table + 128 * w.key_row;
@@ -656,7 +657,8 @@ int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int
     }
   }
   dim3 grid(stream_blocks + d->batch * d->kv_heads * ((rep + 3) / 4));
-  rows_variant(d->dtype, d->md_dtype, flavour == DARTKV_DEQUANT_FP32, rows)<<<grid, kThreads, rows_smem(w, rows), stream>>>(*d, a, w);
+  DARTKV_CUDA_OK(launch_following(rows_variant(d->dtype, d->md_dtype, flavour == DARTKV_DEQUANT_FP32, rows), grid, kThreads, rows_smem(w,
+                                  rows), stream, *d, a, w));
   DARTKV_LAUNCH_OK("decode_rows_kernel");
   return DARTKV_OK;
 }

@@ -286,6 +286,7 @@ template <int DT, int MD, bool FP32>
 __global__ void __launch_bounds__(kThreads, 2) decode_wide_kernel(dartkv_cache_desc d, FastArgs a, WideGeom w) {
   using H = Half2Ops<DT>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
+  wait_previous();
   WideBlockSmem& bs = *reinterpret_cast<WideBlockSmem*>(smem_raw);
   uint8_t* warp_base = smem_raw + ((sizeof(WideBlockSmem) + 127) / 128) * 128;
   float* warp_out = reinterpret_cast<float*>(warp_base);   // merge buffer: aliases the warps' streaming memory
@@ -606,7 +607,8 @@ int dartkv_decode_wide_launch(const dartkv_cache_desc* d, const void* query, int
       if (device >= 0 && device < 64) ready[device].store(true, std::memory_order_release);
     }
   }
-  wide_variant(d->dtype, d->md_dtype, flavour == DARTKV_DEQUANT_FP32)<<<grid, kThreads, smem, stream>>>(*d, a, w);
+  DARTKV_CUDA_OK(launch_following(wide_variant(d->dtype, d->md_dtype, flavour == DARTKV_DEQUANT_FP32), grid, kThreads, smem, stream, *d,
+                                  a, w));
   DARTKV_LAUNCH_OK("decode_wide_kernel");
   return DARTKV_OK;
 }

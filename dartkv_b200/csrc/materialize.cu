@@ -152,6 +152,7 @@ struct MaterializeArgs {
 __global__ void __launch_bounds__(kTileThreads) materialize_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                    const __grid_constant__ MaterializeArgs a) {
   extern __shared__ int s_slot[];
+  wait_previous();
   const int bh = blockIdx.x, side = a.side0 + blockIdx.z, first = a.t0 + blockIdx.y * kTileTokens;
   materialize_tokens(d, bh, side, first, min(a.t1, first + kTileTokens), (int64_t)bh * a.out_tokens - a.out_first, a.flavour,
                      side == 0 ? a.out_k : a.out_v, a.out_dt, s_slot);
@@ -231,6 +232,7 @@ template <int MD, int DT>
 __global__ void __launch_bounds__(kSpanThreads) materialize_spans_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                          const __grid_constant__ MaterializeArgs a, int first_span) {
   extern __shared__ int s_slot[];
+  wait_previous();
   const int bh = blockIdx.x, side = a.side0 + blockIdx.z, span = first_span + blockIdx.y, D = d.head_dim;
   const int span_lo = span == 0 ? 0 : d.sink_tokens + kSpan * (span - 1);
   const int span_hi = span == 0 ? d.sink_tokens : span_lo + kSpan;
@@ -301,10 +303,11 @@ int launch_materialize(const dartkv_cache_desc* d, int side, int sides, int t0, 
     const int end = span_of(t1 - 1) + 1;
     for (int first = span_of(t0); first < end; first += kMaxGridY) {
       const dim3 grid(bh, min(end - first, kMaxGridY), sides);
-      if (d->md_dtype == DARTKV_F16 && d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-      else if (d->md_dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_F16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-      else if (d->dtype == DARTKV_F16) materialize_spans_kernel<DARTKV_BF16, DARTKV_F16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
-      else materialize_spans_kernel<DARTKV_BF16, DARTKV_BF16><<<grid, kSpanThreads, smem, stream>>>(*d, a, first);
+      const bool half_md = d->md_dtype == DARTKV_F16, half = d->dtype == DARTKV_F16;
+      DARTKV_CUDA_OK(launch_following(half_md ? (half ? materialize_spans_kernel<DARTKV_F16,
+                                      DARTKV_F16> : materialize_spans_kernel<DARTKV_F16, DARTKV_BF16>)
+                                              : (half ? materialize_spans_kernel<DARTKV_BF16, DARTKV_F16> : materialize_spans_kernel<DARTKV_BF16, DARTKV_BF16>),
+                                      grid, dim3(kSpanThreads), smem, stream, *d, a, first));
       DARTKV_LAUNCH_OK("materialize_spans_kernel");
     }
     return DARTKV_OK;
@@ -312,7 +315,8 @@ int launch_materialize(const dartkv_cache_desc* d, int side, int sides, int t0, 
   for (int64_t first = t0; first < t1; first += (int64_t)kMaxGridY * kTileTokens) {
     a.t0 = (int)first;
     a.t1 = (int)min((int64_t)t1, first + (int64_t)kMaxGridY * kTileTokens);
-    materialize_kernel<<<dim3(bh, ceil_div(a.t1 - a.t0, kTileTokens), sides), kTileThreads, smem, stream>>>(*d, a);
+    DARTKV_CUDA_OK(launch_following(materialize_kernel, dim3(bh, ceil_div(a.t1 - a.t0, kTileTokens), sides), dim3(kTileThreads), smem,
+                                    stream, *d, a));
     DARTKV_LAUNCH_OK("materialize_kernel");
   }
   return DARTKV_OK;

@@ -64,6 +64,7 @@ static inline unsigned grid_for(int64_t threads, int block) { return (unsigned)(
 // ---------------------------------------------------------------------------- pack / unpack
 __global__ void pack_kernel(const uint8_t* __restrict__ codes, int64_t rows, int64_t n, int bits, int64_t packed_bytes,
                             uint8_t* __restrict__ packed) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= rows * packed_bytes) return;
   int64_t row = tid / packed_bytes, byte = tid % packed_bytes;
@@ -78,6 +79,7 @@ __global__ void pack_kernel(const uint8_t* __restrict__ codes, int64_t rows, int
 
 __global__ void unpack_kernel(const uint8_t* __restrict__ packed, int64_t rows, int64_t packed_bytes, int bits,
                               int64_t count, uint8_t* __restrict__ codes) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= rows * count) return;
   int64_t row = tid / count, j = tid % count;
@@ -92,7 +94,8 @@ extern "C" int dartkv_pack(const uint8_t* codes, int64_t rows, int64_t n, int bi
   if (rows == 0) return DARTKV_OK;
   DARTKV_REQUIRE(codes && packed, "pack received a null pointer");
   int64_t packed_bytes = ceil_div64(n, 8 / bits);
-  pack_kernel<<<grid_for(rows * packed_bytes, 256), 256, 0, (cudaStream_t)stream>>>(codes, rows, n, bits, packed_bytes, packed);
+  DARTKV_CUDA_OK(launch_following(pack_kernel, grid_for(rows * packed_bytes, 256), 256, 0, (cudaStream_t)stream, codes, rows, n, bits,
+                                  packed_bytes, packed));
   DARTKV_LAUNCH_OK("pack_kernel");
   return DARTKV_OK;
 }
@@ -103,7 +106,8 @@ extern "C" int dartkv_unpack(const uint8_t* packed, int64_t rows, int64_t packed
   DARTKV_REQUIRE(rows >= 0 && count > 0 && count <= packed_bytes * (8 / bits), "unpack count exceeds the packed row");
   if (rows == 0) return DARTKV_OK;
   DARTKV_REQUIRE(codes && packed, "unpack received a null pointer");
-  unpack_kernel<<<grid_for(rows * count, 256), 256, 0, (cudaStream_t)stream>>>(packed, rows, packed_bytes, bits, count, codes);
+  DARTKV_CUDA_OK(launch_following(unpack_kernel, grid_for(rows * count, 256), 256, 0, (cudaStream_t)stream, packed, rows, packed_bytes,
+                                  bits, count, codes));
   DARTKV_LAUNCH_OK("unpack_kernel");
   return DARTKV_OK;
 }
@@ -140,6 +144,7 @@ struct QuantArgs {
 };
 
 __global__ void quantize_kernel(QuantArgs a) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = a.outer * a.units * a.inner;
   if (tid >= total) return;
@@ -219,7 +224,7 @@ extern "C" int dartkv_quantize(const void* x, int dtype, int64_t outer, int64_t 
   a.units = ceil_div64(a.padded, a.unit);
   a.values = values; a.scale = scale; a.zero = zero; a.nonfinite = nonfinite;
   int64_t threads = outer * a.units * inner;
-  quantize_kernel<<<grid_for(threads, 128), 128, 0, (cudaStream_t)stream>>>(a);
+  DARTKV_CUDA_OK(launch_following(quantize_kernel, grid_for(threads, 128), 128, 0, (cudaStream_t)stream, a));
   DARTKV_LAUNCH_OK("quantize_kernel");
   return DARTKV_OK;
 }
@@ -228,6 +233,7 @@ __global__ void dequantize_kernel(const uint8_t* __restrict__ values, const void
                                   const void* __restrict__ zero, int md, int64_t outer, int64_t n, int64_t inner,
                                   int bits, int group, int flavour, void* out, int out_dt, int64_t so, int64_t sn,
                                   int64_t si, int64_t groups, int64_t packed_bytes) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= outer * n * inner) return;
   int64_t i = tid % inner;
@@ -264,9 +270,9 @@ extern "C" int dartkv_dequantize(const uint8_t* values, const void* scale, const
   if (made) return made > 0 ? DARTKV_OK : made;
   int64_t groups = ceil_div64(n, group_size);
   int64_t packed_bytes = ceil_div64(groups * group_size, 8 / bits);
-  dequantize_kernel<<<grid_for(outer * n * inner, 256), 256, 0, (cudaStream_t)stream>>>(
-      values, scale, zero, md_dtype, outer, n, inner, bits, group_size, flavour, out, out_dtype, stride_outer,
-      stride_n, stride_inner, groups, packed_bytes);
+  DARTKV_CUDA_OK(launch_following(dequantize_kernel, grid_for(outer * n * inner, 256), 256, 0, (cudaStream_t)stream, values, scale, zero,
+                                  md_dtype, outer, n, inner, bits, group_size, flavour, out, out_dtype, stride_outer, stride_n,
+                                  stride_inner, groups, packed_bytes));
   DARTKV_LAUNCH_OK("dequantize_kernel");
   return DARTKV_OK;
 }
@@ -277,6 +283,7 @@ extern "C" int dartkv_dequantize(const uint8_t* values, const void* scale, const
 // boundaries (the reference accumulates in fp32, with last-bit noise at more of them).
 __global__ void channel_scores_kernel(const void* __restrict__ keys, int dt, int64_t bh, int64_t tokens, int64_t d,
                                       int64_t sbh, int64_t st, int strategy, void* scores) {
+  wait_previous();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= bh * d) return;
   int64_t c = tid % d, r = tid / d;
@@ -314,8 +321,8 @@ extern "C" int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, in
                                               (cudaStream_t)stream);
     if (made) return made > 0 ? DARTKV_OK : made;
   }
-  channel_scores_kernel<<<grid_for(bh * head_dim, 128), 128, 0, (cudaStream_t)stream>>>(
-      keys, dtype, bh, tokens, head_dim, stride_bh, stride_token, strategy, scores);
+  DARTKV_CUDA_OK(launch_following(channel_scores_kernel, grid_for(bh * head_dim, 128), 128, 0, (cudaStream_t)stream, keys, dtype, bh,
+                                  tokens, head_dim, stride_bh, stride_token, strategy, scores));
   DARTKV_LAUNCH_OK("channel_scores_kernel");
   return DARTKV_OK;
 }
@@ -324,6 +331,7 @@ extern "C" int dartkv_channel_scores(const void* keys, int dtype, int64_t bh, in
 __global__ void select_channels_kernel(const void* __restrict__ scores, int dt, int64_t d, int count,
                                        int32_t* __restrict__ indices) {
   extern __shared__ uint32_t s_key[];
+  wait_previous();
   int64_t r = blockIdx.x;
   for (int c = threadIdx.x; c < d; c += blockDim.x) s_key[c] = rank_key(load_f(scores, dt, r * d + c));
   __syncthreads();
@@ -342,8 +350,8 @@ extern "C" int dartkv_select_channels(const void* scores, int dtype, int64_t bh,
   DARTKV_REQUIRE(count >= 0 && count <= head_dim, "count must be in [0, head_dim]");
   if (bh == 0 || count == 0) return DARTKV_OK;
   DARTKV_REQUIRE(scores && indices, "select_channels received a null pointer");
-  select_channels_kernel<<<(unsigned)bh, 128, head_dim * sizeof(float), (cudaStream_t)stream>>>(scores, dtype, head_dim,
-                                                                                             count, indices);
+  DARTKV_CUDA_OK(launch_following(select_channels_kernel, (unsigned)bh, 128, head_dim * sizeof(float), (cudaStream_t)stream, scores,
+                                  dtype, head_dim, count, indices));
   DARTKV_LAUNCH_OK("select_channels_kernel");
   return DARTKV_OK;
 }
@@ -375,6 +383,7 @@ __global__ void quantize_key_mixed_kernel(const void* __restrict__ keys, int dt,
                                           int md, uint8_t* __restrict__ low, uint8_t* __restrict__ high, void* scale,
                                           void* zero, int32_t* nonfinite) {
   extern __shared__ int s_slot[];
+  wait_previous();
   int64_t r = blockIdx.x;
   for (int c = threadIdx.x; c < d; c += blockDim.x) s_slot[c] = -1;
   __syncthreads();
@@ -444,9 +453,9 @@ extern "C" int dartkv_quantize_key_mixed(const void* keys, int dtype, int64_t bh
   if (made) return made > 0 ? DARTKV_OK : made;
   int64_t groups = ceil_div64(tokens, group_size);
   dim3 grid((unsigned)bh, grid_for(head_dim * groups, 128));
-  quantize_key_mixed_kernel<<<grid, 128, head_dim * sizeof(int), (cudaStream_t)stream>>>(
-      keys, dtype, tokens, head_dim, stride_bh, stride_token, group_size, indices, promoted, md_dtype, low, high, scale,
-      zero, nonfinite);
+  DARTKV_CUDA_OK(launch_following(quantize_key_mixed_kernel, grid, 128, head_dim * sizeof(int), (cudaStream_t)stream, keys, dtype,
+                                  tokens, head_dim, stride_bh, stride_token, group_size, indices, promoted, md_dtype, low, high, scale,
+                                  zero, nonfinite));
   DARTKV_LAUNCH_OK("quantize_key_mixed_kernel");
   return DARTKV_OK;
 }
@@ -456,6 +465,7 @@ __global__ void dequantize_key_mixed_kernel(const uint8_t* __restrict__ low, con
                                             const void* __restrict__ zero, int md, int64_t tokens, int64_t d, int group,
                                             int promoted, int flavour, void* out, int out_dt) {
   extern __shared__ int s_slot[];
+  wait_previous();
   int64_t r = blockIdx.x;
   for (int c = threadIdx.x; c < d; c += blockDim.x) s_slot[c] = -1;
   __syncthreads();
@@ -494,8 +504,8 @@ extern "C" int dartkv_dequantize_key_mixed(const uint8_t* low, const uint8_t* hi
                                                flavour, out, out_dtype, tokens * head_dim, head_dim, (cudaStream_t)stream);
   if (made) return made > 0 ? DARTKV_OK : made;
   dim3 grid((unsigned)bh, grid_for(tokens * head_dim, 256));
-  dequantize_key_mixed_kernel<<<grid, 256, head_dim * sizeof(int), (cudaStream_t)stream>>>(
-      low, high, indices, scale, zero, md_dtype, tokens, head_dim, group_size, promoted, flavour, out, out_dtype);
+  DARTKV_CUDA_OK(launch_following(dequantize_key_mixed_kernel, grid, 256, head_dim * sizeof(int), (cudaStream_t)stream, low, high,
+                                  indices, scale, zero, md_dtype, tokens, head_dim, group_size, promoted, flavour, out, out_dtype));
   DARTKV_LAUNCH_OK("dequantize_key_mixed_kernel");
   return DARTKV_OK;
 }

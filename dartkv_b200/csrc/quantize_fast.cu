@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(256, TOK == 32 ? 2 : 4) quantize_columns_kerne
   constexpr int PB = KB == 0 ? 2 : KB, CODE_BITS = KB == 0 ? 4 : KB;
   constexpr int PER_HALF = 16 / PB;
   constexpr uint32_t MAGIC = pair_magic<DT, CODE_BITS>();
+  wait_previous();
   __shared__ int s_slot[KB == 0 ? kSlab : 1];
   __shared__ uint32_t s_mn[4][64], s_mx[4][64];
   const int p = threadIdx.x & 63, split = threadIdx.x >> 6, splits = blockDim.x >> 6;
@@ -176,19 +177,17 @@ __global__ void __launch_bounds__(256, TOK == 32 ? 2 : 4) quantize_columns_kerne
   }
 }
 
+using ColumnsKernel = void (*)(ColumnArgs);
 template <int DT, int KB>
-void launch_columns_of(int tok, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
-  if (tok == 32) quantize_columns_kernel<DT, KB, 32><<<grid, threads, 0, stream>>>(a);
-  else if (tok == 16) quantize_columns_kernel<DT, KB, 16><<<grid, threads, 0, stream>>>(a);
-  else if (tok == 8 && KB >= 4) quantize_columns_kernel<DT, KB, KB >= 4 ? 8 : 0><<<grid, threads, 0, stream>>>(a);
-  else quantize_columns_kernel<DT, KB, 0><<<grid, threads, 0, stream>>>(a);
+ColumnsKernel columns_variant_of(int tok) {
+  if (tok == 32) return quantize_columns_kernel<DT, KB, 32>;
+  if (tok == 16) return quantize_columns_kernel<DT, KB, 16>;
+  return tok == 8 && KB >= 4 ? quantize_columns_kernel<DT, KB, (KB >= 4 ? 8 : 0)> : quantize_columns_kernel<DT, KB, 0>;
 }
 template <int DT>
-void launch_columns(int kb, int tok, dim3 grid, int threads, cudaStream_t stream, const ColumnArgs& a) {
-  if (kb == 0) launch_columns_of<DT, 0>(tok, grid, threads, stream, a);
-  else if (kb == 2) launch_columns_of<DT, 2>(tok, grid, threads, stream, a);
-  else if (kb == 4) launch_columns_of<DT, 4>(tok, grid, threads, stream, a);
-  else launch_columns_of<DT, 8>(tok, grid, threads, stream, a);
+ColumnsKernel columns_variant(int kb, int tok) {
+  return kb == 0 ? columns_variant_of<DT, 0>(tok) : kb == 2 ? columns_variant_of<DT, 2>(tok)
+       : kb == 4 ? columns_variant_of<DT, 4>(tok) : columns_variant_of<DT, 8>(tok);
 }
 
 bool is16(int dt) { return dt == DARTKV_F16 || dt == DARTKV_BF16; }
@@ -212,8 +211,9 @@ int dartkv_quantize_columns_fast(const void* x, int dtype, int64_t outer, int64_
   ColumnArgs a{reinterpret_cast<const uint16_t*>(x), so, sn, (int)n, (int)inner, group, (int)groups,
                groups * (int64_t)words * 4, values, high, indices, promoted, md, scale, zero, nonfinite};
   const dim3 grid((unsigned)groups, (unsigned)slabs, (unsigned)outer);
-  if (dtype == DARTKV_F16) launch_columns<DARTKV_F16>(key_bits, group / splits, grid, 64 * splits, stream, a);
-  else launch_columns<DARTKV_BF16>(key_bits, group / splits, grid, 64 * splits, stream, a);
+  DARTKV_CUDA_OK(launch_following(dtype == DARTKV_F16 ? columns_variant<DARTKV_F16>(key_bits, group / splits)
+                                                      : columns_variant<DARTKV_BF16>(key_bits, group / splits),
+                                  grid, dim3(64 * splits), 0, stream, a));
   DARTKV_LAUNCH_OK("quantize_columns_kernel");
   return 1;
 }
@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
                                                             int group, int md, uint8_t* __restrict__ values, void* scale_out,
                                                             void* zero_out, int32_t* nonfinite) {
   using P = Pack16<DT>;
+  wait_previous();
   // the eighths of a row are numbered through all rows: whole groups in order, so neither the group's number nor this
   // lane's place in it needs a division, and the row only where rows are not contiguous
   const int per_row = n / 8, lanes = group / 8;
@@ -295,12 +296,8 @@ __global__ void __launch_bounds__(256) quantize_rows_kernel(const uint16_t* __re
 }
 
 template <int DT>
-void launch_rows(int bits, unsigned blocks, cudaStream_t stream, const void* x_, int64_t rows, int n, int64_t so, int group, int md,
-                 uint8_t* values, void* scale, void* zero, int32_t* nonfinite) {
-  const uint16_t* x = reinterpret_cast<const uint16_t*>(x_);
-  if (bits == 2) quantize_rows_kernel<DT, 2><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
-  else if (bits == 4) quantize_rows_kernel<DT, 4><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
-  else quantize_rows_kernel<DT, 8><<<blocks, 256, 0, stream>>>(x, rows, n, so, group, md, values, scale, zero, nonfinite);
+auto rows_variant(int bits) {
+  return bits == 2 ? quantize_rows_kernel<DT, 2> : bits == 4 ? quantize_rows_kernel<DT, 4> : quantize_rows_kernel<DT, 8>;
 }
 
 }  // namespace
@@ -313,8 +310,10 @@ int dartkv_quantize_rows_fast(const void* x, int dtype, int64_t rows, int64_t n,
     return 0;
   const int64_t blocks = ceil_div64(rows * (n / 8), 256);
   if (!fits_int(blocks)) return 0;
-  if (dtype == DARTKV_F16) launch_rows<DARTKV_F16>(bits, (unsigned)blocks, stream, x, rows, (int)n, so, group, md, values, scale, zero, nonfinite);
-  else launch_rows<DARTKV_BF16>(bits, (unsigned)blocks, stream, x, rows, (int)n, so, group, md, values, scale, zero, nonfinite);
+  DARTKV_CUDA_OK(launch_following(dtype == DARTKV_F16 ? rows_variant<DARTKV_F16>(bits) : rows_variant<DARTKV_BF16>(bits),
+                                  dim3((unsigned)blocks),
+                                  dim3(256), 0, stream, reinterpret_cast<const uint16_t*>(x), rows, (int)n, so, group, md, values, scale,
+                                  zero, nonfinite));
   DARTKV_LAUNCH_OK("quantize_rows_kernel");
   return 1;
 }
@@ -334,6 +333,7 @@ __global__ void __launch_bounds__(64 * kScoreSplits) score_select_kernel(const u
                                                                          int64_t sbh, int64_t st, int count,
                                                                          uint16_t* scores, int32_t* indices) {
   using P = Pack16<DT>;
+  wait_previous();
   __shared__ double s_sum[kScoreSplits][2][64];
   __shared__ double s_all[kScoreBlocks][128];   // the blocks' sums, in the first one
   __shared__ uint32_t s_key[128];
@@ -402,18 +402,9 @@ int dartkv_score_select_fast(const void* keys, int dtype, int64_t bh, int64_t to
   // block a row 26.5; [4,8,1024,128]: 28.3, one block a row 30.8; whole quantize_key_mixed calls)
   int blocks = 1;
   while (blocks < kScoreBlocks && bh * blocks * 2 <= 2 * dartkv_sm_count() && tokens >= 128 * blocks * 2) blocks *= 2;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((unsigned)(bh * blocks));
-  config.blockDim = dim3(64 * kScoreSplits);
-  config.stream = stream;
-  cudaLaunchAttribute attribute = {};
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = blocks;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  DARTKV_CUDA_OK(cudaLaunchKernelEx(&config, dtype == DARTKV_F16 ? score_select_kernel<DARTKV_F16> : score_select_kernel<DARTKV_BF16>, k,
-                                    tokens, (int)d, sbh, st, count, s, indices));
+  DARTKV_CUDA_OK(launch_clusters(blocks, dtype == DARTKV_F16 ? score_select_kernel<DARTKV_F16> : score_select_kernel<DARTKV_BF16>,
+                                 dim3((unsigned)(bh * blocks)), dim3(64 * kScoreSplits), 0, stream, k, tokens, (int)d, sbh, st, count, s,
+                                 indices));
   DARTKV_LAUNCH_OK("score_select_kernel");
   return 1;
 }
@@ -443,6 +434,7 @@ template <int MD, int OUT, int BITS>
 __global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_constant__ RestoreArgs a) {
   constexpr int PB = BITS == 0 ? 2 : BITS, TOK = 32 / PB;
   constexpr uint32_t MASK = (1u << PB) - 1u;
+  wait_previous();
   __shared__ int s_slot[BITS == 0 ? kSlab : 1];
   const int64_t o = blockIdx.z;
   if (BITS == 0) {
@@ -490,6 +482,7 @@ __global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_const
 template <int MD, int OUT, int BITS>
 __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant__ RestoreArgs a, int64_t total) {
   constexpr uint32_t MASK = (1u << BITS) - 1u;
+  wait_previous();
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= total) return;
   // whole groups follow one another through all rows; divisions in 32 bits where they do
@@ -522,24 +515,24 @@ __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant
 }
 
 template <int MD, int OUT>
-void launch_restore(bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a, int64_t total) {
-  if (columns) {
-    if (bits == 0) restore_columns_kernel<MD, OUT, 0><<<grid, 256, 0, stream>>>(a);
-    else if (bits == 2) restore_columns_kernel<MD, OUT, 2><<<grid, 256, 0, stream>>>(a);
-    else if (bits == 4) restore_columns_kernel<MD, OUT, 4><<<grid, 256, 0, stream>>>(a);
-    else restore_columns_kernel<MD, OUT, 8><<<grid, 256, 0, stream>>>(a);
-  } else {
-    if (bits == 2) restore_rows_kernel<MD, OUT, 2><<<grid, 256, 0, stream>>>(a, total);
-    else if (bits == 4) restore_rows_kernel<MD, OUT, 4><<<grid, 256, 0, stream>>>(a, total);
-    else restore_rows_kernel<MD, OUT, 8><<<grid, 256, 0, stream>>>(a, total);
-  }
+cudaError_t launch_restore(bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a, int64_t total) {
+  if (columns)
+    return launch_following(bits == 0   ? restore_columns_kernel<MD, OUT, 0>
+                            : bits == 2 ? restore_columns_kernel<MD, OUT, 2>
+                            : bits == 4 ? restore_columns_kernel<MD, OUT, 4>
+                                        : restore_columns_kernel<MD, OUT, 8>,
+                            grid, dim3(256), 0, stream, a);
+  return launch_following(bits == 2   ? restore_rows_kernel<MD, OUT, 2>
+                          : bits == 4 ? restore_rows_kernel<MD, OUT, 4>
+                                      : restore_rows_kernel<MD, OUT, 8>,
+                          grid, dim3(256), 0, stream, a, total);
 }
-void launch_restore_typed(int md, int out_dtype, bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a,
-                          int64_t total) {
-  if (md == DARTKV_F16 && out_dtype == DARTKV_F16) launch_restore<DARTKV_F16, DARTKV_F16>(columns, bits, grid, stream, a, total);
-  else if (md == DARTKV_F16) launch_restore<DARTKV_F16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
-  else if (out_dtype == DARTKV_F16) launch_restore<DARTKV_BF16, DARTKV_F16>(columns, bits, grid, stream, a, total);
-  else launch_restore<DARTKV_BF16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
+cudaError_t launch_restore_typed(int md, int out_dtype, bool columns, int bits, dim3 grid, cudaStream_t stream, const RestoreArgs& a,
+                                 int64_t total) {
+  if (md == DARTKV_F16 && out_dtype == DARTKV_F16) return launch_restore<DARTKV_F16, DARTKV_F16>(columns, bits, grid, stream, a, total);
+  if (md == DARTKV_F16) return launch_restore<DARTKV_F16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
+  if (out_dtype == DARTKV_F16) return launch_restore<DARTKV_BF16, DARTKV_F16>(columns, bits, grid, stream, a, total);
+  return launch_restore<DARTKV_BF16, DARTKV_BF16>(columns, bits, grid, stream, a, total);
 }
 
 }  // namespace
@@ -557,7 +550,7 @@ int dartkv_restore_columns_fast(const uint8_t* values, const uint8_t* high, cons
   if (slabs > 65535) return 0;
   RestoreArgs a{values, high, indices, promoted, scale, zero, (int)n, (int)inner, group, (int)groups, flavour, words * 4, so, sn, out};
   const dim3 grid((unsigned)ceil_div64(words, 4), (unsigned)slabs, (unsigned)outer);
-  launch_restore_typed(md, out_dtype, true, key_bits, grid, stream, a, 0);
+  DARTKV_CUDA_OK(launch_restore_typed(md, out_dtype, true, key_bits, grid, stream, a, 0));
   DARTKV_LAUNCH_OK("restore_columns_kernel");
   return 1;
 }
@@ -570,7 +563,7 @@ int dartkv_restore_rows_fast(const uint8_t* values, const void* scale, const voi
   const int64_t total = rows * (n / 8), blocks = ceil_div64(total, 256);
   if (!fits_int(blocks)) return 0;
   RestoreArgs a{values, nullptr, nullptr, 0, scale, zero, (int)n, 1, group, (int)(n / group), flavour, 0, so, 1, out};
-  launch_restore_typed(md, out_dtype, false, bits, dim3((unsigned)blocks), stream, a, total);
+  DARTKV_CUDA_OK(launch_restore_typed(md, out_dtype, false, bits, dim3((unsigned)blocks), stream, a, total));
   DARTKV_LAUNCH_OK("restore_rows_kernel");
   return 1;
 }
