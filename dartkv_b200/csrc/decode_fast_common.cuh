@@ -47,6 +47,19 @@ struct FastArgs {
 // us, shared 18.4, 2 x 6,000 (192) 17.0 and 18.4 (B200).
 inline bool dartkv_few_pages(long long units, int stream_blocks) { return units == stream_blocks && stream_blocks <= dartkv_sm_count(); }
 
+// The pages of one row that a block of the 2-bit kernels works on; tokens before first_live get no weight (left padding) and
+// whole pages of them are not even fetched.
+struct RowPiece {
+  int first_live, begin, end;
+};
+__device__ __forceinline__ RowPiece row_piece(const dartkv_cache_desc& d, const FastArgs& a, int bh, int quad, int quads, int total_pages) {
+  RowPiece p;
+  p.first_live = a.row_start ? max(a.row_start[bh / d.kv_heads], 0) : 0;
+  p.begin = max(4 * quad, p.first_live > d.sink_tokens ? (p.first_live - d.sink_tokens) >> 7 : 0);
+  p.end = min(4 * (quad + quads), total_pages);
+  return p;
+}
+
 __host__ __device__ __forceinline__ int fast_range_end(int sink_tokens, int page_size, int k_end, int v_end,
                                                        int sink_filled) {
   int packed = min(k_end, v_end);
@@ -341,7 +354,8 @@ __device__ __forceinline__ void store_query_compact(uint2* query, const void* q,
 }
 
 // Block merge of the eight warp states: thread = (channel, head parity); partials leave in natural-log units.
-template <bool ROW_GROUPS = false, class BS>
+// WARP_FLOATS: floats from one warp's accumulators ([head][channel]) to the next one's.
+template <bool ROW_GROUPS = false, int WARP_FLOATS = 512, class BS>
 __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, const float* warp_out, int b, int hkv, int rep,
                                             int slot, int head0 = 0) {
   const int tid = threadIdx.x;
@@ -357,7 +371,7 @@ __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, con
       if (mw != -INFINITY) {
         const float wgt = fast_exp2(mw - m);
         l += bs.merge_l[w][r] * wgt;
-        acc += warp_out[(w * 4 + r) * 128 + ch] * wgt;
+        acc += warp_out[w * WARP_FLOATS + r * 128 + ch] * wgt;
       }
     }
     const int64_t row = ((int64_t)b * a.query_heads + hkv * rep + (ROW_GROUPS ? head0 : 0) + r) * a.total_splits + slot;

@@ -48,12 +48,14 @@ struct FusedWarpSmem {
   FusedScratch scratch;
 };
 
+static_assert(sizeof(FusedScratch) >= 512 * sizeof(float), "the scratch of a warp takes its state at the end of a row");
+
 struct FusedBlockSmem {
   uint2 query[128];              // [channel]: the 16-bit query values of the four heads (zero for absent heads)
   float merge_m[kWarps][4];
   float merge_l[kWarps][4];
   int slot_map[128];
-  uint64_t k_bar[kWarps], v_bar[kWarps];   // not beside the staging memory, which becomes the merge buffer
+  uint64_t k_bar[kWarps], v_bar[kWarps];
 };
 
 template <int DT>
@@ -409,13 +411,13 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   extern __shared__ __align__(128) uint8_t smem_raw[];
   wait_previous();
   FusedBlockSmem& bs = *reinterpret_cast<FusedBlockSmem*>(smem_raw + sizeof(FusedWarpSmem) * kWarps);
-  float* warp_out = reinterpret_cast<float*>(smem_raw);   // reused after the page loop: [warp][head][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rep = a.query_heads / d.kv_heads;
 
   if ((int)blockIdx.x >= a.stream_blocks) {
     const int bh = blockIdx.x - a.stream_blocks;
+    float* const warp_out = reinterpret_cast<float*>(smem_raw);   // [warp][head][128]
     dense_block<DT, MD>(d, a, bs, warp_out, bh);
     __syncthreads();
     block_merge(a, bs, warp_out, bh / d.kv_heads, bh % d.kv_heads, rep, 0);
@@ -430,12 +432,11 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   const int fast_end = fast_range_end(d.sink_tokens, d.page_size, k_end, v_end, sink_filled);
   const int total_pages = fast_end > d.sink_tokens ? (fast_end - d.sink_tokens) / 128 : 0;
   constexpr int kMetaBytes = 128 * 2 * GN * 2;
-  int bh = 0;
-  auto issue_keys = [&](int pg) {
+  auto issue_keys = [&](int bh, int pg) {
     mbar_expect_tx(&bs.k_bar[warp], d.key_page_bytes);
     bulk_copy_g2s(ws.keys, d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes, d.key_page_bytes, &bs.k_bar[warp]);
   };
-  auto issue_values = [&](int pg) {
+  auto issue_values = [&](int bh, int pg) {
     mbar_expect_tx(&bs.v_bar[warp], kValueCodes + kMetaBytes);
     const int64_t vrow = (int64_t)bh * d.max_value_tokens + (int64_t)pg * 128;
     bulk_copy_g2s(ws.values, d.v_codes + vrow * 32, kValueCodes, &bs.v_bar[warp]);
@@ -451,43 +452,43 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 
+  int bh = unit / a.quads, quad = unit - bh * a.quads;
+  RowPiece now = row_piece(d, a, bh, quad, min(a.quads - quad, unit_end - unit), total_pages);
+  // this warp's first page is requested before anything else, so its latency overlaps the query load below
+  if (lane == 0 && now.begin + warp < now.end) { issue_keys(bh, now.begin + warp); issue_values(bh, now.begin + warp); }
+  if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane);
+  __syncthreads();
+
   while (unit < unit_end) {
-    bh = unit / a.quads;
-    const int quad_begin = unit - bh * a.quads;
-    const int quad_count = min(a.quads - quad_begin, unit_end - unit);
-    unit += quad_count;
-    // tokens before the row's first live one get no weight: whole pages of them are not even fetched
-    const int row_first = a.row_start ? max(a.row_start[bh / d.kv_heads], 0) : 0;
-    const int p_begin = max(4 * quad_begin, row_first > d.sink_tokens ? (row_first - d.sink_tokens) >> 7 : 0);
-    const int p_end = min(4 * (quad_begin + quad_count), total_pages);
-
-    // this warp's first page is requested before anything else, so its latency overlaps the query load below
-    const int pg0 = p_begin + warp;
-    if (lane == 0 && pg0 < p_end) { issue_keys(pg0); issue_values(pg0); }
-
-    const int b = bh / d.kv_heads, hkv = bh % d.kv_heads;
-    if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)b * a.query_heads + hkv * rep, rep, lane);
-    __syncthreads();
+    unit += min(a.quads - quad, unit_end - unit);
+    quad = 0;
+    // this warp's first page of the next row: requested as soon as its buffers are free, before the rows are merged
+    auto next_row = [&](auto issue) {
+      if (lane != 0 || unit >= unit_end) return;
+      const RowPiece next = row_piece(d, a, bh + 1, 0, min(a.quads, unit_end - unit), total_pages);
+      if (next.begin + warp < next.end) issue(bh + 1, next.begin + warp);
+    };
 
     work.start_row();
     if constexpr (FEW) {
       // the block's only unit: warps w and w + 4 share page w, half of its tokens each
       const int hf = warp >> 2, shared = warp & 3;
       const FusedWarpSmem& page = reinterpret_cast<const FusedWarpSmem*>(smem_raw)[shared];
-      if (p_begin + shared < p_end) {
+      if (now.begin + shared < now.end) {
         ok = mbar_wait(&bs.k_bar[shared], 0) && ok;
         work.fill_table(page.keys, ws.scratch);
         __syncwarp();
         float s_acc[2][4];
         work.template logits<2>(page.keys, ws.scratch, hf, s_acc);
         __syncwarp();
-        work.template softmax<2>(s_acc, hf, row_first - (d.sink_tokens + 128 * (p_begin + shared)), ws.scratch,
+        work.template softmax<2>(s_acc, hf, now.first_live - (d.sink_tokens + 128 * (now.begin + shared)), ws.scratch,
                                  [&] { ok = mbar_wait(&bs.v_bar[shared], 0) && ok; }, page.values);
         __syncwarp();
         work.template weigh_values<2>(page.values, ws.scratch, hf);
       }
     } else {
-      for (int pg = pg0; pg < p_end; pg += kWarps, parity ^= 1) {
+      for (int pg = now.begin + warp; pg < now.end; pg += kWarps, parity ^= 1) {
+        const bool last = pg + kWarps >= now.end;
         ok = mbar_wait(&bs.k_bar[warp], parity) && ok;
         work.fill_table(ws.keys, ws.scratch);
         __syncwarp();
@@ -495,24 +496,34 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
         work.template logits<4>(ws.keys, ws.scratch, 0, s_acc);
         __syncwarp();
         // the keys are consumed: their buffer takes the next page's while the values are worked on
-        if (lane == 0 && pg + kWarps < p_end) issue_keys(pg + kWarps);
-        work.template softmax<4>(s_acc, 0, row_first - (d.sink_tokens + 128 * pg), ws.scratch,
+        if (last) next_row(issue_keys);
+        else if (lane == 0) issue_keys(bh, pg + kWarps);
+        work.template softmax<4>(s_acc, 0, now.first_live - (d.sink_tokens + 128 * pg), ws.scratch,
                                  [&] { ok = mbar_wait(&bs.v_bar[warp], parity) && ok; }, ws.values);
         __syncwarp();
         work.template weigh_values<4>(ws.values, ws.scratch, 0);
         __syncwarp();
-        if (lane == 0 && pg + kWarps < p_end) issue_values(pg + kWarps);
+        if (last) next_row(issue_values);
+        else if (lane == 0) issue_values(bh, pg + kWarps);
       }
     }
 
-    __syncthreads();   // every warp is done with its stages: the staging memory becomes the merge buffer
-    work.hand_over(warp_out + warp * 512);
+    if (now.begin + warp >= now.end) {   // no page of this row for this warp
+      next_row(issue_keys);
+      next_row(issue_values);
+    }
+    // the states meet in the warps' scratch: nothing there is in use between the rows
+    __syncwarp();
+    work.hand_over(reinterpret_cast<float*>(&ws.scratch));
     if (lane < 4) { bs.merge_m[warp][lane] = merge_maximum(work.m_run, work.l_run); bs.merge_l[warp][lane] = work.l_run; }
     __syncthreads();
-    block_merge(a, bs, warp_out, bh / d.kv_heads, bh % d.kv_heads, rep,
-                1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
-    // the merge buffer is staging memory again, the query table may be overwritten
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    block_merge<false, sizeof(FusedWarpSmem) / sizeof(float)>(a, bs, reinterpret_cast<const float*>(&reinterpret_cast<FusedWarpSmem*>(smem_raw)->scratch),
+                                                     bh / d.kv_heads, bh % d.kv_heads, rep,
+                                                     1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
+    if (unit >= unit_end) break;
+    ++bh;
+    now = row_piece(d, a, bh, 0, min(a.quads, unit_end - unit), total_pages);
+    if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane);
     __syncthreads();
   }
   if (!ok && lane == 0) atomicExch(a.status, 1);
