@@ -724,7 +724,8 @@ struct DecodeLayout {
   int quads, stream_blocks;            // tensor-core layouts: four-page units per (batch, kv head), stream blocks
   long long units;
   int total_splits;
-  int row_groups;                      // groups of query rows per KV head that are work rows of their own (layout 4)
+  int row_groups;                      // layout 4: groups of up to eight query rows per KV head
+  int pieces;                          // large calls of more than eight rows (decode_many.cu): blocks per work row, else 0
 };
 
 int dartkv_decode_fast_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
@@ -745,6 +746,10 @@ int dartkv_decode_rows_groups(int rep);
 int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int query_heads, float scale, int flavour, int quads,
                               int stream_blocks, long long units, int total_splits, float* part_m, float* part_l, float* part_acc,
                               int* status, const int32_t* row_start, cudaStream_t stream);
+int dartkv_decode_many_groups(int rep);
+int dartkv_decode_many_pieces(const dartkv_cache_desc* d, int rep, int pages);
+int dartkv_decode_many_launch(const dartkv_cache_desc* d, const void* query, int query_heads, float scale, int pieces, int total_splits,
+                              float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start, cudaStream_t stream);
 int dartkv_decode_wide_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
                               int flavour, int quads, int stream_blocks, long long units, int total_splits,
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
@@ -825,9 +830,25 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
+    if (L.fast == 4 && rep > 8) {
+      // Every block of decode_many.cu works for all rows of a KV head (of a group of up to 32), one page after another: less work,
+      // but a longer chain than that of decode_rows.cu's blocks, which take four pages at a time for eight rows.  It pays where its
+      // blocks, counted once for every eight rows, come near two per SM.  2-bit, 8 KV heads, before and after (B200): 20 rows,
+      // 1 x 4,096 tokens (64 blocks, counted 192) 17.0 and 20.8 us, 1 x 8,192 (384) 23.2 and 21.3, 4 x 2,100 (384) 22.8 and 20.1,
+      // 8 x 4,096 (768) 62.9 and 41.1; 9 rows, 2 x 4,096 (256) 20.8 and 18.5, 8 x 1,100 (256) 22.5 and 17.5.  With two eights of
+      // rows and as many blocks per KV head as a row has slots for, 1 x 16,384 tokens take 23.5 and 27.9.
+      const int groups = dartkv_decode_many_groups(rep), pieces = dartkv_decode_many_pieces(d, rep, pages);
+      const long long blocks = (long long)d->batch * d->kv_heads * groups * pieces;
+      if (10 * blocks * L.row_groups >= 17 * dartkv_sm_count() && (L.row_groups > 2 || pieces < 15)) {
+        L.pieces = pieces;
+        L.stream_blocks = (int)blocks;
+        L.total_splits = pieces + (groups > 1 ? 2 : 1);   // the plan counts in eights of rows, which may lie across two blocks more
+        return L;
+      }
+    }
     const int resident = (L.fast == 3 ? dartkv_decode_wide_blocks_per_sm(d, q_dtype, rep, flavour) : 2) * dartkv_sm_count();
     // dense blocks of the many-row layout (one per four rows): with 2.0 instead of 4.0 8 x 1,177 tokens, 12 rows, take 39.9
-    // instead of 33.8 us and 8 x 4,173 tokens, 20 rows, 73 instead of 77; with 8.0 16 x 2,125 tokens, 8 rows, 48 instead of 44
+    // instead of 33.8 us; with 8.0 16 x 2,125 tokens, 8 rows, 48 instead of 44
     const double block_fixed = 1.75, dense_cost = L.fast == 4 ? 4.0 : 2.0;
     int best_pieces = 1;
     double best_cost = 1e30;
@@ -964,7 +985,13 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   float* part_acc = part_l + rows;
   const int bh = d->batch * d->kv_heads;
   const int D = d->head_dim;
-  if (L.fast == 4) {
+  if (L.pieces) {
+    int rc = dartkv_decode_many_launch(d, query, query_heads, scale, L.pieces, L.total_splits, part_m, part_l, part_acc, status, row_start,
+                                       stream);
+    if (rc) return rc;
+    L.row_groups = dartkv_decode_many_groups(rep);   // the merge finds a row's slots from the work rows
+    L.units = (long long)bh * L.row_groups * L.quads;
+  } else if (L.fast == 4) {
     int rc = dartkv_decode_rows_launch(d, query, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units, L.total_splits, part_m,
                                        part_l, part_acc, status, row_start, stream);
     if (rc) return rc;
@@ -1045,7 +1072,7 @@ extern "C" int dartkv_decode_attention_padded(const dartkv_cache_desc* d, const 
 // Below this many tokens passes of four rows stay, not for speed but for their results: a token's is bit for bit that of a
 // call with this token alone, which many-row blocks with their own order of sums do not give.  Batch 8, 32 heads on 8,
 // 2-bit pages, device time of a call: 600 tokens 2 queries 48 us in passes, 26 us at once, 5 queries 110 / 38; 1,100
-// tokens 50 / 26 and 118 / 40; 4,096 tokens 69 / 44 and 161 / 75 (B200).
+// tokens 50 / 26 and 118 / 40; 4,096 tokens 69 / 44 and 161 / 42 (B200).
 constexpr int kRowsMinTokens = 1024;
 
 extern "C" int dartkv_decode_rows_limit(const dartkv_cache_desc* d, int q_dtype, int flavour, int tokens) {

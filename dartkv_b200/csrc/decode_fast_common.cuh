@@ -328,12 +328,6 @@ __device__ void dense_block(const dartkv_cache_desc& d, const FastArgs& a, BS& b
 }
 
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t d;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-  return d;
-}
-
 // The query of a KV head's group as 16-bit values, the heads of a channel side by side (zero for absent heads), by one warp.
 __device__ __forceinline__ void store_query_compact(uint2* query, const void* q, int64_t first_row, int rep, int lane) {
   uint2 v[4];   // [head]: channels 4 * lane .. + 3

@@ -138,6 +138,11 @@ template <int FROM, int TO> __device__ __forceinline__ uint32_t cast16(uint32_t 
   return pack16<TO>(lo, hi);
 }
 
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
 // (a & b) | c in one LOP3; b and c are kept in registers (a logic op takes at most one immediate)
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;

@@ -230,8 +230,10 @@ int dartkv_decode_attention(const dartkv_cache_desc* desc, const void* query, in
  * per-op flavour (2-bit pages), 2 tensor-core unrounded flavour (2-bit pages), 3 tensor-core kernels for every
  * other packed geometry and the fp32 flavour, 4 (dartkv_decode_plan_rows only) tensor-core kernel for more than four
  * query rows per KV head.  On the tensor-core layouts one unit is four consecutive pages of a row, i.e. of a
- * (batch, kv head), under kernel 4 of one of the ceil(rows per KV head / 8) groups of its query rows; block j of `stream_blocks` owns units [j*units/stream_blocks, (j+1)*units/stream_blocks)
- * and every row is touched by at most total_splits - 1 of them (plus its dense-token block). */
+ * (batch, kv head), under kernel 4 of one of the ceil(rows per KV head / 8) groups of its query rows; block j of `stream_blocks`
+ * owns units [j*units/stream_blocks, (j+1)*units/stream_blocks) and every row is touched by at most total_splits - 1 of them (plus
+ * its dense-token block).  Under kernel 4 with more than eight rows per KV head a block works for all of them (32 at most), on an
+ * even share of the (batch, kv head)'s pages and dense tokens. */
 typedef struct {
   int32_t kernel;
   int32_t quads;          /* units per row */
