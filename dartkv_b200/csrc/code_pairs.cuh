@@ -1,4 +1,5 @@
-// Packed codes of any width to 16-bit numbers, two codes with scales of their own per register (decode_rows.cu, decode_many.cu).
+// Packed codes of any width to 16-bit numbers, two codes with scales of their own per register: MMA operands (decode_rows.cu,
+// decode_many.cu) and restored keys and values (materialize.cu, quantize_fast.cu).
 #pragma once
 
 #include "mma_utils.cuh"
@@ -6,10 +7,12 @@
 namespace {
 
 // scale and zero point of the two elements of a register, made ready for codes at any of the in-mantissa positions.
-// MD: metadata dtype (the arithmetic), OUT: cache dtype (the MMA operand), FP32: the fp32 flavour.
-template <int MD, int OUT, bool FP32>
+// MD: metadata dtype (the arithmetic), OUT: cache dtype (the MMA operand), FP32: the fp32 flavour.  WIDE: any scale, at one
+// operation more (the magic number is subtracted first); without it magic * scale must not overflow.
+template <int MD, int OUT, bool FP32, bool WIDE = false>
 struct PairAffine {
   using H = Half2Ops<MD>;
+  static constexpr bool kFp32 = FP32;
   uint32_t ss, zz, ms[3];
   float s0, s1, z0, z1;
   template <int POSITIONS>
@@ -19,6 +22,7 @@ struct PairAffine {
       unpack16<MD>(zeros, z0, z1);
     } else {
       ss = scales; zz = zeros;
+      if (!WIDE)
 #pragma unroll
         for (int j = 0; j < POSITIONS; ++j) ms[j] = H::mul(ss, H::neg_magic(j));
     }
@@ -26,7 +30,7 @@ struct PairAffine {
   // m = magic(J) + code in both halves
   template <int J>
   __device__ __forceinline__ uint32_t restore(uint32_t m) const {
-    if (!FP32) return cast16<MD, OUT>(H::add(H::fma(m, ss, ms[J]), zz));
+    if (!FP32) return cast16<MD, OUT>(H::add(WIDE ? H::mul(H::add(m, H::neg_magic(J)), ss) : H::fma(m, ss, ms[J]), zz));
     float c0, c1;
     unpack16<MD>(H::add(m, H::neg_magic(J)), c0, c1);
     return pack16<OUT>(__fmaf_rn(c0, s0, z0), __fmaf_rn(c1, s1, z1));
@@ -34,8 +38,8 @@ struct PairAffine {
 };
 
 // eight 2-bit codes per half of x -> eight registers
-template <int MD, int OUT, bool FP32>
-__device__ __forceinline__ void restore_codes2(const CodeConsts<MD>& k, uint32_t x, const PairAffine<MD, OUT, FP32>& a, uint32_t (&r)[8]) {
+template <int MD, int OUT, bool FP32, bool WIDE>
+__device__ __forceinline__ void restore_codes2(const CodeConsts<MD>& k, uint32_t x, const PairAffine<MD, OUT, FP32, WIDE>& a, uint32_t (&r)[8]) {
   constexpr int P0 = Half2Ops<MD>::kFirstPos;
   const uint32_t x0 = align_codes(x, 0, P0), x1 = align_codes(x, 3, P0), x2 = align_codes(x, 6, P0);
   r[0] = a.template restore<0>(and_or(x0, k.mask[0], k.magic[0]));
@@ -49,8 +53,8 @@ __device__ __forceinline__ void restore_codes2(const CodeConsts<MD>& k, uint32_t
 }
 
 // eight codes per half split over a low and a high plane (code = low | high << 2) -> eight registers
-template <int MD, int OUT, bool FP32>
-__device__ __forceinline__ void restore_codes22(const CodeConsts<MD>& k, uint32_t xl, uint32_t xh, const PairAffine<MD, OUT, FP32>& a,
+template <int MD, int OUT, bool FP32, bool WIDE>
+__device__ __forceinline__ void restore_codes22(const CodeConsts<MD>& k, uint32_t xl, uint32_t xh, const PairAffine<MD, OUT, FP32, WIDE>& a,
                                                 uint32_t (&r)[8]) {
   constexpr int P0 = Half2Ops<MD>::kFirstPos;
 #pragma unroll
@@ -62,8 +66,8 @@ __device__ __forceinline__ void restore_codes22(const CodeConsts<MD>& k, uint32_
 }
 
 // four 4-bit codes per half of x -> four registers (bits 4..7 of an fp16 mantissa, 0..3 of a bf16 mantissa: magic(0))
-template <int MD, int OUT, bool FP32>
-__device__ __forceinline__ void restore_codes4(const CodeConsts<MD>& k, uint32_t mask4, uint32_t x, const PairAffine<MD, OUT, FP32>& a,
+template <int MD, int OUT, bool FP32, bool WIDE>
+__device__ __forceinline__ void restore_codes4(const CodeConsts<MD>& k, uint32_t mask4, uint32_t x, const PairAffine<MD, OUT, FP32, WIDE>& a,
                                                uint32_t* r) {
   constexpr int P0 = Half2Ops<MD>::kFirstPos;
 #pragma unroll
@@ -72,8 +76,8 @@ __device__ __forceinline__ void restore_codes4(const CodeConsts<MD>& k, uint32_t
 
 // the four 8-bit codes of a word for each half -> four registers.  Eight bits fit an fp16 mantissa (1024 + code; the magic
 // is subtracted first, 1024 * scale could overflow) but not a bf16 one: there through fp32 (8388608 + code, exact).
-template <int MD, int OUT, bool FP32>
-__device__ __forceinline__ void restore_codes8(uint32_t w0, uint32_t w1, const PairAffine<MD, OUT, FP32>& a, uint32_t* r) {
+template <int MD, int OUT, bool FP32, bool WIDE>
+__device__ __forceinline__ void restore_codes8(uint32_t w0, uint32_t w1, const PairAffine<MD, OUT, FP32, WIDE>& a, uint32_t* r) {
   using H = Half2Ops<MD>;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -85,6 +89,49 @@ __device__ __forceinline__ void restore_codes8(uint32_t w0, uint32_t w1, const P
     } else {
       const uint32_t m = and_or(prmt(w0, w1, j * 0x0011u | (4 + j) * 0x1100u), 0x00FF00FFu, 0x64006400u);
       r[j] = cast16<MD, OUT>(H::add(H::mul(H::add(m, 0xE400E400u), a.ss), a.zz));
+    }
+  }
+}
+
+// The codes of one word of each of two neighbouring columns, BITS wide (0: 2-bit codes with a second plane for promoted columns), in
+// kColumnParts<BITS> parts of N elements: element part * N + u of both columns is r[u].
+template <int BITS> constexpr int kColumnParts = BITS == 8 ? 1 : 2;
+template <int MD, int OUT, bool FP32, int BITS, int N>
+__device__ __forceinline__ void restore_columns(const CodeConsts<MD>& k, const uint32_t (&w)[2], const uint32_t (&high)[2],
+                                                const PairAffine<MD, OUT, FP32, true>& affine, int part, uint32_t (&r)[N]) {
+  static_assert(N * kColumnParts<BITS> == 32 / (BITS == 0 ? 2 : BITS), "a word's elements");
+  if constexpr (BITS == 8) {
+    restore_codes8<MD, OUT>(w[0], w[1], affine, r);
+  } else {
+    const uint32_t sel = part ? 0x7632u : 0x5410u, x = prmt(w[0], w[1], sel);
+    if constexpr (BITS == 0) restore_codes22<MD, OUT>(k, x, prmt(high[0], high[1], sel), affine, r);
+    else if constexpr (BITS == 2) restore_codes2<MD, OUT>(k, x, affine, r);
+    else restore_codes4<MD, OUT>(k, 0x000F000Fu << (2 * Half2Ops<MD>::kFirstPos), x, affine, r);
+  }
+}
+
+// Eight neighbouring codes of a row, BITS wide, of one group.
+template <int MD, int OUT, bool FP32, int BITS>
+__device__ __forceinline__ void restore_row(const CodeConsts<MD>& k, uint64_t codes, uint32_t scale, uint32_t zero, uint32_t (&r)[4]) {
+  constexpr int P0 = Half2Ops<MD>::kFirstPos;
+  PairAffine<MD, OUT, FP32, true> affine;
+  affine.template init<0>(scale * 0x00010001u, zero * 0x00010001u);
+  const uint32_t lo = (uint32_t)codes, hi = (uint32_t)(codes >> 32);
+  if constexpr (BITS == 8) {
+    restore_codes8<MD, OUT>(prmt(lo, hi, 0x6420u), prmt(lo, hi, 0x7531u), affine, r);
+  } else if constexpr (BITS == 4) {
+    // the odd codes move up to the half-word above the even ones: two pairs a word, eight bits apart
+    constexpr uint32_t mask = 0x000F000Fu << (2 * P0);
+    const uint32_t x[2] = {(lo & 0xFFFFu) | ((lo << 12) & 0xFFFF0000u), (lo >> 16) | ((lo >> 4) & 0xFFFF0000u)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = affine.template restore<0>(and_or(align_codes(x[i >> 1], 4 * (i & 1), P0), mask, k.magic[0]));
+  } else {
+    const uint32_t x = lo | (lo << 14);   // pair i four bits on from pair i - 1: positions 0 and 2 of two alignments
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t y = align_codes(x, 4 * i, P0);
+      r[2 * i] = affine.template restore<0>(and_or(y, k.mask[0], k.magic[0]));
+      r[2 * i + 1] = affine.template restore<2>(and_or(y, k.mask[2], k.magic[2]));
     }
   }
 }

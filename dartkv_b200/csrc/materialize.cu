@@ -5,10 +5,12 @@
 // (the span of a key page) of one (batch, head) and side with whole-word reads of the codes and whole-line stores; a
 // thread owns the tokens of one key code word for two neighbouring channels, or eight channels of a value row.
 // Everything else takes materialize_kernel, which walks a tile of tokens element pair by element pair.
-// Bound by the instructions per element and the latency of the codes (issue 62 %), the stores stay in L2: 2 x 20 MB out of
-// 8 MB packed (fp16 [4,8,2500,128], 2-bit + promoted keys) take 23 us, the pass that appends them too 222 us with one
-// block per token (which built the page's slot map 128 times over) and 52 us now (B200).
+// Bound by instructions and the latency of the codes, the stores stay in L2: 2 x 20 MB out of 8 MB packed (fp16 [4,8,2500,128],
+// 2-bit + promoted keys) take 24.7 us element by element and 16.1 with two codes per register (code_pairs.cuh), some 2 us of
+// the difference from the form of the launch; 222 us for the pass that appends them too with one block per token, which built
+// the page's slot map 128 times over (B200).
 
+#include "code_pairs.cuh"
 #include "common.cuh"
 #include "append_common.cuh"
 
@@ -158,20 +160,13 @@ __global__ void __launch_bounds__(kTileThreads) materialize_kernel(const __grid_
                      side == 0 ? a.out_k : a.out_v, a.out_dt, s_slot);
 }
 
-template <int OUT>
-__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
-  uint32_t v;
-  if (OUT == DARTKV_F16) asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
-  else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
-  return v;
-}
-
 // A page of n tokens, the tokens [lo, hi) of it wanted; out: row of the page's first token.  BITS 0: mixed keys.
 template <int MD, int DT, int BITS>
 __device__ __forceinline__ void restore_page(const dartkv_cache_desc& d, const uint8_t* page, int n, int lo, int hi, int flavour,
                                              uint16_t* out, const int* s_slot) {
   constexpr int PB = BITS == 0 ? 2 : BITS, TOK = 32 / PB;
-  constexpr uint32_t MASK = (1u << PB) - 1u;
+  CodeConsts<MD> consts;
+  consts.init();
   const int groups = ceil_div(n, d.key_group), row_words = groups * d.key_group * PB / 32;
   const uint32_t* codes = reinterpret_cast<const uint32_t*>(page);
   const uint32_t* high = reinterpret_cast<const uint32_t*>(page + d.key_off_high);
@@ -179,35 +174,38 @@ __device__ __forceinline__ void restore_page(const dartkv_cache_desc& d, const u
   for (int item = threadIdx.x; item < items; item += kSpanThreads) {
     const int p = item % pairs, w = item / pairs, t = w * TOK, g = t / d.key_group;
     if (t + TOK <= lo || t >= hi) continue;
-    uint32_t code[2], more[2] = {0, 0};
-    float s[2], z[2];
+    uint32_t code[2], more[2] = {0, 0}, s[2], z[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int c = 2 * p + i;
       code[i] = codes[c * row_words + w];
       if (BITS == 0 && s_slot[c] >= 0) more[i] = high[s_slot[c] * row_words + w];
-      s[i] = load_f(page + d.key_off_scale, MD, c * groups + g);
-      z[i] = load_f(page + d.key_off_zero, MD, c * groups + g);
+      s[i] = reinterpret_cast<const uint16_t*>(page + d.key_off_scale)[c * groups + g];
+      z[i] = reinterpret_cast<const uint16_t*>(page + d.key_off_zero)[c * groups + g];
     }
+    constexpr int PARTS = kColumnParts<BITS>, N = TOK / PARTS;
+    uint32_t* to = reinterpret_cast<uint32_t*>(out + (int64_t)t * d.head_dim) + p;
+    auto restore = [&](auto affine) {
+      affine.template init<0>(s[0] | (s[1] << 16), z[0] | (z[1] << 16));
 #pragma unroll
-    for (int u = 0; u < TOK; ++u) {
-      if (t + u < lo || t + u >= hi) continue;
-      float v[2];
+      for (int part = 0; part < PARTS; ++part) {
+        uint32_t v[N];
+        restore_columns<MD, DT, decltype(affine)::kFp32, BITS>(consts, code, more, affine, part, v);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        uint32_t q = (code[i] >> (PB * u)) & MASK;
-        if (BITS == 0) q |= ((more[i] >> (PB * u)) & MASK) << 2;
-        v[i] = affine_restore((float)q, s[i], z[i], MD, DT, flavour);
+        for (int u = 0; u < N; ++u, to += pairs)
+          if (t + part * N + u >= lo && t + part * N + u < hi) *to = v[u];
       }
-      reinterpret_cast<uint32_t*>(out + (int64_t)(t + u) * d.head_dim)[p] = pack_pair<DT>(v[0], v[1]);
-    }
+    };
+    if (flavour == DARTKV_DEQUANT_PER_OP) restore(PairAffine<MD, DT, false, true>());
+    else restore(PairAffine<MD, DT, true, true>());
   }
 }
 
 // Packed value rows [lo, hi) (absolute tokens); out + token * D: the token's output row.
 template <int MD, int DT, int BITS>
 __device__ __forceinline__ void restore_values(const dartkv_cache_desc& d, int bh, int lo, int hi, int flavour, uint16_t* out) {
-  constexpr uint32_t MASK = (1u << BITS) - 1u;
+  CodeConsts<MD> consts;
+  consts.init();
   const int per_row = d.head_dim / 8, items = (hi - lo) * per_row;
   for (int item = threadIdx.x; item < items; item += kSpanThreads) {
     const int t = lo + item / per_row, k = item % per_row, g = 8 * k / d.value_group;
@@ -217,12 +215,11 @@ __device__ __forceinline__ void restore_values(const dartkv_cache_desc& d, int b
     if (BITS == 2) q = reinterpret_cast<const uint16_t*>(codes)[k];
     else if (BITS == 4) q = reinterpret_cast<const uint32_t*>(codes)[k];
     else q = reinterpret_cast<const uint64_t*>(codes)[k];
-    const float s = load_f(d.v_meta, MD, (row * 2 + 0) * d.value_groups + g), z = load_f(d.v_meta, MD, (row * 2 + 1) * d.value_groups + g);
+    const uint16_t* meta = reinterpret_cast<const uint16_t*>(d.v_meta) + row * 2 * d.value_groups + g;
+    const uint32_t s = meta[0], z = meta[d.value_groups];
     uint32_t v[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      v[i] = pack_pair<DT>(affine_restore((float)((uint32_t)(q >> (BITS * 2 * i)) & MASK), s, z, MD, DT, flavour),
-                           affine_restore((float)((uint32_t)(q >> (BITS * (2 * i + 1))) & MASK), s, z, MD, DT, flavour));
+    if (flavour == DARTKV_DEQUANT_PER_OP) restore_row<MD, DT, false, BITS>(consts, q, s, z, v);
+    else restore_row<MD, DT, true, BITS>(consts, q, s, z, v);
     reinterpret_cast<uint4*>(out + (int64_t)t * d.head_dim)[k] = make_uint4(v[0], v[1], v[2], v[3]);
   }
 }

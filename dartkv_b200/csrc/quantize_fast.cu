@@ -6,11 +6,13 @@
 // are split over up to four threads per channel pair, and requested at once where they fit registers, codes gather in
 // registers (quant_math.cuh) and leave as whole words.  fp16 [8,8,1024,128], 2-bit + promoted keys in groups of 128 / 2-bit
 // values, a call of the Python API among others, with its allocations and the check of its input: keys with the selection
-// 33.7 us (36.7 with the tokens of a column group read twice), values 24.3, restoring them 10.7; all four calls with their
-// waits 92.5 us, 503 with one group or element per thread (B200).
+// 33.7 us (36.7 with the tokens of a column group read twice), values 24.3; all four calls with their waits 92.5 us, 503 with one
+// group or element per thread.  The GPU's share of restoring keys is 10.3 us element by element and 6.5 with two codes per
+// register (code_pairs.cuh), of values 8.3 and 4.9, some 2 us of each from the form of the launch (B200).
 
 #include <cooperative_groups.h>
 
+#include "code_pairs.cuh"
 #include "common.cuh"
 #include "quant_math.cuh"
 
@@ -422,18 +424,11 @@ struct RestoreArgs {
   void* out;
 };
 
-template <int MD>
-__device__ __forceinline__ float meta16(const void* p, int64_t i) { return load_f(p, MD, i); }
-
-template <int OUT>
-__device__ __forceinline__ uint32_t pack_pair(float lo, float hi) { return Pack16<OUT>::pack(hi, lo); }
-
 // Groups along a strided axis: a thread restores the tokens of one code word for two neighbouring columns.
 // grid (words / 4, slab of columns, outer), 256 threads = 64 column pairs x 4 words.  BITS 0: mixed keys.
 template <int MD, int OUT, int BITS>
 __global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_constant__ RestoreArgs a) {
   constexpr int PB = BITS == 0 ? 2 : BITS, TOK = 32 / PB;
-  constexpr uint32_t MASK = (1u << PB) - 1u;
   wait_previous();
   __shared__ int s_slot[BITS == 0 ? kSlab : 1];
   const int64_t o = blockIdx.z;
@@ -451,8 +446,7 @@ __global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_const
   if (c0 >= a.inner || t0 >= a.n) return;
   const int g = t0 / a.group;
   const int64_t row = o * a.inner + c0;
-  uint32_t code[2], high[2] = {0, 0};
-  float s[2], z[2];
+  uint32_t code[2], high[2] = {0, 0}, s[2], z[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     code[i] = reinterpret_cast<const uint32_t*>(a.values + (row + i) * a.packed_bytes)[w];
@@ -460,28 +454,31 @@ __global__ void __launch_bounds__(256) restore_columns_kernel(const __grid_const
       const int slot = s_slot[2 * p + i];
       if (slot >= 0) high[i] = reinterpret_cast<const uint32_t*>(a.high + (o * a.promoted + slot) * a.packed_bytes)[w];
     }
-    s[i] = meta16<MD>(a.scale, (row + i) * a.groups + g);
-    z[i] = meta16<MD>(a.zero, (row + i) * a.groups + g);
+    s[i] = reinterpret_cast<const uint16_t*>(a.scale)[(row + i) * a.groups + g];
+    z[i] = reinterpret_cast<const uint16_t*>(a.zero)[(row + i) * a.groups + g];
   }
-  uint32_t* out = reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(a.out) + o * a.so + (int64_t)t0 * a.sn + c0);
+  CodeConsts<MD> consts;
+  consts.init();
+  constexpr int PARTS = kColumnParts<BITS>, N = TOK / PARTS;
+  uint16_t* out = reinterpret_cast<uint16_t*>(a.out) + o * a.so + (int64_t)t0 * a.sn + c0;
+  auto restore = [&](auto affine) {
+    affine.template init<0>(s[0] | (s[1] << 16), z[0] | (z[1] << 16));
 #pragma unroll
-  for (int u = 0; u < TOK; ++u) {
-    if (t0 + u >= a.n) break;
-    float v[2];
+    for (int part = 0; part < PARTS; ++part) {
+      uint32_t v[N];
+      restore_columns<MD, OUT, decltype(affine)::kFp32, BITS>(consts, code, high, affine, part, v);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      uint32_t q = (code[i] >> (PB * u)) & MASK;
-      if (BITS == 0) q |= ((high[i] >> (PB * u)) & MASK) << 2;
-      v[i] = affine_restore((float)q, s[i], z[i], MD, OUT, a.flavour);
+      for (int u = 0; u < N; ++u, out += a.sn)
+        if (t0 + part * N + u < a.n) *reinterpret_cast<uint32_t*>(out) = v[u];
     }
-    *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(out) + (int64_t)u * a.sn) = pack_pair<OUT>(v[0], v[1]);
-  }
+  };
+  if (a.flavour == DARTKV_DEQUANT_PER_OP) restore(PairAffine<MD, OUT, false, true>());
+  else restore(PairAffine<MD, OUT, true, true>());
 }
 
 // Groups along contiguous elements: a thread restores eight of them.
 template <int MD, int OUT, int BITS>
 __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant__ RestoreArgs a, int64_t total) {
-  constexpr uint32_t MASK = (1u << BITS) - 1u;
   wait_previous();
   const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= total) return;
@@ -503,14 +500,12 @@ __global__ void __launch_bounds__(256) restore_rows_kernel(const __grid_constant
   if (BITS == 2) codes = reinterpret_cast<const uint16_t*>(a.values)[id];
   else if (BITS == 4) codes = reinterpret_cast<const uint32_t*>(a.values)[id];
   else codes = reinterpret_cast<const uint64_t*>(a.values)[id];
-  const float s = meta16<MD>(a.scale, g), z = meta16<MD>(a.zero, g);
+  const uint32_t s = reinterpret_cast<const uint16_t*>(a.scale)[g], z = reinterpret_cast<const uint16_t*>(a.zero)[g];
+  CodeConsts<MD> consts;
+  consts.init();
   uint32_t v[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float lo = affine_restore((float)((uint32_t)(codes >> (BITS * 2 * i)) & MASK), s, z, MD, OUT, a.flavour);
-    const float hi = affine_restore((float)((uint32_t)(codes >> (BITS * (2 * i + 1))) & MASK), s, z, MD, OUT, a.flavour);
-    v[i] = pack_pair<OUT>(lo, hi);
-  }
+  if (a.flavour == DARTKV_DEQUANT_PER_OP) restore_row<MD, OUT, false, BITS>(consts, codes, s, z, v);
+  else restore_row<MD, OUT, true, BITS>(consts, codes, s, z, v);
   *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + at) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
