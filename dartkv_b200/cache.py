@@ -515,6 +515,11 @@ class DartKVCache:
     def get(self) -> Tuple[torch.Tensor, torch.Tensor]:
         if self._life.seen == 0:
             raise RuntimeError("DartKVCache is empty; call update() before get()")
+        made = _lib.HOST.get(ctypes.addressof(self._desc), self._life.seen, self._device.index)
+        if made is not None:            # not on another device than the current one
+            if type(made) is int:
+                check(made)
+            return made
         b, h, d = self._shape
         keys = torch.empty((b, h, self._life.seen, d), dtype=self._dtype, device=self._device)
         values = torch.empty_like(keys)

@@ -143,9 +143,29 @@ at::ScalarType scalar_type(int code) {
   return code == DARTKV_F32 ? at::kFloat : code == DARTKV_F16 ? at::kHalf : at::kBFloat16;
 }
 
+// Several tensors in one allocation, each from a multiple of 512 bytes on (as the allocator would place them).
+struct Block {
+  int64_t size = 0;
+  at::Tensor memory;
+  int64_t add(at::IntArrayRef shape, at::ScalarType type) {
+    const int64_t at = size;
+    size += (c10::multiply_integers(shape) * (int64_t)c10::elementSize(type) + 511) / 512 * 512;
+    return at;
+  }
+  void allocate(const at::TensorOptions& bytes) { memory = at::empty({size}, bytes); }
+  at::Tensor view(int64_t at, at::IntArrayRef shape, at::ScalarType type) const {
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(memory.storage()), memory.key_set(), c10::scalarTypeToTypeMeta(type));
+    t.unsafeGetTensorImpl()->set_storage_offset(at / (int64_t)c10::elementSize(type));
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(shape);
+    return t;
+  }
+};
+
 // allocate(desc, device_index, key_pages, value_rows): the pools of a new cache, in the order of `kPoolNames` on the
 // Python side, with the descriptor's pointers set; None when the device is not the current one.  Only the state words
-// and the finite-input flag start at zero (one fill for both); everything else is written before it is read.
+// and the finite-input flag start at zero (one memset for both); everything else is written before it is read.  Pools that
+// never grow share one allocation, and so do those of the values, which grow together: an allocation of each pool's own and a
+// fill kernel take 20.6 us of host time, this 8.3.
 PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 4) { PyErr_SetString(PyExc_TypeError, "allocate takes 4 arguments"); return nullptr; }
@@ -155,16 +175,31 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (device != c10::cuda::current_device()) Py_RETURN_NONE;
   try {
     const int64_t b = d->batch, h = d->kv_heads, hd = d->head_dim, sinks = d->sink_tokens > 0 ? d->sink_tokens : 1;
-    const auto options = at::TensorOptions().device(at::Device(at::kCUDA, (c10::DeviceIndex)device));
-    const auto dense = options.dtype(scalar_type(d->dtype));
-    at::Tensor words = at::zeros({64}, options.dtype(at::kInt)), table = at::empty({2, pages}, options.dtype(at::kInt));
+    const auto bytes = at::TensorOptions().device(at::Device(at::kCUDA, (c10::DeviceIndex)device)).dtype(at::kByte);
+    const auto dense = scalar_type(d->dtype), md = scalar_type(d->md_dtype);
+    const int64_t ring = d->ring_tokens;
+    Block fixed, table, values;
+    const int64_t k_sink = fixed.add({b, h, sinks, hd}, dense), v_sink = fixed.add({b, h, sinks, hd}, dense),
+                  k_ring = fixed.add({b, h, ring, hd}, dense), v_ring = fixed.add({b, h, ring, hd}, dense),
+                  state = fixed.add({32}, at::kInt), nonfinite = fixed.add({1}, at::kInt),
+                  start = table.add({pages}, at::kInt), tokens = table.add({pages}, at::kInt),
+                  codes = values.add({b, h, rows, d->value_row_bytes}, at::kByte), meta = values.add({b, h, rows, 2, d->value_groups}, md);
+    fixed.allocate(bytes);
+    table.allocate(bytes);
+    values.allocate(bytes);
     at::Tensor pools[] = {
-        at::empty({b, h, sinks, hd}, dense), at::empty({b, h, sinks, hd}, dense),
-        at::empty({b, h, d->ring_tokens, hd}, dense), at::empty({b, h, d->ring_tokens, hd}, dense),
-        words.narrow(0, 0, 32), words.narrow(0, 32, 1),
-        at::empty({b, h, pages, d->key_page_bytes}, options.dtype(at::kByte)), table.select(0, 0), table.select(0, 1),
-        at::empty({b, h, rows, d->value_row_bytes}, options.dtype(at::kByte)),
-        at::empty({b, h, rows, 2, d->value_groups}, options.dtype(scalar_type(d->md_dtype)))};
+        fixed.view(k_sink, {b, h, sinks, hd}, dense), fixed.view(v_sink, {b, h, sinks, hd}, dense),
+        fixed.view(k_ring, {b, h, ring, hd}, dense), fixed.view(v_ring, {b, h, ring, hd}, dense),
+        fixed.view(state, {32}, at::kInt), fixed.view(nonfinite, {1}, at::kInt),
+        at::empty({b, h, pages, d->key_page_bytes}, bytes), table.view(start, {pages}, at::kInt), table.view(tokens, {pages}, at::kInt),
+        values.view(codes, {b, h, rows, d->value_row_bytes}, at::kByte), values.view(meta, {b, h, rows, 2, d->value_groups}, md)};
+    // from the state words to the end of the flag behind them
+    const cudaError_t err = cudaMemsetAsync(pools[4].data_ptr(), 0, (size_t)(nonfinite - state) + sizeof(int32_t),
+                                            (cudaStream_t)stream_of(pools[4]));
+    if (err != cudaSuccess) {
+      PyErr_Format(PyExc_RuntimeError, "CUDA error while clearing a new cache's state: %s", cudaGetErrorString(err));
+      return nullptr;
+    }
     d->k_sink = pools[0].data_ptr(); d->v_sink = pools[1].data_ptr();
     d->k_ring = pools[2].data_ptr(); d->v_ring = pools[3].data_ptr();
     d->state = (int32_t*)pools[4].data_ptr();
@@ -254,19 +289,116 @@ PyObject* tensors(std::initializer_list<at::Tensor> list) {
 
 bool dense_here(const at::Tensor& t) { return t.is_contiguous() && on_current_device(t); }
 
-// quantize(data, bits, group, axis, metadata dtype code, division, check) -> (values, scale, zero); data contiguous
+// get(desc, tokens, device_index) -> (keys, values): the whole cache materialized; None when the device is not the current one.
+PyObject* get(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 3) { PyErr_SetString(PyExc_TypeError, "get takes 3 arguments"); return nullptr; }
+  auto* d = static_cast<const dartkv_cache_desc*>(PyLong_AsVoidPtr(args[0]));
+  const int64_t tokens = PyLong_AsLongLong(args[1]);
+  const long device = PyLong_AsLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (device != c10::cuda::current_device()) Py_RETURN_NONE;
+  const auto options = at::TensorOptions().dtype(scalar_type(d->dtype)).device(at::Device(at::kCUDA, (c10::DeviceIndex)device));
+  at::Tensor keys = at::empty({d->batch, d->kv_heads, tokens, d->head_dim}, options), values = at::empty(keys.sizes(), options);
+  const int rc = dartkv_cache_materialize_both(d, 0, (int32_t)tokens, DARTKV_DEQUANT_PER_OP, keys.data_ptr(), values.data_ptr(), d->dtype,
+                                               stream_of(keys));
+  if (rc != 0) return PyLong_FromLong(rc);
+  return tensors({keys, values});
+  END_HANDLE_TH_ERRORS
+}
+
+// the shape in a Python tuple of integers; false when it is not one
+bool shape_of(PyObject* tuple, at::SmallVector<int64_t, 6>& shape) {
+  if (!PyTuple_Check(tuple)) return false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(tuple); ++i) {
+    shape.push_back(PyLong_AsLongLong(PyTuple_GET_ITEM(tuple, i)));
+    if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+  }
+  return true;
+}
+
+// dequantize(values, scale, zero, original shape, axis, bits, group, flavour, output dtype code) -> tensor
+PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 9) { PyErr_SetString(PyExc_TypeError, "dequantize takes 9 arguments"); return nullptr; }
+  at::SmallVector<int64_t, 6> shape;
+  for (int i = 0; i < 3; ++i)
+    if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
+  const at::Tensor &values = THPVariable_Unpack(args[0]), &scale = THPVariable_Unpack(args[1]), &zero = THPVariable_Unpack(args[2]);
+  if (!shape_of(args[3], shape)) Py_RETURN_NONE;
+  int64_t axis = PyLong_AsLongLong(args[4]);
+  const int bits = (int)PyLong_AsLong(args[5]);
+  const int64_t group = PyLong_AsLongLong(args[6]);
+  const int flavour = (int)PyLong_AsLong(args[7]), code = (int)PyLong_AsLong(args[8]);
+  if (PyErr_Occurred()) return nullptr;
+  const int64_t dims = (int64_t)shape.size();
+  if (axis < 0) axis += dims;
+  const int md = dtype_code(scale.scalar_type());
+  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || zero.scalar_type() != scale.scalar_type() || axis < 0 || axis >= dims ||
+      group < 1 || group > INT32_MAX || values.scalar_type() != at::kByte || !dense_here(values) || !dense_here(scale) || !dense_here(zero))
+    Py_RETURN_NONE;
+  int64_t outer = 1, inner = 1;
+  for (int64_t i = 0; i < axis; ++i) outer *= shape[i];
+  for (int64_t i = axis + 1; i < dims; ++i) inner *= shape[i];
+  const int64_t len = shape[axis];
+  at::Tensor out = at::empty(shape, values.options().dtype(scalar_type(code)).requires_grad(false));
+  const int rc = dartkv_dequantize((const uint8_t*)values.data_ptr(), scale.data_ptr(), zero.data_ptr(), md, outer, len, inner, bits, (int)group,
+                                   flavour, out.data_ptr(), code, len * inner, inner, 1, stream_of(values));
+  if (rc != 0) return PyLong_FromLong(rc);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// dequantize_mixed(low, high, indices, scale, zero, original shape, group, flavour, output dtype code) -> tensor
+PyObject* dequantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (n != 9) { PyErr_SetString(PyExc_TypeError, "dequantize_mixed takes 9 arguments"); return nullptr; }
+  at::SmallVector<int64_t, 6> shape;
+  for (int i = 0; i < 5; ++i)
+    if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
+  const at::Tensor &low = THPVariable_Unpack(args[0]), &high = THPVariable_Unpack(args[1]), &index = THPVariable_Unpack(args[2]),
+                   &scale = THPVariable_Unpack(args[3]), &zero = THPVariable_Unpack(args[4]);
+  if (!shape_of(args[5], shape) || shape.size() != 4) Py_RETURN_NONE;
+  const int64_t group = PyLong_AsLongLong(args[6]);
+  const int flavour = (int)PyLong_AsLong(args[7]), code = (int)PyLong_AsLong(args[8]);
+  if (PyErr_Occurred()) return nullptr;
+  const int md = dtype_code(scale.scalar_type());
+  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || zero.scalar_type() != scale.scalar_type() || group < 1 || group > INT32_MAX ||
+      low.scalar_type() != at::kByte || high.scalar_type() != at::kByte || index.scalar_type() != at::kInt || index.dim() < 1 ||
+      !dense_here(low) || !dense_here(high) || !dense_here(index) || !dense_here(scale) || !dense_here(zero))
+    Py_RETURN_NONE;
+  const int64_t promoted = index.size(-1);
+  at::Tensor out = at::empty(shape, low.options().dtype(scalar_type(code)).requires_grad(false));
+  const int rc = dartkv_dequantize_key_mixed((const uint8_t*)low.data_ptr(), promoted ? (const uint8_t*)high.data_ptr() : nullptr,
+                                             promoted ? (const int32_t*)index.data_ptr() : nullptr, scale.data_ptr(), zero.data_ptr(), md,
+                                             shape[0] * shape[1], shape[2], shape[3], (int)group, (int)promoted, flavour, out.data_ptr(), code,
+                                             stream_of(low));
+  if (rc != 0) return PyLong_FromLong(rc);
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// quantize(data, bits, group, axis, metadata dtype code (-1: the data's own, or fp32), division, check) -> (values, scale, zero)
 PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 7) { PyErr_SetString(PyExc_TypeError, "quantize takes 7 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
+  for (int i = 1; i < 7; ++i)
+    if (!PyLong_Check(args[i])) Py_RETURN_NONE;
   const at::Tensor& x = THPVariable_Unpack(args[0]);
-  const int bits = (int)PyLong_AsLong(args[1]);
+  const int64_t bits_asked = PyLong_AsLongLong(args[1]);
   const int64_t group = PyLong_AsLongLong(args[2]);
-  const int64_t axis = PyLong_AsLongLong(args[3]);
-  const int md = (int)PyLong_AsLong(args[4]), division = (int)PyLong_AsLong(args[5]), wanted = (int)PyLong_AsLong(args[6]);
-  if (PyErr_Occurred()) return nullptr;
+  int64_t axis = PyLong_AsLongLong(args[3]);
+  int md = (int)PyLong_AsLong(args[4]);
+  const int division = (int)PyLong_AsLong(args[5]), wanted = (int)PyLong_AsLong(args[6]);
+  if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }   // a number that no C integer holds
   const int code = dtype_code(x.scalar_type());
-  if (code < 0 || !dense_here(x) || x.numel() == 0 || group > INT32_MAX) Py_RETURN_NONE;
+  if (code < 0 || !dense_here(x) || x.numel() == 0 || group < 1 || group > INT32_MAX || md < -1 || division < 0 ||
+      (bits_asked != 2 && bits_asked != 4 && bits_asked != 8) || axis < -x.dim() || axis >= x.dim())
+    Py_RETURN_NONE;
+  const int bits = (int)bits_asked;
+  if (axis < 0) axis += x.dim();
+  if (md < 0) md = code;   // fp16 and bf16 keep their own, fp32 data fp32
   int64_t outer = 1, inner = 1;
   at::SmallVector<int64_t, 6> shape;
   for (int64_t i = 0; i < x.dim(); ++i) {
@@ -334,6 +466,9 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 PyMethodDef methods[] = {
+    {"get", (PyCFunction)(void (*)(void))get, METH_FASTCALL, "keys and values of a whole cache"},
+    {"dequantize", (PyCFunction)(void (*)(void))dequantize, METH_FASTCALL, "group-wise dequantizer"},
+    {"dequantize_mixed", (PyCFunction)(void (*)(void))dequantize_mixed, METH_FASTCALL, "mixed key dequantizer"},
     {"quantize", (PyCFunction)(void (*)(void))quantize, METH_FASTCALL, "group-wise quantizer"},
     {"quantize_mixed", (PyCFunction)(void (*)(void))quantize_mixed, METH_FASTCALL, "mixed key quantizer"},
     {"allocate", (PyCFunction)(void (*)(void))allocate, METH_FASTCALL, "the pools of a new cache"},

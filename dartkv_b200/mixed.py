@@ -72,8 +72,14 @@ class MixedQuantizedKey:
         return mask
 
     def dequantize(self, *, dtype: Optional[torch.dtype] = None, flavour: int = _lib.DEQUANT_PER_OP) -> torch.Tensor:
-        device = require_cuda(self.low_values, self.scale, self.zero_point)
         out_dtype = dtype or self.output_dtype
+        made = _lib.HOST.dequantize_mixed(self.low_values, self.high_values, self.channel_indices, self.scale, self.zero_point,
+                                          self.original_shape, self.group_size, flavour, _lib.DTYPE_CODE.get(out_dtype, -1))
+        if made is not None:            # whatever the native path leaves (and every error) is handled below
+            if type(made) is int:
+                check(made)
+            return made
+        device = require_cuda(self.low_values, self.scale, self.zero_point)
         if out_dtype not in _lib.DTYPE_CODE:
             raise TypeError(f"unsupported output dtype {out_dtype}")
         b, h, t, d = self.original_shape
@@ -166,6 +172,18 @@ def select_key_channels(
     return mask, indices
 
 
+def _mixed(made, keys: torch.Tensor, group_size: int) -> MixedQuantizedKey:
+    """The result of the native path, or its error."""
+
+    if made is False:
+        raise ValueError("key_states must contain finite values")
+    if type(made) is int:
+        check(made)
+    low, high, indices, scale, zero = made
+    shape = tuple(keys.shape)
+    return MixedQuantizedKey(low, high, indices, scale, zero, shape, -(-shape[2] // group_size) * group_size, group_size, 2, 4, keys.dtype)
+
+
 def quantize_key_mixed(
     key_states: torch.Tensor,
     *,
@@ -183,6 +201,14 @@ def quantize_key_mixed(
     host synchronization of the finite-input check.
     """
 
+    if indices is None and strategy == "magnitude" and promote_bits == 4 and isinstance(group_size, int) and group_size > 0 \
+            and key_states.ndim == 4 and 0.0 <= promote_ratio <= 1.0:
+        # an ordinary call; whatever the native path leaves (and every error) is handled below
+        count, metadata = promoted_count(key_states.shape[3], promote_ratio), metadata_dtype or key_states.dtype
+        if 0 < count < key_states.shape[3] and metadata in _lib.DTYPE_CODE:
+            made = _lib.HOST.quantize_mixed(key_states, group_size, count, _lib.DTYPE_CODE[metadata], None, int(check_finite))
+            if made is not None:
+                return _mixed(made, key_states, group_size)
     if key_states.ndim != 4:
         raise ValueError("key_states must have shape [B, H, T, D]")
     if not torch.is_floating_point(key_states):
@@ -208,16 +234,8 @@ def quantize_key_mixed(
         _, indices = select_key_channels(keys, promote_ratio, strategy=strategy)
     idx32 = None if select_here else indices.to(device=device, dtype=torch.int32).contiguous()
     made = _lib.HOST.quantize_mixed(keys, group_size, count, _lib.DTYPE_CODE[meta_dtype], idx32, int(check_finite))
-    if made is False:
-        raise ValueError("key_states must contain finite values")
-    if type(made) is int:
-        check(made)
     if made is not None:
-        low, high, idx32, scale, zero = made
-        return MixedQuantizedKey(
-            low_values=low, high_values=high, channel_indices=idx32, scale=scale, zero_point=zero,
-            original_shape=(batch, heads, tokens, head_dim), padded_tokens=-(-tokens // group_size) * group_size,
-            group_size=group_size, low_bits=2, promote_bits=promote_bits, output_dtype=keys.dtype)
+        return _mixed(made, keys, group_size)
     if select_here:
         idx32 = select_key_channels(keys, promote_ratio, strategy=strategy)[1].to(torch.int32).contiguous()
     promoted = idx32.shape[-1]

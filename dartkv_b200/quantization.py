@@ -16,6 +16,8 @@ from . import _lib
 from ._lib import LIB, check, ptr, require_cuda, stream_ptr, device_guard
 
 _SUPPORTED_BITS = (2, 4, 8)
+_DIVISION_CODE = {"true": _lib.DIV_TRUE, "reciprocal": _lib.DIV_RECIPROCAL}
+_METADATA_CODE = {None: -1, **_lib.DTYPE_CODE}
 
 
 def _validate_bits(bits: int) -> None:
@@ -120,8 +122,14 @@ class QuantizedTensor:
         the metadata dtype (the PyTorch path, default) or one fp32 multiply-add (its Triton path).
         """
 
-        device = require_cuda(self.values, self.scale, self.zero_point)
         out_dtype = dtype or self.output_dtype
+        made = _lib.HOST.dequantize(self.values, self.scale, self.zero_point, self.original_shape, self.axis, self.bits, self.group_size,
+                                    flavour, _lib.DTYPE_CODE.get(out_dtype, -1))
+        if made is not None:            # whatever the native path leaves (and every error) is handled below
+            if type(made) is int:
+                check(made)
+            return made
+        device = require_cuda(self.values, self.scale, self.zero_point)
         if out_dtype not in _lib.DTYPE_CODE:
             raise TypeError(f"unsupported output dtype {out_dtype}")
         axis = self.axis if self.axis >= 0 else len(self.original_shape) + self.axis
@@ -147,6 +155,20 @@ class QuantizedTensor:
             axis=self.axis)
 
 
+def _quantized(made, data: torch.Tensor, bits: int, group_size: int, axis: int) -> "QuantizedTensor":
+    """The result of the native path, or its error."""
+
+    if made is False:
+        raise ValueError("quantize expects all values to be finite")
+    if type(made) is int:
+        check(made)
+    values, scale, zero = made
+    shape = tuple(data.shape)
+    axis %= len(shape)
+    padded, vpb = -(-shape[axis] // group_size) * group_size, 8 // bits
+    return QuantizedTensor(values, scale, zero, shape, shape[axis], padded, -(-padded // vpb) * vpb, group_size, bits, data.dtype, axis)
+
+
 def quantize(
     data: torch.Tensor,
     *,
@@ -165,6 +187,10 @@ def quantize(
     finite-input check needs.
     """
 
+    made = _lib.HOST.quantize(data, bits, group_size, axis, _METADATA_CODE.get(metadata_dtype, -2), _DIVISION_CODE.get(division, -1),
+                              int(check_finite))
+    if made is not None:                # an ordinary call; whatever the native path leaves (and every error) is handled below
+        return _quantized(made, data, bits, group_size, axis)
     _validate_bits(bits)
     if not isinstance(group_size, int) or group_size <= 0:
         raise ValueError(f"group_size must be a positive integer, got {group_size}")
@@ -195,18 +221,9 @@ def quantize(
     vpb = 8 // bits
     packed_dim = ((padded_dim + vpb - 1) // vpb) * vpb
     moved_shape = tuple(s for i, s in enumerate(original_shape) if i != axis)
-    made = _lib.HOST.quantize(data, bits, group_size, axis, _lib.DTYPE_CODE[meta_dtype],
-                              _lib.DIV_TRUE if division == "true" else _lib.DIV_RECIPROCAL, int(check_finite))
-    if made is False:
-        raise ValueError("quantize expects all values to be finite")
-    if type(made) is int:
-        check(made)
+    made = _lib.HOST.quantize(data, bits, group_size, axis, _lib.DTYPE_CODE[meta_dtype], _DIVISION_CODE[division], int(check_finite))
     if made is not None:
-        values, scale, zero = made
-        return QuantizedTensor(
-            values=values, scale=scale, zero_point=zero, original_shape=original_shape, original_dim=n,
-            padded_dim=padded_dim, packed_dim=packed_dim, group_size=group_size, bits=bits, output_dtype=data.dtype,
-            axis=axis)
+        return _quantized(made, data, bits, group_size, axis)
     values = torch.empty((*moved_shape, packed_dim // vpb), dtype=torch.uint8, device=device)
     scale = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)
     zero = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)
