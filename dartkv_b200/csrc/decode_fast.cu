@@ -71,6 +71,10 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
   int unit = (int)((int64_t)sb * a.units / a.stream_blocks);   // the host keeps the unit count below 2^31
   const int unit_end = (int)((int64_t)(sb + 1) * a.units / a.stream_blocks);
   WarpSmem& ws = reinterpret_cast<WarpSmem*>(smem_raw)[warp];
+  int bh = unit / a.quads, quad = unit - bh * a.quads;
+  // the row's first live token, its query and the state are requested together
+  const int first_live = first_live_token(d, a, bh);
+  const QueryPair first_query = load_query(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, tid);
   const int k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
   const int fast_end = fast_range_end(d.sink_tokens, d.page_size, k_end, v_end, sink_filled);
   const int total_pages = fast_end > d.sink_tokens ? (fast_end - d.sink_tokens) / 128 : 0;
@@ -96,11 +100,10 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 
-  int bh = unit / a.quads, quad = unit - bh * a.quads;
-  RowPiece now = row_piece(d, a, bh, quad, min(a.quads - quad, unit_end - unit), total_pages);
+  RowPiece now = row_piece(d, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
   // this warp's first page is requested before anything else, so its latency overlaps the query load below
   if (lane == 0 && now.begin + warp < now.end) { issue_keys(bh, now.begin + warp); issue_values(bh, now.begin + warp); }
-  store_query(bs.q32, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, tid, kThreads);
+  store_query(bs.q32, first_query, tid);
   __syncthreads();
 
   while (unit < unit_end) {
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
     // this warp's first page of the next row: requested as soon as its buffers are free, before the rows are merged
     auto next_row = [&](auto issue) {
       if (lane != 0 || unit >= unit_end) return;
-      const RowPiece next = row_piece(d, a, bh + 1, 0, min(a.quads, unit_end - unit), total_pages);
+      const RowPiece next = row_piece(d, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
       if (next.begin + warp < next.end) issue(bh + 1, next.begin + warp);
     };
 
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
                                                      1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
     if (unit >= unit_end) break;
     ++bh;
-    now = row_piece(d, a, bh, 0, min(a.quads, unit_end - unit), total_pages);
-    store_query(bs.q32, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, tid, kThreads);
+    now = row_piece(d, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
+    store_query(bs.q32, load_query(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, tid), tid);
     __syncthreads();
   }
   if (!ok && lane == 0) atomicExch(a.status, 1);

@@ -428,6 +428,10 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   int unit = (int)((int64_t)sb * a.units / a.stream_blocks);   // the host keeps the unit count below 2^31
   const int unit_end = (int)((int64_t)(sb + 1) * a.units / a.stream_blocks);
   FusedWarpSmem& ws = reinterpret_cast<FusedWarpSmem*>(smem_raw)[warp];
+  int bh = unit / a.quads, quad = unit - bh * a.quads;
+  // the row's first live token, its query and the state are requested together
+  const int first_live = first_live_token(d, a, bh);
+  const QueryWords first_query = load_query_compact(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, warp == 0 ? rep : 0, lane);
   const int k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
   const int fast_end = fast_range_end(d.sink_tokens, d.page_size, k_end, v_end, sink_filled);
   const int total_pages = fast_end > d.sink_tokens ? (fast_end - d.sink_tokens) / 128 : 0;
@@ -452,11 +456,10 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 
-  int bh = unit / a.quads, quad = unit - bh * a.quads;
-  RowPiece now = row_piece(d, a, bh, quad, min(a.quads - quad, unit_end - unit), total_pages);
+  RowPiece now = row_piece(d, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
   // this warp's first page is requested before anything else, so its latency overlaps the query load below
   if (lane == 0 && now.begin + warp < now.end) { issue_keys(bh, now.begin + warp); issue_values(bh, now.begin + warp); }
-  if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane);
+  if (warp == 0) store_query_compact(bs.query, first_query, lane);
   __syncthreads();
 
   while (unit < unit_end) {
@@ -465,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
     // this warp's first page of the next row: requested as soon as its buffers are free, before the rows are merged
     auto next_row = [&](auto issue) {
       if (lane != 0 || unit >= unit_end) return;
-      const RowPiece next = row_piece(d, a, bh + 1, 0, min(a.quads, unit_end - unit), total_pages);
+      const RowPiece next = row_piece(d, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
       if (next.begin + warp < next.end) issue(bh + 1, next.begin + warp);
     };
 
@@ -522,8 +525,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
                                                      1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
     if (unit >= unit_end) break;
     ++bh;
-    now = row_piece(d, a, bh, 0, min(a.quads, unit_end - unit), total_pages);
-    if (warp == 0) store_query_compact(bs.query, a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane);
+    now = row_piece(d, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
+    if (warp == 0) store_query_compact(bs.query, load_query_compact(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane), lane);
     __syncthreads();
   }
   if (!ok && lane == 0) atomicExch(a.status, 1);

@@ -278,15 +278,22 @@ struct PageWork {
   }
 };
 
-// the query of a KV head's group, pre-shifted for the block-diagonal operand: [channel][2 * head + j']
-__device__ __forceinline__ void store_query(uint32_t (*q32)[8], const void* q, int64_t first_row, int rep, int tid, int threads) {
-  for (int i = tid; i < 4 * 128; i += threads) {
-    const int r = i >> 7, ch = i & 127;
-    uint32_t v = 0;
-    if (r < rep) v = reinterpret_cast<const uint16_t*>(q)[(first_row + r) * 128 + ch];
-    q32[ch][2 * r] = v;
-    q32[ch][2 * r + 1] = v << 16;
+// the query of a KV head's group, pre-shifted for the block-diagonal operand: [channel][2 * head + j'].  A thread has a channel of
+// heads r and r + 2 (zero for absent heads).
+struct QueryPair { uint32_t value[2]; };
+__device__ __forceinline__ QueryPair load_query(const void* q, int64_t first_row, int rep, int tid) {
+  QueryPair v;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = (tid >> 7) + 2 * i;
+    v.value[i] = r < rep ? reinterpret_cast<const uint16_t*>(q)[(first_row + r) * 128 + (tid & 127)] : 0u;
   }
+  return v;
+}
+__device__ __forceinline__ void store_query(uint32_t (*q32)[8], const QueryPair& v, int tid) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    *reinterpret_cast<uint2*>(&q32[tid & 127][2 * ((tid >> 7) + 2 * i)]) = make_uint2(v.value[i], v.value[i] << 16);
 }
 
 }  // namespace
