@@ -286,10 +286,13 @@ template <int MD> __device__ __forceinline__ float load_md(const void* p, int64_
 
 // Uniform key pages of few tokens: what decode_generic_kernel does, one tile of 32 tokens per block, with the chain of memory
 // latencies cut to two.  Every lane finds the place of its own token (sink, page, dense tail), so a tile is not cut at segment
-// edges; pages are found without a search where there are at most 32; the metadata dtype is a template argument (loads behind a
-// run-time choice of dtype are not batched); the tile's values, packed or dense, are requested with its keys.  The blocks of a
-// (batch, KV head), a.cluster of them, are a cluster that merges its results through distributed shared memory.
-template <int REP, int MD>
+// edges; pages are found without a search where there are at most 32; the tile's values, packed or dense, are requested with
+// its keys.  The blocks of a (batch, KV head), a.cluster of them, are a cluster that merges its results through distributed
+// shared memory.  What such a call waits for longest is its own instructions, each of which runs once: so the metadata dtype and
+// whether the cache is fp32 are template arguments (F32), what concerns a token (packed or dense, flavour, ring row) is found
+// once by its lane and kept as bits, and addresses of a thread's tokens and channels are a first one plus steps.  [1,8,256,128]
+// fp32, 2-bit: 12.5 us, with all of that found again for every element 15.0 us (of which requesting the values took 4.7).
+template <int REP, int MD, bool F32>
 __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __grid_constant__ dartkv_cache_desc d,
                                                                       const __grid_constant__ GenericArgs a) {
   extern __shared__ float smem[];
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
   float* s_l = s_m + REP;
   static_assert(GEN_WARPS * GEN_TILE <= GEN_THREADS, "partial logits and sums share memory");
 
-  const int split = blockIdx.x % a.cluster, bh = blockIdx.x / a.cluster;
+  const int tiles = a.cluster ? a.cluster : a.total_splits, split = blockIdx.x % tiles, bh = blockIdx.x / tiles;
   const int b = bh / d.kv_heads, h = bh % d.kv_heads;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int seen = d.state[0], pages = d.state[1], k_end = d.state[2], v_end = d.state[3], sink_filled = d.state[4];
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
   float acc[REP];
 #pragma unroll
   for (int r = 0; r < REP; ++r) acc[r] = 0.0f;
-  const int bits = d.key_bits, vpb = 8 / bits, vbits = d.value_bits, per = 8 / vbits, vg = vc / d.value_group;
+  const int bits = d.key_bits, vbits = d.value_bits, vg = vc / d.value_group;   // 2, 4 or 8 bits: no code lies across bytes
   const uint32_t mask = (1u << bits) - 1u, vmask = (1u << vbits) - 1u;
   auto value_flavour = [&](int tok) -> int {             // see decode_generic_kernel
     if (a.flavour == DARTKV_DEQUANT_PER_OP || d.regular_pages) return a.flavour;
@@ -339,7 +342,8 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
     const int tok = lo + min(lane, nt - 1);              // lanes past the tile repeat its last token
     // ---- the place of this lane's key
     const bool packed = tok >= sink_filled && tok < k_end;
-    int page_first = 0, page_n = 1, pg = 0, key_flavour = a.flavour;
+    int page_first = 0, page_n = 1, pg = 0;
+    bool key_per_op = a.flavour == DARTKV_DEQUANT_PER_OP;
     if (by_lane) {
       for (int i = 0; i < pages; ++i) {
         const int f = __shfl_sync(0xffffffffu, my_first, i), n = __shfl_sync(0xffffffffu, my_tokens, i);
@@ -355,40 +359,53 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
       page_n = d.page_tokens[pg];
     }
     const uint8_t* page = d.k_pages + ((int64_t)bh * d.max_key_pages + pg) * d.key_page_bytes;
-    if (a.flavour != DARTKV_DEQUANT_PER_OP && packed && page_first < v_end) {   // see decode_generic_kernel
+    if (!key_per_op && packed && page_first < v_end) {   // see decode_generic_kernel
       const int next_value_edge = d.sink_tokens + ((page_first - d.sink_tokens) / d.page_size + 1) * d.page_size;
-      if (min(next_value_edge, v_end) < page_first + page_n) key_flavour = DARTKV_DEQUANT_PER_OP;
+      key_per_op = min(next_value_edge, v_end) < page_first + page_n;
     }
+    // ---- bits of the tile's tokens: values packed, and restored with per-op rounding
+    const uint32_t value_packed = __ballot_sync(0xffffffffu, tok >= sink_filled && tok < v_end);
+    const uint32_t value_per_op = __ballot_sync(0xffffffffu, a.flavour == DARTKV_DEQUANT_PER_OP || value_flavour(tok) == DARTKV_DEQUANT_PER_OP);
     // ---- the tile's values are requested, kAhead of this thread's tokens at a time, the first ones before the keys are
-    // waited for.  A dense value takes the scale's register.  One copy of this code serves all of a tile's tokens: instruction
-    // fetch is the longest stall of such a call.  Dense [1,8,20,256] fp32, one query row per KV head: 20.5 us with dense values
-    // loaded one by one behind the softmax, 21.2 with a second copy of the code for the first tokens, 16.4 so.  Sixteen ahead
-    // with more query rows: 16 rows of that shape 37.2 us instead of 33.1.
+    // waited for.  A dense value takes the scale's register.  One copy of this code serves all of a tile's tokens.  Dense
+    // [1,8,20,256] fp32, one query row per KV head: 20.5 us with dense values loaded one by one behind the softmax, 21.2 with a
+    // second copy of the code for the first tokens, 16.4 so.  Sixteen ahead with more query rows: 16 rows of that shape 37.2 us
+    // instead of 33.1.
     constexpr int kAhead = REP <= 4 ? 16 : 8;
     uint32_t v_code[kAhead];
     float v_scale[kAhead], v_zero[kAhead];
-    auto value_packed = [&](int t) { return t >= sink_filled && t < v_end; };
-    auto request = [&](int base, auto dense) {
+    const int64_t row0 = (int64_t)bh * d.max_value_tokens + (lo - d.sink_tokens);   // of the tile's first token, whether packed or not
+    const uint8_t* const codes0 = d.v_codes + row0 * d.value_row_bytes + (vc * vbits >> 3);
+    const int meta_step = 2 * d.value_groups, ring_row = lo % d.ring_tokens;
+    const int64_t meta0 = row0 * meta_step + vg;
+    const int64_t sink0 = ((int64_t)bh * d.sink_tokens + lo) * D + vc, ring0 = (int64_t)bh * d.ring_tokens * D + vc;
+    auto dense = [&](const void* p, int64_t i) { return F32 ? reinterpret_cast<const float*>(p)[i] : load_f(p, d.dtype, i); };
+    auto request_values = [&](int base) {
 #pragma unroll
       for (int i = 0; i < kAhead; ++i) {
-        const int tt = vsplit + (base + i) * vsplits, t = lo + tt;
+        const int tt = vsplit + (base + i) * vsplits;
         v_code[i] = 0; v_scale[i] = v_zero[i] = 0.0f;
-        if (tt < nt && value_packed(t)) {
-          const int64_t row = (int64_t)bh * d.max_value_tokens + (t - d.sink_tokens);
-          v_code[i] = d.v_codes[row * d.value_row_bytes + vc / per];
-          v_scale[i] = load_md<MD>(d.v_meta, (row * 2 + 0) * d.value_groups + vg);
-          v_zero[i] = load_md<MD>(d.v_meta, (row * 2 + 1) * d.value_groups + vg);
-        } else if (tt < nt) {
-          v_scale[i] = t < sink_filled ? dense(d.v_sink, ((int64_t)bh * d.sink_tokens + t) * D + vc)
-                                       : dense(d.v_ring, ((int64_t)bh * d.ring_tokens + (t % d.ring_tokens)) * D + vc);
+        if (tt < nt) {
+          if ((value_packed >> tt) & 1u) {
+            v_code[i] = codes0[tt * d.value_row_bytes];
+            v_scale[i] = load_md<MD>(d.v_meta, meta0 + tt * meta_step);
+            v_zero[i] = load_md<MD>(d.v_meta, meta0 + tt * meta_step + d.value_groups);
+          } else if (lo + tt < sink_filled) {
+            v_scale[i] = dense(d.v_sink, sink0 + tt * D);
+          } else {
+            int row = ring_row + tt;
+            while (row >= d.ring_tokens) row -= d.ring_tokens;
+            v_scale[i] = dense(d.v_ring, ring0 + row * D);
+          }
         }
       }
     };
-    auto request_values = [&](int base) {
-      if (d.dtype == DARTKV_F32) request(base, [](const void* p, int64_t i) { return reinterpret_cast<const float*>(p)[i]; });
-      else request(base, [&](const void* p, int64_t i) { return load_f(p, d.dtype, i); });
-    };
     if (vsplit < vsplits) request_values(0);
+    auto restore = [&](uint32_t code, float s, float z, bool per_op) {
+      if (!F32) return affine_restore((float)code, s, z, MD, d.dtype, per_op ? DARTKV_DEQUANT_PER_OP : a.flavour);
+      const float rounded = rnd<MD>(__fadd_rn(rnd<MD>(__fmul_rn((float)code, s)), z)), fused = __fmaf_rn((float)code, s, z);
+      return per_op ? rounded : fused;   // fp32 caches round neither result again
+    };
     // ---- partial logits of this warp's channels
     float dot[REP];
 #pragma unroll
@@ -399,37 +416,30 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
     };
     if (packed) {
       const int j = tok - page_first, g = j / d.key_group, G = ceil_div(page_n, d.key_group);
-      const int row_bytes = ceil_div(G * d.key_group, vpb);
-      const uint8_t* codes = page + j / vpb;
-      const int shift = (j % vpb) * bits;
+      const int row_bytes = (G * d.key_group * bits + 7) >> 3;
+      const uint8_t* codes = page + (j * bits >> 3) + warp * row_bytes;
+      const int shift = j * bits & 7;
       const uint8_t *scale = page + d.key_off_scale, *zero = page + d.key_off_zero;
-#pragma unroll 2
+#pragma unroll 1
       for (int c0 = warp; c0 < D; c0 += 8 * GEN_WARPS) {
         uint32_t code[8];
         float s[8], z[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 8; ++i) {   // channels past the last one repeat it
           const int c = min(c0 + i * GEN_WARPS, D - 1);
-          code[i] = codes[c * row_bytes];
+          code[i] = codes[(c - warp) * row_bytes];
           s[i] = load_md<MD>(scale, c * G + g);
           z[i] = load_md<MD>(zero, c * G + g);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-          if (c0 + i * GEN_WARPS < D)
-            add(c0 + i * GEN_WARPS, affine_restore((float)((code[i] >> shift) & mask), s[i], z[i], MD, d.dtype, key_flavour));
+          if (c0 + i * GEN_WARPS < D) add(c0 + i * GEN_WARPS, restore((code[i] >> shift) & mask, s[i], z[i], key_per_op));
       }
     } else {
       const void* rows = tok < sink_filled ? d.k_sink : d.k_ring;
       const int64_t row = tok < sink_filled ? (int64_t)bh * d.sink_tokens + tok : (int64_t)bh * d.ring_tokens + tok % d.ring_tokens;
-      if (d.dtype == DARTKV_F32) {
-        const float* k = reinterpret_cast<const float*>(rows) + row * D;
-#pragma unroll 16
-        for (int c = warp; c < D; c += GEN_WARPS) add(c, k[c]);
-      } else {
 #pragma unroll 8
-        for (int c = warp; c < D; c += GEN_WARPS) add(c, load_f(rows, d.dtype, row * D + c));
-      }
+      for (int c = warp; c < D; c += GEN_WARPS) add(c, dense(rows, row * D + c));
     }
 #pragma unroll
     for (int r = 0; r < REP; ++r) s_part[(warp * REP + r) * GEN_TILE + lane] = dot[r];
@@ -453,16 +463,16 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
     __syncthreads();
     // ---- values
     if (vsplit < vsplits) {
-      const int vshift = (vc % per) * vbits;
+      const int vshift = vc * vbits & 7;
 #pragma unroll 1
       for (int base = 0; vsplit + base * vsplits < nt; base += kAhead) {
         if (base > 0) request_values(base);
 #pragma unroll
         for (int i = 0; i < kAhead; ++i) {
-          const int tt = vsplit + (base + i) * vsplits, t = lo + tt;
+          const int tt = vsplit + (base + i) * vsplits;
           if (tt >= nt) break;
-          const float v = value_packed(t) ? affine_restore((float)((v_code[i] >> vshift) & vmask), v_scale[i], v_zero[i], MD, d.dtype, value_flavour(t))
-                                          : v_scale[i];
+          const float v = (value_packed >> tt) & 1u ? restore((v_code[i] >> vshift) & vmask, v_scale[i], v_zero[i], (value_per_op >> tt) & 1u)
+                                                    : v_scale[i];
 #pragma unroll
           for (int r = 0; r < REP; ++r) acc[r] = fmaf(r < rep ? s_p[tt * REP + r] : 0.0f, v, acc[r]);
         }
@@ -483,6 +493,17 @@ __global__ void __launch_bounds__(GEN_THREADS, 2) decode_tiles_kernel(const __gr
       for (int s = 0; s < vsplits; ++s) acc[r] += s_part[(s * REP + r) * D + vc];
       s_part[r * D + vc] = acc[r];   // nobody else reads these entries before the cluster meets
     }
+  if (a.cluster == 0) {   // more tiles than a cluster has blocks: a partial each, for the merge kernel
+#pragma unroll
+    for (int r = 0; r < REP; ++r) {
+      if (r < rep) {
+        const int64_t row = ((int64_t)b * a.query_heads + h * rep + r) * a.total_splits + split;
+        if (tid == 0) { a.part_m[row] = s_l[r] == s_l[r] ? s_m[r] : s_l[r]; a.part_l[row] = s_l[r]; }   // see decode_generic_kernel
+        if (vsplit == 0) a.part_acc[row * D + vc] = acc[r];
+      }
+    }
+    return;
+  }
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
@@ -515,18 +536,19 @@ static size_t tiles_smem(int D, int rep) {
 }
 
 using GenericKernel = void (*)(const dartkv_cache_desc, const GenericArgs);
-template <int MD>
+template <int MD, bool F32>
 static GenericKernel tiles_variant_of(int rep) {
   switch (rep) {
-    case 1: return decode_tiles_kernel<1, MD>;
-    case 2: return decode_tiles_kernel<2, MD>;
-    case 4: return decode_tiles_kernel<4, MD>;
-    case 8: return decode_tiles_kernel<8, MD>;
-    default: return decode_tiles_kernel<16, MD>;
+    case 1: return decode_tiles_kernel<1, MD, F32>;
+    case 2: return decode_tiles_kernel<2, MD, F32>;
+    case 4: return decode_tiles_kernel<4, MD, F32>;
+    case 8: return decode_tiles_kernel<8, MD, F32>;
+    default: return decode_tiles_kernel<16, MD, F32>;
   }
 }
+template <bool F32>
 static GenericKernel tiles_variant(int md, int rep) {
-  return md == DARTKV_F32 ? tiles_variant_of<DARTKV_F32>(rep) : md == DARTKV_F16 ? tiles_variant_of<DARTKV_F16>(rep) : tiles_variant_of<DARTKV_BF16>(rep);
+  return md == DARTKV_F32 ? tiles_variant_of<DARTKV_F32, F32>(rep) : md == DARTKV_F16 ? tiles_variant_of<DARTKV_F16, F32>(rep) : tiles_variant_of<DARTKV_BF16, F32>(rep);
 }
 
 // shared memory of decode_generic_kernel<REP>; the sums of up to GEN_THREADS channels reuse the partial logits
@@ -1008,16 +1030,18 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     a.row_start = row_start;
     DARTKV_REQUIRE(L.generic_splits <= 65535, "too many splits");
     const int padded_rep = rep <= 1 ? 1 : rep <= 2 ? 2 : rep <= 4 ? 4 : rep <= 8 ? 8 : 16;
-    // Uniform pages of up to eight tiles, a block each: decode_tiles_kernel, whose blocks of a KV head are a cluster (of the
-    // portable size) and two of which fit an SM.  [1,8,256,128] fp32, 2-bit: 31.2 us through decode_generic_kernel and a merge
-    // launch, 16.4 here.  More blocks than two per SM gain nothing or lose: 64 rows of 160 tokens (320 blocks) 22.6 us there and
-    // 24.6 as tiles with 64 channels, 32.8 and 30.8 with 128; 192 rows of 96 tokens (576 blocks) 24.6 and 42.8.
-    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_chunk == GEN_TILE && L.generic_splits <= 8 &&
-                       bh * L.generic_splits <= 2 * dartkv_sm_count();
-    a.cluster = tiles ? L.generic_splits : 0;
+    // Uniform pages where a block has one tile at most go to decode_tiles_kernel.  Its blocks of a KV head are a cluster (of the
+    // portable size) and finish the row where there are up to eight of them and all are resident; clusters that wait for room cost
+    // more than partials and a merge.  Calls of 16-bit caches with more blocks than that stay with decode_generic_kernel.  fp32, 128
+    // channels: [1,8,256] 12.5 us (31.2 in decode_generic_kernel), [1,8,1000] 25.1 -> 16.7, [4,8,300] (320 blocks) 31.8 -> 18.8, [24,8,96] (576
+    // blocks) 24.4 there, 32.7 in clusters of three and 22.4 as partials; 16 bits, 64 channels, [128,8,20] 27.9 and 30.9 (B200).
+    const long long blocks = (long long)bh * L.generic_splits;
+    const bool resident = blocks <= 2 * dartkv_sm_count();
+    const bool tiles = d->key_mode == DARTKV_QUANTIZED_PAGE && L.generic_chunk == GEN_TILE && (resident || d->dtype == DARTKV_F32);
+    a.cluster = tiles && L.generic_splits <= 8 && (resident || L.generic_splits == 1) ? L.generic_splits : 0;
     a.out = peers ? nullptr : out;
     const size_t smem = tiles ? tiles_smem(D, padded_rep) : generic_smem(D, padded_rep);
-    const GenericKernel kernel = tiles ? tiles_variant(d->md_dtype, padded_rep) : padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
+    const GenericKernel kernel = tiles ? (d->dtype == DARTKV_F32 ? tiles_variant<true>(d->md_dtype, padded_rep) : tiles_variant<false>(d->md_dtype, padded_rep)) : padded_rep == 1 ? decode_generic_kernel<1> : padded_rep == 2 ? decode_generic_kernel<2>
                       : padded_rep == 4 ? decode_generic_kernel<4> : padded_rep == 8 ? decode_generic_kernel<8> : decode_generic_kernel<16>;
     if (smem > 48 * 1024) DARTKV_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (a.cluster) {
@@ -1025,6 +1049,9 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
       DARTKV_LAUNCH_OK("decode_tiles_kernel");
       if (!peers) return DARTKV_OK;
       L.total_splits = 1;
+    } else if (tiles) {
+      DARTKV_CUDA_OK(launch_following(kernel, dim3((unsigned)(bh * L.generic_splits)), dim3(GEN_THREADS), smem, stream, *d, a));
+      DARTKV_LAUNCH_OK("decode_tiles_kernel");
     } else {
       DARTKV_CUDA_OK(launch_following(kernel, dim3(bh, L.generic_splits), GEN_THREADS, smem, stream, *d, a));
       DARTKV_LAUNCH_OK("decode_generic_kernel");
