@@ -745,6 +745,7 @@ struct DecodeLayout {
   int fast;                            // tensor-core kernel for the packed pages: 1 per-op rounded, 2 unrounded fp32
   int quads, stream_blocks;            // tensor-core layouts: four-page units per (batch, kv head), stream blocks
   long long units;
+  int unit_pages, row_units;           // pages of the units that are dealt out, four or eight, and such units per row
   int total_splits;
   int row_groups;                      // layout 4: groups of up to eight query rows per KV head
   int pieces;                          // large calls of more than eight rows (decode_many.cu): blocks per work row, else 0
@@ -752,12 +753,12 @@ struct DecodeLayout {
 
 int dartkv_decode_fast_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
 int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
-                              int flavour, int quads, int stream_blocks, long long units, int total_splits,
+                              int flavour, int unit_pages, int quads, int stream_blocks, long long units, int total_splits,
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                               cudaStream_t stream);
 int dartkv_decode_fused32_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
 int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
-                                 int flavour, int quads, int stream_blocks, long long units, int total_splits,
+                                 int flavour, int unit_pages, int quads, int stream_blocks, long long units, int total_splits,
                                  float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                               cudaStream_t stream);
 
@@ -815,6 +816,57 @@ static int generic_splits_for(int bh, int tokens) {
   return min(max(1, (148 * 4 + bh - 1) / bh), max(1, (tokens + GEN_TILE - 1) / GEN_TILE));
 }
 
+// Work split of the 2-bit kernels.  Two families are compared with a cost model in rounds of eight pages, one per warp:
+//   aligned    rows * s blocks, s = 1..16 pieces per row, in units of four pages;
+//   unaligned  one block per resident slot, in units of eight pages: a block may finish one row and start the next (at most 15
+//              blocks touch a row), and what it does of a row is whole rounds but for the row's last one.
+// Of a round beside another block on the SM, a round alone takes 0.6, one of four pages whose warps have a page each 0.7 (shared by two
+// warps, alone, 0.3), a row that a block touches 0.3 more, the dense block of a row 0.7 of a slot's time, and up to 0.45 where
+// dense blocks are left over for a second turn; the unaligned family counts 1 % more.  Fitted to 88 shapes (8 to 1,024 rows, 4 to
+// 255 pages, both kernels), of which the model's choice takes 0.2 % more than the best of both families on average and 4 % at most;
+// in units of four pages and with the constants of kernels of four pages a round 8 x 2,200 tokens took 17.2 us and not 14.5, unrounded
+// 16 x 2,200 19.2 and not 15.6, 32 x 8,192 86.2 and not 82.9, 24 x 6,001 55.6 and not 52.6.  Aligned and unaligned: batch 128, 32,768
+// tokens 1,054 and 1,075, 112 x 10,000 364 and 321 (B200).
+static void two_bit_split(DecodeLayout& L, int bh, int pages, int resident, const char* force) {
+  constexpr double kRow = 0.3, kDense = 0.7, kAlone = 0.6, kShared = 0.3, kHalf = 0.7, kTail = 0.45, kAcross = 1.01;
+  const bool force_unaligned = force && force[0] == 'u', force_aligned = force && force[0] == 'a';
+  const int sms = dartkv_sm_count();
+  int best_pieces = 1;
+  double best_cost = 1e30;
+  for (int q = max(1, (L.quads + 15) / 16); q <= L.quads; ++q) {
+    const int pieces = (L.quads + q - 1) / q;
+    const long long blocks = (long long)bh * pieces;
+    const bool alone = blocks <= sms;
+    const double rounds = (q == 1 ? (alone ? kShared : kHalf) : (q + 1) / 2 * (alone ? kAlone : 1.0)) + kRow;
+    const double left_over = blocks + bh > resident ? (double)(blocks + bh - resident) / sms : 0.0;
+    const double by_waves = (double)((blocks + resident - 1) / resident) * rounds + kTail * (left_over < 1.0 ? left_over : 1.0);
+    const double by_work = (double)bh * (pieces * rounds + kDense) / resident;
+    const double cost = by_waves > by_work ? by_waves : by_work;
+    if (cost < best_cost - 1e-9) { best_cost = cost; best_pieces = pieces; }
+  }
+  L.unit_pages = 4;
+  L.row_units = L.quads;
+  L.stream_blocks = bh * best_pieces;
+  L.total_splits = best_pieces + 1;
+  const int octs = (pages + 7) / 8;
+  const long long units = (long long)bh * octs, min_share = (octs + 14) / 15;
+  long long blocks = min((long long)resident, units / min_share);
+  if (force_unaligned && strchr(force, ':')) {
+    const long long wanted = atoll(strchr(force, ':') + 1);
+    if (wanted >= 1 && wanted < blocks) blocks = wanted;
+  }
+  if (blocks < 1 || force_aligned) return;
+  const double share = (double)((units + blocks - 1) / blocks);
+  const double cost = kAcross * (share * (blocks <= sms ? kAlone : 1.0) + kRow * (share / octs + 1.0) + (double)bh * kDense / resident);
+  if (cost >= best_cost && !force_unaligned) return;
+  L.unit_pages = 8;
+  L.row_units = octs;
+  L.stream_blocks = (int)blocks;
+  // slots of a row: the blocks that touch it, counted in the units that are dealt out and in those of four pages that a plan reports
+  const long long w8 = units / blocks, w4 = max(1ll, L.units / blocks);
+  L.total_splits = (int)max((octs + w8 - 2) / w8, (L.quads + w4 - 2) / w4) + 2;
+}
+
 // rows_call: the call came through dartkv_decode_attention_rows, the only one that runs more than four query rows per
 // KV head on the tensor cores
 static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int query_heads, int flavour, int tokens,
@@ -823,6 +875,7 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
   const int rep = query_heads / d->kv_heads;
   int bh = d->batch * d->kv_heads;
   L.row_groups = 1;
+  L.unit_pages = 4;
   L.fast = rows_call && rep > 4 && dartkv_decode_rows_supported(d, q_dtype, rep, flavour) ? 4 : 0;
   if (L.fast == 4) {
     L.row_groups = dartkv_decode_rows_groups(rep);
@@ -839,16 +892,15 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     bh = d->batch * d->kv_heads;
   }
   if (L.fast) {
-    // One unit = four consecutive pages of a (batch, kv head).  The units of all rows are dealt out evenly to
-    // `stream_blocks` blocks.  Two families of splits are compared with a cost model in units of a round of four pages
+    // One unit = four consecutive pages of a (batch, kv head).  The units of all rows are dealt out evenly to `stream_blocks`
+    // blocks (two_bit_split() for the 2-bit kernels).  Two families of splits are compared with a cost model in units of a round of four pages
     // (a block costs its rounds plus 1.75 per row it touches: query load, first-page latency, merge of its eight warps;
     // the dense block of a row about 2; blocks run in waves of two per SM):
     //   aligned    rows * s blocks, s = 1..16 pieces per row;
     //   unaligned  one block per resident slot, a block may finish one row and start the next (at most 16 blocks
     //              touch a row); measured ~3 % slower per unit than aligned blocks, but it fills every slot when
     //              the rows do not (e.g. 256 rows on 296 slots: 9 % faster at context 32768).
-    // The constants were fitted to B200 timings of kernels that put two warps on each of a round's four pages, as
-    // decode_rows and decode_wide do.  The 2-bit kernels take eight pages a round; they have not been refitted to them.
+    // The constants were fitted to B200 timings.
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
@@ -869,6 +921,14 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
       }
     }
     const int resident = (L.fast == 3 ? dartkv_decode_wide_blocks_per_sm(d, q_dtype, rep, flavour) : 2) * dartkv_sm_count();
+    // "aligned" | "unaligned" | "unaligned:<blocks>" overrides the model (tests exercise both families, and
+    // blocks that span several rows, with it): set through dartkv_decode_split_override(), or once per process
+    // from the environment variable DARTKV_DECODE_SPLIT
+    const char* force = split_override();
+    if (L.fast == 1 || L.fast == 2) {
+      two_bit_split(L, bh, pages, resident, force);
+      return L;
+    }
     // dense blocks of the many-row layout (one per four rows): with 2.0 instead of 4.0 8 x 1,177 tokens, 12 rows, take 39.9
     // instead of 33.8 us; with 8.0 16 x 2,125 tokens, 8 rows, 48 instead of 44
     const double block_fixed = 1.75, dense_cost = L.fast == 4 ? 4.0 : 2.0;
@@ -889,10 +949,6 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
       const long long min_share = (L.quads + 14) / 15;
       long long blocks = resident;
       if (blocks > L.units / min_share) blocks = L.units / min_share;
-      // "aligned" | "unaligned" | "unaligned:<blocks>" overrides the model (tests exercise both families, and
-      // blocks that span several rows, with it): set through dartkv_decode_split_override(), or once per process
-      // from the environment variable DARTKV_DECODE_SPLIT
-      const char* force = split_override();
       const bool force_unaligned = force && force[0] == 'u', force_aligned = force && force[0] == 'a';
       if (force_unaligned && strchr(force, ':')) {
         const long long wanted = atoll(strchr(force, ':') + 1);
@@ -1018,9 +1074,15 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
                                        part_l, part_acc, status, row_start, stream);
     if (rc) return rc;
   } else if (L.fast) {
-    int rc = (L.fast == 3 ? dartkv_decode_wide_launch : L.fast == 2 ? dartkv_decode_fused32_launch : dartkv_decode_fast_launch)(
-        d, query, q_dtype, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units, L.total_splits, part_m,
-        part_l, part_acc, status, row_start, stream);
+    if (L.unit_pages == 8) {   // what kernel and merge find a row's blocks from
+      L.quads = L.row_units;
+      L.units = (long long)bh * L.row_units;
+    }
+    int rc = L.fast == 3 ? dartkv_decode_wide_launch(d, query, q_dtype, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units,
+                                                     L.total_splits, part_m, part_l, part_acc, status, row_start, stream)
+                         : (L.fast == 2 ? dartkv_decode_fused32_launch : dartkv_decode_fast_launch)(
+                               d, query, q_dtype, query_heads, scale, flavour, L.unit_pages, L.quads, L.stream_blocks, L.units, L.total_splits,
+                               part_m, part_l, part_acc, status, row_start, stream);
     if (rc) return rc;
   } else {
     GenericArgs a;

@@ -3,7 +3,7 @@
 // 32 promoted 2+2-bit channels), 16-bit data whose metadata has the same dtype, up to 4 query heads
 // per KV head.  Everything else takes the generic kernel in decode_attention.cu.
 //
-// Work split: one unit = four consecutive pages of a (batch, kv head) row.  The units of all rows are dealt out
+// Work split: one unit = four or eight consecutive pages of a (batch, kv head) row.  The units of all rows are dealt out
 // evenly to the stream blocks (aligned to rows, or one block per resident slot whose share may run from one
 // row into the next; the host chooses).  A warp of a block's eight takes every eighth page of the block's run by itself
 // (decode_page.cuh), from buffers of its own that bulk async copies fill, completion on an mbarrier: the keys' buffer is
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
     return;
   }
 
-  // ---- stream block: an even share of all (row, four-page unit) work, possibly spanning several rows
+  // ---- stream block: an even share of all (row, unit) work, possibly spanning several rows
   const int sb = blockIdx.x;
   int unit = (int)((int64_t)sb * a.units / a.stream_blocks);   // the host keeps the unit count below 2^31
   const int unit_end = (int)((int64_t)(sb + 1) * a.units / a.stream_blocks);
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 
-  RowPiece now = row_piece(d, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
+  RowPiece now = row_piece(d, a, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
   // this warp's first page is requested before anything else, so its latency overlaps the query load below
   if (lane == 0 && now.begin + warp < now.end) { issue_keys(bh, now.begin + warp); issue_values(bh, now.begin + warp); }
   store_query(bs.q32, first_query, tid);
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
     // this warp's first page of the next row: requested as soon as its buffers are free, before the rows are merged
     auto next_row = [&](auto issue) {
       if (lane != 0 || unit >= unit_end) return;
-      const RowPiece next = row_piece(d, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
+      const RowPiece next = row_piece(d, a, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
       if (next.begin + warp < next.end) issue(bh + 1, next.begin + warp);
     };
 
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fast_kernel(dartkv_cache_d
                                                      1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
     if (unit >= unit_end) break;
     ++bh;
-    now = row_piece(d, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
+    now = row_piece(d, a, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
     store_query(bs.q32, load_query(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, tid), tid);
     __syncthreads();
   }
@@ -230,14 +230,14 @@ static FastKernel fast_variant(bool few, int md, int dtype, int value_groups, in
 }
 
 int dartkv_decode_fast_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
-                              int flavour, int quads, int stream_blocks, long long units, int total_splits,
+                              int flavour, int unit_pages, int quads, int stream_blocks, long long units, int total_splits,
                               float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                               cudaStream_t stream) {
   (void)q_dtype;
   FastArgs a{query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l, part_acc, status,
-             row_start};
+             row_start, unit_pages};
   dim3 grid(stream_blocks + d->batch * d->kv_heads);
-  const bool few = dartkv_few_pages(units, stream_blocks);
+  const bool few = dartkv_few_pages(unit_pages, units, stream_blocks);
   {
     // the shared-memory opt-in is per device and per kernel: ask once per device (the flags are atomic; two threads
     // that race on a device's first call both set the attribute, which is harmless)

@@ -25,10 +25,10 @@ struct FastArgs {
   int query_heads;
   float scale;
   int flavour;
-  // Work split: one unit = four consecutive pages of one (batch, kv head) (a round of the four warp pairs of decode_rows and
-  // decode_wide, half a round of the eight warps of the 2-bit kernels); the units of all (batch, kv head) rows, `quads` each,
-  // are dealt out evenly to `stream_blocks` blocks, so a block may finish one row and start the next.  Partial slot 0 of a row
-  // belongs to its dense-token block, slot 1 + k to the k-th stream block that touches the row.
+  // Work split: one unit = `unit_pages` consecutive pages of one (batch, kv head): four (a round of the four warp pairs of
+  // decode_rows and decode_wide) or, in the 2-bit kernels, eight (a round of their eight warps); the units of all (batch, kv
+  // head) rows, `quads` each, are dealt out evenly to `stream_blocks` blocks, so a block may finish one row and start the next.
+  // Partial slot 0 of a row belongs to its dense-token block, slot 1 + k to the k-th stream block that touches the row.
   int quads, stream_blocks;
   long long units;
   int total_splits;
@@ -38,6 +38,7 @@ struct FastArgs {
   int* status;
   // optional [batch] first live token of every batch row (left padding): tokens before it get no weight
   const int32_t* row_start;
+  int unit_pages;
 };
 
 // Calls of the 2-bit kernels whose blocks have one unit each, four pages at most, and an SM each: a warp per page would leave
@@ -45,7 +46,9 @@ struct FastArgs {
 // 32 heads on 8: 16 x 160 tokens 14.3 -> 12.3 us, 8 x 800 14.1 -> 12.9, 4 x 2,080 13.5 -> 13.1; unrounded 12.3 -> 10.3, 12.3 ->
 // 11.2, 11.8 -> 11.3.  Two blocks on an SM keep it busy, and the second table of a page costs: 4 x 4,128 tokens (256 blocks) 17.5
 // us, shared 18.4, 2 x 6,000 (192) 17.0 and 18.4 (B200).
-inline bool dartkv_few_pages(long long units, int stream_blocks) { return units == stream_blocks && stream_blocks <= dartkv_sm_count(); }
+inline bool dartkv_few_pages(int unit_pages, long long units, int stream_blocks) {
+  return unit_pages == 4 && units == stream_blocks && stream_blocks <= dartkv_sm_count();
+}
 
 // The pages of one row that a block of the 2-bit kernels works on; tokens before first_live get no weight (left padding) and
 // whole pages of them are not even fetched.
@@ -55,11 +58,11 @@ struct RowPiece {
 __device__ __forceinline__ int first_live_token(const dartkv_cache_desc& d, const FastArgs& a, int bh) {
   return a.row_start ? max(a.row_start[bh / d.kv_heads], 0) : 0;
 }
-__device__ __forceinline__ RowPiece row_piece(const dartkv_cache_desc& d, int first_live, int quad, int quads, int total_pages) {
+__device__ __forceinline__ RowPiece row_piece(const dartkv_cache_desc& d, const FastArgs& a, int first_live, int quad, int quads, int total_pages) {
   RowPiece p;
   p.first_live = first_live;
-  p.begin = max(4 * quad, p.first_live > d.sink_tokens ? (p.first_live - d.sink_tokens) >> 7 : 0);
-  p.end = min(4 * (quad + quads), total_pages);
+  p.begin = max(a.unit_pages * quad, p.first_live > d.sink_tokens ? (p.first_live - d.sink_tokens) >> 7 : 0);
+  p.end = min(a.unit_pages * (quad + quads), total_pages);
   return p;
 }
 

@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
   bool ok = true;
   uint32_t parity = 0;   // of the pages this warp has consumed so far
 
-  RowPiece now = row_piece(d, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
+  RowPiece now = row_piece(d, a, first_live, quad, min(a.quads - quad, unit_end - unit), total_pages);
   // this warp's first page is requested before anything else, so its latency overlaps the query load below
   if (lane == 0 && now.begin + warp < now.end) { issue_keys(bh, now.begin + warp); issue_values(bh, now.begin + warp); }
   if (warp == 0) store_query_compact(bs.query, first_query, lane);
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
     // this warp's first page of the next row: requested as soon as its buffers are free, before the rows are merged
     auto next_row = [&](auto issue) {
       if (lane != 0 || unit >= unit_end) return;
-      const RowPiece next = row_piece(d, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
+      const RowPiece next = row_piece(d, a, first_live_token(d, a, bh + 1), 0, min(a.quads, unit_end - unit), total_pages);
       if (next.begin + warp < next.end) issue(bh + 1, next.begin + warp);
     };
 
@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_fused32_kernel(dartkv_cach
                                                      1 + sb - dartkv_block_of_unit((int64_t)bh * a.quads, a.stream_blocks, a.units));
     if (unit >= unit_end) break;
     ++bh;
-    now = row_piece(d, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
+    now = row_piece(d, a, first_live_token(d, a, bh), 0, min(a.quads, unit_end - unit), total_pages);
     if (warp == 0) store_query_compact(bs.query, load_query_compact(a.q, (int64_t)(bh / d.kv_heads) * a.query_heads + bh % d.kv_heads * rep, rep, lane), lane);
     __syncthreads();
   }
@@ -587,14 +587,14 @@ static FusedKernel fused_variant(bool few, int dtype, int md, int value_groups, 
 }
 
 int dartkv_decode_fused32_launch(const dartkv_cache_desc* d, const void* query, int q_dtype, int query_heads, float scale,
-                                 int flavour, int quads, int stream_blocks, long long units, int total_splits,
+                                 int flavour, int unit_pages, int quads, int stream_blocks, long long units, int total_splits,
                                  float* part_m, float* part_l, float* part_acc, int* status, const int32_t* row_start,
                                  cudaStream_t stream) {
   (void)q_dtype;
   FastArgs a{query, query_heads, scale, flavour, quads, stream_blocks, units, total_splits, part_m, part_l, part_acc, status,
-             row_start};
+             row_start, unit_pages};
   dim3 grid(stream_blocks + d->batch * d->kv_heads);
-  const bool few = dartkv_few_pages(units, stream_blocks);
+  const bool few = dartkv_few_pages(unit_pages, units, stream_blocks);
   {
     // the shared-memory opt-in is per device and per kernel: ask once per device (the flags are atomic; two threads
     // that race on a device's first call both set the attribute, which is harmless)
