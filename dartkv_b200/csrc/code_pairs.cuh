@@ -115,7 +115,7 @@ template <int MD, int OUT, bool FP32, int BITS>
 __device__ __forceinline__ void restore_row(const CodeConsts<MD>& k, uint64_t codes, uint32_t scale, uint32_t zero, uint32_t (&r)[4]) {
   constexpr int P0 = Half2Ops<MD>::kFirstPos;
   PairAffine<MD, OUT, FP32, true> affine;
-  affine.template init<0>(scale * 0x00010001u, zero * 0x00010001u);
+  affine.template init<0>(low_twice(scale), low_twice(zero));
   const uint32_t lo = (uint32_t)codes, hi = (uint32_t)(codes >> 32);
   if constexpr (BITS == 8) {
     restore_codes8<MD, OUT>(prmt(lo, hi, 0x6420u), prmt(lo, hi, 0x7531u), affine, r);

@@ -173,7 +173,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_many_kernel(const __grid_c
       restore_codes8<MD, DT, false>(codes.z, codes.w, affine, r + 4);
     }
   };
-  auto twice = [](uint32_t x) { return x * 0x00010001u; };
   using KeyWord = typename CodeWord<KB>::type;
   using ValueWord = typename CodeWord<VB>::type;
   constexpr int kKeyPositions = KB == 2 ? 3 : 1, kValuePositions = VB == 2 ? 3 : VB == 4 ? 1 : 0;
@@ -201,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_many_kernel(const __grid_c
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       Affine affine;
-      affine.template init<kKeyPositions>(twice(ss[i]), twice(zz[i]));
+      affine.template init<kKeyPositions>(low_twice(ss[i]), low_twice(zz[i]));
       uint32_t r[8];
       restore(x[i], affine, r);
       if (promoted[i] != step) store_tile(to + 32 * i * kTileRow, r);   // else made below
@@ -210,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_many_kernel(const __grid_c
       for (int s = 4 * warp + sub; s < K; s += 32) {
         const int ch = reinterpret_cast<const int32_t*>(k_stage + d.key_off_index)[s] & 127;
         Affine affine;
-        affine.template init<2>(twice(lds_u16(k_stage + d.key_off_scale + 2 * ch)), twice(lds_u16(k_stage + d.key_off_zero + 2 * ch)));
+        affine.template init<2>(low_twice(lds_u16(k_stage + d.key_off_scale + 2 * ch)), low_twice(lds_u16(k_stage + d.key_off_zero + 2 * ch)));
         uint32_t r[8];
         restore_codes22<MD, DT, false>(cc, lds_u32(k_stage + 32 * ch + 4 * word), lds_u32(k_stage + d.key_off_high + 32 * s + 4 * word), affine, r);
         store_tile(sm.keys + ch * kTileRow + 32 * word, r);
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_many_kernel(const __grid_c
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       Affine affine;
-      affine.template init<kValuePositions>(twice(ss[i]), twice(zz[i]));
+      affine.template init<kValuePositions>(low_twice(ss[i]), low_twice(zz[i]));
       uint32_t r[8];
       restore(x[i], affine, r);
       store_tile(to + 32 * i * kTileRow, r);

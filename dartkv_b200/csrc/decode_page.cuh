@@ -36,8 +36,6 @@ __device__ __forceinline__ void cast_registers(uint32_t (&r)[N]) {
   }
 }
 
-__device__ __forceinline__ uint32_t low_twice(uint32_t x) { return prmt(x, x, 0x1010u); }
-__device__ __forceinline__ uint32_t high_twice(uint32_t x) { return prmt(x, x, 0x3232u); }
 
 // DT = metadata dtype (the arithmetic of the dequantization), OUT = cache dtype (the MMA operands): when they differ
 // every dequantized register is cast, as the reference casts its dequantized pages (src/dart/quantization.py:103-106).
@@ -48,10 +46,11 @@ template <int DT, int OUT, int GN, int KP>
 struct PageWork {
   using H = Half2Ops<DT>;
   using HO = Half2Ops<OUT>;
-  // Unrolling, for whole pages: longer bodies (12 and 8 steps) cost 5 us of instruction fetch on the first pages of a call,
-  // shorter ones expose shared-memory latency (batch 128, 32,768 tokens: 1,089 us; with single promoted steps 1,107, with
-  // single steps throughout 1,116, with two of P.V 1,077, though with fp16 scales beside bf16 1,536 instead of 1,524).
-  static constexpr int kPromUnroll = 4, kQkUnroll = 4, kPvUnroll = 1;
+  // Unrolling, for whole pages: longer bodies cost instruction fetch on the first pages of a call, shorter ones expose
+  // shared-memory latency.  Batch 128, 32,768 tokens: 1,026 us; with two promoted steps 1,042, with two or six of the other
+  // logits' 1,035 and 1,037, with two of P.V 1,027.  fp16 scales beside bf16, 32 x 8,192 tokens: two of the other logits' steps
+  // 112.3 us, four 114.5.
+  static constexpr int kPromUnroll = 4, kQkUnroll = DT == OUT ? 4 : 2, kPvUnroll = 1;
   CodeConsts<DT> cc;
   const dartkv_cache_desc& d;
   const uint8_t* q_thread;   // this thread's column of the query: + 32 * channel
