@@ -28,7 +28,7 @@ CODE_DTYPE = {v: k for k, v in DTYPE_CODE.items()}
 EXPORTS = (
     "dartkv_last_error", "dartkv_version", "dartkv_launch_count", "dartkv_pack", "dartkv_unpack", "dartkv_quantize", "dartkv_dequantize",
     "dartkv_channel_scores", "dartkv_select_channels", "dartkv_promote_channels", "dartkv_quantize_key_mixed", "dartkv_dequantize_key_mixed",
-    "dartkv_cache_geometry", "dartkv_cache_append", "dartkv_cache_materialize", "dartkv_cache_materialize_both", "dartkv_decode_workspace_bytes",
+    "dartkv_cache_geometry", "dartkv_cache_clear", "dartkv_cache_append", "dartkv_cache_materialize", "dartkv_cache_materialize_both", "dartkv_decode_workspace_bytes",
     "dartkv_decode_attention", "dartkv_decode_plan", "dartkv_decode_plan_rows", "dartkv_decode_status", "dartkv_builtin_scratch_bytes",
     "dartkv_decode_attention_builtin_scratch", "dartkv_shard_range", "dartkv_decode_split_override",
     "dartkv_lifecycle_plan", "dartkv_cache_append_step", "dartkv_decode_attention_scatter",
@@ -132,6 +132,7 @@ def _load() -> ctypes.CDLL:
     lib.dartkv_quantize_key_mixed.argtypes = [p, i32, i64, i64, i64, i64, i64, i32, p, i32, i32, p, p, p, p, p, p]
     lib.dartkv_dequantize_key_mixed.argtypes = [p, p, p, p, p, i32, i64, i64, i64, i32, i32, i32, p, i32, p]
     lib.dartkv_cache_geometry.argtypes = [POINTER(CacheDesc)]
+    lib.dartkv_cache_clear.argtypes = [POINTER(CacheDesc), p, p]
     lib.dartkv_cache_append.argtypes = [POINTER(CacheDesc), POINTER(AppendPlan), p, p, i64, i64, i64, p, p, p]
     lib.dartkv_cache_materialize.argtypes = [POINTER(CacheDesc), i32, c_int32, c_int32, i32, p, i32, p]
     lib.dartkv_cache_materialize_both.argtypes = [POINTER(CacheDesc), c_int32, c_int32, i32, p, p, i32, p]

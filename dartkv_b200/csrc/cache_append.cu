@@ -7,6 +7,21 @@
 
 static inline int align16(int v) { return (v + 15) & ~15; }
 
+// One warp: a memset in its place is not followed as closely by the append (bulk append of [16,8,4096,128] with its new cache
+// 74.1 us, this 72.0; B200).
+__global__ void clear_state_kernel(int32_t* state, int32_t* nonfinite) {
+  wait_previous();
+  state[threadIdx.x] = 0;
+  if (threadIdx.x == 0 && nonfinite) *nonfinite = 0;
+}
+
+extern "C" int dartkv_cache_clear(const dartkv_cache_desc* d, int32_t* nonfinite, void* stream) {
+  DARTKV_REQUIRE(d != nullptr && d->state != nullptr, "cache_clear received a null pointer");
+  DARTKV_CUDA_OK(launch_following(clear_state_kernel, 1, 32, 0, (cudaStream_t)stream, d->state, nonfinite));
+  DARTKV_LAUNCH_OK("clear_state_kernel");
+  return DARTKV_OK;
+}
+
 extern "C" int dartkv_cache_geometry(dartkv_cache_desc* d) {
   DARTKV_REQUIRE(d != nullptr, "null descriptor");
   DARTKV_REQUIRE(d->batch > 0 && d->kv_heads > 0 && d->head_dim > 0, "batch, kv_heads and head_dim must be positive");

@@ -163,7 +163,7 @@ struct Block {
 
 // allocate(desc, device_index, key_pages, value_rows): the pools of a new cache, in the order of `kPoolNames` on the
 // Python side, with the descriptor's pointers set; None when the device is not the current one.  Only the state words
-// and the finite-input flag start at zero (one memset for both); everything else is written before it is read.  Pools that
+// and the finite-input flag start at zero (one launch for both); everything else is written before it is read.  Pools that
 // never grow share one allocation, and so do those of the values, which grow together: an allocation of each pool's own and a
 // fill kernel take 20.6 us of host time, this 8.3.
 PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -193,13 +193,6 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
         fixed.view(state, {32}, at::kInt), fixed.view(nonfinite, {1}, at::kInt),
         at::empty({b, h, pages, d->key_page_bytes}, bytes), table.view(start, {pages}, at::kInt), table.view(tokens, {pages}, at::kInt),
         values.view(codes, {b, h, rows, d->value_row_bytes}, at::kByte), values.view(meta, {b, h, rows, 2, d->value_groups}, md)};
-    // from the state words to the end of the flag behind them
-    const cudaError_t err = cudaMemsetAsync(pools[4].data_ptr(), 0, (size_t)(nonfinite - state) + sizeof(int32_t),
-                                            (cudaStream_t)stream_of(pools[4]));
-    if (err != cudaSuccess) {
-      PyErr_Format(PyExc_RuntimeError, "CUDA error while clearing a new cache's state: %s", cudaGetErrorString(err));
-      return nullptr;
-    }
     d->k_sink = pools[0].data_ptr(); d->v_sink = pools[1].data_ptr();
     d->k_ring = pools[2].data_ptr(); d->v_ring = pools[3].data_ptr();
     d->state = (int32_t*)pools[4].data_ptr();
@@ -207,6 +200,7 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
     d->page_start = (int32_t*)pools[7].data_ptr(); d->page_tokens = (int32_t*)pools[8].data_ptr();
     d->v_codes = (uint8_t*)pools[9].data_ptr(); d->v_meta = pools[10].data_ptr();
     d->max_key_pages = (int32_t)pages; d->max_value_tokens = (int32_t)rows;
+    if (dartkv_cache_clear(d, (int32_t*)pools[5].data_ptr(), stream_of(pools[4])) != 0) Py_RETURN_NONE;   // Python allocates again, or raises
     constexpr int kPools = sizeof(pools) / sizeof(pools[0]);
     PyObject* out = PyTuple_New(kPools);
     if (!out) return nullptr;

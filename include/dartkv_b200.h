@@ -144,6 +144,8 @@ typedef struct dartkv_cache_desc {
 
 /* Fill the byte-geometry fields from the configuration fields. */
 int dartkv_cache_geometry(dartkv_cache_desc* desc);
+/* Clears a new cache's 32 state words and its finite-input flag (may be NULL), on the stream. */
+int dartkv_cache_clear(const dartkv_cache_desc* desc, int32_t* nonfinite, void* stream);
 
 /* One append step, planned on the host (the lifecycle rules of src/dart/cache.py:168-190,403-470
  * are integer bookkeeping) and executed by the device: tokens [chunk_start, chunk_start+chunk_tokens)
