@@ -21,13 +21,17 @@
 //   * the probabilities travel as a high and a low 16-bit part: side by side in the eight columns with up to four
 //     query rows (columns 4..7 repeat rows 0..3, so the same lane sees both), in MMAs of their own with more.
 //   * the two warps of a pair share a staged page and split its tokens; nothing is exchanged between them.
+//   * uniform pages take the channels in their order: the query rows wait as MMA operands, code addresses are constants, and a
+//     table entry holds the parameters of both channel pairs of a k-step (64.9 us, with the promoted pages' row offsets in the
+//     table, to 61.3 at the size below; two steps unrolled, four 63.5).  Value parameters of groups of 64 in one wide load and a
+//     select instead of four narrow ones: 62.3, the registers run out.
 // Staging is by bulk copies on mbarriers, keys and values separately: with one buffer each (4-bit pages) the next
 // page's keys arrive during P.V and its values during the logits, two blocks per SM stay resident.
 //
-// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 70 us here (the query
-// rows in M instead of N needed 64 + 32 accumulators and spilled: 88 us).  Two query tokens on batch 8, 4,096 tokens,
+// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 61 us here (the query
+// rows in M instead of N needed 64 + 32 accumulators and spilled).  Two query tokens on batch 8, 4,096 tokens,
 // 2-bit: 69 us as two passes of decode_fast.cu, 44 us here in one launch.  One
-// query token on the 2-bit pages of decode_fast.cu stays there: 1,089 us against 1,462 us at batch 128, 32,768 tokens.
+// query token on the 2-bit pages of decode_fast.cu stays there: 1,026 us against 1,462 us at batch 128, 32,768 tokens.
 
 #include <atomic>
 
@@ -93,7 +97,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
   extern __shared__ __align__(128) uint8_t smem_raw[];
   wait_previous();
   RowsSmem<R>& bs = *reinterpret_cast<RowsSmem<R>*>(smem_raw);
-  uint8_t* q_table = smem_raw + (sizeof(RowsSmem<R>) + 127) / 128 * 128;   // [channel] rows of w.key_row bytes: 8 columns
+  uint8_t* q_table = smem_raw + (sizeof(RowsSmem<R>) + 127) / 128 * 128;   // [channel] rows of w.key_row bytes: 8 columns; uniform pages: [k-step][lane] operands
   uint8_t* pair_base = q_table + 128 * w.key_row;
   float* warp_out = reinterpret_cast<float*>(pair_base);   // merge buffer: aliases the staging memory
 
@@ -155,7 +159,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
     mbar_fence_init();
   }
   __syncthreads();
-  const int K = w.key_kind == 22 ? d.promoted : 0;
+  const bool uniform = w.key_kind != 22;
+  const int K = uniform ? 0 : d.promoted;
   const int prom_steps = (K + 15) >> 4;
   const float scale2 = a.scale * kLog2e;
   const int vgroup = (16 * g) / d.value_group;
@@ -193,7 +198,9 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
       const int col = i >> 7, ch = i & 127, r = R == 4 ? col & 3 : col;
       uint16_t v = 0;
       if (r < rows) v = reinterpret_cast<const uint16_t*>(a.q)[(first_row + r) * 128 + ch];
-      *reinterpret_cast<uint16_t*>(q_table + ch * w.key_row + 2 * col) = v;
+      // uniform pages: a lane's operand of a k-step as it goes into the MMA
+      const int at = uniform ? 8 * (32 * (ch >> 4) + 4 * col + (ch & 3)) + 2 * ((ch >> 2) & 3) : ch * w.key_row + 2 * col;
+      *reinterpret_cast<uint16_t*>(q_table + at) = v;
     }
     __syncthreads();
 
@@ -239,14 +246,21 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
           if (!((flags >> (8 * i)) & 1u)) order[min(pos++, 127)] = (uint8_t)(4 * lane + i);
         __syncwarp();
       }
+      auto param = [&](int off, int c0, int c1) { return prmt(lds_u16(blob + off + 2 * c0), lds_u16(blob + off + 2 * c1), 0x5410u); };
+      if (uniform) {
+        // channels in their order: one entry holds both pairs of a k-step and lane of a quad
+        const int ch = 16 * (lane >> 2) + c;
+        table[lane] = make_uint4(param(d.key_off_scale, ch, ch + 4), param(d.key_off_zero, ch, ch + 4),
+                                 param(d.key_off_scale, ch + 8, ch + 12), param(d.key_off_zero, ch + 8, ch + 12));
+      } else {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int f = lane + 32 * i;
-        const int p0 = 16 * (f >> 3) + 8 * ((f >> 2) & 1) + (f & 3);
-        const int ch0 = K > 0 ? order[p0] : p0, ch1 = K > 0 ? order[p0 + 4] : p0 + 4;
-        const uint32_t ss = prmt(lds_u16(blob + d.key_off_scale + 2 * ch0), lds_u16(blob + d.key_off_scale + 2 * ch1), 0x5410u);
-        const uint32_t zz = prmt(lds_u16(blob + d.key_off_zero + 2 * ch0), lds_u16(blob + d.key_off_zero + 2 * ch1), 0x5410u);
-        table[f] = make_uint4(ss, zz, (uint32_t)(ch0 * w.key_row), (uint32_t)(ch1 * w.key_row));
+        for (int i = 0; i < 2; ++i) {
+          const int f = lane + 32 * i;
+          const int p0 = 16 * (f >> 3) + 8 * ((f >> 2) & 1) + (f & 3);
+          const int ch0 = order[p0], ch1 = order[p0 + 4];
+          table[f] = make_uint4(param(d.key_off_scale, ch0, ch1), param(d.key_off_zero, ch0, ch1), (uint32_t)(ch0 * w.key_row),
+                                (uint32_t)(ch1 * w.key_row));
+        }
       }
       __syncwarp();
 
@@ -256,28 +270,46 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
       for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) s_acc[mt][i] = 0.0f;
-      auto multiply = [&](const uint4& ea, const uint4& eb, const uint32_t (&ra)[8], const uint32_t (&rb)[8]) {
-        const uint32_t b0 = prmt(lds_u16(q_thread + ea.z), lds_u16(q_thread + ea.w), 0x5410u);
-        const uint32_t b1 = prmt(lds_u16(q_thread + eb.z), lds_u16(q_thread + eb.w), 0x5410u);
+      auto products = [&](const uint32_t (&ra)[8], const uint32_t (&rb)[8], uint32_t b0, uint32_t b1) {
 #pragma unroll
         for (int mt = 0; mt < 4; ++mt) HO::mma(s_acc[mt], ra[2 * mt], ra[2 * mt + 1], rb[2 * mt], rb[2 * mt + 1], b0, b1);
       };
+      auto multiply = [&](const uint4& ea, const uint4& eb, const uint32_t (&ra)[8], const uint32_t (&rb)[8]) {
+        products(ra, rb, prmt(lds_u16(q_thread + ea.z), lds_u16(q_thread + ea.w), 0x5410u),
+                 prmt(lds_u16(q_thread + eb.z), lds_u16(q_thread + eb.w), 0x5410u));
+      };
+      const uint2* const q_ready = reinterpret_cast<const uint2*>(q_table) + lane;
       if (w.key_kind == 4) {
-        const uint8_t* codes = blob + 8 * g + 4 * hf;
+        const uint8_t* codes = blob + 64 * c + 8 * g + 4 * hf;
 #pragma unroll 2
-        for (int i = 0; i < 8; ++i) {
-          const uint4 ea = table[8 * i + c], eb = table[8 * i + 4 + c];
+        for (int i = 0; i < 8; ++i, codes += 16 * 64) {
+          const uint4 e = table[4 * i + c];
+          const uint2 q = q_ready[32 * i];
           uint32_t ra[8], rb[8];
           Affine aff;
-          aff.template init<1>(ea.x, ea.y);
-          uint32_t w0 = lds_u32(codes + ea.z), w1 = lds_u32(codes + ea.w);
+          aff.template init<1>(e.x, e.y);
+          uint32_t w0 = lds_u32(codes), w1 = lds_u32(codes + 4 * 64);
           restore_codes4<MD, DT, FP32>(cc, mask4, prmt(w0, w1, 0x5410u), aff, ra);
           restore_codes4<MD, DT, FP32>(cc, mask4, prmt(w0, w1, 0x7632u), aff, ra + 4);
-          aff.template init<1>(eb.x, eb.y);
-          w0 = lds_u32(codes + eb.z); w1 = lds_u32(codes + eb.w);
+          aff.template init<1>(e.z, e.w);
+          w0 = lds_u32(codes + 8 * 64); w1 = lds_u32(codes + 12 * 64);
           restore_codes4<MD, DT, FP32>(cc, mask4, prmt(w0, w1, 0x5410u), aff, rb);
           restore_codes4<MD, DT, FP32>(cc, mask4, prmt(w0, w1, 0x7632u), aff, rb + 4);
-          multiply(ea, eb, ra, rb);
+          products(ra, rb, q.x, q.y);
+        }
+      } else if (w.key_kind == 2) {
+        const uint8_t* codes = blob + 32 * c + 4 * g + 2 * hf;
+#pragma unroll 2
+        for (int i = 0; i < 8; ++i, codes += 16 * 32) {
+          const uint4 e = table[4 * i + c];
+          const uint2 q = q_ready[32 * i];
+          uint32_t ra[8], rb[8];
+          Affine aff;
+          aff.template init<3>(e.x, e.y);
+          restore_codes2<MD, DT, FP32>(cc, prmt(lds_u16(codes), lds_u16(codes + 4 * 32), 0x5410u), aff, ra);
+          aff.template init<3>(e.z, e.w);
+          restore_codes2<MD, DT, FP32>(cc, prmt(lds_u16(codes + 8 * 32), lds_u16(codes + 12 * 32), 0x5410u), aff, rb);
+          products(ra, rb, q.x, q.y);
         }
       } else {
         const uint8_t* codes = blob + 4 * g + 2 * hf;
