@@ -18,7 +18,8 @@
 // operand register, address arithmetic, shifts; packed 16-bit arithmetic: two per register), and four warps per scheduler to
 // keep them so.  Batch 128, 32,768 tokens: 1,144 us with two warps per page that split the logits by channels, the rest by
 // tokens, and met twice per page; 1,089 us with a warp per page, which fills one table instead of two and exchanges nothing
-// (B200; the instructions of a launch went from 3,340 to 3,287 per page).
+// (B200; the instructions of a launch went from 3,340 to 3,287 per page); 1,026 us now (states merged beside the next row's
+// pages, shorter dense blocks, half-register operands).
 // Algorithmic HBM bytes per page and (batch, kv head): 10880.
 
 #include <atomic>
