@@ -1057,8 +1057,11 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   const int64_t rows = (int64_t)d->batch * query_heads * L.total_splits;
   DARTKV_REQUIRE(workspace_bytes >= layout_bytes(d, query_heads, L), "decode workspace too small: need %lld bytes",
                  (long long)layout_bytes(d, query_heads, L));
+  DARTKV_REQUIRE((uintptr_t)workspace % 4 == 0, "the decode workspace must be 4-byte aligned");
+  // The status word and the counter of finished blocks, then the partials, which move two floats at a time: from a multiple of eight
+  // bytes on, wherever the workspace begins.
   int* status = reinterpret_cast<int*>(workspace);
-  float* part_m = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 16);
+  float* part_m = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 16 - (uintptr_t)workspace % 8);
   float* part_l = part_m + rows;
   float* part_acc = part_l + rows;
   const int bh = d->batch * d->kv_heads;
@@ -1122,7 +1125,7 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
   {
     const bool few = L.total_splits <= kFewSplits;
     // few slots a row of a tensor-core layout (128 channels, 16 bits): a warp per row, which moves four channels at a time
-    if (L.fast && L.total_splits <= kRowSlots && !peers && (uintptr_t)out % 8 == 0 && (uintptr_t)part_acc % 8 == 0 &&
+    if (L.fast && L.total_splits <= kRowSlots && !peers && (uintptr_t)out % 8 == 0 &&
         rows / L.total_splits < (1ll << 31)) {
       const int out_rows = (int)(rows / L.total_splits);
       DARTKV_CUDA_OK(launch_following(decode_merge_rows_kernel, dim3((out_rows + 7) / 8), dim3(256), 0, stream, part_m, part_l, part_acc,

@@ -398,7 +398,7 @@ __device__ __forceinline__ void block_merge(const FastArgs& a, const BS& bs, con
       a.part_m[row] = merge_maximum(m == -INFINITY ? -INFINITY : m * 0.6931471805599453f, l);
       a.part_l[row] = l;
     }
-    *reinterpret_cast<float2*>(a.part_acc + row * 128 + ch) = make_float2(acc0, acc1);   // 8-byte aligned like the scratch
+    *reinterpret_cast<float2*>(a.part_acc + row * 128 + ch) = make_float2(acc0, acc1);   // the partials begin at a multiple of eight bytes
   }
 }
 

@@ -219,7 +219,7 @@ int dartkv_cache_materialize_both(const dartkv_cache_desc* desc, int32_t t0, int
  * query/out [B,Hq,D] (q_dtype, contiguous; the query 4-byte aligned where a tensor-core kernel serves the call,
  * else -1 is returned).
  * workspace: split-K scratch of at least dartkv_decode_workspace_bytes(desc, Hq, max_tokens) bytes
- * for any call with tokens <= max_tokens; zero it once after allocating (its first word is a status
+ * for any call with tokens <= max_tokens, 4-byte aligned (else -1 is returned); zero it once after allocating (its first word is a status
  * word that a kernel sets if a bounded wait on an async copy ran out).
  * tokens: tokens currently in the cache (sizes the split grid; the kernels read the exact count and
  * the page metadata from desc->state on the device). */

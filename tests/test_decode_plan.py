@@ -134,6 +134,15 @@ def test_a_query_from_an_odd_element_on_is_refused_before_any_launch(kwargs, fla
         assert call(*args) == _lib.EINVAL and "aligned" in _lib.last_error()
 
 
+@pytest.mark.parametrize("query_heads,dtype", [(4, _lib.BF16), (4, _lib.F32)])
+def test_a_workspace_from_an_odd_byte_on_is_refused_before_any_launch(query_heads, dtype):
+    d = make_desc(1, 1, dtype=dtype)
+    for offset in (1, 2, 3, 6):
+        assert LIB.dartkv_decode_attention(ctypes.byref(d), 0x20000000, dtype, query_heads, 0.1, _lib.DEQUANT_PER_OP, 5000,
+                                           0x30000000 + offset, 1 << 40, 0x40000000, None) == _lib.EINVAL
+        assert "workspace" in _lib.last_error()
+
+
 def test_the_scratch_of_a_class_of_widths_serves_every_width_in_it():
     # calls of 5..8, 9..16, ... query heads per KV head share the buffer of the widest
     for kwargs in (dict(), dict(value_bits=4, key_bits=4, promoted=0), dict(value_group=32), dict(dtype=_lib.F32)):
