@@ -743,11 +743,11 @@ __global__ void __launch_bounds__(256) decode_merge_rows_kernel(const float* __r
 struct DecodeLayout {
   int generic_splits, generic_chunk;   // generic kernel over the whole range (fallback)
   int fast;                            // tensor-core kernel for the packed pages: 1 per-op rounded, 2 unrounded fp32
-  int quads, stream_blocks;            // tensor-core layouts: four-page units per (batch, kv head), stream blocks
-  long long units;
-  int unit_pages, row_units;           // pages of the units that are dealt out, four or eight, and such units per row
+  int quads, stream_blocks;            // tensor-core layouts: units per work row, stream blocks
+  long long units;                     // of all work rows: (batch, kv head, group of the head's query rows)
+  int unit_pages;                      // pages of a unit, four or eight
   int total_splits;
-  int row_groups;                      // layout 4: groups of up to eight query rows per KV head
+  int row_groups;                      // layout 4: groups of the query rows of a KV head, else 1
   int pieces;                          // large calls of more than eight rows (decode_many.cu): blocks per work row, else 0
 };
 
@@ -844,8 +844,6 @@ static void two_bit_split(DecodeLayout& L, int bh, int pages, int resident, cons
     const double cost = by_waves > by_work ? by_waves : by_work;
     if (cost < best_cost - 1e-9) { best_cost = cost; best_pieces = pieces; }
   }
-  L.unit_pages = 4;
-  L.row_units = L.quads;
   L.stream_blocks = bh * best_pieces;
   L.total_splits = best_pieces + 1;
   const int octs = (pages + 7) / 8;
@@ -860,11 +858,11 @@ static void two_bit_split(DecodeLayout& L, int bh, int pages, int resident, cons
   const double cost = kAcross * (share * (blocks <= sms ? kAlone : 1.0) + kRow * (share / octs + 1.0) + (double)bh * kDense / resident);
   if (cost >= best_cost && !force_unaligned) return;
   L.unit_pages = 8;
-  L.row_units = octs;
+  L.quads = octs;
+  L.units = units;
   L.stream_blocks = (int)blocks;
-  // slots of a row: the blocks that touch it, counted in the units that are dealt out and in those of four pages that a plan reports
-  const long long w8 = units / blocks, w4 = max(1ll, L.units / blocks);
-  L.total_splits = (int)max((octs + w8 - 2) / w8, (L.quads + w4 - 2) / w4) + 2;
+  const long long w = units / blocks;   // smallest share of a block
+  L.total_splits = (int)((octs + w - 2) / w + 1) + 1;
 }
 
 // rows_call: the call came through dartkv_decode_attention_rows, the only one that runs more than four query rows per
@@ -912,11 +910,13 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
       // 8 x 4,096 (768) 62.9 and 41.1; 9 rows, 2 x 4,096 (256) 20.8 and 18.5, 8 x 1,100 (256) 22.5 and 17.5.  With two eights of
       // rows and as many blocks per KV head as a row has slots for, 1 x 16,384 tokens take 23.5 and 27.9.
       const int groups = dartkv_decode_many_groups(rep), pieces = dartkv_decode_many_pieces(d, rep, pages);
-      const long long blocks = (long long)d->batch * d->kv_heads * groups * pieces;
+      const long long work_rows = (long long)d->batch * d->kv_heads * groups, blocks = work_rows * pieces;
       if (10 * blocks * L.row_groups >= 17 * dartkv_sm_count() && (L.row_groups > 2 || pieces < 15)) {
         L.pieces = pieces;
+        L.row_groups = groups;
+        L.units = work_rows * L.quads;
         L.stream_blocks = (int)blocks;
-        L.total_splits = pieces + (groups > 1 ? 2 : 1);   // the plan counts in eights of rows, which may lie across two blocks more
+        L.total_splits = pieces + 1;
         return L;
       }
     }
@@ -1017,6 +1017,8 @@ static int decode_plan_impl(const dartkv_cache_desc* d, int q_dtype, int query_h
   out->units = L.fast ? L.units : 0;
   out->generic_splits = L.fast ? 0 : L.generic_splits;
   out->generic_chunk = L.fast ? 0 : L.generic_chunk;
+  out->unit_pages = L.fast && !L.pieces ? L.unit_pages : 0;
+  out->row_groups = L.fast ? L.row_groups : 0;
   return DARTKV_OK;
 }
 
@@ -1070,17 +1072,11 @@ static int decode_attention_impl(const dartkv_cache_desc* d, const void* query, 
     int rc = dartkv_decode_many_launch(d, query, query_heads, scale, L.pieces, L.total_splits, part_m, part_l, part_acc, status, row_start,
                                        stream);
     if (rc) return rc;
-    L.row_groups = dartkv_decode_many_groups(rep);   // the merge finds a row's slots from the work rows
-    L.units = (long long)bh * L.row_groups * L.quads;
   } else if (L.fast == 4) {
     int rc = dartkv_decode_rows_launch(d, query, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units, L.total_splits, part_m,
                                        part_l, part_acc, status, row_start, stream);
     if (rc) return rc;
   } else if (L.fast) {
-    if (L.unit_pages == 8) {   // what kernel and merge find a row's blocks from
-      L.quads = L.row_units;
-      L.units = (long long)bh * L.row_units;
-    }
     int rc = L.fast == 3 ? dartkv_decode_wide_launch(d, query, q_dtype, query_heads, scale, flavour, L.quads, L.stream_blocks, L.units,
                                                      L.total_splits, part_m, part_l, part_acc, status, row_start, stream)
                          : (L.fast == 2 ? dartkv_decode_fused32_launch : dartkv_decode_fast_launch)(

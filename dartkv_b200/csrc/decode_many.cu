@@ -585,7 +585,7 @@ int dartkv_decode_many_pieces(const dartkv_cache_desc* d, int rep, int pages) {
   const int quads = (pages + 3) / 4;
   int best = 1;
   double best_cost = 1e30;
-  for (int pieces = 1; pieces <= (w.groups > 1 ? 15 : 16) && pieces <= quads; ++pieces) {
+  for (int pieces = 1; pieces <= 16 && pieces <= quads; ++pieces) {
     const double share = (pages + 1 + pieces - 1) / pieces + 2.0;
     const double cost = share * ((rows * pieces + resident - 1) / resident);
     if (cost < best_cost - 1e-9) { best_cost = cost; best = pieces; }

@@ -26,7 +26,7 @@ void dartkv_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed);
 extern "C" long long dartkv_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 extern "C" const char* dartkv_last_error(void) { return g_error; }
-extern "C" int dartkv_version(void) { return 110; }
+extern "C" int dartkv_version(void) { return 111; }
 
 // ---------------------------------------------------------------------------- sharding rule (host arithmetic)
 // Every (batch row, KV head) is independent on this path, so ranks own rectangles of rows x heads.  The batch is

@@ -231,19 +231,21 @@ int dartkv_decode_attention(const dartkv_cache_desc* desc, const void* query, in
  * the reference: it exists so that integrators and tests can see the plan).  kernel: 0 generic, 1 tensor-core
  * per-op flavour (2-bit pages), 2 tensor-core unrounded flavour (2-bit pages), 3 tensor-core kernels for every
  * other packed geometry and the fp32 flavour, 4 (dartkv_decode_plan_rows only) tensor-core kernel for more than four
- * query rows per KV head.  On the tensor-core layouts one unit is four consecutive pages of a row, i.e. of a
- * (batch, kv head), under kernel 4 of one of the ceil(rows per KV head / 8) groups of its query rows; block j of `stream_blocks`
- * owns units [j*units/stream_blocks, (j+1)*units/stream_blocks) and every row is touched by at most total_splits - 1 of them (plus
- * its dense-token block).  Under kernel 4 with more than eight rows per KV head a block works for all of them (32 at most), on an
- * even share of the (batch, kv head)'s pages and dense tokens. */
+ * query rows per KV head.  On the tensor-core layouts a work row is a (batch, kv head), under kernel 4 one of `row_groups` groups of
+ * its query rows, and a unit is `unit_pages` consecutive pages of a work row, four or eight; block j of `stream_blocks` owns units
+ * [j*units/stream_blocks, (j+1)*units/stream_blocks) and every work row is touched by at most total_splits - 1 of them (plus its
+ * dense-token block).  Large calls of kernel 4 with more than eight rows per KV head report unit_pages 0: every work row has
+ * stream_blocks / (units / quads) blocks of its own, which take even shares of its pages and of its dense tokens. */
 typedef struct {
   int32_t kernel;
-  int32_t quads;          /* units per row */
+  int32_t quads;          /* units per work row */
   int32_t stream_blocks;
   int32_t total_splits;   /* partial slots per (batch, query head) row of the workspace */
-  int64_t units;          /* rows * quads */
+  int64_t units;          /* work rows * quads */
   int32_t generic_splits; /* generic kernel only */
   int32_t generic_chunk;
+  int32_t unit_pages;
+  int32_t row_groups;
 } dartkv_decode_plan_info;
 int dartkv_decode_plan(const dartkv_cache_desc* desc, int q_dtype, int query_heads, int flavour, int tokens,
                        dartkv_decode_plan_info* out);

@@ -41,8 +41,20 @@ def plan(d, q_dtype, hq, flavour, tokens):
     return info
 
 
-ROWS = [(1, 1), (1, 8), (2, 8), (3, 2), (16, 8), (32, 8), (37, 8), (128, 8), (512, 8)]
-TOKENS = [1, 31, 32, 33, 159, 160, 161, 32 + 4 * 128, 32 + 5 * 128 + 77, 8192, 32768, 131072]
+def pages_of_blocks(info, row, pages):
+    """The pages of a work row that each block works on, as the kernels find them."""
+    parts = []
+    for j in range(info.stream_blocks):
+        begin, end = j * info.units // info.stream_blocks, (j + 1) * info.units // info.stream_blocks
+        begin, end = max(begin - row * info.quads, 0), min(end - row * info.quads, info.quads)
+        if begin < end:
+            parts.append(range(info.unit_pages * begin, min(info.unit_pages * end, pages)))
+    return parts
+
+
+ROWS = [(1, 1), (1, 8), (2, 8), (3, 2), (5, 2), (10, 2), (6, 8), (16, 8), (32, 8), (37, 8), (128, 8), (512, 8)]
+TOKENS = [1, 31, 32, 33, 159, 160, 161, 32 + 4 * 128, 32 + 5 * 128 + 77, 8192, 32 + 116 * 128, 32 + 225 * 128, 32 + 228 * 128, 32768,
+          32 + 289 * 128, 131072]
 
 
 @pytest.mark.parametrize("split", [None, "aligned", "unaligned", "unaligned:7", "unaligned:3"])
@@ -55,7 +67,8 @@ def test_tensor_core_plans_stay_inside_their_partial_slots(flavour, split, decod
         assert info.kernel == (1 if flavour == _lib.DEQUANT_PER_OP else 2)
         rows = batch * heads
         pages = max(1, (tokens - 32) // 128)
-        assert info.quads == (pages + 3) // 4
+        assert info.unit_pages in (4, 8) and info.row_groups == 1
+        assert info.quads == -(-pages // info.unit_pages)
         assert info.units == rows * info.quads
         assert 1 <= info.stream_blocks <= info.units
         assert 2 <= info.total_splits <= 17
@@ -70,8 +83,23 @@ def test_tensor_core_plans_stay_inside_their_partial_slots(flavour, split, decod
             last = block_of_unit(row * info.quads + info.quads - 1, info.stream_blocks, info.units)
             assert edges[first] <= row * info.quads < edges[first + 1]
             assert 1 + (last - first + 1) <= info.total_splits
+        if rows <= 64:
+            for row in range(rows):
+                parts = pages_of_blocks(info, row, pages)
+                assert [p for part in parts for p in part] == list(range(pages)) and 1 + len(parts) <= info.total_splits
         need = 16 + batch * 4 * heads * info.total_splits * (2 + 128) * 4
         assert LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), 4 * heads, tokens) >= need
+
+
+@pytest.mark.parametrize("flavour", [_lib.DEQUANT_PER_OP, _lib.DEQUANT_FUSED])
+def test_slots_are_those_of_the_units_that_are_dealt_out(flavour):
+    # units of eight pages whose shares end inside a row: counted in units of four, 5 x 2 rows of 225 to 228 pages took 21 slots, more
+    # than the merge of tensor-core layouts is made for, and 6 x 8 of 289 to 296 nine, one more than the warp-per-row merge takes
+    for (batch, heads), pages, most in (((5, 2), range(225, 229), 17), ((10, 2), range(225, 229), 17), ((6, 8), range(289, 297), 8)):
+        for n in pages:
+            info = plan(make_desc(batch, heads), _lib.BF16, 4 * heads, flavour, 32 + 128 * n)
+            assert info.total_splits <= most
+            assert all(1 + len(pages_of_blocks(info, row, n)) <= info.total_splits for row in range(batch * heads))
 
 
 def test_other_geometries_take_the_general_tensor_core_kernel():
@@ -172,8 +200,10 @@ def test_many_row_plans_stay_inside_their_partial_slots(split, decode_split):
         for rep in (5, 7, 8, 9, 16, 17, 20, 31, 33, 49, 57, 64):
             assert plan(d, _lib.BF16, rep * heads, _lib.DEQUANT_PER_OP, tokens).kernel == 0      # the ordinary entry point
             check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, rep * heads, _lib.DEQUANT_PER_OP, tokens, ctypes.byref(info)))
-            groups = -(-rep // 8)
-            rows = batch * heads * groups
+            # groups of eight query rows, or of 32 where a block restores a page once for all rows of a group
+            assert info.row_groups == (-(-rep // 8) if info.unit_pages else -(-rep // 32))
+            assert info.unit_pages == 4 or (info.unit_pages == 0 and rep > 8)
+            rows = batch * heads * info.row_groups
             assert info.kernel == 4 and info.quads == ((tokens - 32) // 128 + 3) // 4 and info.units == rows * info.quads
             assert 1 <= info.stream_blocks <= info.units and 2 <= info.total_splits <= 17
             sample = range(rows) if rows <= 64 else (0, 1, rows // 3, rows // 2, rows - 2, rows - 1)
@@ -181,6 +211,9 @@ def test_many_row_plans_stay_inside_their_partial_slots(split, decode_split):
                 first = block_of_unit(row * info.quads, info.stream_blocks, info.units)
                 last = block_of_unit(row * info.quads + info.quads - 1, info.stream_blocks, info.units)
                 assert 1 + (last - first + 1) <= info.total_splits
+                if info.unit_pages == 0:   # blocks of one work row each, as many for every row
+                    assert (first, last) == (row * (info.stream_blocks // rows), (row + 1) * (info.stream_blocks // rows) - 1)
+            assert info.unit_pages == 4 or info.stream_blocks % rows == 0 and info.total_splits == 1 + info.stream_blocks // rows
             need = 16 + batch * rep * heads * info.total_splits * (2 + 128) * 4
             assert LIB.dartkv_decode_workspace_bytes(ctypes.byref(d), rep * heads, tokens) >= need
         # up to four rows, and what the many-row kernel does not take, run as through the ordinary entry point
