@@ -902,7 +902,8 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
-    if (L.fast == 4 && rep > 8) {
+    // (sinks and rings from any multiple of 8 bytes on serve decode_rows.cu, decode_many.cu reads them 16 bytes at a time)
+    if (L.fast == 4 && rep > 8 && ((uintptr_t)d->k_sink | (uintptr_t)d->v_sink | (uintptr_t)d->k_ring | (uintptr_t)d->v_ring) % 16 == 0) {
       // Every block of decode_many.cu works for all rows of a KV head (of a group of up to 32), one page after another: less work,
       // but a longer chain than that of decode_rows.cu's blocks, which take four pages at a time for eight rows.  It pays where its
       // blocks, counted once for every eight rows, come near two per SM.  2-bit, 8 KV heads, before and after (B200): 20 rows,

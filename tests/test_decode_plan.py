@@ -222,3 +222,12 @@ def test_many_row_plans_stay_inside_their_partial_slots(split, decode_split):
             check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, hq, flavour, tokens, ctypes.byref(info)))
             ordinary = plan(d, _lib.BF16, hq, flavour, tokens)
             assert bytes(info) == bytes(ordinary)
+
+
+@pytest.mark.parametrize("pool", ["k_sink", "v_sink", "k_ring", "v_ring"])
+def test_dense_pools_that_sixteen_byte_loads_cannot_read_stay_with_the_narrower_kernel(pool):
+    d, info = make_desc(8, 8), DecodePlanInfo()
+    for offset, unit_pages in ((0, 0), (8, 4), (16, 0)):
+        setattr(d, pool, 0x70000000 + offset)
+        check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, 20 * 8, _lib.DEQUANT_PER_OP, 4096, ctypes.byref(info)))
+        assert info.kernel == 4 and info.unit_pages == unit_pages
