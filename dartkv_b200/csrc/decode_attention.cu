@@ -909,10 +909,13 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
       // blocks, counted once for every eight rows, come near two per SM.  2-bit, 8 KV heads, before and after (B200): 20 rows,
       // 1 x 4,096 tokens (64 blocks, counted 192) 17.0 and 20.8 us, 1 x 8,192 (384) 23.2 and 21.3, 4 x 2,100 (384) 22.8 and 20.1,
       // 8 x 4,096 (768) 62.9 and 41.1; 9 rows, 2 x 4,096 (256) 20.8 and 18.5, 8 x 1,100 (256) 22.5 and 17.5.  With two eights of
-      // rows and as many blocks per KV head as a row has slots for, 1 x 16,384 tokens take 23.5 and 27.9.
+      // rows and as many blocks per KV head as a row has slots for, 1 x 16,384 tokens take 23.5 and 27.9.  Nor does it pay where
+      // decode_rows.cu has room for all of its units and dense blocks at once: 64 rows, 1 x 1,100 tokens (128 units and 128 dense
+      // blocks, 32 blocks here) 14.4 and 21.6, 48 rows, 1 x 2,100 (288 together) 18.4 and 19.2; 2 x 1,100 (384) 22.6 and 19.2.
+      const long long at_once = (long long)bh * min(L.quads, 16) + (long long)d->batch * d->kv_heads * ((rep + 3) / 4);
       const int groups = dartkv_decode_many_groups(rep), pieces = dartkv_decode_many_pieces(d, rep, pages);
       const long long work_rows = (long long)d->batch * d->kv_heads * groups, blocks = work_rows * pieces;
-      if (10 * blocks * L.row_groups >= 17 * dartkv_sm_count() && (L.row_groups > 2 || pieces < 15)) {
+      if (10 * blocks * L.row_groups >= 17 * dartkv_sm_count() && (L.row_groups > 2 || pieces < 15) && at_once > 2 * dartkv_sm_count()) {
         L.pieces = pieces;
         L.row_groups = groups;
         L.units = work_rows * L.quads;

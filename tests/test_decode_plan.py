@@ -231,3 +231,11 @@ def test_dense_pools_that_sixteen_byte_loads_cannot_read_stay_with_the_narrower_
         setattr(d, pool, 0x70000000 + offset)
         check(LIB.dartkv_decode_plan_rows(ctypes.byref(d), _lib.BF16, 20 * 8, _lib.DEQUANT_PER_OP, 4096, ctypes.byref(info)))
         assert info.kernel == 4 and info.unit_pages == unit_pages
+
+
+@pytest.mark.parametrize("batch,rep,tokens,once_for_all", [(1, 64, 1100, False), (1, 48, 2100, False), (2, 48, 1100, True), (1, 64, 2100, True),
+                                                           (8, 20, 4096, True), (1, 20, 4096, False), (8, 9, 1100, True)])
+def test_pages_are_restored_once_for_all_rows_where_that_is_faster(batch, rep, tokens, once_for_all):
+    info = DecodePlanInfo()
+    check(LIB.dartkv_decode_plan_rows(ctypes.byref(make_desc(batch, 8)), _lib.BF16, 8 * rep, _lib.DEQUANT_PER_OP, tokens, ctypes.byref(info)))
+    assert (info.unit_pages == 0) == once_for_all
