@@ -20,7 +20,8 @@ HOST_SOURCE = os.path.join(CSRC, "host_path.cpp")
 HOST_PATH = os.path.join(PACKAGE_DIR, "_dartkv_host.so")
 HOST_STAMP = os.path.join(PACKAGE_DIR, "build", "host_path.stamp")   # what the extension was built against
 SOURCES = ("quantize.cu", "quantize_fast.cu", "cache_append.cu", "append_fast.cu", "materialize.cu", "decode_attention.cu", "decode_fast.cu", "decode_fused32.cu",
-           "decode_wide.cu", "decode_rows.cu", "decode_many.cu")
+           "decode_wide.cu", "decode_rows.cu", "decode_many.cu", "decode_many_bf16.cu", "decode_many_bf16_f16.cu", "decode_many_f16_bf16.cu",
+           "decode_many_f16.cu")
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",

@@ -1,5 +1,5 @@
 // Packed codes of any width to 16-bit numbers, two codes with scales of their own per register: MMA operands (decode_rows.cu,
-// decode_many.cu) and restored keys and values (materialize.cu, quantize_fast.cu).
+// decode_many.cuh) and restored keys and values (materialize.cu, quantize_fast.cu).
 #pragma once
 
 #include "mma_utils.cuh"

@@ -748,7 +748,7 @@ struct DecodeLayout {
   int unit_pages;                      // pages of a unit, four or eight
   int total_splits;
   int row_groups;                      // layout 4: groups of the query rows of a KV head, else 1
-  int pieces;                          // large calls of more than eight rows (decode_many.cu): blocks per work row, else 0
+  int pieces;                          // large calls of more than eight rows (decode_many.cuh): blocks per work row, else 0
 };
 
 int dartkv_decode_fast_supported(const dartkv_cache_desc* d, int q_dtype, int query_heads);
@@ -902,9 +902,9 @@ static DecodeLayout decode_layout(const dartkv_cache_desc* d, int q_dtype, int q
     const int pages = max(1, (tokens - d->sink_tokens) / d->page_size);
     L.quads = (pages + 3) / 4;
     L.units = (long long)bh * L.quads;
-    // (sinks and rings from any multiple of 8 bytes on serve decode_rows.cu, decode_many.cu reads them 16 bytes at a time)
+    // (sinks and rings from any multiple of 8 bytes on serve decode_rows.cu, decode_many.cuh reads them 16 bytes at a time)
     if (L.fast == 4 && rep > 8 && ((uintptr_t)d->k_sink | (uintptr_t)d->v_sink | (uintptr_t)d->k_ring | (uintptr_t)d->v_ring) % 16 == 0) {
-      // Every block of decode_many.cu works for all rows of a KV head (of a group of up to 32), one page after another: less work,
+      // Every block of decode_many.cuh works for all rows of a KV head (of a group of up to 32), one page after another: less work,
       // but a longer chain than that of decode_rows.cu's blocks, which take four pages at a time for eight rows.  It pays where its
       // blocks, counted once for every eight rows, come near two per SM.  2-bit, 8 KV heads, before and after (B200): 20 rows,
       // 1 x 4,096 tokens (64 blocks, counted 192) 17.0 and 20.8 us, 1 x 8,192 (384) 23.2 and 21.3, 4 x 2,100 (384) 22.8 and 20.1,

@@ -3,6 +3,8 @@
 // that handles dense tokens, and the block-level merge of the warps' online-softmax states.
 #pragma once
 
+#include <atomic>
+
 #include "common.cuh"
 #include "mma_utils.cuh"
 
@@ -39,6 +41,23 @@ struct FastArgs {
   // optional [batch] first live token of every batch row (left padding): tokens before it get no weight
   const int32_t* row_start;
   int unit_pages;
+};
+
+// Opt-in to more than 48 KB of shared memory, once per device and kernel, for the kernel that is launched only: every kernel
+// that is touched gets loaded.  Two threads that race on a device's first call both set the attribute, which is harmless.
+template <int KERNELS>
+struct SharedMemoryOptIn {
+  std::atomic<bool> done[64][KERNELS];
+  template <class Kernel>
+  cudaError_t operator()(int index, Kernel kernel, int bytes) {
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    const bool known = device >= 0 && device < 64;
+    if (err != cudaSuccess || (known && done[device][index].load(std::memory_order_acquire))) return err;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (err == cudaSuccess && known) done[device][index].store(true, std::memory_order_release);
+    return err;
+  }
 };
 
 // Calls of the 2-bit kernels whose blocks have one unit each, four pages at most, and an SM each: a warp per page would leave

@@ -4,7 +4,7 @@
 // geometries of decode_wide.cu that fit this description, and calls with more than four query rows per KV head
 // (several query tokens at once, wide GQA groups), which otherwise take one call per four rows.  More than eight rows
 // are split into groups of equal size; a group is a row of work like a (batch, KV head) pair, so all of them run in
-// one launch and find each other's pages in L2.  decode_many.cu takes such calls where they are large.
+// one launch and find each other's pages in L2.  decode_many.cuh takes such calls where they are large.
 //
 // What bounds it: as in decode_fast.cu, the dependent phases of a page (order, table, logits, softmax, P.V) at four warps
 // per scheduler, here with instruction fetch as the largest stall; time moves with the number of instructions (three
