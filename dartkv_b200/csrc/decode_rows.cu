@@ -33,8 +33,6 @@
 // 2-bit: 69 us as two passes of decode_fast.cu, 44 us here in one launch.  One
 // query token on the 2-bit pages of decode_fast.cu stays there: 1,026 us against 1,462 us at batch 128, 32,768 tokens.
 
-#include <atomic>
-
 #include "decode_fast_common.cuh"
 #include "code_pairs.cuh"
 
@@ -88,8 +86,10 @@ __device__ __forceinline__ void rows_merge(const FastArgs& a, const RowsSmem<R>&
   }
 }
 
-// R: most query rows of a group, 4 or 8.
-template <int DT, int MD, bool FP32, int R>
+// R: most query rows of a group, 4 or 8.  UNIFORM: no promoted channels; in one kernel with them the two forms take each other's registers and
+// instruction fetch: promoted 2-bit pages with fp16 metadata beside bf16, eight rows, 16 x 16,384 tokens 166 us, apart 156; 4-bit, four
+// rows, 94.7 and 93.5 (B200).
+template <int DT, int MD, bool FP32, int R, bool UNIFORM>
 __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_desc d, FastArgs a, RowsGeom w) {
   using H = Half2Ops<MD>;
   using HO = Half2Ops<DT>;
@@ -159,8 +159,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
     mbar_fence_init();
   }
   __syncthreads();
-  const bool uniform = w.key_kind != 22;
-  const int K = uniform ? 0 : d.promoted;
+  const int K = UNIFORM ? 0 : d.promoted;
   const int prom_steps = (K + 15) >> 4;
   const float scale2 = a.scale * kLog2e;
   const int vgroup = (16 * g) / d.value_group;
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
       uint16_t v = 0;
       if (r < rows) v = reinterpret_cast<const uint16_t*>(a.q)[(first_row + r) * 128 + ch];
       // uniform pages: a lane's operand of a k-step as it goes into the MMA
-      const int at = uniform ? 8 * (32 * (ch >> 4) + 4 * col + (ch & 3)) + 2 * ((ch >> 2) & 3) : ch * w.key_row + 2 * col;
+      const int at = UNIFORM ? 8 * (32 * (ch >> 4) + 4 * col + (ch & 3)) + 2 * ((ch >> 2) & 3) : ch * w.key_row + 2 * col;
       *reinterpret_cast<uint16_t*>(q_table + at) = v;
     }
     __syncthreads();
@@ -222,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
 
       // ---- contraction order of the channels (promoted slots first), then one entry per channel pair: a k-step is
       // sixteen positions, lane c of a quad takes positions (c, c + 4) and (c + 8, c + 12) of it
-      if (K > 0) {
+      if constexpr (!UNIFORM) {
         reinterpret_cast<uint32_t*>(flag)[lane] = 0;
         __syncwarp();
         const int32_t* idx = reinterpret_cast<const int32_t*>(blob + d.key_off_index);
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
         __syncwarp();
       }
       auto param = [&](int off, int c0, int c1) { return prmt(lds_u16(blob + off + 2 * c0), lds_u16(blob + off + 2 * c1), 0x5410u); };
-      if (uniform) {
+      if constexpr (UNIFORM) {
         // channels in their order: one entry holds both pairs of a k-step and lane of a quad
         const int ch = 16 * (lane >> 2) + c;
         table[lane] = make_uint4(param(d.key_off_scale, ch, ch + 4), param(d.key_off_zero, ch, ch + 4),
@@ -278,8 +277,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
         products(ra, rb, prmt(lds_u16(q_thread + ea.z), lds_u16(q_thread + ea.w), 0x5410u),
                  prmt(lds_u16(q_thread + eb.z), lds_u16(q_thread + eb.w), 0x5410u));
       };
-      const uint2* const q_ready = reinterpret_cast<const uint2*>(q_table) + lane;
-      if (w.key_kind == 4) {
+      if (UNIFORM && w.key_kind == 4) {
+        const uint2* const q_ready = reinterpret_cast<const uint2*>(q_table) + lane;
         const uint8_t* codes = blob + 64 * c + 8 * g + 4 * hf;
 #pragma unroll 2
         for (int i = 0; i < 8; ++i, codes += 16 * 64) {
@@ -297,7 +296,8 @@ __global__ void __launch_bounds__(kThreads, 2) decode_rows_kernel(dartkv_cache_d
           restore_codes4<MD, DT, FP32>(cc, mask4, prmt(w0, w1, 0x7632u), aff, rb + 4);
           products(ra, rb, q.x, q.y);
         }
-      } else if (w.key_kind == 2) {
+      } else if (UNIFORM) {
+        const uint2* const q_ready = reinterpret_cast<const uint2*>(q_table) + lane;
         const uint8_t* codes = blob + 32 * c + 4 * g + 2 * hf;
 #pragma unroll 2
         for (int i = 0; i < 8; ++i, codes += 16 * 32) {
@@ -542,15 +542,16 @@ RowsGeom rows_geometry_for(const dartkv_cache_desc* d, int rows) {
 }
 
 using RowsKernel = void (*)(dartkv_cache_desc, FastArgs, RowsGeom);
-template <int DT, int MD>
+template <int DT, int MD, bool UNIFORM>
 RowsKernel rows_variant_of(bool fp32, int rows) {
-  if (rows == 8) return decode_rows_kernel<DT, MD, false, 8>;
-  return fp32 ? decode_rows_kernel<DT, MD, true, 4> : decode_rows_kernel<DT, MD, false, 4>;
+  if (rows == 8) return decode_rows_kernel<DT, MD, false, 8, UNIFORM>;
+  return fp32 ? decode_rows_kernel<DT, MD, true, 4, UNIFORM> : decode_rows_kernel<DT, MD, false, 4, UNIFORM>;
 }
+template <bool UNIFORM>
 RowsKernel rows_variant(int dtype, int md, bool fp32, int rows) {
   if (dtype == DARTKV_BF16)
-    return md == DARTKV_BF16 ? rows_variant_of<DARTKV_BF16, DARTKV_BF16>(fp32, rows) : rows_variant_of<DARTKV_BF16, DARTKV_F16>(fp32, rows);
-  return md == DARTKV_BF16 ? rows_variant_of<DARTKV_F16, DARTKV_BF16>(fp32, rows) : rows_variant_of<DARTKV_F16, DARTKV_F16>(fp32, rows);
+    return md == DARTKV_BF16 ? rows_variant_of<DARTKV_BF16, DARTKV_BF16, UNIFORM>(fp32, rows) : rows_variant_of<DARTKV_BF16, DARTKV_F16, UNIFORM>(fp32, rows);
+  return md == DARTKV_BF16 ? rows_variant_of<DARTKV_F16, DARTKV_BF16, UNIFORM>(fp32, rows) : rows_variant_of<DARTKV_F16, DARTKV_F16, UNIFORM>(fp32, rows);
 }
 
 }  // namespace
@@ -582,23 +583,13 @@ int dartkv_decode_rows_launch(const dartkv_cache_desc* d, const void* query, int
   RowsGeom w = rows_geometry_for(d, rows);
   w.groups = dartkv_decode_rows_groups(rep);
   w.group_rows = (rep + w.groups - 1) / w.groups;
-  {
-    // the shared-memory opt-in is per device and per kernel: ask once per device
-    static std::atomic<bool> ready[64];
-    int device = 0;
-    DARTKV_CUDA_OK(cudaGetDevice(&device));
-    if (device < 0 || device >= 64 || !ready[device].load(std::memory_order_acquire)) {
-      for (int dt : {DARTKV_BF16, DARTKV_F16})
-        for (int md : {DARTKV_BF16, DARTKV_F16})
-          for (int variant : {0, 4, 8})
-            DARTKV_CUDA_OK(cudaFuncSetAttribute(rows_variant(dt, md, variant == 0, variant ? variant : 4),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, 113 * 1024));
-      if (device >= 0 && device < 64) ready[device].store(true, std::memory_order_release);
-    }
-  }
+  const bool uniform = w.key_kind != 22, fp32 = flavour == DARTKV_DEQUANT_FP32;
+  const RowsKernel kernel = (uniform ? rows_variant<true> : rows_variant<false>)(d->dtype, d->md_dtype, fp32, rows);
+  static SharedMemoryOptIn<4 * 3 * 2> opt_in;
+  DARTKV_CUDA_OK(opt_in((2 * (d->dtype == DARTKV_BF16) + (d->md_dtype == DARTKV_BF16)) * 6 + (rows == 8 ? 2 : fp32 ? 1 : 0) * 2 + uniform, kernel,
+                        113 * 1024));
   dim3 grid(stream_blocks + d->batch * d->kv_heads * ((rep + 3) / 4));
-  DARTKV_CUDA_OK(launch_following(rows_variant(d->dtype, d->md_dtype, flavour == DARTKV_DEQUANT_FP32, rows), grid, kThreads, rows_smem(w,
-                                  rows), stream, *d, a, w));
+  DARTKV_CUDA_OK(launch_following(kernel, grid, kThreads, rows_smem(w, rows), stream, *d, a, w));
   DARTKV_LAUNCH_OK("decode_rows_kernel");
   return DARTKV_OK;
 }
