@@ -44,6 +44,17 @@ long device_argument(PyObject* const* args, Py_ssize_t n, Py_ssize_t at, const a
   return n > at ? PyLong_AsLong(args[at]) : (long)t.device().index();
 }
 
+// A call into the C ABI with the interpreter unlocked: a launch that waits for room in the queue must not stop the other
+// Python threads.
+template <class Call>
+int unlocked(Call call) {
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = call();
+  Py_END_ALLOW_THREADS
+  return rc;
+}
+
 void* stream_of(const at::Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 // append(keys, values, desc, lifecycle_config, lifecycle_state, plan, nonfinite[, device]) -> return code or kSlowPath
@@ -74,15 +85,12 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (k.size(i) == 1) stride[i] = 0;
   }
   if (k.stride(3) != 1 || v.stride(3) != 1) return PyLong_FromLong(kSlowPath);
-  int rc;
   const void *kp = k.data_ptr(), *vp = v.data_ptr();
   void* stream = stream_of(k);
   const int chunk = (int)k.size(2);
-  Py_BEGIN_ALLOW_THREADS
-  rc = dartkv_cache_append_step(desc, cfg, state, kp, vp, chunk, stride[0], stride[1], stride[2], nullptr, nonfinite,
-                                plan, stream);
-  Py_END_ALLOW_THREADS
-  return PyLong_FromLong(rc);
+  return PyLong_FromLong(unlocked([&] {
+    return dartkv_cache_append_step(desc, cfg, state, kp, vp, chunk, stride[0], stride[1], stride[2], nullptr, nonfinite, plan, stream);
+  }));
   END_HANDLE_TH_ERRORS
 }
 
@@ -130,11 +138,10 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const void* qp = dense.defined() ? dense.data_ptr() : q.data_ptr();
   at::Tensor out = at::empty(q.sizes(), q.options().requires_grad(false).memory_format(at::MemoryFormat::Contiguous));
   void* op = out.data_ptr();
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = (rep > 4 ? dartkv_decode_attention_rows : dartkv_decode_attention_padded)(desc, qp, code, (int)query_heads, (float)scale, (int)flavour, (int)tokens, row_start,
-                                      workspace, workspace_bytes, op, stream);
-  Py_END_ALLOW_THREADS
+  const int rc = unlocked([&] {
+    return (rep > 4 ? dartkv_decode_attention_rows : dartkv_decode_attention_padded)(
+        desc, qp, code, (int)query_heads, (float)scale, (int)flavour, (int)tokens, row_start, workspace, workspace_bytes, op, stream);
+  });
   if (rc != 0) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -186,7 +193,9 @@ PyObject* allocate(PyObject*, PyObject* const* args, Py_ssize_t n) {
     d->page_start = (int32_t*)pools[7].data_ptr(); d->page_tokens = (int32_t*)pools[8].data_ptr();
     d->v_codes = (uint8_t*)pools[9].data_ptr(); d->v_meta = pools[10].data_ptr();
     d->max_key_pages = (int32_t)pages; d->max_value_tokens = (int32_t)rows;
-    if (dartkv_cache_clear(d, (int32_t*)pools[5].data_ptr(), stream_of(pools[4])) != 0) Py_RETURN_NONE;   // Python allocates again, or raises
+    auto* flag = (int32_t*)pools[5].data_ptr();
+    void* stream = stream_of(pools[4]);
+    if (unlocked([&] { return dartkv_cache_clear(d, flag, stream); }) != 0) Py_RETURN_NONE;   // Python allocates again, or raises
     constexpr int kPools = sizeof(pools) / sizeof(pools[0]);
     PyObject* out = PyTuple_New(kPools);
     if (!out) return nullptr;
@@ -208,7 +217,8 @@ PyObject* scratch(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   if (bytes < 16 || device != c10::cuda::current_device()) Py_RETURN_NONE;
   at::Tensor buffer = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
-  const cudaError_t err = cudaMemsetAsync(buffer.data_ptr(), 0, 16, (cudaStream_t)stream_of(buffer));
+  void *at = buffer.data_ptr(), *stream = stream_of(buffer);
+  const cudaError_t err = (cudaError_t)unlocked([&] { return (int)cudaMemsetAsync(at, 0, 16, (cudaStream_t)stream); });
   if (err != cudaSuccess) {
     PyErr_Format(PyExc_RuntimeError, "CUDA error while clearing decode scratch: %s", cudaGetErrorString(err));
     return nullptr;
@@ -239,10 +249,7 @@ int32_t* host_flag() {
 // What a call with a finite-input check returns: the tuple, a return code, or False where the input was not finite.
 PyObject* finish(PyObject* tuple, int rc, const int32_t* flag, void* stream) {
   if (rc == 0 && flag) {
-    cudaError_t err;
-    Py_BEGIN_ALLOW_THREADS
-    err = cudaStreamSynchronize((cudaStream_t)stream);
-    Py_END_ALLOW_THREADS
+    const cudaError_t err = (cudaError_t)unlocked([&] { return (int)cudaStreamSynchronize((cudaStream_t)stream); });
     if (err != cudaSuccess) {
       Py_DECREF(tuple);
       PyErr_Format(PyExc_RuntimeError, "CUDA error while waiting for the finite-input check: %s", cudaGetErrorString(err));
@@ -280,8 +287,8 @@ PyObject* get(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (device != c10::cuda::current_device()) Py_RETURN_NONE;
   const auto options = at::TensorOptions().dtype(scalar_type(d->dtype)).device(at::Device(at::kCUDA, (c10::DeviceIndex)device));
   at::Tensor keys = at::empty({d->batch, d->kv_heads, tokens, d->head_dim}, options), values = at::empty(keys.sizes(), options);
-  const int rc = dartkv_cache_materialize_both(d, 0, (int32_t)tokens, DARTKV_DEQUANT_PER_OP, keys.data_ptr(), values.data_ptr(), d->dtype,
-                                               stream_of(keys));
+  void *kp = keys.data_ptr(), *vp = values.data_ptr(), *stream = stream_of(keys);
+  const int rc = unlocked([&] { return dartkv_cache_materialize_both(d, 0, (int32_t)tokens, DARTKV_DEQUANT_PER_OP, kp, vp, d->dtype, stream); });
   if (rc != 0) return PyLong_FromLong(rc);
   return tensors({keys, values});
   END_HANDLE_TH_ERRORS
@@ -322,8 +329,11 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   for (int64_t i = axis + 1; i < dims; ++i) inner *= shape[i];
   const int64_t len = shape[axis];
   at::Tensor out = at::empty(shape, values.options().dtype(scalar_type(code)).requires_grad(false));
-  const int rc = dartkv_dequantize((const uint8_t*)values.data_ptr(), scale.data_ptr(), zero.data_ptr(), md, outer, len, inner, bits, (int)group,
-                                   flavour, out.data_ptr(), code, len * inner, inner, 1, stream_of(values));
+  const void *vp = values.data_ptr(), *sp = scale.data_ptr(), *zp = zero.data_ptr();
+  void *op = out.data_ptr(), *stream = stream_of(values);
+  const int rc = unlocked([&] {
+    return dartkv_dequantize((const uint8_t*)vp, sp, zp, md, outer, len, inner, bits, (int)group, flavour, op, code, len * inner, inner, 1, stream);
+  });
   if (rc != 0) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -349,10 +359,13 @@ PyObject* dequantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Py_RETURN_NONE;
   const int64_t promoted = index.size(-1);
   at::Tensor out = at::empty(shape, low.options().dtype(scalar_type(code)).requires_grad(false));
-  const int rc = dartkv_dequantize_key_mixed((const uint8_t*)low.data_ptr(), promoted ? (const uint8_t*)high.data_ptr() : nullptr,
-                                             promoted ? (const int32_t*)index.data_ptr() : nullptr, scale.data_ptr(), zero.data_ptr(), md,
-                                             shape[0] * shape[1], shape[2], shape[3], (int)group, (int)promoted, flavour, out.data_ptr(), code,
-                                             stream_of(low));
+  const void *lp = low.data_ptr(), *hp = promoted ? high.data_ptr() : nullptr, *ip = promoted ? index.data_ptr() : nullptr;
+  const void *sp = scale.data_ptr(), *zp = zero.data_ptr();
+  void *op = out.data_ptr(), *stream = stream_of(low);
+  const int rc = unlocked([&] {
+    return dartkv_dequantize_key_mixed((const uint8_t*)lp, (const uint8_t*)hp, (const int32_t*)ip, sp, zp, md, shape[0] * shape[1], shape[2], shape[3],
+                                       (int)group, (int)promoted, flavour, op, code, stream);
+  });
   if (rc != 0) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -395,8 +408,11 @@ PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   int32_t* flag = wanted ? host_flag() : nullptr;
   if (wanted && !flag) Py_RETURN_NONE;
   void* stream = stream_of(x);
-  const int rc = dartkv_quantize(x.data_ptr(), code, outer, len, inner, len * inner, inner, 1, bits, (int)group, md, division,
-                                 (uint8_t*)values.data_ptr(), scale.data_ptr(), zero.data_ptr(), flag, stream);
+  const void* xp = x.data_ptr();
+  void *vp = values.data_ptr(), *sp = scale.data_ptr(), *zp = zero.data_ptr();
+  const int rc = unlocked([&] {
+    return dartkv_quantize(xp, code, outer, len, inner, len * inner, inner, 1, bits, (int)group, md, division, (uint8_t*)vp, sp, zp, flag, stream);
+  });
   return finish(tensors({values, scale, zero}), rc, flag, stream);
   END_HANDLE_TH_ERRORS
 }
@@ -424,8 +440,10 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (index.scalar_type() != at::kInt || !dense_here(index)) Py_RETURN_NONE;
   } else {
     index = at::empty({b, h, count}, options.dtype(at::kInt));
+    const void* kp = k.data_ptr();
+    auto* ip = (int32_t*)index.data_ptr();
     auto promote = [&](void* scores) {
-      return dartkv_promote_channels(k.data_ptr(), code, b * h, t, d, t * d, d, (int)count, scores, (int32_t*)index.data_ptr(), stream);
+      return unlocked([&] { return dartkv_promote_channels(kp, code, b * h, t, d, t * d, d, (int)count, scores, ip, stream); });
     };
     rc = promote(nullptr);   // enough where one launch does it
     if (rc == DARTKV_ELIMIT) rc = promote(at::empty({b, h, d}, options).data_ptr());
@@ -438,9 +456,12 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor zero = at::empty({b, h, d, groups}, options.dtype(scalar_type(md)));
   int32_t* flag = wanted ? host_flag() : nullptr;
   if (wanted && !flag) Py_RETURN_NONE;
-  rc = dartkv_quantize_key_mixed(k.data_ptr(), code, b * h, t, d, t * d, d, (int)group,
-                                 promoted ? (const int32_t*)index.data_ptr() : nullptr, (int)promoted, md, (uint8_t*)low.data_ptr(),
-                                 promoted ? (uint8_t*)high.data_ptr() : nullptr, scale.data_ptr(), zero.data_ptr(), flag, stream);
+  const void *kp = k.data_ptr(), *ip = promoted ? index.data_ptr() : nullptr;
+  void *lp = low.data_ptr(), *hp = promoted ? high.data_ptr() : nullptr, *sp = scale.data_ptr(), *zp = zero.data_ptr();
+  rc = unlocked([&] {
+    return dartkv_quantize_key_mixed(kp, code, b * h, t, d, t * d, d, (int)group, (const int32_t*)ip, (int)promoted, md, (uint8_t*)lp, (uint8_t*)hp,
+                                     sp, zp, flag, stream);
+  });
   return finish(tensors({low, high, index, scale, zero}), rc, flag, stream);
   END_HANDLE_TH_ERRORS
 }
