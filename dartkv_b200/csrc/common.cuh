@@ -155,7 +155,7 @@ static inline cudaError_t launch_clusters(int cluster, void (*kernel)(Params...)
   attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
   config.attrs = attributes;
   config.numAttrs = cluster > 0 ? 2 : 1;
-  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, Params(args)...);
+  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
   if (err != cudaSuccess) cudaGetLastError();   // reported by the caller, not left for the next one who asks
   return err;
 }
