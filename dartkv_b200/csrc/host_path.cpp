@@ -44,15 +44,22 @@ long device_argument(PyObject* const* args, Py_ssize_t n, Py_ssize_t at, const a
   return n > at ? PyLong_AsLong(args[at]) : (long)t.device().index();
 }
 
-// A call into the C ABI with the interpreter unlocked: a launch that waits for room in the queue must not stop the other
-// Python threads.
+// The interpreter stays unlocked as long as one of these lives.  Every launch runs so: one that waits for room in the queue must
+// not stop the other Python threads.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
 template <class Call>
-int unlocked(Call call) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = call();
-  Py_END_ALLOW_THREADS
-  return rc;
+auto unlocked(Call call) {
+  const Unlocked scope;
+  return call();
+}
+// the tensor itself where it is contiguous, else a copy
+at::Tensor dense_of(const at::Tensor& t) {
+  if (t.is_contiguous()) return t;
+  const Unlocked scope;
+  return t.detach().contiguous();
 }
 
 void* stream_of(const at::Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
@@ -132,10 +139,9 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     row_start = r.data_ptr<int32_t>();
   }
   // the kernels read the query two channels at a time: a 16-bit view from an odd element on is copied too
-  at::Tensor dense;
-  if (!q.is_contiguous()) dense = q.detach().contiguous();
-  else if ((uintptr_t)q.data_ptr() % 4) dense = q.detach().clone();
-  const void* qp = dense.defined() ? dense.data_ptr() : q.data_ptr();
+  at::Tensor dense = dense_of(q);
+  if ((uintptr_t)dense.data_ptr() % 4) dense = unlocked([&] { return q.detach().clone(); });
+  const void* qp = dense.data_ptr();
   at::Tensor out = at::empty(q.sizes(), q.options().requires_grad(false).memory_format(at::MemoryFormat::Contiguous));
   void* op = out.data_ptr();
   const int rc = unlocked([&] {
@@ -218,7 +224,7 @@ PyObject* scratch(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (bytes < 16 || device != c10::cuda::current_device()) Py_RETURN_NONE;
   at::Tensor buffer = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
   void *at = buffer.data_ptr(), *stream = stream_of(buffer);
-  const cudaError_t err = (cudaError_t)unlocked([&] { return (int)cudaMemsetAsync(at, 0, 16, (cudaStream_t)stream); });
+  const cudaError_t err = unlocked([&] { return cudaMemsetAsync(at, 0, 16, (cudaStream_t)stream); });
   if (err != cudaSuccess) {
     PyErr_Format(PyExc_RuntimeError, "CUDA error while clearing decode scratch: %s", cudaGetErrorString(err));
     return nullptr;
@@ -249,7 +255,7 @@ int32_t* host_flag() {
 // What a call with a finite-input check returns: the tuple, a return code, or False where the input was not finite.
 PyObject* finish(PyObject* tuple, int rc, const int32_t* flag, void* stream) {
   if (rc == 0 && flag) {
-    const cudaError_t err = (cudaError_t)unlocked([&] { return (int)cudaStreamSynchronize((cudaStream_t)stream); });
+    const cudaError_t err = unlocked([&] { return cudaStreamSynchronize((cudaStream_t)stream); });
     if (err != cudaSuccess) {
       Py_DECREF(tuple);
       PyErr_Format(PyExc_RuntimeError, "CUDA error while waiting for the finite-input check: %s", cudaGetErrorString(err));
@@ -273,8 +279,6 @@ PyObject* tensors(std::initializer_list<at::Tensor> list) {
   for (const at::Tensor& t : list) PyTuple_SET_ITEM(out, i++, THPVariable_Wrap(t));
   return out;
 }
-
-bool dense_here(const at::Tensor& t) { return t.is_contiguous() && on_current_device(t); }
 
 // get(desc, tokens, device_index) -> (keys, values): the whole cache materialized; None when the device is not the current one.
 PyObject* get(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -311,7 +315,7 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::SmallVector<int64_t, 6> shape;
   for (int i = 0; i < 3; ++i)
     if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
-  const at::Tensor &values = THPVariable_Unpack(args[0]), &scale = THPVariable_Unpack(args[1]), &zero = THPVariable_Unpack(args[2]);
+  const at::Tensor &values_given = THPVariable_Unpack(args[0]), &scale_given = THPVariable_Unpack(args[1]), &zero_given = THPVariable_Unpack(args[2]);
   if (!shape_of(args[3], shape)) Py_RETURN_NONE;
   int64_t axis = PyLong_AsLongLong(args[4]);
   const int bits = (int)PyLong_AsLong(args[5]);
@@ -320,10 +324,12 @@ PyObject* dequantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   const int64_t dims = (int64_t)shape.size();
   if (axis < 0) axis += dims;
-  const int md = dtype_code(scale.scalar_type());
-  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || zero.scalar_type() != scale.scalar_type() || axis < 0 || axis >= dims ||
-      group < 1 || group > INT32_MAX || values.scalar_type() != at::kByte || !dense_here(values) || !dense_here(scale) || !dense_here(zero))
+  const int md = dtype_code(scale_given.scalar_type());
+  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || zero_given.scalar_type() != scale_given.scalar_type() || axis < 0 || axis >= dims ||
+      group < 1 || group > INT32_MAX || values_given.scalar_type() != at::kByte || !on_current_device(values_given) ||
+      !on_current_device(scale_given) || !on_current_device(zero_given))
     Py_RETURN_NONE;
+  const at::Tensor values = dense_of(values_given), scale = dense_of(scale_given), zero = dense_of(zero_given);
   int64_t outer = 1, inner = 1;
   for (int64_t i = 0; i < axis; ++i) outer *= shape[i];
   for (int64_t i = axis + 1; i < dims; ++i) inner *= shape[i];
@@ -346,17 +352,20 @@ PyObject* dequantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::SmallVector<int64_t, 6> shape;
   for (int i = 0; i < 5; ++i)
     if (!THPVariable_Check(args[i])) Py_RETURN_NONE;
-  const at::Tensor &low = THPVariable_Unpack(args[0]), &high = THPVariable_Unpack(args[1]), &index = THPVariable_Unpack(args[2]),
-                   &scale = THPVariable_Unpack(args[3]), &zero = THPVariable_Unpack(args[4]);
+  const at::Tensor* given[5];
+  for (int i = 0; i < 5; ++i) given[i] = &THPVariable_Unpack(args[i]);
   if (!shape_of(args[5], shape) || shape.size() != 4) Py_RETURN_NONE;
   const int64_t group = PyLong_AsLongLong(args[6]);
   const int flavour = (int)PyLong_AsLong(args[7]), code = (int)PyLong_AsLong(args[8]);
   if (PyErr_Occurred()) return nullptr;
-  const int md = dtype_code(scale.scalar_type());
-  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || zero.scalar_type() != scale.scalar_type() || group < 1 || group > INT32_MAX ||
-      low.scalar_type() != at::kByte || high.scalar_type() != at::kByte || index.scalar_type() != at::kInt || index.dim() < 1 ||
-      !dense_here(low) || !dense_here(high) || !dense_here(index) || !dense_here(scale) || !dense_here(zero))
+  const int md = dtype_code(given[3]->scalar_type());
+  if (code < DARTKV_F32 || code > DARTKV_BF16 || md < 0 || given[4]->scalar_type() != given[3]->scalar_type() || group < 1 || group > INT32_MAX ||
+      given[0]->scalar_type() != at::kByte || given[1]->scalar_type() != at::kByte || given[2]->scalar_type() != at::kInt || given[2]->dim() < 1)
     Py_RETURN_NONE;
+  for (const at::Tensor* t : given)
+    if (!on_current_device(*t)) Py_RETURN_NONE;
+  const at::Tensor low = dense_of(*given[0]), high = dense_of(*given[1]), index = dense_of(*given[2]), scale = dense_of(*given[3]),
+                   zero = dense_of(*given[4]);
   const int64_t promoted = index.size(-1);
   at::Tensor out = at::empty(shape, low.options().dtype(scalar_type(code)).requires_grad(false));
   const void *lp = low.data_ptr(), *hp = promoted ? high.data_ptr() : nullptr, *ip = promoted ? index.data_ptr() : nullptr;
@@ -371,24 +380,26 @@ PyObject* dequantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// quantize(data, bits, group, axis, metadata dtype code (-1: the data's own, or fp32), division, check) -> (values, scale, zero)
+// quantize(data, bits, group, axis, metadata dtype code (-1: the data's own, or fp32), division, check) -> (values, scale, zero);
+// data of any strides, as for the other functional calls: a strided one that came back to Python to be copied there would cross twice
 PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 7) { PyErr_SetString(PyExc_TypeError, "quantize takes 7 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
   for (int i = 1; i < 7; ++i)
     if (!PyLong_Check(args[i])) Py_RETURN_NONE;
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const at::Tensor& given = THPVariable_Unpack(args[0]);
   const int64_t bits_asked = PyLong_AsLongLong(args[1]);
   const int64_t group = PyLong_AsLongLong(args[2]);
   int64_t axis = PyLong_AsLongLong(args[3]);
   int md = (int)PyLong_AsLong(args[4]);
   const int division = (int)PyLong_AsLong(args[5]), wanted = (int)PyLong_AsLong(args[6]);
   if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }   // a number that no C integer holds
-  const int code = dtype_code(x.scalar_type());
-  if (code < 0 || !dense_here(x) || x.numel() == 0 || group < 1 || group > INT32_MAX || md < -1 || division < 0 ||
-      (bits_asked != 2 && bits_asked != 4 && bits_asked != 8) || axis < -x.dim() || axis >= x.dim())
+  const int code = dtype_code(given.scalar_type());
+  if (code < 0 || !on_current_device(given) || given.numel() == 0 || group < 1 || group > INT32_MAX || md < -1 || division < 0 ||
+      (bits_asked != 2 && bits_asked != 4 && bits_asked != 8) || axis < -given.dim() || axis >= given.dim())
     Py_RETURN_NONE;
+  const at::Tensor x = dense_of(given);
   const int bits = (int)bits_asked;
   if (axis < 0) axis += x.dim();
   if (md < 0) md = code;   // fp16 and bf16 keep their own, fp32 data fp32
@@ -418,17 +429,18 @@ PyObject* quantize(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // quantize_mixed(keys, group, promoted count, metadata dtype code, indices | None, check)
-//   -> (low, high, indices, scale, zero); keys [B,H,T,D] contiguous, indices int32 contiguous
+//   -> (low, high, indices, scale, zero); keys [B,H,T,D], indices int32 contiguous
 PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 6) { PyErr_SetString(PyExc_TypeError, "quantize_mixed takes 6 arguments"); return nullptr; }
   if (!THPVariable_Check(args[0])) Py_RETURN_NONE;
-  const at::Tensor& k = THPVariable_Unpack(args[0]);
+  const at::Tensor& given = THPVariable_Unpack(args[0]);
   const int64_t group = PyLong_AsLongLong(args[1]), count = PyLong_AsLongLong(args[2]);
   const int md = (int)PyLong_AsLong(args[3]), wanted = (int)PyLong_AsLong(args[5]);
   if (PyErr_Occurred()) return nullptr;
-  const int code = dtype_code(k.scalar_type());
-  if (code < 0 || !dense_here(k) || k.dim() != 4 || k.numel() == 0 || group > INT32_MAX) Py_RETURN_NONE;
+  const int code = dtype_code(given.scalar_type());
+  if (code < 0 || !on_current_device(given) || given.dim() != 4 || given.numel() == 0 || group > INT32_MAX) Py_RETURN_NONE;
+  const at::Tensor k = dense_of(given);
   const int64_t b = k.size(0), h = k.size(1), t = k.size(2), d = k.size(3), groups = (t + group - 1) / group, packed = (group + 3) / 4;
   const auto options = k.options().requires_grad(false);
   void* stream = stream_of(k);
@@ -437,7 +449,7 @@ PyObject* quantize_mixed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (args[4] != Py_None) {
     if (!THPVariable_Check(args[4])) Py_RETURN_NONE;
     index = THPVariable_Unpack(args[4]);
-    if (index.scalar_type() != at::kInt || !dense_here(index)) Py_RETURN_NONE;
+    if (index.scalar_type() != at::kInt || !index.is_contiguous() || !on_current_device(index)) Py_RETURN_NONE;
   } else {
     index = at::empty({b, h, count}, options.dtype(at::kInt));
     const void* kp = k.data_ptr();

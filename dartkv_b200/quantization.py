@@ -221,9 +221,6 @@ def quantize(
     vpb = 8 // bits
     packed_dim = ((padded_dim + vpb - 1) // vpb) * vpb
     moved_shape = tuple(s for i, s in enumerate(original_shape) if i != axis)
-    made = _lib.HOST.quantize(data, bits, group_size, axis, _lib.DTYPE_CODE[meta_dtype], _DIVISION_CODE[division], int(check_finite))
-    if made is not None:
-        return _quantized(made, data, bits, group_size, axis)
     values = torch.empty((*moved_shape, packed_dim // vpb), dtype=torch.uint8, device=device)
     scale = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)
     zero = torch.empty((*moved_shape, groups), dtype=meta_dtype, device=device)

@@ -1,4 +1,5 @@
-"""Calls that go through the native host path against the same calls in forms that it leaves to Python, and errors that stay what they were."""
+"""Calls that go through the native host path against the same calls with strided tensors and in forms that it leaves to Python, and errors
+that stay what they were."""
 
 import pytest
 import torch
@@ -24,8 +25,11 @@ def test_quantize_and_back(axis, metadata, dtype):
     assert ours.axis == strided.axis == axis % 4 and ours.original_shape == (2, 3, 40, 64) and ours.scale.dtype == (metadata or dtype)
     assert (ours.original_dim, ours.padded_dim, ours.packed_dim, ours.groups) == (strided.original_dim, strided.padded_dim, strided.packed_dim, strided.groups)
     back = ours.dequantize()
-    ours.values = torch.stack((ours.values, ours.values), -1)[..., 0]       # not contiguous: restored through Python
-    assert not ours.values.is_contiguous() and torch.equal(ours.dequantize(), back)
+    for name in ("values", "scale", "zero_point"):
+        setattr(ours, name, torch.stack((getattr(ours, name),) * 2, -1)[..., 0])
+        assert not getattr(ours, name).is_contiguous() and torch.equal(ours.dequantize(), back)
+    ours.original_shape = list(ours.original_shape)                         # not a tuple: restored through Python
+    assert torch.equal(ours.dequantize(), back)
     assert ours.dequantize(dtype=torch.bfloat16).dtype == torch.bfloat16
 
 
@@ -35,8 +39,33 @@ def test_mixed_keys_and_back():
     for name in ("low_values", "high_values", "channel_indices", "scale", "zero_point"):
         assert torch.equal(getattr(ours, name), getattr(strided, name))
     back = ours.dequantize()
-    ours.channel_indices = ours.channel_indices.long()
+    for name in ("low_values", "high_values", "channel_indices", "scale", "zero_point"):
+        setattr(ours, name, torch.stack((getattr(ours, name),) * 2, -1)[..., 0])
+        assert not getattr(ours, name).is_contiguous() and torch.equal(ours.dequantize(), back)
+    ours.channel_indices = ours.channel_indices.long()                      # restored through Python
     assert torch.equal(ours.dequantize(), back)
+
+
+def test_strided_tensors_cross_into_native_code_once(monkeypatch):
+    data = randn(2, 3, 64, 32).transpose(1, 2).contiguous().transpose(1, 2)
+    packed, mixed = dart.quantize(data), dart.quantize_key_mixed(data, group_size=32)
+    packed.values, mixed.low_values = (torch.stack((t, t), -1)[..., 0] for t in (packed.values, mixed.low_values))
+    crossed = []
+
+    class Host:
+        def __getattr__(self, name):
+            def call(*args):
+                crossed.append(name)
+                return getattr(host, name)(*args)
+            return call
+
+    host = dart._lib.HOST
+    monkeypatch.setattr(dart._lib, "HOST", Host())
+    monkeypatch.setattr(dart.quantization, "LIB", None)                     # nothing is left to do through ctypes
+    monkeypatch.setattr(dart.mixed, "LIB", None)
+    for call in (lambda: dart.quantize(data), lambda: dart.quantize_key_mixed(data, group_size=32), packed.dequantize, mixed.dequantize):
+        call()
+    assert crossed == ["quantize", "quantize_mixed", "dequantize", "dequantize_mixed"]
 
 
 @pytest.mark.parametrize("call,error,text", [
