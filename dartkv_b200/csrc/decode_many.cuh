@@ -173,7 +173,6 @@ __global__ void __launch_bounds__(kThreads, 2) decode_many_kernel(const __grid_c
   const float scale2 = a.scale * kLog2e;
   const int K = key2 ? w.promoted : 0;
   bool ok = true;
-  uint32_t parity = 0;
 
   // sixteen codes of a row, in one word, two or four
   auto restore = [&](auto codes, const Affine& affine, uint32_t (&r)[8]) {
@@ -569,19 +568,20 @@ size_t many_smem(const dartkv_cache_desc* d, const ManyGeom& w) {
   return nt <= 2 ? many_smem_of<2>(d, w) : nt == 3 ? many_smem_of<3>(d, w) : many_smem_of<4>(d, w);
 }
 
+// Not for 8-bit values beside 4-bit keys: such pages leave no room for two blocks of decode_rows.cu, whose geometries these are.
 using ManyKernel = void (*)(dartkv_cache_desc, FastArgs, ManyGeom);
 template <int DT, int MD, int NT>
 ManyKernel many_variant_of(int kb, int vb) {
   if (kb == 2) return vb == 2 ? decode_many_kernel<DT, MD, NT, 2, 2> : vb == 4 ? decode_many_kernel<DT, MD, NT, 2, 4> : decode_many_kernel<DT, MD, NT, 2, 8>;
-  return vb == 2 ? decode_many_kernel<DT, MD, NT, 4, 2> : vb == 4 ? decode_many_kernel<DT, MD, NT, 4, 4> : decode_many_kernel<DT, MD, NT, 4, 8>;
+  return vb == 2 ? decode_many_kernel<DT, MD, NT, 4, 2> : decode_many_kernel<DT, MD, NT, 4, 4>;
 }
 template <int DT, int MD>
 ManyKernel many_variant(int nt, int kb, int vb) {
   return nt <= 2 ? many_variant_of<DT, MD, 2>(kb, vb) : nt == 3 ? many_variant_of<DT, MD, 3>(kb, vb) : many_variant_of<DT, MD, 4>(kb, vb);
 }
 
-// Launches the kernel of these types.  The 18 kernels of a pair of types are a translation unit (decode_many_*.cu): a module is loaded as a
-// whole by the first call that reaches it, which took 37 ms with all 72 in one and every one's attribute set, 27 ms with
+// Launches the kernel of these types.  The 15 kernels of a pair of types are a translation unit (decode_many_*.cu): a module is loaded as a
+// whole by the first call that reaches it, which took 37 ms with all of them in one and every one's attribute set, 27 ms with
 // the attribute of one and 4 ms so.
 template <int DT, int MD>
 int many_launch(const DecodeManyCall& c) {
@@ -594,8 +594,8 @@ int many_launch(const DecodeManyCall& c) {
                    c.status, c.row_start};
   const int kb = w.promoted ? 2 : d->key_bits, vb = d->value_bits, nt = max(2, (w.group_rows + 7) / 8);
   const ManyKernel kernel = many_variant<DT, MD>(nt, kb, vb);
-  static SharedMemoryOptIn<3 * 2 * 3> opt_in;
-  DARTKV_CUDA_OK(opt_in(((nt - 2) * 2 + (kb == 4)) * 3 + (vb == 2 ? 0 : vb == 4 ? 1 : 2), kernel, 160 * 1024));
+  static SharedMemoryOptIn<3 * 5> opt_in;
+  DARTKV_CUDA_OK(opt_in((nt - 2) * 5 + (kb == 4 ? 3 : 0) + (vb == 2 ? 0 : vb == 4 ? 1 : 2), kernel, 160 * 1024));
   DARTKV_CUDA_OK(launch_following(kernel, dim3(work_rows * c.pieces), dim3(kThreads), many_smem(d, w), c.stream, *d, a, w));
   DARTKV_LAUNCH_OK("decode_many_kernel");
   return DARTKV_OK;

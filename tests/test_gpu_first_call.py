@@ -27,7 +27,7 @@ print("TOOK", 1e3 * took)
 
 
 def test_first_call_of_many_rows():
-    # 37 ms with all 72 variants loaded, about 1 ms with one: the fastest of three processes counts
+    # 37 ms with all variants in one module, about 4 ms with those of a pair of types: the fastest of three processes counts
     took = []
     for _ in range(3):
         done = subprocess.run([sys.executable, "-c", CODE], capture_output=True, text=True, timeout=300,
