@@ -129,8 +129,8 @@ __host__ __device__ __forceinline__ int dartkv_block_of_unit(int64_t x, int bloc
 }
 
 // ---------------------------------------------------------------------------- overlapped launches
-// Every kernel is launched with programmatic stream serialization, and wait_previous() is the first statement of each (nothing
-// may be read or written before it): it returns once the grids before this one have ended and their memory is visible.  Calls
+// Every kernel is launched with programmatic stream serialization, and calls wait_previous() before it reads or writes any memory
+// (only arithmetic on its parameters may come before, as in decode_merge_rows_kernel): it returns once the grids before this one have ended and their memory is visible.  Calls
 // here are a few to some tens of microseconds of kernel, so the gap between two of them counts.  A plainly launched kernel
 // starts at a multiple of 1 or 2 us after the one before it: kernels that spin for 5, 7.3 and 11.1 us come every 8.2, 10.2 and
 // 14.3 us, so launched every 5.6, 7.9 and 11.7 us.  No kernel lets its successor in before it has ended

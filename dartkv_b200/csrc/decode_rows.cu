@@ -28,7 +28,7 @@
 // Staging is by bulk copies on mbarriers, keys and values separately: with one buffer each (4-bit pages) the next
 // page's keys arrive during P.V and its values during the logits, two blocks per SM stay resident.
 //
-// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 61 us here (the query
+// B200: 4-bit fp16 pages, batch 24, 6,001 tokens, 32 heads on 8: 115 us through decode_wide.cu, 60 us here (the query
 // rows in M instead of N needed 64 + 32 accumulators and spilled).  Two query tokens on batch 8, 4,096 tokens,
 // 2-bit: 69 us as two passes of decode_fast.cu, 44 us here in one launch.  One
 // query token on the 2-bit pages of decode_fast.cu stays there: 1,026 us against 1,462 us at batch 128, 32,768 tokens.
