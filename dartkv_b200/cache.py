@@ -515,7 +515,8 @@ class DartKVCache:
     def get(self) -> Tuple[torch.Tensor, torch.Tensor]:
         if self._life.seen == 0:
             raise RuntimeError("DartKVCache is empty; call update() before get()")
-        made = _lib.HOST.get(ctypes.addressof(self._desc), self._life.seen, self._device.index)
+        desc = self._desc               # kept until the call returns: another thread may clear the cache meanwhile
+        made = _lib.HOST.get(ctypes.addressof(desc), self._life.seen, self._device.index)
         if made is not None:            # not on another device than the current one
             if type(made) is int:
                 check(made)

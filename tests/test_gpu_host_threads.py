@@ -1,7 +1,10 @@
-"""A native call whose launch waits for room in the GPU's queue leaves the other Python threads running."""
+"""A native call whose launch waits for room in the GPU's queue leaves the other Python threads running, whatever they do meanwhile."""
 
+import gc
 import threading
 import time
+import types
+import weakref
 
 import pytest
 import torch
@@ -54,3 +57,18 @@ def test_other_threads_run_while_a_launch_waits(name):
     assert not error, error
     assert last - start > 0.4                      # the thread did wait for the GPU
     assert longest < 0.2, longest                  # and this one did not
+
+
+def test_the_descriptor_outlives_a_call_that_reads_it(monkeypatch):
+    cache = calls()["get"].__self__
+    desc, seen = weakref.ref(cache._desc), []
+
+    def get(*args):
+        cache.clear()                              # what another thread may do while the interpreter is unlocked
+        gc.collect()
+        seen.append(desc() is not None)
+        return ()
+
+    monkeypatch.setattr(dart._lib, "HOST", types.SimpleNamespace(get=get))
+    cache.get()
+    assert seen == [True]
